@@ -1,7 +1,7 @@
 """The work a program hands to this framework, as measured cases.
 
-Two kinds of entry are used, as programs use them: the contract (compile -> materialize -> prepared submissions, or a
-GraphSession) with weights as resident buffers, and the kernel-level entries on the caller's own buffers and stream. A
+Two kinds of entry are used, as programs use them: the contract (compile -> materialize -> submissions, prepared ones for
+host inputs, or a GraphSession) with weights as resident buffers, and the kernel-level entries on the caller's own buffers and stream. A
 case whose weights would stay in the L2 cache between passes runs several layers' worth of them in one pass.
 """
 import ctypes as C
@@ -215,7 +215,7 @@ def _stream():
 
 
 def _contract_chain(st, program, per_layer, out_name, out_shape, out_dtype):
-    """One materialised program, one prepared binding set for each layer's resident buffers."""
+    """One materialised program, one binding set for each layer's resident buffers; results stay resident."""
     sess = api.ArtifactSession.compile(program, _dev())
     slots = {b["name"]: b["binding"] for b in program.buffers()}
     counts = {b["name"]: b["count"] for b in program.buffers()}
@@ -227,9 +227,7 @@ def _contract_chain(st, program, per_layer, out_name, out_shape, out_dtype):
             bs.insert_resident(slots[name], h)
         h, view = st.resident(shape=(max(counts[out_name], n_out),), dtype=out_dtype)
         bs.insert_resident(slots[out_name], h)
-        prepared = sess.prepare(bs)
-        st.chain.append(prepared)
-        st.close.append(prepared.free)
+        st.chain.append(bs)
         st.outputs.append(view[:n_out].view(out_shape))
     torch.cuda.synchronize()
     return st
@@ -351,9 +349,7 @@ def run(st):
         st.graph.replay()
         return {"hidden": st.hidden[-1], "first": st.hidden[0]}
     if kind in ("int4_contract", "affine", "k_quant"):
-        pending = []
-        for prepared in st.chain:
-            pending.append(prepared.submit(after=pending[-1] if pending else None))
+        pending = [st.session.submit(bs, leave_resident=True) for bs in st.chain]  # an instance's submissions run in order
         for sub in pending:
             sub.wait()
         return st.outputs
