@@ -313,6 +313,9 @@ cudaError_t dispatch(vyb_instance* inst, void* const* b, cudaStream_t s) {
         case OpKind::Int8Pack: return launch_int8_pack((const uint32_t*)b[0], (uint32_t*)b[1], u[0], s);
         case OpKind::LinearRows: {
             const bool has_bias = u[5] != 0;
+            if (u[4] && !has_bias && rt_dtype(u[3]) != 0 && dense_rows_supported(b[0], b[1], u[0], u[1], u[2]))
+                return launch_dense_rows(b[0], b[1], b[2], u[0], u[1], u[2], rt_dtype(u[3]) == 2,
+                                         inst->dev->prop.multiProcessorCount, s, inst->status_dev);
             return launch_linear_rows(b[0], b[1], has_bias ? b[2] : nullptr, has_bias ? b[3] : b[2], u[0], u[1], u[2],
                                       rt_dtype(u[3]), u[4], s);
         }
