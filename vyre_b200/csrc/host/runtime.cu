@@ -101,7 +101,8 @@ struct vyb_instance {
     std::vector<DeviceBuf> temps;
     void* scratch = nullptr;  // op-specific device scratch, sized at materialisation
     size_t scratch_len = 0;
-    uint32_t* status_dev = nullptr;   // 4 words, raised by kernels whose bounded waits ran out
+    uint32_t* status_dev = nullptr;   // 4 words, raised by kernels whose bounded waits ran out; a submission's own slot while it is enqueued
+    uint32_t injected_status = 0;     // word that the next submission reports (vyb_instance_inject_status)
     uint32_t* status_host = nullptr;  // pinned mirror
 
     // events are recycled: creating and destroying three per submission costs more than the launch itself
@@ -898,16 +899,33 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
             sub->outputs.push_back(o);
         }
     }
+    // Kernels raise their status words (only when a bounded wait runs out) straight in this submission's own mapped pinned
+    // slot, so a word raised by one submission is never reported for another and nothing has to be copied or cleared on the
+    // stream between two submissions: the copy and the memset that did it kept consecutive kernels about 20 us apart.
+    sub->status_host = static_cast<uint32_t*>(inst->acquire_pinned(16));
+    void* own_status = nullptr;
+    if (!sub->status_host || cudaHostGetDevicePointer(&own_status, sub->status_host, 0) != cudaSuccess) {
+        cudaGetLastError();
+        cleanup();
+        return fail_oom(16, 0);
+    }
+    std::memset(sub->status_host, 0, 16);
+    sub->status_host[0] = inst->injected_status;
+    inst->injected_status = 0;
     sub->start = inst->acquire_event(true);  // inst->mu is held for the whole submission
     sub->end = inst->acquire_event(true);
     sub->done = inst->acquire_event(false);
     cudaEventRecord(sub->start, inst->stream);
     cudaGetLastError();  // a non-sticky error left by an unrelated earlier call must not be blamed on this launch
+    uint32_t* const shared_status = inst->status_dev;
+    inst->status_dev = static_cast<uint32_t*>(own_status);
     cudaError_t e = dispatch(inst, slot_ptr, inst->stream);
+    inst->status_dev = shared_status;
     cudaEventRecord(sub->end, inst->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(inst->stream);
+        inst->injected_status = sub->status_host[0];  // nothing ran: the next submission reports it
         cleanup();
         inst->release_event(sub->start, true);
         inst->release_event(sub->end, true);
@@ -917,14 +935,6 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
     }
     for (auto& o : sub->outputs)
         if (o.host) cudaMemcpyAsync(o.host, o.dev_ptr, o.len, cudaMemcpyDeviceToHost, inst->stream);
-    // every submission reads the status words into its OWN pinned slot and clears them on the stream right after,
-    // so a word raised by one submission is never reported for another
-    sub->status_host = static_cast<uint32_t*>(inst->acquire_pinned(16));
-    if (sub->status_host) {
-        sub->status_host[0] = 0;
-        cudaMemcpyAsync(sub->status_host, inst->status_dev, 16, cudaMemcpyDeviceToHost, inst->stream);
-        cudaMemsetAsync(inst->status_dev, 0, 16, inst->stream);
-    }
     cudaEventRecord(sub->done, inst->stream);
     inst->refs.fetch_add(1);  // released by the completion (or by a failed wait)
     *submission = sub.release();
@@ -936,10 +946,8 @@ int32_t vyb_instance_inject_status(vyb_instance* inst, uint32_t word) {
     if (!inst) return fail_invalid_program("Fix: pass a non-null instance.");
     std::lock_guard<std::mutex> ilk(inst->mu);
     cudaSetDevice(inst->dev->ordinal);
-    // stream-ordered, like a kernel whose bounded wait ran out: the next submission on this instance reads it
-    cudaError_t e = cudaMemcpyAsync(inst->status_dev, &word, 4, cudaMemcpyHostToDevice, inst->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(inst->stream);
-    if (e != cudaSuccess) return fail_dispatch(int(e), "status injection failed: " + cuda_msg(e));
+    // like a kernel whose bounded wait ran out in the next submission on this instance
+    inst->injected_status = word;
     clear_error();
     return VYB_OK;
 }
