@@ -1,0 +1,60 @@
+"""The int4 linear at 5 to 64 rows on the tensor cores with weights unpacked into tensor memory: exact weights, f32 sums."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+import vyre_b200 as vb
+from vyre_b200 import api, ffi, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    d = vb.Device.acquire(0)
+    yield d
+    d.release()
+
+
+def reference(x, w, s, m, n, k):
+    q = np.stack((w & 15, w >> 4), axis=-1).reshape(n, k).astype(np.float64) - 8.0
+    wf = q * np.repeat(synth.bf16_bits_to_f32(s).astype(np.float64), 128, axis=1)
+    xf = synth.bf16_bits_to_f32(x).astype(np.float64)
+    return xf @ wf.T, np.abs(xf) @ np.abs(wf).T
+
+
+def check(got, want, mags, k, f32):
+    # f32 sums in any order: k 2^-24 of the summed magnitudes at most; bf16 outputs add one rounding
+    assert np.all(np.abs(got - want) <= k * 2.0 ** -24 * mags + (0.0 if f32 else 2.0 ** -8) * np.abs(want))
+
+
+# every column class (16, 48, 64) at its edges, one to eight k parts, tails in n, fewer k blocks than pipeline stages
+@pytest.mark.parametrize("m,n,k,f32", [(9, 200, 1024, True), (16, 4096, 2048, False), (17, 130, 1024, True), (48, 1000, 3072, False), (49, 260, 4096, True),
+                                       (64, 128, 7168, False), (12, 14336, 1024, True), (33, 20000, 1024, False)])
+def test_batched_decode_through_the_contract(dev, m, n, k, f32):
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=m + n)
+    x[0, :128] = oracle.f32_to_bf16_bits(oracle.bf16_bits_to_f32(x[0, :128]) * np.float32(2.0 ** 14))  # a group of outliers
+    prog = api.linear_int4_grouped_rowmajor("x", "w", "s", "o", m, k, n, 128, ffi.DT_F32 if f32 else ffi.DT_BF16)
+    out = vb.ArtifactSession.compile(prog, dev).run_host([x, w.view(np.uint32), s])[0]
+    got = (np.frombuffer(out, np.float32) if f32 else oracle.bf16_bits_to_f32(np.frombuffer(out, np.uint16))).reshape(m, n).astype(np.float64)
+    check(got, *reference(x, w, s, m, n, k), k, f32)
+
+
+@pytest.mark.parametrize("m,n,k,f32", [(5, 300, 6144, False), (8, 4096, 14336, False), (2, 140, 8192, True), (8, 64, 6144, True), (1, 200, 1024, False),
+                                       (3, 72, 3072, True), (8, 1000, 5120, False)])
+def test_long_rows_beyond_four_at_kernel_level_in_a_chain(m, n, k, f32):
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=k)
+    t = [torch.from_numpy(v).cuda() for v in (x.view(np.int16), w, s.view(np.int16))]
+    ys = [torch.zeros(m, n, dtype=torch.float32 if f32 else torch.bfloat16, device="cuda") for _ in range(3)]
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    for y in ys:  # consecutive launches overlap (constant weights)
+        ffi.check(ffi.lib().vyb_k_int4_gemv_ex(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), y.data_ptr(), m, n, k, 128,
+                                               ffi.DT_F32 if f32 else ffi.DT_BF16, 1, C.c_void_p(torch.cuda.current_stream().cuda_stream), status.data_ptr()))
+    torch.cuda.synchronize()
+    assert status.tolist() == [0] * 4
+    for y in ys:
+        assert torch.equal(y, ys[0])
+    check(ys[0].double().cpu().numpy(), *reference(x, w, s, m, n, k), k, f32)

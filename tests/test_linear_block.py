@@ -52,7 +52,7 @@ def test_builder_slots_and_errors():
     (1, 14336, True, False, 1),     # ... the norm of a long row does not
     (1, 14336, True, True, 9),
     (5, 8192, False, True, 1),
-    (1, 3072, True, True, 1),       # other k: the bulk-copy GEMV
+    (1, 3072, True, True, 1),       # other k: the tensor-memory kernel
     (256, 4096, True, True, 2),     # prefill
     (1, 96, True, True, 0),
 ])
