@@ -99,29 +99,24 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
     bool ok = true;
     if (warp == 0) {
-        for (uint32_t i = 0; i < kbs && ok; ++i) {
-            const uint32_t s = i % p.stages;
-            if (i >= p.stages) ok = mbar_wait(smem_u32(&bars->empty[s]), ((i / p.stages) - 1) & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (ok && lane == 0) {
-                const uint32_t bar = smem_u32(&bars->full[s]), dst = smem_u32(tiles + s * stage_bytes);
+        if (elect_one()) {
+            for (uint32_t i = 0; i < kbs; ++i) {
+                const uint32_t s = i % p.stages, bar = smem_u32(&bars->full[s]), dst = smem_u32(tiles + s * stage_bytes);
+                if (i >= p.stages && !mbar_wait(smem_u32(&bars->empty[s]), ((i / p.stages) - 1) & 1, abort_flag)) break;
                 mbar_arrive_expect_tx(bar, stage_bytes);
                 tma_load_2d(dst, &map_w, int((kb0 + i) * BK), int(n0), bar);
                 tma_load_2d(dst + A_BYTES, &map_x, int((kb0 + i) * BK), int(r0), bar);
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else if (warp == 1) {
         // M = 128 weight rows, N = bn activation rows; c f32, a / b both bf16 or both f16
         const uint32_t idesc = (1u << 4) | (p.f16 ? 0u : (1u << 7) | (1u << 10)) | ((p.bn >> 3) << 17) | (uint32_t(BM >> 4) << 24);
-        for (uint32_t i = 0; i < kbs && ok; ++i) {
-            const uint32_t s = i % p.stages;
-            ok = mbar_wait(smem_u32(&bars->full[s]), (i / p.stages) & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            if (lane == 0) {
-                const uint32_t src = smem_u32(tiles + s * stage_bytes);
+        if (elect_one()) {
+            for (uint32_t i = 0; i < kbs; ++i) {
+                const uint32_t s = i % p.stages, src = smem_u32(tiles + s * stage_bytes);
+                if (!mbar_wait(smem_u32(&bars->full[s]), (i / p.stages) & 1, abort_flag)) break;
+                tc_fence_after();
                 const uint64_t da = smem_desc_sw128(src), db = smem_desc_sw128(src + A_BYTES);
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k)
@@ -129,8 +124,8 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 tc_commit(smem_u32(&bars->empty[s]));
                 if (i + 1 == kbs) tc_commit(smem_u32(&bars->acc_full));
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     auto store = [&](uint32_t row, uint32_t col, float v) {
         // the reference flushes subnormal f32 results before it rounds to the storage type

@@ -183,87 +183,87 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int deq_idx = dequant_index(warp);
     if (warp == TMA_WARP) {
         // ------------------------------------ TMA producer ------------------------------------
-        uint32_t a_it = 0, r_it = 0, r_tile = pair, r_blk = 0;
-        bool ok = true;
-        for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
-            const TileCoord c = coord(tile);
-            const int m0 = int(c.mt * 2 * BM + rank * BM);
-            for (uint32_t kb = 0; kb < k_blocks && ok; ++kb, ++a_it) {
-                while (ok && r_tile < total_tiles && r_it <= a_it / RAW_KB + RAW_AHEAD) {
-                    const uint32_t rs = r_it % RAW_STAGES;
-                    if (r_it >= RAW_STAGES)
-                        ok = mbar_wait(smem_u32(&bars->raw_empty[rs]), ((r_it / RAW_STAGES) - 1) & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    if (lane == 0) {
+        if (elect_one()) {
+            uint32_t a_it = 0, r_it = 0, r_tile = pair, r_blk = 0;
+            uint32_t as = 0, a_parity = 1;
+            bool ok = true;
+            for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
+                const TileCoord c = coord(tile);
+                const int m0 = int(c.mt * 2 * BM + rank * BM);
+                for (uint32_t kb = 0; kb < k_blocks; ++kb, ++a_it) {
+                    while (r_tile < total_tiles && r_it <= a_it / RAW_KB + RAW_AHEAD) {
+                        const uint32_t rs = r_it % RAW_STAGES;
+                        if (r_it >= RAW_STAGES && !mbar_wait(smem_u32(&bars->raw_empty[rs]), ((r_it / RAW_STAGES) - 1) & 1, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
                         const uint32_t bar = smem_u32(&bars->raw_full[rs]);
                         mbar_arrive_expect_tx(bar, raw_bytes);
                         tma_load_2d(smem_u32(tiles + RAW_RING + rs * RAW_BYTES), &map_w, int(r_blk * RAW_KB * (BK / 2)),
                                     int(weight_row0(coord(r_tile))), bar);
+                        ++r_it;
+                        if (++r_blk == raw_blocks) {
+                            r_blk = 0;
+                            r_tile += pairs;
+                        }
                     }
-                    __syncwarp();
-                    ++r_it;
-                    if (++r_blk == raw_blocks) {
-                        r_blk = 0;
-                        r_tile += pairs;
+                    if (!ok) break;
+                    if (a_it >= A_STAGES && !mbar_wait(smem_u32(&bars->empty[as]), a_parity, abort_flag)) {
+                        ok = false;
+                        break;
                     }
-                }
-                if (!ok) break;
-                const uint32_t as = a_it % A_STAGES;
-                if (a_it >= A_STAGES) ok = mbar_wait(smem_u32(&bars->empty[as]), ((a_it / A_STAGES) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (lane == 0) {
                     // both CTAs' activation boxes count on the leader's barrier; the leader posts the expectation
                     const uint32_t leader_bar = mapa(smem_u32(&bars->a_full[as]), 0);
                     if (rank == 0) mbar_arrive_expect_tx(smem_u32(&bars->a_full[as]), 2 * A_BYTES);
                     tma_load_2d_pair(smem_u32(tiles + A_RING + as * A_BYTES), &map_x, int(kb * BK), m0, leader_bar);
+                    if (++as == uint32_t(A_STAGES)) {
+                        as = 0;
+                        a_parity ^= 1;
+                    }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp == MMA_WARP) {
         // ------------------------------------ MMA issuer (leader CTA only) ------------------------------------
-        if (rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = idesc_bf16_f32(2 * BM, p.bn);
-            uint32_t it = 0, local = 0;
+            uint32_t s = 0, parity = 0, local = 0;
             bool ok = true;
             for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
                 const uint32_t acc = local & 1;
-                if (local >= 2) ok = mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
+                if (local >= 2 && !mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * MAX_BN;
-                for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const uint32_t as = it % A_STAGES, bs = it % B_STAGES;
-                    ok = mbar_wait(smem_u32(&bars->a_full[as]), (it / A_STAGES) & 1, abort_flag);
-                    ok = ok && mbar_wait(smem_u32(&bars->b_full[bs]), (it / B_STAGES) & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (lane == 0) {
-                        const uint64_t da = smem_desc_sw128(smem_u32(tiles + A_RING + as * A_BYTES));
-                        const uint64_t db = smem_desc_sw128(smem_u32(tiles + B_RING + bs * B_BYTES));
-#pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k)
-                            mma_f16_pair(d_tmem, smem_desc_advance(da, k * UMMA_K * 2), smem_desc_advance(db, k * UMMA_K * 2),
-                                         idesc, (kb | uint32_t(k)) != 0);
-                        // free the stage in both CTAs
-                        const uint32_t em = smem_u32(&bars->empty[as]);
-                        tc_commit_pair(em);
-                        tc_commit_pair(mapa(em, 1));
+                for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait2(smem_u32(&bars->a_full[s]), parity, smem_u32(&bars->b_full[s]), parity, abort_flag)) {
+                        ok = false;
+                        break;
                     }
-                    __syncwarp();
+                    tc_fence_after();
+                    const uint64_t da = smem_desc_sw128(smem_u32(tiles + A_RING + s * A_BYTES));
+                    const uint64_t db = smem_desc_sw128(smem_u32(tiles + B_RING + s * B_BYTES));
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        mma_f16_pair(d_tmem, smem_desc_advance(da, k * UMMA_K * 2), smem_desc_advance(db, k * UMMA_K * 2),
+                                     idesc, (kb | uint32_t(k)) != 0);
+                    // free the stage in both CTAs
+                    const uint32_t em = smem_u32(&bars->empty[s]);
+                    tc_commit_pair(em);
+                    tc_commit_pair(mapa(em, 1));
+                    if (++s == uint32_t(STAGES)) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
-                if (ok && lane == 0) {
+                if (ok) {
                     const uint32_t af = smem_u32(&bars->acc_full[acc]);
                     tc_commit_pair(af);
                     tc_commit_pair(mapa(af, 1));
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (is_epilogue_warp(warp)) {
         // ------------------------------------ epilogue warps ------------------------------------
         const uint32_t quad = warp & 3;  // TMEM lane quarter this warp may read

@@ -82,66 +82,70 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const uint32_t tmem_base = bars->tmem_base;
 
     if (warp == TMA_WARP) {
-        uint32_t it = 0;
-        bool ok = true;
-        for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
-            const int m0 = int((tile % m_tiles) * 2 * BM + rank * BM);
-            const int n0 = int((tile / m_tiles) * BN + rank * (BN / 2));
-            for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-                const uint32_t s = it % STAGES;
-                if (it >= STAGES) ok = mbar_wait(smem_u32(&bars->empty[s]), ((it / STAGES) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (lane == 0) {
+        if (elect_one()) {
+            uint32_t s = 0, parity = 1;  // of the stage's previous release; the first round finds the stages free
+            bool ok = true, first = true;
+            for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
+                const int m0 = int((tile % m_tiles) * 2 * BM + rank * BM);
+                const int n0 = int((tile / m_tiles) * BN + rank * (BN / 2));
+                for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+                    if (!first && !mbar_wait(smem_u32(&bars->empty[s]), parity, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
                     const uint32_t leader_bar = mapa(smem_u32(&bars->full[s]), 0);
                     if (rank == 0) mbar_arrive_expect_tx(smem_u32(&bars->full[s]), 2 * STAGE_BYTES);
                     uint8_t* st = tiles + size_t(s) * STAGE_BYTES;
                     tma_load_2d_pair(smem_u32(st), &map_a, int(kb * BK), m0, leader_bar);
                     tma_load_2d_pair(smem_u32(st + A_BYTES), &map_w, int(kb * BK), n0, leader_bar);
+                    if (++s == uint32_t(STAGES)) {
+                        s = 0;
+                        first = false;
+                        parity ^= 1;
+                    }
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp == MMA_WARP) {
-        if (rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t idesc = idesc_s8_s32(2 * BM, BN);
-            uint32_t it = 0, local = 0;
+            uint32_t s = 0, parity = 0, local = 0;
             bool ok = true;
             for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
                 const uint32_t acc = local & 1;
-                if (local >= 2) ok = mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
+                if (local >= 2 && !mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag)) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + acc * BN;
-                for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const uint32_t s = it % STAGES;
-                    ok = mbar_wait(smem_u32(&bars->full[s]), (it / STAGES) & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (lane == 0) {
-                        const uint8_t* st = tiles + size_t(s) * STAGE_BYTES;
-                        const uint64_t da = smem_desc_sw128(smem_u32(st));
-                        const uint64_t db = smem_desc_sw128(smem_u32(st + A_BYTES));
-#pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k)
-                            mma_i8_pair(d_tmem, smem_desc_advance(da, k * UMMA_K), smem_desc_advance(db, k * UMMA_K), idesc,
-                                        (kb | uint32_t(k)) != 0);
-                        const uint32_t em = smem_u32(&bars->empty[s]);
-                        tc_commit_pair(em);
-                        tc_commit_pair(mapa(em, 1));
+                for (uint32_t kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait(smem_u32(&bars->full[s]), parity, abort_flag)) {
+                        ok = false;
+                        break;
                     }
-                    __syncwarp();
+                    tc_fence_after();
+                    const uint8_t* st = tiles + size_t(s) * STAGE_BYTES;
+                    const uint64_t da = smem_desc_sw128(smem_u32(st));
+                    const uint64_t db = smem_desc_sw128(smem_u32(st + A_BYTES));
+#pragma unroll
+                    for (int k = 0; k < BK / UMMA_K; ++k)
+                        mma_i8_pair(d_tmem, smem_desc_advance(da, k * UMMA_K), smem_desc_advance(db, k * UMMA_K), idesc,
+                                    (kb | uint32_t(k)) != 0);
+                    const uint32_t em = smem_u32(&bars->empty[s]);
+                    tc_commit_pair(em);
+                    tc_commit_pair(mapa(em, 1));
+                    if (++s == uint32_t(STAGES)) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
-                if (ok && lane == 0) {
+                if (ok) {
                     const uint32_t af = smem_u32(&bars->acc_full[acc]);
                     tc_commit_pair(af);
                     tc_commit_pair(mapa(af, 1));
                 }
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (is_epilogue_warp(warp)) {
         const uint32_t quad = warp & 3;
         uint32_t local = 0;
