@@ -92,6 +92,28 @@ def test_moe_ffn_empty_and_crowded_experts():
     check_against_oracle(got[0][sel], got[1][sel], got[2][sel], *want, x[sel], wr)
 
 
+# few rows per expert (weights unpacked into tensor memory): one row, full and ragged chunks of 32 and 64 rows, an expert with
+# several chunks beside empty ones, groups of 64, 128 and 192
+@pytest.mark.parametrize("tokens,hidden,inter,experts,topk,group,crowded", [(1, 256, 256, 64, 1, 128, False), (40, 768, 768, 8, 2, 192, True),
+                                                                           (90, 256, 512, 8, 2, 64, True), (33, 512, 256, 2, 2, 128, False),
+                                                                           (128, 256, 768, 4, 4, 128, False)])
+def test_moe_ffn_few_rows_per_expert(tokens, hidden, inter, experts, topk, group, crowded):
+    rng = np.random.default_rng(tokens)
+    x, wr, w13, _, w2, _ = synth.moe_ffn_inputs(tokens, hidden, inter, experts, seed=tokens)
+    s13 = synth.f32_to_bf16_bits(rng.uniform(1e-3, 2e-2, size=(experts, 2, inter, hidden // group)).astype(np.float32))
+    s2 = synth.f32_to_bf16_bits(rng.uniform(1e-3, 2e-2, size=(experts, hidden, inter // group)).astype(np.float32))
+    if crowded:  # every token picks the same experts
+        x = synth.f32_to_bf16_bits(np.abs(synth.bf16_bits_to_f32(x)))
+        wrf = np.zeros((experts, hidden), np.float32)
+        wrf[3] = 1.0
+        wr = synth.f32_to_bf16_bits(wrf)
+    else:
+        wr = synth.f32_to_bf16_bits(synth.bf16_bits_to_f32(wr) * np.float32(25.0))
+    got = run_kernel_level(x, wr, w13, s13, w2, s2, tokens, hidden, inter, experts, topk, group)
+    want = oracle.moe_ffn_int4(x, wr, w13, s13, w2, s2, np.arange(tokens), hidden, inter, experts, topk, group=group, mode=1)
+    check_against_oracle(*got, *want, x, wr)
+
+
 def test_moe_ffn_contract_path_matches_kernel_level_and_is_deterministic():
     tokens, hidden, inter, experts, topk = 200, 256, 512, 8, 2
     x, wr, w13, s13, w2, s2 = synth.moe_ffn_inputs(tokens, hidden, inter, experts, seed=9)

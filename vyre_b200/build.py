@@ -46,6 +46,7 @@ SOURCES = {
     "kernels/int4_prefill_tcgen05.cu": [],
     "kernels/int4_gemm_pair_tcgen05.cu": [],
     "kernels/dense_rows_tcgen05.cu": [],
+    "kernels/moe_skinny_tcgen05.cu": [],
     "kernels/moe_ffn.cu": [],
     "kernels/allgather_push.cu": [],
     "kernels/moe_ep.cu": [],

@@ -191,6 +191,11 @@ cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float
 // dtype: 0 = f32, 1 = bf16, 2 = f16
 cudaError_t launch_linear_rows(const void* x, const void* w, const void* bias, void* out, uint32_t rows,
                                uint32_t in_dim, uint32_t out_dim, uint32_t dtype, uint32_t out_in, cudaStream_t s);
+// grouped expert GEMMs for few rows per expert (moe_skinny_tcgen05.cu); plan: moe_plan_kernel's words; wide: 64 activation rows
+// per item instead of 32
+cudaError_t launch_moe_skinny(const void* x_sorted, const void* w, const void* scales, void* y, const uint32_t* plan, uint32_t max_rows,
+                              uint32_t n, uint32_t k, uint32_t group, uint32_t experts, bool glu, bool wide, int sm_count, cudaStream_t stream,
+                              uint32_t* status);
 // linear_rows at size with 16-bit [out, in] weights (dense_rows_tcgen05.cu): tensor cores, f32 sums in another order
 bool dense_rows_supported(const void* x, const void* w, uint32_t rows, uint32_t in_dim, uint32_t out_dim);
 cudaError_t launch_dense_rows(const void* x, const void* w, void* out, uint32_t rows, uint32_t in_dim, uint32_t out_dim, bool f16,

@@ -25,6 +25,7 @@ namespace vybk {
 namespace {
 
 constexpr uint32_t ROW_TILE = 256;       // rows per CTA-pair tile of the grouped GEMM
+constexpr uint32_t SKINNY_ROWS = 128;    // average rows per expert up to which the skinny expert GEMMs run
 constexpr uint32_t MAX_EXPERTS = 64;
 constexpr uint32_t MAX_TOPK = 8;
 constexpr uint32_t PAD_TOKEN = 0xFFFFFFFFu;
@@ -169,7 +170,8 @@ cudaError_t launch_router_gate(const uint16_t* x, const uint16_t* w_router, uint
 }
 
 // ---- plan: expert segments, tile table, deterministic row positions (single CTA) -------------------------------------
-// plan words: [0] number of 256-row tiles, [1 .. 1+E] segment starts (rows), then tile_expert[max_tiles].
+// plan words: [0] number of 256-row tiles, [1 .. E] segment starts (rows; the low eight bits hold the padding rows at the
+// segment's end), [1+E] end of the last segment, then tile_expert[max_tiles].
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, uint32_t* __restrict__ pos,
                 uint32_t* __restrict__ row_token, uint32_t tokens, uint32_t experts, uint32_t topk, uint32_t max_rows) {
@@ -189,8 +191,8 @@ moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, u
         uint32_t* tile_expert = plan + 2 + experts;
         for (uint32_t e = 0; e < experts; ++e) {
             s_start[e] = start;
-            plan[1 + e] = start;
             const uint32_t padded = (s_count[e] + ROW_TILE - 1) / ROW_TILE * ROW_TILE;
+            plan[1 + e] = start | (padded - s_count[e]);  // segment starts are multiples of 256
             for (uint32_t r = 0; r < padded; r += ROW_TILE) tile_expert[tile++] = e;
             start += padded;
         }
@@ -237,20 +239,28 @@ moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, u
     }
 }
 
-// ---- gather: expert-sorted activation rows (padding rows are zero) ---------------------------------------------------
+// ---- gather: expert-sorted activation rows ---------------------------------------------------
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ row_token, const uint32_t* __restrict__ plan,
-                  uint16_t* __restrict__ xg, uint32_t hidden, uint32_t experts) {
+                  uint16_t* __restrict__ xg, uint32_t hidden, uint32_t experts, bool skinny) {
     const uint32_t rows = plan[1 + experts];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t p = blockIdx.x * 8 + warp; p < rows; p += gridDim.x * 8) {
         const uint32_t t = row_token[p];
         uint4* dst = reinterpret_cast<uint4*>(xg + size_t(p) * hidden);
         if (t == PAD_TOKEN) {
-            for (uint32_t c = lane; c < hidden / 8; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
+            // the skinny GEMMs never store what they compute for padding rows (columns of their tiles)
+            if (!skinny)
+                for (uint32_t c = lane; c < hidden / 8; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
         } else {
             const uint4* src = reinterpret_cast<const uint4*>(x + size_t(t) * hidden);
-            for (uint32_t c = lane; c < hidden / 8; c += 32) dst[c] = src[c];
+            for (uint32_t c = lane; c < hidden / 8; c += 32) {
+                uint4 v = src[c];
+                if (skinny)  // k order 0 4 1 5 2 6 3 7, in which the skinny GEMMs unpack weights
+                    v = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410),
+                                   __byte_perm(v.y, v.w, 0x7632));
+                dst[c] = v;
+            }
         }
     }
 }
@@ -362,10 +372,23 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
                                        routing_idx, routing_w, tokens, hidden, experts, topk, sm_count, stream);
     if (e != cudaSuccess) return e;
     moe_plan_kernel<<<1, 1024, 0, stream>>>(routing_idx, plan, pos, row_token, tokens, experts, topk, L.max_rows);
+    const bool skinny = uint64_t(tokens) * topk <= uint64_t(experts) * SKINNY_ROWS;
     moe_gather_kernel<<<sm_count * 4, 256, 0, stream>>>(static_cast<const uint16_t*>(x_bf16), row_token, plan, xg, hidden,
-                                                        experts);
+                                                        experts, skinny);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    // Few rows per expert: weight rows on the M side, unpacked into tensor memory (8 experts, 4096 / 14336, top-2: 272 against
+    // 784 us at 64 tokens, 636 against 795 us at 512 = 128 rows per expert; 730 against 810 us at 768, where the pair GEMM's
+    // 256-row tiles are filled and its share of the time no longer grows).
+    if (skinny) {
+        const bool wide = uint64_t(tokens) * topk > uint64_t(experts) * 20;  // at 20 rows on average the fullest expert still fits 32
+        e = launch_moe_skinny(xg, w13, s13, h, plan, L.max_rows, inter, hidden, group, experts, true, wide, sm_count, stream, status);
+        if (e == cudaSuccess)
+            e = launch_moe_skinny(h, w2, s2, y, plan, L.max_rows, hidden, inter, group, experts, false, wide, sm_count, stream, status);
+        if (e != cudaSuccess) return e;
+        moe_combine_kernel<<<sm_count * 4, 256, 0, stream>>>(y, pos, routing_w, static_cast<uint16_t*>(out_bf16), tokens, hidden, topk);
+        return cudaGetLastError();
+    }
     // h = swiglu(xg . W1^T, xg . W3^T) per expert
     e = launch_int4_gemm_pair(xg, w13, s13, h, L.max_rows, inter, hidden, group, 0, 1, experts, tile_expert, plan, inter,
                               sm_count, stream, status);
