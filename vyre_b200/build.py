@@ -36,6 +36,7 @@ SOURCES = {
     "host/runtime.cu": [],
     "kernels/ref_ops.cu": ["-ftz=true", "-prec-div=true", "-prec-sqrt=true", "-fmad=false"],
     "kernels/dropin_fast.cu": ["-ftz=true", "-fmad=false"],
+    "kernels/affine_grouped_mma.cu": ["-ftz=true", "-fmad=false"],
     "kernels/int4_gemv.cu": [],
     "kernels/int4_gemv_halfsm.cu": [],
     "kernels/int4_gemv_batch8.cu": [],

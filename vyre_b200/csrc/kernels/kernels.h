@@ -186,6 +186,11 @@ bool i4_matvec_fast_supported(uint32_t batch, uint32_t rows, uint32_t cols);
 cudaError_t launch_affine_grouped_fast(const float* x, const uint32_t* w, const float* scale, const uint32_t* zp,
                                        const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                        uint32_t batch, int sm_count, cudaStream_t s);
+// the same operator with tensor-core sums (affine_grouped_mma.cu); launch_affine_grouped_fast routes to it
+bool affine_grouped_mma_supported(const void* x, const void* w, const void* scale, const void* zp, uint32_t in_dim, uint32_t out_dim,
+                                  uint32_t group);
+cudaError_t launch_affine_grouped_mma(const float* x, const uint32_t* w, const float* scale, const uint32_t* zp, const float* b, float* out,
+                                      uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t batch, int sm_count, cudaStream_t s);
 cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float* scales, float* out, uint32_t batch,
                                   uint32_t rows, uint32_t cols, cudaStream_t s);
 // dtype: 0 = f32, 1 = bf16, 2 = f16
