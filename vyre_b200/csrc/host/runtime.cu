@@ -347,7 +347,7 @@ cudaError_t dispatch(vyb_instance* inst, void* const* b, cudaStream_t s) {
         case OpKind::KQuantLinear:
             if (inst->variant == KV_K_QUANT_WORD_COLUMNS && k_quant_linear_fast_supported(u[0], u[1], u[2]))
                 return launch_k_quant_linear_fast((const float*)b[0], (const uint32_t*)b[1], (const float*)b[2], (const float*)b[3],
-                                                  (const float*)b[4], (float*)b[5], (float*)inst->scratch, u[0], u[1], u[2],
+                                                  (const float*)b[4], (float*)b[5], u[0], u[1], u[2],
                                                   inst->dev->prop.multiProcessorCount, s);
             return launch_k_quant_linear((const float*)b[0], (const uint32_t*)b[1], (const float*)b[2], (const float*)b[3],
                                          (const float*)b[4], (float*)b[5], u[0], u[1], u[2], s);
@@ -427,7 +427,6 @@ size_t scratch_bytes_for(const Program& p) {
     switch (p.kind) {
         case OpKind::ExpertMlp: return size_t(p.params.u[1]) * 4;
         case OpKind::LinearInt8Dynamic: return size_t(p.params.u[0]) * p.params.u[1];
-        case OpKind::KQuantLinear: return vybk::k_quant_linear_fast_scratch_bytes(p.params.u[1]);
         case OpKind::LinearInt4Block:  // the normalised activations, when the norm runs as its own kernel
             return (p.params.u[5] & 1u) ? size_t(p.params.u[0]) * p.params.u[1] * 2 : 0;
         case OpKind::MoeFfnInt4:

@@ -389,114 +389,203 @@ cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float
 
 
 // ---- GGML K-quant linear at size (vyre-libs/src/nn/quant/ggml.rs:217-333) ------------------------------------------------
-// The weight stream is k-major with neighbouring outputs in neighbouring nibbles (2-bit fields for Q2_K), so a thread owns
-// FOUR neighbouring packed word COLUMNS (one 16-byte load per k row: 32 outputs for Q4_K, 64 for Q2_K) and a warp reads 512
-// contiguous bytes of one k row. The k range is cut into up to K_QUANT_K_CHUNKS chunks across blockIdx.y so that decode
-// shapes fill the GPU and every thread has eight independent 16-byte loads in flight (the loop is latency-bound
-// otherwise); inside a block eight k slices are folded through shared memory in slice order, the chunk's partial row goes
-// to scratch, and a second launch adds the chunks in chunk order and the bias (deterministic).
-// out[i] = b[i] + sum_k x[k] * (q * scale + min) with scale and minimum applied per word (x * scale once, x * min once):
-// the reference's map in another summation order.
-template <int BITS, int KS>
-__global__ void __launch_bounds__(32 * KS) k_quant_linear_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ packed,
-                                                                      const float* __restrict__ scales, const float* __restrict__ mins,
-                                                                      float* __restrict__ partial, uint32_t in_dim, uint32_t out_dim,
-                                                                      uint32_t k_per_chunk) {
-    constexpr int VPW = 32 / BITS;                  // outputs per packed word
-    constexpr int OPT = 4 * VPW;                    // outputs per thread
-    constexpr uint32_t BLOCK = BITS == 4 ? 32 : 16; // weights per scale / min
-    extern __shared__ float red[];                  // [KS][32][OPT + 1]: a thread's row padded by one word, no bank conflicts
+// out[i] = b[i] + sum_k x[k] * (q * scale + min): scale and minimum belong to one k and 32 (16 for Q2_K) neighbouring outputs, so
+// a thread multiplies x[k] with both once per word row and spends a byte permutation, a subtraction and an FMA on a weight. The
+// weight stream is k-major with neighbouring outputs in neighbouring fields: a thread owns W neighbouring packed word columns (a
+// warp reads 128 W contiguous bytes of a k row); the eight warps of a block and the blocks of a cluster split k, and a set of
+// word rows is under way while the one before is summed. Slices are folded through shared memory in warp order and then over the
+// cluster in rank order (distributed shared memory; deterministic, no scratch, one launch).
+// What bounds it: those instructions (about four per weight) and the latency of the next set; HBM alone would take 6.7 us at
+// 4096 x 14336 Q4_K. Measured per linear in a chain of submissions, before (k chunks to scratch, a second launch that folds them)
+// and now: Q4_K 4096 -> 14336 48 / 29 us, 14336 -> 4096 53 / 49 us, Q2_K 4096 -> 14336 53 / 30 us.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float peer_f32(const float* p, uint32_t rank) {
+    uint32_t a = uint32_t(__cvta_generic_to_shared(p));
+    float v;
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}" : "=f"(v) : "r"(a), "r"(rank) : "memory");
+    return v;
+}
+
+constexpr int KQ_WARPS = 8, KQ_MAX_SPLIT = 8;
+
+// grid x = column blocks * split, cluster = split
+template <int BITS, int W>
+__global__ void __launch_bounds__(32 * KQ_WARPS, 2) k_quant_linear_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ packed,
+                                                                              const float* __restrict__ scales, const float* __restrict__ mins,
+                                                                              const float* __restrict__ b, float* __restrict__ out,
+                                                                              uint32_t in_dim, uint32_t out_dim, uint32_t split) {
+    constexpr int VPW = 32 / BITS, OPT = W * VPW;         // outputs per packed word, per thread
+    constexpr uint32_t BLOCK = BITS == 4 ? 32 : 16;       // weights per scale / min
+    constexpr int SPT = OPT <= int(BLOCK) ? 1 : OPT / int(BLOCK);  // scales a thread needs per k row
+    constexpr int OPS = OPT / SPT;                        // outputs per scale
+    constexpr int ROWS = OPT == 8 ? 8 : OPT == 16 ? 6 : 3;              // word rows fetched together, one set ahead of the one that is summed
+    constexpr uint32_t FIELD = (1u << BITS) - 1u, SPREAD = FIELD * 0x01010101u;
+    extern __shared__ float red[];                        // [KQ_WARPS][32][OPT + 1], then [32 * OPT] sums of this block
     constexpr uint32_t PITCH = 32 * (OPT + 1);
-    const uint32_t tx = threadIdx.x, ky = threadIdx.y;
-    const uint32_t quads_per_row = out_dim / OPT;
-    const uint32_t quad = blockIdx.x * 32 + tx;
-    const uint32_t k_begin = blockIdx.y * k_per_chunk, k_end = min(in_dim, k_begin + k_per_chunk);
+    float* sums = red + KQ_WARPS * PITCH;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = blockIdx.x % split, xb = blockIdx.x / split;
+    const uint32_t col = xb * 32 + lane;                  // this thread's group of W word columns
+    const uint32_t cols = out_dim / OPT;
+    const bool active = col < cols;
+    const uint32_t k_per = (in_dim + split - 1) / split, k_begin = min(in_dim, rank * k_per), k_end = min(in_dim, k_begin + k_per);
     float acc[OPT];
 #pragma unroll
-    for (int j = 0; j < OPT; ++j) acc[j] = 0.f;
-    if (quad < quads_per_row) {
-        const uint32_t i0 = quad * OPT;
-        const uint4* wp = reinterpret_cast<const uint4*>(packed);
-#pragma unroll 8
-        for (uint32_t k = k_begin + ky; k < k_end; k += KS) {
-            const uint4 w4 = __ldg(wp + size_t(k) * quads_per_row + quad);
-            const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-            const float xk = __ldg(x + k);
-            const size_t lin = size_t(k) * out_dim + i0;
+    for (int j = 0; j < OPT; ++j) acc[j] = 0.0f;
+    const uint32_t* wp = packed + size_t(col) * W;
+    const size_t row_words = out_dim / VPW, row_scales = out_dim / BLOCK;  // out_dim is a multiple of 4 VPW: whole blocks per row
+    const size_t s0 = size_t(col) * OPT / BLOCK;
+    struct Rows {
+        uint32_t words[ROWS][W];
+        float sc[ROWS][SPT], mn[ROWS][SPT], xk[ROWS];
+    };
+    auto fetch = [&](uint32_t k0, Rows& t) {
 #pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                const uint32_t blk = uint32_t((lin + w * VPW) / BLOCK);
-                const float xs = xk * __ldg(scales + blk), xm = xk * __ldg(mins + blk);
+        for (int r = 0; r < ROWS; ++r) {
+            const uint32_t k = min(k0 + r, in_dim - 1);  // past this block's range: reloaded, times zero
+            const uint32_t* src = wp + size_t(k) * row_words;
+            if constexpr (W == 2) {
+                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+                t.words[r][0] = v.x; t.words[r][1] = v.y;
+            } else {
+                t.words[r][0] = __ldg(src);
+            }
+            t.xk[r] = k0 + r < k_end ? __ldg(x + k) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < SPT; ++j) {
+                t.sc[r][j] = __ldg(scales + size_t(k) * row_scales + s0 + j);
+                t.mn[r][j] = __ldg(mins + size_t(k) * row_scales + s0 + j);
+            }
+        }
+    };
+    auto add = [&](uint32_t k0, const Rows& t) {
+        float part[OPT];  // the set's own sums: short chains keep the f32 rounding below that of one long chain per slice
+#pragma unroll
+        for (int j = 0; j < OPT; ++j) part[j] = 0.0f;
+        float part_low[SPT];
+#pragma unroll
+        for (int j = 0; j < SPT; ++j) part_low[j] = 0.0f;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            if (k0 + r >= k_end) break;
+            float xs[SPT];
+#pragma unroll
+            for (int j = 0; j < SPT; ++j) {
+                xs[j] = t.xk[r] * t.sc[r][j];
+                part_low[j] = fmaf(t.xk[r], t.mn[r][j], part_low[j]);
+            }
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                // the fields of all bytes at once: field j is byte j / (8 / BITS) of spread j % (8 / BITS)
+                constexpr int PER_BYTE = 8 / BITS;
+                uint32_t spread[PER_BYTE];
+#pragma unroll
+                for (int q = 0; q < PER_BYTE; ++q) spread[q] = (t.words[r][w] >> (BITS * q)) & SPREAD;
 #pragma unroll
                 for (int j = 0; j < VPW; ++j) {
-                    // the field as an f32 without an integer conversion: 2^23 + q has q in its low mantissa bits
-                    const float q = __uint_as_float(0x4B000000u | ((words[w] >> (j * BITS)) & ((1u << BITS) - 1u))) - 8388608.0f;
-                    acc[w * VPW + j] = fmaf(q, xs, acc[w * VPW + j] + xm);
+                    // the field as an f32 without an integer conversion: 0x4B0000nn is 2^23 + nn, and the subtraction is exact
+                    const float q = __uint_as_float(__byte_perm(spread[j % PER_BYTE], 0x4B000000u, 0x7540 + j / PER_BYTE)) - 8388608.0f;
+                    part[w * VPW + j] = fmaf(q, xs[(w * VPW + j) / OPS], part[w * VPW + j]);
                 }
             }
         }
+#pragma unroll
+        for (int j = 0; j < OPT; ++j) acc[j] += part[j] + part_low[j / OPS];
+    };
+    if (active) {
+        constexpr uint32_t STEP = KQ_WARPS * ROWS;
+        uint32_t k0 = k_begin + warp * ROWS;
+        Rows even, odd;
+        if (k0 < k_end) fetch(k0, even);
+        while (k0 < k_end) {
+            if (k0 + STEP < k_end) fetch(k0 + STEP, odd);
+            add(k0, even);
+            k0 += STEP;
+            if (k0 >= k_end) break;
+            if (k0 + STEP < k_end) fetch(k0 + STEP, even);
+            add(k0, odd);
+            k0 += STEP;
+        }
     }
 #pragma unroll
-    for (int j = 0; j < OPT; ++j) red[ky * PITCH + tx * (OPT + 1) + j] = acc[j];
+    for (int j = 0; j < OPT; ++j) red[warp * PITCH + lane * (OPT + 1) + j] = acc[j];
     __syncthreads();
-    for (uint32_t o = ky * 32 + tx; o < 32 * OPT; o += 32 * KS) {
-        const uint32_t i = blockIdx.x * 32 * OPT + o;
-        if (i >= out_dim) continue;
+    for (uint32_t o = threadIdx.x; o < 32 * OPT; o += 32 * KQ_WARPS) {
         float sum = 0.f;
 #pragma unroll
-        for (int s = 0; s < KS; ++s) sum += red[s * PITCH + (o / OPT) * (OPT + 1) + o % OPT];
-        partial[size_t(blockIdx.y) * out_dim + i] = sum;
+        for (int s = 0; s < KQ_WARPS; ++s) sum += red[s * PITCH + (o / OPT) * (OPT + 1) + o % OPT];
+        sums[o] = sum;
     }
-}
-
-__global__ void k_quant_fold_kernel(const float* __restrict__ partial, const float* __restrict__ b, float* __restrict__ out,
-                                    uint32_t out_dim, uint32_t chunks) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= out_dim) return;
-    float sum = 0.f;
-#pragma unroll 16
-    for (uint32_t c = 0; c < chunks; ++c) sum += __ldg(partial + size_t(c) * out_dim + i);
-    out[i] = sum + b[i];
+    cluster_barrier();
+    for (uint32_t o = rank * 32 + lane + warp * 32 * split; o < 32 * OPT; o += 32 * split * KQ_WARPS) {
+        const uint32_t i = xb * 32 * OPT + o;
+        if (i >= out_dim) continue;
+        float part[KQ_MAX_SPLIT];
+#pragma unroll
+        for (uint32_t q = 0; q < KQ_MAX_SPLIT; ++q)
+            if (q < split) part[q] = peer_f32(sums + o, q);
+        float sum = part[0];
+#pragma unroll
+        for (uint32_t q = 1; q < KQ_MAX_SPLIT; ++q)
+            if (q < split) sum += part[q];
+        out[i] = sum + b[i];
+    }
+    cluster_barrier();  // no block leaves while another still reads its sums
 }
 
 bool k_quant_linear_fast_supported(uint32_t in_dim, uint32_t out_dim, uint32_t bits) {
     return (bits == 4 || bits == 2) && in_dim >= 1 && out_dim >= 1 && out_dim % (4 * (32 / bits)) == 0;
 }
 
-size_t k_quant_linear_fast_scratch_bytes(uint32_t out_dim) { return size_t(K_QUANT_K_CHUNKS) * out_dim * 4; }
-
-cudaError_t launch_k_quant_linear_fast(const float* x, const uint32_t* packed, const float* scales, const float* mins,
-                                       const float* b, float* out, float* partial, uint32_t in_dim, uint32_t out_dim,
-                                       uint32_t bits, int sm_count, cudaStream_t s) {
-    constexpr int KS = 8;
-    const uint32_t opt = 4 * (32 / bits);
-    const uint32_t xblocks = (out_dim / opt + 31) / 32;
-    // about two blocks per SM, 64 k rows per chunk at least (eight loads in flight per thread)
-    uint32_t chunks = (2u * uint32_t(sm_count) + xblocks - 1) / xblocks;
-    chunks = chunks > K_QUANT_K_CHUNKS ? K_QUANT_K_CHUNKS : chunks;
-    const uint32_t by_rows = (in_dim + 63) / 64;
-    chunks = chunks > by_rows ? by_rows : chunks;
-    const uint32_t k_per_chunk = (in_dim + chunks - 1) / chunks;
-    chunks = (in_dim + k_per_chunk - 1) / k_per_chunk;
-    const dim3 grid(xblocks, chunks), block(32, KS);
-    const size_t smem = size_t(KS) * 32 * (opt + 1) * 4;
+namespace {
+template <int BITS, int W>
+cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b, float* out,
+                               uint32_t in_dim, uint32_t out_dim, uint32_t split, cudaStream_t s) {
+    constexpr uint32_t OPT = W * (32 / BITS);
+    constexpr int SMEM = int((KQ_WARPS * 32 * (OPT + 1) + 32 * OPT) * 4);
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
-    cudaError_t de = cudaGetDevice(&dev);
-    if (de != cudaSuccess) return de;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        cudaError_t e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<2, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(size_t(KS) * 32 * 65 * 4));
+        e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((out_dim / OPT + 31) / 32 * split);
+    cfg.blockDim = dim3(32 * KQ_WARPS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = split;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_quant_linear_fast_kernel<BITS, W>, x, packed, scales, mins, b, out, in_dim, out_dim, split);
+}
+}  // namespace
+
+cudaError_t launch_k_quant_linear_fast(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b,
+                                       float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, int sm_count, cudaStream_t s) {
+    // one word column per thread unless that fills a third of the SMs by itself; then two. Two blocks share an SM; clusters do not
+    // pack every SM of a GPC, so nine tenths of the slots are counted on.
+    const uint32_t vpw = 32 / bits, blocks1 = (out_dim / vpw + 31) / 32;
+    const bool pair = blocks1 > uint32_t(sm_count) / 3;
+    const uint32_t blocks = pair ? (out_dim / (2 * vpw) + 31) / 32 : blocks1;
+    uint32_t split = uint32_t(sm_count) * 9 / 5 / blocks;
+    if (split > uint32_t(KQ_MAX_SPLIT)) split = KQ_MAX_SPLIT;
+    if (split > (in_dim + 63) / 64) split = (in_dim + 63) / 64;  // every warp has rows
+    if (split < 1) split = 1;
     if (bits == 4)
-        k_quant_linear_fast_kernel<4, KS><<<grid, block, smem, s>>>(x, packed, scales, mins, partial, in_dim, out_dim, k_per_chunk);
-    else
-        k_quant_linear_fast_kernel<2, KS><<<grid, block, smem, s>>>(x, packed, scales, mins, partial, in_dim, out_dim, k_per_chunk);
-    k_quant_fold_kernel<<<(out_dim + 255) / 256, 256, 0, s>>>(partial, b, out, out_dim, chunks);
-    return cudaGetLastError();
+        return pair ? launch_k_quant_cfg<4, 2>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
+                    : launch_k_quant_cfg<4, 1>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
+    return pair ? launch_k_quant_cfg<2, 2>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
+                : launch_k_quant_cfg<2, 1>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
 }
 
 }  // namespace vybk

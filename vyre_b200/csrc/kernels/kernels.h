@@ -222,14 +222,11 @@ cudaError_t launch_rms_norm(const void* input, const void* weight, const void* g
 // GGML K-quants with per-block f32 scale / min sidecars; bits = 4 (Q4_K) or 2 (Q2_K)
 cudaError_t launch_k_quant_unpack(const uint32_t* packed, const float* scales, const float* mins, float* out, uint32_t n,
                                   uint32_t bits, cudaStream_t s);
-// K-quant linear at size (dropin_fast.cu; kernel variant 7): out_dim a multiple of the outputs of four packed words; `partial`
-// is scratch of k_quant_linear_fast_scratch_bytes(out_dim) bytes (one partial output row per k chunk)
-constexpr uint32_t K_QUANT_K_CHUNKS = 64;
+// K-quant linear at size (dropin_fast.cu; kernel variant 7): out_dim a multiple of the outputs of four packed words
 bool k_quant_linear_fast_supported(uint32_t in_dim, uint32_t out_dim, uint32_t bits);
-size_t k_quant_linear_fast_scratch_bytes(uint32_t out_dim);
 cudaError_t launch_k_quant_linear_fast(const float* x, const uint32_t* packed, const float* scales, const float* mins,
-                                       const float* b, float* out, float* partial, uint32_t in_dim, uint32_t out_dim,
-                                       uint32_t bits, int sm_count, cudaStream_t s);
+                                       const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, int sm_count,
+                                       cudaStream_t s);
 cudaError_t launch_k_quant_linear(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b,
                                   float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, cudaStream_t s);
 // hidden_scratch: f32 [hidden]
