@@ -66,3 +66,28 @@ def test_wide_quantiser_equals_the_rule(m, k):
     q, s = torch.empty(m, k, dtype=torch.int8, device="cuda"), torch.empty(m, device="cuda")
     ffi.check(ffi.lib().vyb_k_quantize_per_token_int8(xt.data_ptr(), q.data_ptr(), s.data_ptr(), m, k, torch.cuda.current_stream().cuda_stream))
     assert np.array_equal(q.cpu().numpy(), want_q.reshape(m, k)) and np.array_equal(s.cpu().numpy(), want_s)
+
+
+# the register forms (16 and 32 elements a thread) and the loop: one summation order, restated here
+@pytest.mark.parametrize("rows,hidden,dtype", [(3, 2048, BF16), (2, 4100, F32), (1, 4096, F16), (5, 8192, BF16), (2, 8200, F32)])
+def test_long_row_norm_in_registers_has_the_tree_bits(dev, rows, hidden, dtype):
+    rng = np.random.default_rng(hidden)
+    x = to_bits(rng.standard_normal((rows, hidden)).astype(np.float32), dtype)
+    w = to_bits((1.0 + 0.1 * rng.standard_normal(hidden)).astype(np.float32), dtype)
+    got = np.frombuffer(vb.ArtifactSession.compile(api.learned_rms_norm("x", "w", "o", rows, hidden, 1e-5, dtype), dev).run_host([x, w])[0], x.dtype)
+    v = to_f32(x, dtype).reshape(rows, hidden)
+    part = np.zeros((rows, 256), np.float32)
+    for c in range(0, hidden, 256):  # thread t adds the squares of elements t, t + 256, ...
+        blk = v[:, c:c + 256]
+        part[:, :blk.shape[1]] = part[:, :blk.shape[1]] + blk * blk
+    part = part.reshape(rows, 8, 32)
+    for o in (16, 8, 4, 2, 1):
+        part = part + part[:, :, np.arange(32) ^ o]
+    total = np.zeros(rows, np.float32)
+    for i in range(8):
+        total = total + part[:, i, 0]
+    inv = np.float32(1.0) / np.sqrt(total / np.float32(hidden) + np.float32(1e-5))
+    n = v * inv[:, None]
+    n = to_f32(to_bits(n, dtype), dtype) if dtype != F32 else n
+    want = to_bits(n * to_f32(w, dtype), dtype)
+    assert np.array_equal(got.reshape(rows, hidden), want)

@@ -457,6 +457,48 @@ __global__ void __launch_bounds__(256) rms_norm_tree_kernel(const void* input, c
     }
 }
 
+// The same bits for rows of up to 256 V elements without a gate: a thread's elements (and the weights that they meet) are loaded
+// at once and stay in registers between the sum and the products; the sum runs over them in the order above. What bounds the
+// kernel is latency: with a handful of rows the loop above waits for each of its loads in turn (16 at 4096 elements, twice).
+// Measured, 8 rows of 4096 bf16 (ncu, cold): 11.0 -> 8.4 us; four decode blocks at 8 rows 221 -> 216 us.
+template <int V>
+__global__ void __launch_bounds__(256) rms_norm_tree_regs_kernel(const void* input, const void* weight, void* out, uint32_t hidden, float eps,
+                                                                 uint32_t dt, uint32_t wdt) {
+    __shared__ float warp_sum[8];
+    const size_t base = size_t(blockIdx.x) * hidden;
+    float x[V], w[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const uint32_t c = threadIdx.x + 256 * i;
+        x[i] = c < hidden ? load_typed(input, base + c, dt) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const uint32_t c = threadIdx.x + 256 * i;
+        w[i] = c < hidden ? load_typed(weight, c, wdt) : 0.0f;
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+        if (threadIdx.x + 256 * i < hidden) sum = fadd(sum, fmul(x[i], x[i]));
+    for (int o = 16; o > 0; o >>= 1) sum = fadd(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    float total = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) total = fadd(total, warp_sum[i]);
+    const float inv = fdiv(1.0f, __fsqrt_rn(fadd(fdiv(total, float(hidden)), eps)));
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const uint32_t c = threadIdx.x + 256 * i;
+        if (c >= hidden) continue;
+        float normalized = fmul(x[i], inv);
+        if (dt == 1) normalized = __bfloat162float(__float2bfloat16_rn(normalized));
+        else if (dt == 2) normalized = __half2float(__float2half_rn(normalized));
+        store_typed(out, base + c, dt, fmul(normalized, w[i]));
+    }
+}
+
 // vyre-libs/src/nn/quant/ggml.rs:28-120 and 217-333. bits = 4: blocks of 32 weights in 4 words; bits = 2: blocks of 16 in 1
 __device__ __forceinline__ uint32_t k_quant_value(const uint32_t* packed, uint32_t linear, uint32_t bits, uint32_t* block) {
     const uint32_t block_size = bits == 4 ? 32u : 16u, values_per_byte = 8u / bits, words_per_block = bits == 4 ? 4u : 1u;
@@ -622,7 +664,11 @@ cudaError_t launch_residual_add(const void* residual, const void* branch, void* 
 }
 cudaError_t launch_rms_norm(const void* input, const void* weight, const void* gate, void* out, uint32_t rows, uint32_t hidden,
                             float eps, uint32_t dtype, uint32_t weight_dtype, bool tree, cudaStream_t s) {
-    if (tree) rms_norm_tree_kernel<<<rows, 256, 0, s>>>(input, weight, gate, out, hidden, eps, dtype, weight_dtype);
+    if (tree && !gate && hidden <= 4096)
+        rms_norm_tree_regs_kernel<16><<<rows, 256, 0, s>>>(input, weight, out, hidden, eps, dtype, weight_dtype);
+    else if (tree && !gate && hidden <= 8192)
+        rms_norm_tree_regs_kernel<32><<<rows, 256, 0, s>>>(input, weight, out, hidden, eps, dtype, weight_dtype);
+    else if (tree) rms_norm_tree_kernel<<<rows, 256, 0, s>>>(input, weight, gate, out, hidden, eps, dtype, weight_dtype);
     else rms_norm_kernel<<<rows, 256, 0, s>>>(input, weight, gate, out, hidden, eps, dtype, weight_dtype);
     return cudaGetLastError();
 }
