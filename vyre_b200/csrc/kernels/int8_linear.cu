@@ -124,15 +124,32 @@ __global__ void __launch_bounds__(WPB * 32) int8_weight_only_tiled_kernel(const 
                 }
             }
         }
+        // 32 sums of 32 lanes' parts: every halving exchanges half of the values with the lane's partner, so that lane l ends up
+        // with the sum of value l (31 shuffles, the same additions in the same tree as one butterfly per value)
+        static_assert(MB * CPW == 32, "a lane per sum");
+        float v[32];
 #pragma unroll
-        for (int c = 0; c < CPW; ++c) {
-            const float s = col0 + c < n ? scale[col0 + c] : 0.0f;
+        for (int j = 0; j < MB; ++j)
 #pragma unroll
-            for (int j = 0; j < MB; ++j) {
-                float v = acc[j][c];
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == 0 && m0 + j < m && col0 + c < n) y[size_t(m0 + j) * n + col0 + c] = v * s;
+            for (int c = 0; c < CPW; ++c) v[j * CPW + c] = acc[j][c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < o; ++i) {
+                const float keep = upper ? v[i + o] : v[i], send = upper ? v[i] : v[i + o];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
+        }
+        // through shared memory, so that eight lanes store 32 contiguous bytes of a row: the output may be mapped host memory, where
+        // 16384 four-byte stores took longer than the rest of the kernel (16 x 1024 x 1024 from and to host: 60 -> 46 us a call)
+        __syncthreads();
+        const uint32_t j = lane / CPW, c = lane % CPW;
+        xs[j * (WPB * CPW) + warp * CPW + c] = v[0] * (col0 + c < n ? scale[col0 + c] : 0.0f);
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < MB * WPB * CPW; i += WPB * 32) {
+            const uint32_t row = m0 + i / (WPB * CPW), col = blockIdx.x * (WPB * CPW) + i % (WPB * CPW);
+            if (row < m && col < n) y[size_t(row) * n + col] = xs[i];
         }
     }
 }
