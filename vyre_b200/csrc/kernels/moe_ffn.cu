@@ -265,13 +265,19 @@ moe_gather_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ r
     }
 }
 
+// Units of SEG 16-byte chunks of a row, so that a few rows still spread over the SMs: 64 tokens of 4096 elements as a warp per
+// row are sixteen dependent round trips (14.5 us, cold); in units 4.4 us. 4096 tokens: 19.3 / 18.6 us.
+constexpr uint32_t SEG = 64;  // two chunks per lane
+
 // ---- combine: out[t] = bf16( sum_j w[t,j] * y[pos[t,j]] ), slots in selection order, separate multiply and add -------
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const uint16_t* __restrict__ y, const uint32_t* __restrict__ pos, const float* __restrict__ wts,
                    uint16_t* __restrict__ out, uint32_t tokens, uint32_t hidden, uint32_t topk) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (uint32_t t = blockIdx.x * 8 + warp; t < tokens; t += gridDim.x * 8) {
-        for (uint32_t c = lane; c < hidden / 8; c += 32) {
+    const uint32_t chunks = hidden / 8, segs = (chunks + SEG - 1) / SEG;
+    for (uint64_t unit = blockIdx.x * 8 + warp; unit < uint64_t(tokens) * segs; unit += gridDim.x * 8) {
+        const uint32_t t = uint32_t(unit / segs), seg = uint32_t(unit % segs), c1 = min(chunks, (seg + 1) * SEG);
+        for (uint32_t c = seg * SEG + lane; c < c1; c += 32) {
             float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (uint32_t j = 0; j < topk; ++j) {
                 const float w = wts[size_t(t) * topk + j];
