@@ -12,8 +12,8 @@
 // four activation boxes by TMA; sixteen warps unpack (four for each 128 weight rows x 128 k of a stage: eight warps took 219 us
 // where sixteen took 180, latency is half of a stage); one thread issues the MMAs; warps 20-23 drain the accumulators of the
 // previous item (two sets).
-// Measured (8 experts, 4096 / 14336, 64 tokens x 2, cold): gate / up GEMM 399 -> 165 us, down GEMM 377 -> 83 us; the layer
-// 774 -> 272 us at 64 tokens, 268 -> 160 us at one. The unpacking still issues 27 instructions a word (15 of them the
+// Measured (8 experts, 4096 / 14336, 64 tokens x 2, cold): gate / up GEMM 399 -> 150 us, down GEMM 377 -> 76 us; the layer
+// 774 -> 267 us at 64 tokens, 268 -> 160 us at one. The unpacking still issues 27 instructions a word (15 of them the
 // conversion) and keeps the logic pipe 70 % busy; the packed bytes alone would take 108 us.
 // Inside every eight k the activations lie in the order 0 4 1 5 2 6 3 7 (the gather and the glu epilogue write them so): that
 // is the order in which a shift and a mask unpack a word, 15 instructions per eight weights instead of 17, 7 of them on the
