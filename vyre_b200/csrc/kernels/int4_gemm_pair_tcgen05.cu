@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
 // one byte (two nibbles, k even in the low one) -> two bf16 (k, k+1) = bf16((q - 8) * s), natural order
 __device__ __forceinline__ uint32_t dequant_byte(uint32_t byte_in_low, uint32_t s2) {
     // 0x1001 spreads the byte so that the low nibble sits at bits 0-3 and the high nibble at bits 16-19
-    const uint32_t t = ((byte_in_low * 0x1001u) & 0x000F000Fu) | 0x43004300u;  // (128 + q_k, 128 + q_k+1) exactly
+    const uint32_t t = and_or(byte_in_low * 0x1001u, 0x000F000Fu, 0x43004300u);  // (128 + q_k, 128 + q_k+1) exactly
     return bf16x2_mul(bf16x2_sub(t, 0x43084308u), s2);                            // exact q - 8, one rounding of the product
 }
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }

@@ -278,10 +278,10 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t w = words[j];
-                    uint32_t t0 = (w & 0x000F000Fu) | 0x43004300u;          // (k0, k4) as 128+q
-                    uint32_t t1 = ((w >> 4) & 0x000F000Fu) | 0x43004300u;   // (k1, k5)
-                    uint32_t t2 = ((w >> 8) & 0x000F000Fu) | 0x43004300u;   // (k2, k6)
-                    uint32_t t3 = ((w >> 12) & 0x000F000Fu) | 0x43004300u;  // (k3, k7)
+                    uint32_t t0 = and_or(w, 0x000F000Fu, 0x43004300u);          // (k0, k4) as 128+q
+                    uint32_t t1 = and_or(w >> 4, 0x000F000Fu, 0x43004300u);   // (k1, k5)
+                    uint32_t t2 = and_or(w >> 8, 0x000F000Fu, 0x43004300u);   // (k2, k6)
+                    uint32_t t3 = and_or(w >> 12, 0x000F000Fu, 0x43004300u);  // (k3, k7)
                     t0 = bf16x2_mul(bf16x2_sub(t0, 0x43084308u), s2);       // exact q-8, then one rounding of (q-8)*s
                     t1 = bf16x2_mul(bf16x2_sub(t1, 0x43084308u), s2);
                     t2 = bf16x2_mul(bf16x2_sub(t2, 0x43084308u), s2);
