@@ -20,8 +20,8 @@
 // its weights while this one drains. Few weight tiles: the k range of a tile is split over a cluster, the partial sums are
 // added in rank order over distributed shared memory (deterministic, no workspace).
 //
-// Measured (64-launch graphs over rotating weights): 14336 x 4096 at 48 rows 15.7 us (six launches of the 8-row kernel: 91 us),
-// at 64 rows 19 us, at 16 rows 14.0 us; 4096 x 14336 at 8 rows 13.7 us (two launches of the four-row k-block form: 26.6 us).
+// Measured (64-launch graphs over rotating weights): 14336 x 4096 at 48 rows 15.1 us (six launches of the 8-row kernel: 91 us),
+// at 64 rows 17.2 us, at 16 rows 14.4 us; 4096 x 14336 at 8 rows 13.7 us (two launches of the four-row k-block form: 26.6 us).
 // At 3 to 8 rows of 4096 k the 8-row kernel (10.8 us) is the faster one and stays.
 //
 // Every wait is bounded; on expiry a status word is raised, the CTA drains and frees its TMEM. No multicast.
@@ -53,11 +53,14 @@ struct Cfg {
     static constexpr int STAGE_BYTES = RAW_BYTES + B_BYTES;
     static constexpr bool HALF = BN <= 16;  // two CTAs per SM
     static constexpr int STAGES = BN == 48 ? 5 : 4;
-    static constexpr int A_SLOTS = HALF ? 3 : 4;  // unpacked groups in tensor memory, 64 columns each
+    // Groups that one pass of the MMA loop takes (its waits and commits cost more than its MMAs): both of a stage where a CTA has
+    // all of an SM's tensor memory (64 rows: 14336 x 4096 19.1 -> 17.2 us, 4096 x 14336 21.8 -> 16.0, 28672 x 8192 85 -> 58). A_SLOTS passes' unpacked weights and two passes' accumulators are held.
+    static constexpr int PASS = HALF ? 1 : 2;
+    static constexpr int A_SLOTS = HALF ? 3 : 2;
     static constexpr int TMEM_COLS = HALF ? 256 : 512;
-    static constexpr int A_COL = 2 * BN;          // the two accumulators come first
+    static constexpr int A_COL = 2 * PASS * BN;   // the accumulators come first
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + CTRL_BYTES + ALIGN_SLACK;
-    static_assert(A_COL + A_SLOTS * 64 <= TMEM_COLS, "tensor memory");
+    static_assert(A_COL + A_SLOTS * PASS * 64 <= TMEM_COLS, "tensor memory");
     static_assert(SMEM_BYTES <= (HALF ? 113 * 1024 : 227 * 1024), "shared memory");
     static_assert(BN * BM * 4 <= STAGES * STAGE_BYTES, "the partial tile reuses the stages");
 };
@@ -101,7 +104,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_init(smem_u32(&bars->empty[s]), 9);  // eight unpack warps and the MMAs
         }
         for (int s = 0; s < C::A_SLOTS; ++s) {
-            mbar_init(smem_u32(&bars->a_full[s]), 4);
+            mbar_init(smem_u32(&bars->a_full[s]), 4 * C::PASS);
             mbar_init(smem_u32(&bars->a_empty[s]), 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -155,21 +158,25 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         constexpr uint32_t idesc = idesc_bf16_f32(BM, BN);
         if (elect_one()) {
             uint32_t s = 0, slot = 0, a_parity = 0;
-            for (uint32_t gi = 0; gi < 2 * kbs; ++gi) {
-                const uint32_t buf = gi & 1;
+            for (uint32_t it = 0; it < 2 / C::PASS * kbs; ++it) {
+                const uint32_t set = it & 1;
                 // the unpack warps saw the whole stage land before they arrived here: no wait of its own for x
-                if (!(gi < 2 ? mbar_wait(smem_u32(&bars->a_full[slot]), a_parity, abort_flag)
-                             : mbar_wait2(smem_u32(&bars->a_full[slot]), a_parity, smem_u32(&bars->d_empty[buf]), ((gi >> 1) - 1) & 1, abort_flag))) break;
+                if (!(it < 2 ? mbar_wait(smem_u32(&bars->a_full[slot]), a_parity, abort_flag)
+                             : mbar_wait2(smem_u32(&bars->a_full[slot]), a_parity, smem_u32(&bars->d_empty[set]), ((it >> 1) - 1) & 1, abort_flag))) break;
                 tc_fence_after();
-                const uint32_t b = smem_u32(tiles + s * C::STAGE_BYTES + RAW_BYTES) + buf * 2 * BN * 128;
-                const uint64_t db0 = smem_desc_sw128(b), db1 = smem_desc_sw128(b + BN * 128);
 #pragma unroll
-                for (int k = 0; k < GROUP / UMMA_K; ++k)
-                    mma_f16_ts(tmem + buf * BN, tmem + C::A_COL + slot * 64 + k * (UMMA_K / 2),
-                               smem_desc_advance(k < 4 ? db0 : db1, (k & 3) * UMMA_K * 2), idesc, k != 0);
+                for (int h = 0; h < C::PASS; ++h) {
+                    const uint32_t half = C::PASS == 2 ? uint32_t(h) : set;  // which group of the stage
+                    const uint32_t b = smem_u32(tiles + s * C::STAGE_BYTES + RAW_BYTES) + half * 2 * BN * 128;
+                    const uint64_t db0 = smem_desc_sw128(b), db1 = smem_desc_sw128(b + BN * 128);
+#pragma unroll
+                    for (int k = 0; k < GROUP / UMMA_K; ++k)
+                        mma_f16_ts(tmem + (set * C::PASS + h) * BN, tmem + C::A_COL + (slot * C::PASS + h) * 64 + k * (UMMA_K / 2),
+                                   smem_desc_advance(k < 4 ? db0 : db1, (k & 3) * UMMA_K * 2), idesc, k != 0);
+                }
                 tc_commit(smem_u32(&bars->a_empty[slot]));
-                tc_commit(smem_u32(&bars->d_full[buf]));
-                if (buf == 1) {
+                tc_commit(smem_u32(&bars->d_full[set]));
+                if (C::PASS == 2 || set == 1) {
                     tc_commit(smem_u32(&bars->empty[s]));
                     s = s + 1 == uint32_t(C::STAGES) ? 0u : s + 1;
                 }
@@ -184,7 +191,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // ---- unpack: a thread per weight row; warps 4-7 the even groups, 8-11 the odd ones ----
         const uint32_t half = (warp >> 2) - 1, quad = warp & 3, r = quad * 32 + lane;
         for (uint32_t i = 0; i < kbs && ok; ++i) {
-            const uint32_t s = i % C::STAGES, gi = 2 * i + half, slot = gi % C::A_SLOTS;
+            const uint32_t s = i % C::STAGES, it = C::PASS == 2 ? i : 2 * i + half, slot = it % C::A_SLOTS;
             ok = mbar_wait(smem_u32(&bars->full[s]), (i / C::STAGES) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -194,11 +201,11 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             for (uint32_t j = 0; j < 4; ++j) raw[j] = *reinterpret_cast<const uint4*>(row + (((half * 4 + j) ^ (r & 7u)) << 4));
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->empty[s]));  // the packed bytes are in registers
-            if (gi >= uint32_t(C::A_SLOTS)) ok = mbar_wait(smem_u32(&bars->a_empty[slot]), ((gi / C::A_SLOTS) - 1) & 1, abort_flag);
+            if (it >= uint32_t(C::A_SLOTS)) ok = mbar_wait(smem_u32(&bars->a_empty[slot]), ((it / C::A_SLOTS) - 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t dst = tmem + ((quad * 32) << 16) + C::A_COL + slot * 64;
+            const uint32_t dst = tmem + ((quad * 32) << 16) + C::A_COL + (slot * C::PASS + (C::PASS == 2 ? half : 0)) * 64;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t a[32];
@@ -236,18 +243,25 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (i + AHEAD < kbs) queue[d] = __ldg(sp + i + AHEAD);
 #pragma unroll
                 for (uint32_t buf = 0; buf < 2; ++buf) {
-                    ok = ok && mbar_wait(smem_u32(&bars->d_full[buf]), i & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    tc_fence_after();
+                    // PASS = 1: one accumulator per group, set = group parity; PASS = 2: both groups' accumulators, set = stage parity
+                    const uint32_t set = C::PASS == 2 ? i & 1 : buf;
+                    if (C::PASS == 1 || buf == 0) {
+                        ok = ok && mbar_wait(smem_u32(&bars->d_full[set]), (C::PASS == 2 ? i >> 1 : i) & 1, abort_flag);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
                     const float s = __uint_as_float(buf ? pair & 0xFFFF0000u : pair << 16);
                     uint32_t v[BN / 16][16];
 #pragma unroll
-                    for (int c = 0; c < BN / 16; ++c) tmem_ld_32x16(tmem + ((quad * 32) << 16) + buf * BN + c * 16, v[c]);
+                    for (int c = 0; c < BN / 16; ++c)
+                        tmem_ld_32x16(tmem + ((quad * 32) << 16) + (C::PASS == 2 ? set * 2 + buf : set) * BN + c * 16, v[c]);
                     tmem_ld_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&bars->d_empty[buf]));
+                    if (C::PASS == 1 || buf == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->d_empty[set]));
+                    }
 #pragma unroll
                     for (int c = 0; c < BN; ++c) acc[c] = fmaf(s, __uint_as_float(v[c / 16][c % 16]), acc[c]);
                 }
