@@ -56,6 +56,69 @@ def test_tensor_core_sums(dev, shape):
     assert np.all(np.abs(got - want) <= (g + k // g + 8) * 2.0 ** -24 * mags)
 
 
+# several output tiles per block (the next tile's words are fetched under this one's stores, the reduction buffer is used again), with one
+# and with several k chunks: up to two rows, sixteen rows a block, eight rows a block with two k slices
+@pytest.mark.parametrize("shape", [(512, 40000, 32, 1), (8192, 28676, 128, 1), (256, 20000, 64, 60), (1024, 19300, 32, 50), (256, 12900, 64, 20), (2048, 12804, 64, 17)])
+def test_blocks_that_walk_several_tiles(dev, shape):
+    test_tensor_core_sums(dev, shape)
+
+
+# outputs that are no multiple of four: the f32 kernels, whole rows in shared memory up to four batch rows
+@pytest.mark.parametrize("shape", [(4096, 4098, 128, 1), (4096, 4098, 64, 1), (4096, 2050, 128, 2), (4096, 2050, 64, 2), (4096, 2050, 128, 3), (4096, 1026, 64, 4),
+                                   (4096, 1026, 128, 9)])
+def test_other_output_counts_take_the_f32_kernels(dev, shape):
+    test_tensor_core_sums(dev, shape)
+
+
+def definition(x, w, s, z, bias, k, n, g, b):
+    """The sums in 64 bits, and the summed magnitudes of their terms."""
+    q = ((w.reshape(k // 8, 1, n) >> (4 * np.arange(8, dtype=np.uint32))[None, :, None]) & 15).reshape(k, n).astype(np.float64)
+    rep = lambda v: np.repeat(v.reshape(-1, n).astype(np.float64), g, axis=0)  # noqa: E731
+    wd, xd = (q - rep(z)) * rep(s), x.reshape(b, k).astype(np.float64)
+    return xd @ wd + bias, np.abs(xd) @ (16.0 * rep(s)) + np.abs(bias)
+
+
+@pytest.mark.parametrize("shape", [(4096, 4096, 128, 1), (1024, 4096, 64, 6), (1024, 4096, 128, 33)])
+def test_group_sums_that_overflow_follow_the_definition(dev, shape):
+    """Finite activations whose group sums, which meet their scale late, overflow where every scaled weight times x is finite."""
+    k, n, g, b = shape
+    x, w, s, z, bias = make(k, n, g, b, 11, False)
+    x = np.random.default_rng(5).standard_normal(b * k).astype(np.float32)
+    w[:] = 0xFFFFFFFF
+    z[:] = 1  # every weight is 14 s
+    s[:] = np.float32(1e-3)
+    x[:k] = 0
+    x[[0, 1, 2, g + 3]] = 1e38, 7e37, -9e37, 5e37
+    want, mags = definition(x, w, s, z, bias, *shape)
+    assert np.all(np.isfinite(want.astype(np.float32)))
+    got = run(dev, (x, w, s, z, bias), *shape)
+    assert np.all(np.abs(got - want) <= (g + k // g + 8) * 2.0 ** -24 * mags)
+
+
+def test_scales_whose_zero_point_product_overflows_follow_the_definition(dev):
+    k, n, g, b = 1024, 4096, 64, 6
+    x, w, s, z, bias = make(k, n, g, b, 12, False)
+    x = np.abs(x) * np.float32(1e-12)
+    at = 3 * n + np.array([5, 4095])
+    s[at], z[at] = 1e30, 2 ** 31  # the weights of that group are -infinity
+    got, want = run(dev, (x, w, s, z, bias), k, n, g, b), oracle.linear_4bit_affine_grouped(x, w, s, z, bias, k, n, g, batch=b).reshape(b, n)
+    assert np.all(np.isneginf(want[:, [5, 4095]])) and np.array_equal(np.isneginf(got), np.isneginf(want))
+
+
+@pytest.mark.parametrize("shape", [(4096, 4096, 128, 1), (1024, 4096, 64, 6), (1024, 4096, 128, 33)])
+@pytest.mark.parametrize("size", [1e-30, 1e-32, 1e-33])
+def test_small_activations_keep_their_bits(dev, shape, size):
+    """The residuals of the split become subnormal here; flushed, sixteen bits of an activation or fewer would be left."""
+    k, n, g, b = shape
+    x, w, s, z, bias = make(k, n, g, b, 13, False)
+    x = (np.random.default_rng(6).standard_normal(b * k) * size).astype(np.float32)
+    s, bias = s * np.float32(4096.0), np.zeros_like(bias)
+    want, mags = definition(x, w, s, z, bias, *shape)
+    got = run(dev, (x, w, s, z, bias), *shape)
+    # the sums' bound, and 2^-133 of every activation times its weight (|q - zp| <= 15)
+    assert np.all(np.abs(got - want) <= (g + k // g + 8) * 2.0 ** -24 * mags + 2.0 ** -133 * 15.0 * k * float(s.max()))
+
+
 def test_values_that_do_not_split_follow_the_definition(dev):
     k, n, g, b = 1024, 4096, 128, 6
     x, w, s, z, bias = make(k, n, g, b, 3, True)

@@ -7,14 +7,17 @@
 //
 // What bounds it: at decode batches the weights' bytes, then the instructions per weight. The f32 kernels of dropin_fast.cu
 // spend an extraction, a subtraction and an FMA on every weight and batch row. Here a weight is unpacked once into a bf16 pair
-// (q - 8 is exact) for mma.sync.m16n8k16, and the f32 activation is three bf16 numbers (24 significant bits: the split is
-// exact), each a B column of its own. Products are exact, sums are f32 per group; scale and zero point are applied once per group and column.
+// (q - 8 is exact) for mma.sync.m16n8k16, and the f32 activation is three bf16 numbers (24 significant bits), each a B column of
+// its own. The split is exact from 2^-110 on and leaves less than 2^-133 below (its residuals keep their subnormals).
+// Products are exact, sums are f32 per group; scale and zero point are applied once per group and column.
 // The fragments need no shuffles: k labels inside an MMA are a dummy index, so a lane's word (8 k of one output) IS its A
 // fragment of two MMAs, and the activations are staged in the matching order (one 16-byte shared load per lane and word).
 // A lane loads 4 (2) neighbouring outputs of a word row, a warp four rows of 128 (64) bytes, four steps ahead.
 // Measured: see launch_affine_grouped_mma.
 //
-// A tile with an activation that is not finite (or rounds to infinity in bf16) is computed by the definition in f32 instead.
+// An output that does not come out finite is computed again by the definition in f32: a group sum meets its scale late, so that it
+// can overflow (activations from about 1e35 on, or not finite) where the definition, which scales every weight first, does not.
+// A scale of 2^95 and more, whose product with a zero point of 32 bits can overflow in the definition alone, counts as one.
 // Replaces, at size, the generated kernel of vyre-libs/src/nn/linear/inner/linear_4bit.rs:399-775.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -48,6 +51,18 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 __device__ __forceinline__ uint32_t bf16_bits(float v) { return uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(v))); }
 __device__ __forceinline__ float from_bits(uint32_t b) { return __uint_as_float(b << 16); }
+// subnormal operands and results kept (this file's own arithmetic flushes them)
+__device__ __forceinline__ float sub_keep(float a, float b) {
+    float d;
+    asm("sub.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float add_keep(float a, float b) {
+    float d;
+    asm("add.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
 
 // R: 16-output MMA tiles per warp (4: a lane loads 16 bytes of a word row, 2: 8 bytes).
 // NB: blocks of eight batch rows; the three parts of a block are an 8-column tile each, so a lane holds all parts of its rows.
@@ -76,9 +91,8 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
     // columns of a word row are permuted with it: a quarter warp reads two columns of four word rows
     auto slot = [](uint32_t kw, uint32_t col) { return kw * COLS + (col & ~7u) + ((col & 7u) ^ ((kw & 3u) << 1)); };
 
-    // a word row of 8 k of one batch row -> its three bf16 parts in the staged order; false when an element does not split
+    // a word row of 8 k of one batch row -> its three bf16 parts in the staged order
     auto stage = [&](uint32_t k0, uint32_t kc) {
-        bool fine = true;
         const uint32_t kws = kc / 8;
         for (uint32_t e = threadIdx.x; e < kws * (NB == 0 ? 3 : ROWS); e += THREADS) {
             const uint32_t kw = e % kws, r = e / kws;
@@ -90,9 +104,8 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const uint32_t p0 = bf16_bits(v[i]);
-                    fine = fine && (p0 & 0x7F80u) != 0x7F80u;
-                    const float r1 = __fsub_rn(v[i], from_bits(p0));
-                    const uint32_t p1 = bf16_bits(r1), p2 = bf16_bits(__fsub_rn(r1, from_bits(p1)));
+                    const float r1 = sub_keep(v[i], from_bits(p0));
+                    const uint32_t p1 = bf16_bits(r1), p2 = bf16_bits(sub_keep(r1, from_bits(p1)));
                     part[0][i & 3] |= p0 << ((i >> 2) * 16);
                     part[1][i & 3] |= p1 << ((i >> 2) * 16);
                     part[2][i & 3] |= p2 << ((i >> 2) * 16);
@@ -102,7 +115,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
             for (uint32_t q = 0; q < 3; ++q)  // rows past the batch (and the two spare columns of NB = 0) are zero
                 if (column(r, q) < COLS) xs[slot(kw, column(r, q))] = make_uint4(part[q][0], part[q][1], part[q][2], part[q][3]);
         }
-        const bool all_fine = !__syncthreads_or(!fine);
+        __syncthreads();
         for (uint32_t e = threadIdx.x; e < (kc / group) * SUMS; e += THREADS) {
             const uint32_t c = e % SUMS, kw0 = (e / SUMS) * (group / 8);
             float sum = 0.0f;
@@ -112,12 +125,11 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     const uint4 v = xs[slot(kw0 + j, NB == 0 ? c : column(c, q))];
                     const uint32_t r[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) sum += __uint_as_float(r[i] << 16) + __uint_as_float(r[i] & 0xFFFF0000u);
+                    for (int i = 0; i < 4; ++i) sum = add_keep(sum, add_keep(__uint_as_float(r[i] << 16), __uint_as_float(r[i] & 0xFFFF0000u)));
                 }
             xsum[e] = sum;
         }
         __syncthreads();
-        return all_fine;
     };
 
     // where this warp reads: its outputs (MMA tile i has na + i in row g and nz + i in row g + 8) and its run of groups
@@ -171,10 +183,9 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
         return v;
     };
 
-    bool fine = true;
     if (one_chunk && blockIdx.x < tiles) {
         aim(blockIdx.x, 0);  // the first weights are under way while the activations are staged
-        fine = stage(0, in_dim);
+        stage(0, in_dim);
     }
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         float acc[R][AC][4];
@@ -182,11 +193,12 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
         for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int c = 0; c < int(AC); ++c) acc[i][c][0] = acc[i][c][1] = acc[i][c][2] = acc[i][c][3] = 0.0f;
+        float top[2] = {0.0f, 0.0f};  // largest scale of this lane's outputs (NaN takes no part; it makes the sum NaN)
         for (uint32_t k0 = 0; k0 < in_dim; k0 += chunk) {
             if (!one_chunk) {
                 aim(tile, k0);
                 __syncthreads();
-                fine = stage(k0, min(chunk, in_dim - k0)) && fine;
+                stage(k0, min(chunk, in_dim - k0));
             }
             __align__(16) float sa[R], sz[R];
             __align__(16) uint32_t za[R], zz[R];
@@ -213,6 +225,11 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                         if (in_z) {
                             columns4(scale + at + nz, sz);
                             columns4(zp + at + nz, zz);
+                        }
+#pragma unroll
+                        for (int i = 0; i < R; ++i) {
+                            top[0] = fmaxf(top[0], fabsf(sa[i]));
+                            top[1] = fmaxf(top[1], fabsf(sz[i]));
                         }
                     }
                     const uint32_t kw = kw_first + st * 4;
@@ -254,6 +271,13 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                 }
             }
         }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (top[h] >= 0x1p95f)
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+#pragma unroll
+                    for (int c = 0; c < int(AC); ++c) acc[i][c][2 * h] = acc[i][c][2 * h + 1] = __uint_as_float(0x7FC00000u);
         const uint32_t oa = na, oz = nz;
         const bool have_a = in_a, have_z = in_z;
         if (one_chunk && tile + gridDim.x < tiles) aim(tile + gridDim.x, 0);  // the next tile's first weights, under this one's stores
@@ -267,7 +291,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     if (r >= nb || !(j < 2 ? have_a : have_z)) continue;
 #pragma unroll
                     for (int i = 0; i < R; ++i)
-                        out[size_t(b0 + r) * out_dim + n + i] = bias[n + i] + (fine ? acc[i][c][j] : by_definition(r, n + i));
+                        out[size_t(b0 + r) * out_dim + n + i] = bias[n + i] + (finite(acc[i][c][j]) ? acc[i][c][j] : by_definition(r, n + i));
                 }
         } else {
             // sum the k slices (and, with NB = 0, the parts) in a fixed order
@@ -288,15 +312,12 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                 const uint32_t j = e % (WN * TILE), r = e / (WN * TILE), n = tile * WN * TILE + j;
                 if (n >= out_dim) continue;
                 float v = 0.0f;
-                if (fine) {
 #pragma unroll
-                    for (int q = 0; q < WK; ++q) {
-                        const float* p = red + (((j / TILE) * WK + q) * TILE + j % TILE) * PITCH;
-                        v += NB == 0 ? (p[3 * r] + p[3 * r + 1]) + p[3 * r + 2] : p[r];
-                    }
-                } else {
-                    v = by_definition(r, n);
+                for (int q = 0; q < WK; ++q) {
+                    const float* p = red + (((j / TILE) * WK + q) * TILE + j % TILE) * PITCH;
+                    v += NB == 0 ? (p[3 * r] + p[3 * r + 1]) + p[3 * r + 2] : p[r];
                 }
+                if (!finite(v)) v = by_definition(r, n);
                 out[size_t(b0 + r) * out_dim + n] = bias[n] + v;
             }
             __syncthreads();
