@@ -676,8 +676,9 @@ int32_t vyb_k_tensor_peak(uint32_t int8, uint32_t iters, void* stream, uint32_t*
  * the half-SM integer kernel, three to eight rows one launch on the f16 tensor path; k a larger multiple of 2048 is
  * cut into k blocks inside one launch, which keeps a workspace per (device, stream) allocated on the first call that
  * is not under stream capture (a first call under capture runs one launch per k block with a stream-ordered scratch
- * allocation instead) and takes up to four rows (f32 outputs: one); more rows of it, and other k, run one launch of the
- * kernel that unpacks weights into tensor memory (no workspace). Launches that share a stream are ordered; graphs captured
+ * allocation instead) and takes up to four rows a launch (f32 outputs: one); more bf16 rows of it, and most bf16 shapes of
+ * other k, run one launch of the kernel that unpacks weights into tensor memory (no workspace). Other k with f32 outputs, or
+ * with few outputs, run the bulk-copy integer kernel: the group sums of f32 outputs are exact except on the f16 tensor path. Launches that share a stream are ordered; graphs captured
  * on one stream must not be replayed concurrently on two streams when they hold long-row launches (they share that
  * stream's workspace). */
 int32_t vyb_k_int4_gemv(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m,

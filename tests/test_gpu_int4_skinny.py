@@ -58,3 +58,37 @@ def test_long_rows_beyond_four_at_kernel_level_in_a_chain(m, n, k, f32):
     for y in ys:
         assert torch.equal(y, ys[0])
     check(ys[0].double().cpu().numpy(), *reference(x, w, s, m, n, k), k, f32)
+
+
+# f32 outputs: the sum of a 128-k group is exact, so large activations that cancel inside their group leave no trace in its small ones.
+# (Whole rows of 2048 and 4096 beyond one row run on the f16 tensor path, whose group sums are f32.)
+@pytest.mark.parametrize("m,n,k", [(1, 300, 1024), (3, 64, 3072), (8, 200, 5120), (2, 140, 6144), (5, 72, 14336), (12, 96, 3072), (33, 40, 8192)])
+def test_f32_outputs_have_exact_group_sums(dev, m, n, k):
+    rng = np.random.default_rng(m + k)
+    xs = rng.integers(-100, 101, size=(m, k // 128, 128)).astype(np.float32)  # exact in bf16
+    big = (rng.integers(64, 256, size=(m, k // 128, 32)) * 4096).astype(np.float32)
+    xs[:, :, 64:96], xs[:, :, 96:] = big, -big
+    q = rng.integers(0, 16, size=(n, k // 128, 128), dtype=np.uint8)
+    q[:, :, 96:] = q[:, :, 64:96]
+    x = synth.f32_to_bf16_bits(xs.reshape(m, k))
+    qf = q.reshape(n, k)
+    w = (qf[:, 0::2] | (qf[:, 1::2] << 4)).astype(np.uint8)
+    s = synth.f32_to_bf16_bits(rng.uniform(1e-3, 2e-2, size=(n, k // 128)).astype(np.float32))
+    prog = api.linear_int4_grouped_rowmajor("x", "w", "s", "o", m, k, n, 128, ffi.DT_F32)
+    got = np.frombuffer(vb.ArtifactSession.compile(prog, dev).run_host([x, w.view(np.uint32), s])[0], np.float32).reshape(m, n)
+    sums = np.einsum("mgk,ngk->mng", xs.astype(np.float64), q.astype(np.float64) - 8.0)  # the groups' sums, exact
+    terms = sums * synth.bf16_bits_to_f32(s).reshape(n, -1).astype(np.float64)
+    # roundings: scale times sum, then one addition for each group and a handful for the parts of a row
+    assert np.all(np.abs(got - terms.sum(axis=2)) <= (k // 128 + 24) * 2.0 ** -24 * np.abs(terms).sum(axis=2))
+
+
+# bf16 rows of 1024 and 3072 on both sides of the line between the bulk-copy and the tensor-memory kernel
+@pytest.mark.parametrize("m,n,k", [(1, 2368, 1024), (8, 2369, 1024), (2, 130, 3072), (3, 130, 3072), (1, 2400, 3072)])
+def test_small_bf16_shapes_on_both_sides_of_the_line(m, n, k):
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=k + n)
+    t = [torch.from_numpy(v).cuda() for v in (x.view(np.int16), w, s.view(np.int16))]
+    y = torch.zeros(m, n, dtype=torch.bfloat16, device="cuda")
+    ffi.check(ffi.lib().vyb_k_int4_gemv(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), y.data_ptr(), m, n, k, 128, ffi.DT_BF16,
+                                        C.c_void_p(torch.cuda.current_stream().cuda_stream), None))
+    torch.cuda.synchronize()
+    check(y.double().cpu().numpy(), *reference(x, w, s, m, n, k), k, False)

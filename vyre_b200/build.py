@@ -38,6 +38,7 @@ SOURCES = {
     "kernels/dropin_fast.cu": ["-ftz=true", "-fmad=false"],
     "kernels/affine_grouped_mma.cu": ["-ftz=true", "-fmad=false"],
     "kernels/int4_gemv.cu": [],
+    "kernels/int4_gemv_bulk.cu": [],
     "kernels/int4_gemv_halfsm.cu": [],
     "kernels/int4_gemv_batch8.cu": [],
     "kernels/int4_skinny_tcgen05.cu": [],

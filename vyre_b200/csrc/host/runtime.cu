@@ -265,8 +265,9 @@ cudaError_t run_int4_linear(vyb_instance* inst, uint32_t variant, const void* x,
         return launch_int4_prefill(x, w, scale, y, batch, n, k, group, out_f32, inst->dev->prop.multiProcessorCount, s,
                                    inst->status_dev);
     if (variant == KV_INT4_GEMV_TMA && int4_gemv_supported(std::min(batch, 8u), n, k, group)) {
-        if (batch > 8 && int4_skinny_supported(x, w, scale, batch, n, k, group))  // one launch reads the weights once for all rows
-            return launch_int4_skinny(x, w, scale, y, batch, n, k, out_f32, inst->dev->prop.multiProcessorCount, s, inst->status_dev, false);
+        // bf16 outputs: one launch reads the weights once for all rows (f32 outputs keep the eight-row kernels' sums, see launch_int4_gemv)
+        if (batch > 8 && !out_f32 && int4_skinny_supported(x, w, scale, batch, n, k, group))
+            return launch_int4_skinny(x, w, scale, y, batch, n, k, inst->dev->prop.multiProcessorCount, s, inst->status_dev, false);
         for (uint32_t b0 = 0; b0 < batch; b0 += 8) {
             const uint32_t mb = std::min(8u, batch - b0);
             cudaError_t e = launch_int4_gemv((const uint16_t*)x + size_t(b0) * k, w, scale, (uint8_t*)y + size_t(b0) * n * out_elem,

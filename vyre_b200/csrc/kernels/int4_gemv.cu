@@ -59,18 +59,15 @@ bool int4_gemv_supported(uint32_t m, uint32_t n, uint32_t k, uint32_t group) {
 cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m,
                              uint32_t n, uint32_t k, uint32_t out_f32, int sm_count, cudaStream_t stream,
                              uint32_t* status, bool constant_weights) {
-    // Whole rows of 2048 or 4096 k: the half-SM kernel, whose launches overlap on every SM. bf16 outputs go four batch
-    // rows at a time (26-bit block-floating activations, 57-bit for a single row); f32 outputs one row at a time, so
-    // that every row gets the single-row precision.
-    // Rows of 6144, 8192, ... (multiples of 2048 beyond 4096): the half-SM kernel per k block, sums carried in f32. bf16
-    // outputs four batch rows at a time, f32 outputs one row at a time (single-row precision), like the whole-row path.
-    // More rows than one launch of it takes (f32 outputs: from two rows): one launch on the tensor cores with the weights in
-    // tensor memory, which reads them once (4096 x 14336 at 8 rows: 13.7 us against 26.6 us).
-    if (int4_gemv_kblocks_supported(1, n, k, 128) && m > (out_f32 ? 1u : 4u) && int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
-        return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, out_f32, sm_count, stream, status, constant_weights);
+    const size_t out_elem = out_f32 ? 4 : 2;
+    const uint32_t step = out_f32 ? 1 : 4;  // rows per launch of the half-SM kernel: f32 outputs get the single-row precision
+    // Rows of 6144, 8192, ... (multiples of 2048 beyond 4096): the half-SM kernel per k block, sums carried in f32. More bf16 rows
+    // than one launch of it takes: one launch on the tensor cores with the weights in tensor memory, which reads them once (4096 x
+    // 14336 at 8 rows: 13.7 us against 26.6 us). f32 outputs stay: the integer sums of a group are exact, the tensor cores' are
+    // not (activations of widely different size, relative error against 64-bit sums: 0.8e-7 against 1.4 to 2.0e-7).
     if (int4_gemv_kblocks_supported(1, n, k, 128)) {
-        const size_t out_elem = out_f32 ? 4 : 2;
-        const uint32_t step = out_f32 ? 1 : 4;
+        if (!out_f32 && m > 4 && int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
+            return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, sm_count, stream, status, constant_weights);
         for (uint32_t b0 = 0; b0 < m; b0 += step) {
             const uint32_t mb = m - b0 < step ? m - b0 : step;
             cudaError_t e = launch_int4_gemv_kblocks(static_cast<const uint16_t*>(x_bf16) + size_t(b0) * k, w_packed, scale_bf16,
@@ -80,12 +77,12 @@ cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const voi
         }
         return cudaSuccess;
     }
-    // Three to eight batch rows (f32 outputs: from two rows): one launch on the f16 tensor path, eight batch rows per MMA
+    // Whole rows of 2048 or 4096 k. Three to eight batch rows (f32 outputs: from two rows): one launch on the f16 tensor path, eight
+    // batch rows per MMA
     if (m >= (out_f32 ? 2u : 3u) && int4_gemv_batch8_supported(m, n, k, 128))
         return launch_int4_gemv_batch8(x_bf16, w_packed, scale_bf16, y, m, n, k, out_f32, sm_count, stream, constant_weights);
+    // ... fewer: the half-SM kernel, whose launches overlap on every SM (26-bit block-floating activations, 57-bit for a single row)
     if (int4_gemv_halfsm_supported(1, n, k, 128)) {
-        const size_t out_elem = out_f32 ? 4 : 2;
-        const uint32_t step = out_f32 ? 1 : 4;
         for (uint32_t b0 = 0; b0 < m; b0 += step) {
             const uint32_t mb = m - b0 < step ? m - b0 : step;
             cudaError_t e = launch_int4_gemv_halfsm(static_cast<const uint16_t*>(x_bf16) + size_t(b0) * k, w_packed, scale_bf16,
@@ -95,11 +92,15 @@ cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const voi
         }
         return cudaSuccess;
     }
-    // Other k (odd multiples of 1024): the same tensor-memory kernel at every m (14336 x 5120 at 8 rows: 16.5 us against 47.5 us of
-    // an mbarrier-pipelined bulk-copy kernel that this one replaced, 4096 x 11264 at one row: 11.9 against 22.7 us).
-    if (int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
-        return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, out_f32, sm_count, stream, status, constant_weights);
-    return cudaErrorNotSupported;  // the callers check the operands' alignment
+    // Other k (odd multiples of 1024). bf16 outputs: the tensor-memory kernel (14336 x 5120 at 8 rows: 16.5 us against 47.5 us of the
+    // bulk-copy kernel, 4096 x 11264 at one row: 11.9 against 22.7 us), except where a row is one k block of the bulk-copy kernel and every SM has
+    // one 16-row tile of it at most: there it needs no cluster reduction (2048 x 1024 at one row 6.4 against 8.3 us, at eight 7.3 against
+    // 7.9; 2048 x 3072 at one row 6.4 against 8.5, but 8.3 against 7.6 at 128 x 3072 and four). f32 outputs: the bulk-copy kernel, for its exact
+    // group sums (activations of widely different size: error 0.6 to 1.0e-7 against 1.1 to 2.9e-7).
+    const bool small = n <= 16 * uint32_t(sm_count) && (k == 1024 || (k == 3072 && m <= 2));
+    if (!out_f32 && !small && int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
+        return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, sm_count, stream, status, constant_weights);
+    return launch_int4_gemv_bulk(x_bf16, w_packed, scale_bf16, y, m, n, k, out_f32, sm_count, stream, status, constant_weights);
 }
 
 cudaError_t launch_int4_linear_generic(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y,
