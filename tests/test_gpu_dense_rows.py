@@ -55,6 +55,23 @@ def test_tiled_rows_keep_the_reference_order_bits(dev, rows, k, n, dtype, out_in
     assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
 
 
+# the tiled kernel's range: from 2^14 outputs (f32 [out, in]), 2^16 (16 bits), 2^18 and 2^19 ([in, out]), one and four rows a warp, with and
+# without a bias, tails in rows, outputs and k
+@pytest.mark.parametrize("rows,k,n,dtype,out_in,bias", [(5, 33, 3300, F32, True, False), (4, 35, 4100, F32, True, False), (4, 5, 65600, F32, False, True),
+                                                        (17, 100, 3900, BF16, True, False), (66, 9, 4100, F32, False, True), (129, 5, 4100, F16, False, False),
+                                                        (70, 37, 3800, F32, False, False)])
+def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
+    rng = np.random.default_rng(rows + k)
+    x = to_bits(rng.standard_normal((rows, k)).astype(np.float32), dtype)
+    w = to_bits(rng.standard_normal((n, k) if out_in else (k, n)).astype(np.float32), dtype)
+    b = to_bits(rng.standard_normal(n).astype(np.float32), dtype) if bias else None
+    make = api.linear_rows_no_bias_out_in_typed if out_in else api.linear_rows_no_bias_typed
+    prog = api.linear_rows("x", "w", "b", "out", rows, k, n) if bias else make("x", "w", "out", rows, k, n, dtype)
+    got = np.frombuffer(vb.ArtifactSession.compile(prog, dev).run_host([x, w] + ([b] if bias else []))[0], x.dtype)
+    want = oracle.linear_rows(x, w, b, rows, k, n, dtype=ODT[dtype], weight_out_in=out_in)
+    assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
+
+
 @pytest.mark.parametrize("m,k", [(1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
 def test_wide_quantiser_equals_the_rule(m, k):
     import torch

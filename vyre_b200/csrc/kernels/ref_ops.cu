@@ -169,7 +169,7 @@ __global__ void linear_rows_kernel(const void* x, const void* w, const void* bia
 // own), for calls that fill the GPU: a block owns 64 outputs x 4 RT rows and stages 32 k of both operands in shared memory, so
 // weights are read along their rows (the kernel above reads them a row apart per lane and once per activation row) and a
 // staged weight serves RT rows. What bounds it is the order itself: in_dim dependent additions, 4 cycles each, and two
-// f32 instructions per product. Measured (ncu, 16 rows x 4096 -> 14336): the kernel above 3528 us.
+// f32 instructions per product. Where it is the faster one: launch_linear_rows.
 template <int RT>
 __global__ void __launch_bounds__(128) linear_rows_tiled_kernel(const void* __restrict__ x, const void* __restrict__ w,
                                                                 const void* __restrict__ bias, void* __restrict__ out,
@@ -620,9 +620,16 @@ cudaError_t launch_int8_pack(const uint32_t* in, uint32_t* out, uint32_t n, cuda
 }
 cudaError_t launch_linear_rows(const void* x, const void* w, const void* bias, void* out, uint32_t rows,
                                uint32_t in_dim, uint32_t out_dim, uint32_t dtype, uint32_t out_in, cudaStream_t s) {
-    // the tiled form from 2^18 products on (below that one block's staging costs what the whole call does); it has the same bits
+    // The tiled form (same bits) where the plain kernel is bound by its throughput and not by its chain of dependent additions, which is
+    // the shorter one. Plain: 280 products a ns with [out, in] weights (neighbouring lanes a row apart), 2900 with [in, out], 33 to
+    // 52 ns a step of the chain; tiled: 55 to 66 ns a step, 140 with 16-bit operands. Measured, plain / tiled, us: f32 [out, in]
+    // 64 x 4096 x 64 203 / 269, 16 x 512 x 512 38 / 40, 4 x 4096 x 4096 317 / 222, 16 x 2048 x 2048 285 / 140, 64 x 4096 x 4096 3870 / 316;
+    // 16 bits [out, in] (without tensor cores) 16 x 100 x 3000 17 / 21, 64 x 100 x 3000 38 / 21; f32 [in, out] 16 x 4096 x 4096
+    // 200 / 271, 64 x 4096 x 4096 369 / 315; 16 bits [in, out] 64 x 4096 x 4096 418 / 638, 256 x 2048 x 2048 401 / 348.
+    const uint64_t outputs = uint64_t(rows) * out_dim;
     const int rt = rows <= 4 ? 1 : 4;
-    if (uint64_t(rows) * in_dim * out_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
+    const uint64_t from = out_in ? (dtype == 0 ? 1u << 14 : 1u << 16) : dtype == 0 ? 1u << 18 : 1u << 19;
+    if (outputs >= from && outputs * in_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
         const dim3 grid((out_dim + 63) / 64, (rows + 4 * rt - 1) / (4 * rt));
         if (rt == 1) linear_rows_tiled_kernel<1><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
         else linear_rows_tiled_kernel<4><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
