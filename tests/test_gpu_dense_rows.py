@@ -86,7 +86,8 @@ def test_wide_quantiser_equals_the_rule(m, k):
 
 
 # the register forms (16 and 32 elements a thread) and the loop: one summation order, restated here
-@pytest.mark.parametrize("rows,hidden,dtype", [(3, 2048, BF16), (2, 4100, F32), (1, 4096, F16), (5, 8192, BF16), (2, 8200, F32)])
+@pytest.mark.parametrize("rows,hidden,dtype", [(3, 2048, BF16), (2, 4100, F32), (1, 4096, F16), (5, 8192, BF16), (2, 8200, F32),
+                                               (296, 2052, BF16), (297, 2052, BF16)])
 def test_long_row_norm_in_registers_has_the_tree_bits(dev, rows, hidden, dtype):
     rng = np.random.default_rng(hidden)
     x = to_bits(rng.standard_normal((rows, hidden)).astype(np.float32), dtype)
