@@ -72,7 +72,7 @@ def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
     assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
 
 
-@pytest.mark.parametrize("m,k", [(1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
+@pytest.mark.parametrize("m,k", [(2, 512), (2, 520), (4097, 896), (4097, 904), (1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
 def test_wide_quantiser_equals_the_rule(m, k):
     import torch
     rng = np.random.default_rng(k)
