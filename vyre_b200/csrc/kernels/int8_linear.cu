@@ -76,11 +76,12 @@ __global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* __re
 // activation rows through L1 for its one output channel (64 KB per warp, 64 MB per launch at the benchmark size, which is
 // what its time goes to). Here a block of four warps loads a 16-row x 1024-k activation tile once, each warp owns TWO
 // output channels (an activation register feeds two weights), a lane takes four consecutive k per step so that the
-// float4 reads of a warp are conflict-free and its weight reads are one 128-byte line per channel.
+// float4 reads of a warp are conflict-free and its weight reads are one 128-byte line per channel. Three blocks fit an SM's shared
+// memory: told so, the compiler takes the registers it needs (held to 64 for eight blocks it spilled: 256 x 4096 x 1024 441 us).
 constexpr int KC = 1024;   // k per shared-memory tile
 constexpr int CPW = 2;     // output channels per warp
 constexpr int WPB = 4;     // warps per block
-__global__ void __launch_bounds__(WPB * 32) int8_weight_only_tiled_kernel(const float* __restrict__ x, const int8_t* __restrict__ w,
+__global__ void __launch_bounds__(WPB * 32, 3) int8_weight_only_tiled_kernel(const float* __restrict__ x, const int8_t* __restrict__ w,
                                                                           const float* __restrict__ scale, float* __restrict__ y,
                                                                           uint32_t m, uint32_t n, uint32_t k) {
     extern __shared__ __align__(16) float xs[];  // [MB][KC]
