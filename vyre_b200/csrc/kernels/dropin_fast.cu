@@ -397,7 +397,7 @@ cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float
 // cluster in rank order (distributed shared memory; deterministic, no scratch, one launch).
 // What bounds it: those instructions (about four per weight) and the latency of the next set; HBM alone would take 6.7 us at
 // 4096 x 14336 Q4_K. Measured per linear in a chain of submissions, before (k chunks to scratch, a second launch that folds them)
-// and now: Q4_K 4096 -> 14336 48 / 29 us, 14336 -> 4096 53 / 49 us, Q2_K 4096 -> 14336 53 / 30 us.
+// and now: Q4_K 4096 -> 14336 48 / 29 us, Q2_K 4096 -> 14336 53 / 30 us; rule and figures for long k: launch_k_quant_linear_fast.
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -409,7 +409,7 @@ __device__ __forceinline__ float peer_f32(const float* p, uint32_t rank) {
     return v;
 }
 
-constexpr int KQ_WARPS = 8, KQ_MAX_SPLIT = 8;
+constexpr int KQ_WARPS = 8, KQ_MAX_SPLIT = 16;
 
 // grid x = column blocks * split, cluster = split
 template <int BITS, int W>
@@ -552,6 +552,7 @@ cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const flo
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
         e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
@@ -573,13 +574,16 @@ cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const flo
 cudaError_t launch_k_quant_linear_fast(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b,
                                        float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, int sm_count, cudaStream_t s) {
     // one word column per thread unless that fills a third of the SMs by itself; then two. Two blocks share an SM; clusters do not
-    // pack every SM of a GPC, so nine tenths of the slots are counted on.
+    // pack every SM of a GPC, so nine tenths of the slots are counted on. Sixteen parts where all clusters of sixteen are at work at
+    // once, else eight at most (clusters of 9 to 15 leave too many SMs of a GPC empty): with eight, few outputs and a long k took
+    // longer than in the two launches before (us, those / eight parts: Q4_K 14336 x 4096 34 / 43, 28672 x 512 35 / 44, Q2_K 28672 x 512 46 / 60).
     const uint32_t vpw = 32 / bits, blocks1 = (out_dim / vpw + 31) / 32;
     const bool pair = blocks1 > uint32_t(sm_count) / 3;
     const uint32_t blocks = pair ? (out_dim / (2 * vpw) + 31) / 32 : blocks1;
     uint32_t split = uint32_t(sm_count) * 9 / 5 / blocks;
-    if (split > uint32_t(KQ_MAX_SPLIT)) split = KQ_MAX_SPLIT;
     if (split > (in_dim + 63) / 64) split = (in_dim + 63) / 64;  // every warp has rows
+    if (split >= uint32_t(KQ_MAX_SPLIT)) split = KQ_MAX_SPLIT;
+    else if (split > 8) split = 8;
     if (split < 1) split = 1;
     if (bits == 4)
         return pair ? launch_k_quant_cfg<4, 2>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
