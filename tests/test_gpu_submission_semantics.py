@@ -54,6 +54,33 @@ def test_each_submission_reports_its_own_status(dev):
     assert c.wait().output(3) == want                     # and b's failure does not leak into c
 
 
+def test_refused_resident_bindings_leave_the_device_usable(dev):
+    """A resident buffer that is too small, or already freed, is an error of that submission and nothing else: no lock stays held and
+    the buffers bound before it are released."""
+    m, n, k = 1, 512, 4096
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=15)
+    sess = gemv_session(dev, m, n, k)
+    hx, hw, hs, small = dev.resident_from(x), dev.resident_from(w.view(np.uint32)), dev.resident_from(s), dev.allocate_resident(64)
+
+    def bind(scale):
+        bs = vb.BindingSet(sess.artifact.digest())
+        for slot, h in ((0, hx), (1, hw), (2, scale)):
+            bs.insert_resident(slot, h)
+        return bs
+
+    want = sess.submit(bind(hs)).wait().output(3)
+    for use in (sess.submit, sess.prepare):
+        with pytest.raises(vb.BackendError, match="holds 64 bytes but the program needs"):
+            use(bind(small))
+    dev.free_resident(small)
+    for use in (sess.submit, sess.prepare):
+        with pytest.raises(vb.BackendError, match="unknown or already freed"):
+            use(bind(small))
+    assert sess.submit(bind(hs)).wait().output(3) == want
+    for h in (hx, hw, hs):
+        dev.free_resident(h)  # refused while a submission holds them
+
+
 def test_prepared_submissions_equal_ordinary_ones(dev):
     m, n, k = 2, 777, 4096
     x, w, s = synth.int4_linear_inputs(m, n, k, seed=13)

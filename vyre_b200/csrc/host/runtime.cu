@@ -820,18 +820,20 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         void* dev_ptr = nullptr;
         bool resident = false;
         if (b && b->kind == VYB_BIND_RESIDENT) {
-            std::lock_guard<std::mutex> lk(d->mu);
+            std::unique_lock<std::mutex> lk(d->mu);
             Resident* r = nullptr;
             if (int32_t rc = d->resolve(b->resident, "CUDA resident dispatch", &r)) {
+                lk.unlock();  // cleanup takes it
                 cleanup();
                 return rc;
             }
             // an output may be bound with its logical (trimmed) size; inputs need the declared size
-            const size_t min_len = bd.access == VYB_ACCESS_OUTPUT ? logical : need;
-            if (r->len < min_len) {
+            const size_t min_len = bd.access == VYB_ACCESS_OUTPUT ? logical : need, len = r->len;
+            if (len < min_len) {
+                lk.unlock();
                 cleanup();
                 return fail_invalid_program("Fix: resident buffer bound to `" + bd.name + "` holds " +
-                                            std::to_string(r->len) + " bytes but the program needs " +
+                                            std::to_string(len) + " bytes but the program needs " +
                                             std::to_string(min_len) + "; allocate the declared size.");
             }
             r->inflight++;
@@ -1115,9 +1117,10 @@ int32_t vyb_prepare(vyb_instance* inst, const uint8_t artifact_digest[32], const
         void* dev_ptr = nullptr;
         void* direct_host = nullptr;
         if (b && b->kind == VYB_BIND_RESIDENT) {
-            std::lock_guard<std::mutex> lk(d->mu);
+            std::unique_lock<std::mutex> lk(d->mu);
             Resident* r = nullptr;
             if (int32_t rc = d->resolve(b->resident, "CUDA resident dispatch", &r)) {
+                lk.unlock();  // undo takes it
                 undo();
                 return rc;
             }
