@@ -580,9 +580,9 @@ int32_t vyb_prepared_submit(vyb_prepared* prepared, const vyb_binding* host_upda
 int32_t vyb_prepared_submit_after(vyb_prepared* prepared, const vyb_submission* after, const vyb_binding* host_updates,
                                   size_t n_updates, vyb_submission** submission);
 int32_t vyb_prepared_free(vyb_prepared* prepared);
-/* Host-side injection for recovery tests, like vyb_device_mark_lost: writes `word` into the instance's kernel
- * status words exactly where a kernel whose bounded wait ran out would raise it; the NEXT submission on the
- * instance then fails with DispatchFailed and later ones succeed again. No device fault is provoked. */
+/* Injection for recovery tests, like vyb_device_mark_lost: the NEXT submission on the instance runs a one-thread kernel
+ * first that raises `word` exactly where and as a kernel whose bounded wait ran out would; that submission then fails with
+ * DispatchFailed and later ones succeed again. No device fault is provoked. */
 int32_t vyb_instance_inject_status(vyb_instance* instance, uint32_t word);
 /* Submission::is_ready / wait (artifact_lifecycle.rs:112-117); wait consumes the submission */
 int32_t vyb_submission_is_ready(const vyb_submission* s);

@@ -45,8 +45,8 @@ def test_each_submission_reports_its_own_status(dev):
     want = sess.submit(bs).wait().output(3)
     a = sess.submit(bs)                                   # healthy, still to be waited for
     ffi.check(ffi.lib().vyb_instance_inject_status(sess.instance._h, 64))  # as if the NEXT kernel's bounded wait ran out
-    b = sess.submit(bs)                                   # reads the raised word
-    c = sess.submit(bs)                                   # healthy again: b cleared the word on the stream
+    b = sess.submit(bs)                                   # a kernel of b raises the word in b's own mapped slot
+    c = sess.submit(bs)                                   # healthy again: c has a slot of its own
     assert a.wait().output(3) == want                     # a is not blamed for b
     with pytest.raises(vb.BackendError, match="bounded device-side wait") as e:
         b.wait()

@@ -102,8 +102,7 @@ struct vyb_instance {
     void* scratch = nullptr;  // op-specific device scratch, sized at materialisation
     size_t scratch_len = 0;
     uint32_t* status_dev = nullptr;   // 4 words, raised by kernels whose bounded waits ran out; a submission's own slot while it is enqueued
-    uint32_t injected_status = 0;     // word that the next submission reports (vyb_instance_inject_status)
-    uint32_t* status_host = nullptr;  // pinned mirror
+    uint32_t injected_status = 0;     // word that a kernel of the next submission raises (vyb_instance_inject_status)
 
     // events are recycled: creating and destroying three per submission costs more than the launch itself
     std::vector<cudaEvent_t> timing_events, plain_events;
@@ -182,7 +181,6 @@ void instance_unref(vyb_instance* i) {
     for (auto& b : i->temps) cudaFree(b.ptr);
     if (i->scratch) cudaFree(i->scratch);
     if (i->status_dev) cudaFree(i->status_dev);
-    if (i->status_host) cudaFreeHost(i->status_host);
     device_unref(i->dev);
     delete i;
 }
@@ -205,7 +203,7 @@ struct vyb_submission {
     std::vector<void*> staged;  // pinned copies of the caller's host inputs (the BindingSet owns its bytes)
     std::vector<OutputSlot> outputs;
     std::vector<uint64_t> resident_ids;
-    uint32_t* status_host = nullptr;  // this submission's own pinned copy of the kernel status words
+    uint32_t* status_host = nullptr;  // this submission's own mapped pinned slot for the kernel status words
     vyb_prepared* prepared = nullptr;  // set when the submission replays a prepared graph (buffers belong to it)
     bool consumed = false;
 };
@@ -255,6 +253,9 @@ bool overwrites_every_output_byte(const Program& p) {
             return false;
     }
 }
+
+// What a kernel does whose bounded wait ran out (vyb_instance_inject_status)
+__global__ void raise_status_kernel(uint32_t* status, uint32_t word) { atomicOr(status, word); }
 
 // The int4 group-quantized projection y[batch][n] = x[batch][k] W^T by the kernel the payload names
 cudaError_t run_int4_linear(vyb_instance* inst, uint32_t variant, const void* x, const void* w, const void* scale, void* y,
@@ -728,12 +729,10 @@ int32_t vyb_materialize(vyb_device* d, const vyb_artifact* artifact, const vyb_p
     }
     e = cudaMalloc(reinterpret_cast<void**>(&inst->status_dev), 16);
     if (e == cudaSuccess) e = cudaMemset(inst->status_dev, 0, 16);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&inst->status_host), 16, cudaHostAllocDefault);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail_dispatch(int(e), "status buffer allocation failed: " + cuda_msg(e));
     }
-    std::memset(inst->status_host, 0, 16);
     d->refs.fetch_add(1);
     *instance = inst.release();
     clear_error();
@@ -905,7 +904,7 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
     }
     // Kernels raise their status words (only when a bounded wait runs out) straight in this submission's own mapped pinned
     // slot, so a word raised by one submission is never reported for another and nothing has to be copied or cleared on the
-    // stream between two submissions: the copy and the memset that did it kept consecutive kernels about 20 us apart.
+    // stream between two submissions: the copy and the memset that did it took 12 us of every submission in a chain.
     sub->status_host = static_cast<uint32_t*>(inst->acquire_pinned(16));
     void* own_status = nullptr;
     if (!sub->status_host || cudaHostGetDevicePointer(&own_status, sub->status_host, 0) != cudaSuccess) {
@@ -914,8 +913,6 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         return fail_oom(16, 0);
     }
     std::memset(sub->status_host, 0, 16);
-    sub->status_host[0] = inst->injected_status;
-    inst->injected_status = 0;
     sub->start = inst->acquire_event(true);  // inst->mu is held for the whole submission
     sub->end = inst->acquire_event(true);
     sub->done = inst->acquire_event(false);
@@ -923,13 +920,14 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
     cudaGetLastError();  // a non-sticky error left by an unrelated earlier call must not be blamed on this launch
     uint32_t* const shared_status = inst->status_dev;
     inst->status_dev = static_cast<uint32_t*>(own_status);
+    if (inst->injected_status) raise_status_kernel<<<1, 1, 0, inst->stream>>>(inst->status_dev, inst->injected_status);
     cudaError_t e = dispatch(inst, slot_ptr, inst->stream);
     inst->status_dev = shared_status;
     cudaEventRecord(sub->end, inst->stream);
+    if (e == cudaSuccess) inst->injected_status = 0;  // else the next submission reports it
     if (e != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(inst->stream);
-        inst->injected_status = sub->status_host[0];  // nothing ran: the next submission reports it
         cleanup();
         inst->release_event(sub->start, true);
         inst->release_event(sub->end, true);
@@ -950,7 +948,7 @@ int32_t vyb_instance_inject_status(vyb_instance* inst, uint32_t word) {
     if (!inst) return fail_invalid_program("Fix: pass a non-null instance.");
     std::lock_guard<std::mutex> ilk(inst->mu);
     cudaSetDevice(inst->dev->ordinal);
-    // like a kernel whose bounded wait ran out in the next submission on this instance
+    // a kernel of the next submission on this instance raises it, as one whose bounded wait ran out does
     inst->injected_status = word;
     clear_error();
     return VYB_OK;
