@@ -92,3 +92,35 @@ def test_small_bf16_shapes_on_both_sides_of_the_line(m, n, k):
                                         C.c_void_p(torch.cuda.current_stream().cuda_stream), None))
     torch.cuda.synchronize()
     check(y.double().cpu().numpy(), *reference(x, w, s, m, n, k), k, False)
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 40000, 6144), (1, 40000, 5120), (3, 1000, 5120)])
+def test_one_sm_is_left_free_on_request(m, n, k):
+    """VYB_LAUNCH_LEAVE_ONE_SM: no launch has more blocks than the other SMs hold at once; the outputs are the same bits."""
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=k)
+    t = [torch.from_numpy(v).cuda() for v in (x.view(np.int16), w, s.view(np.int16))]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    stream = torch.cuda.Stream()
+
+    def launch(y, flags):
+        ffi.check(ffi.lib().vyb_k_int4_gemv_ex(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), y.data_ptr(), m, n, k, 128, ffi.DT_BF16, flags,
+                                               C.c_void_p(stream.cuda_stream), None))
+
+    ys = [torch.zeros(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    launch(ys[0], 0)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        launch(ys[1], ffi.LAUNCH_LEAVE_ONE_SM)
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, count = rt.cudaGraphGetNodes(raw, 0)
+    err, nodes, count = rt.cudaGraphGetNodes(raw, count)
+    assert int(err) == 0 and count >= 1
+    for node in nodes[:count]:
+        err, params = rt.cudaGraphKernelNodeGetParams(node)
+        assert int(err) == 0 and params.gridDim.x * params.gridDim.y <= 2 * (sms - 1)
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))

@@ -80,6 +80,7 @@ struct Params {
     __nv_bfloat16* y;
     uint32_t* status;
     uint32_t m, n, k, split;
+    uint32_t tile0;          // first weight tile of this launch
 };
 
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
@@ -97,7 +98,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     Bars* bars = reinterpret_cast<Bars*>(tiles + C::STAGES * C::STAGE_BYTES);
     volatile unsigned int* abort_flag = &bars->abort_flag;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t part = blockIdx.x % p.split, n0 = (blockIdx.x / p.split) * BM;
+    const uint32_t part = blockIdx.x % p.split, n0 = (p.tile0 + blockIdx.x / p.split) * BM;
     const uint32_t blocks = p.k / KB, base = blocks / p.split, rem = blocks % p.split;
     const uint32_t kb0 = part * base + min(part, rem), kbs = base + (part < rem ? 1u : 0u);
 
@@ -339,7 +340,6 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, int sm_cou
     if (!encode_tensor_map_2d(&mw, w, p.n, p.k / 2, 1, BM, KB / 2, true) || !encode_tensor_map_2d(&mx, x, p.m, p.k, 2, BN, 64, true))
         return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles * p.split);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = stream;
@@ -351,7 +351,18 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, int sm_cou
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = constant_weights ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, int4_skinny_kernel<BN>, mw, mx, p);
+    // A caller that wants an SM left free (sm_count below the device's, VYB_LAUNCH_LEAVE_ONE_SM) gets launches that fit the other SMs at once:
+    // a second wave of one launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const uint32_t step = sm_count < sms && tiles > slots ? slots : tiles;
+    for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
+        cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split);
+        e = cudaLaunchKernelEx(&cfg, int4_skinny_kernel<BN>, mw, mx, p);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
