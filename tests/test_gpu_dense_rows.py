@@ -35,12 +35,38 @@ def test_sixteen_bit_rows_on_the_tensor_cores(dev, rows, k, n, dtype):
     x = to_bits(rng.standard_normal((rows, k)).astype(np.float32), dtype)
     w = to_bits((rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32), dtype)
     sess = vb.ArtifactSession.compile(api.linear_rows_no_bias_out_in_typed("x", "w", "out", rows, k, n, dtype), dev)
+    assert sess.kernel_variant() == 10
     got = to_f32(np.frombuffer(sess.run_host([x, w])[0], np.uint16), dtype).reshape(rows, n)
     want = to_f32(x, dtype).astype(np.float64) @ to_f32(w, dtype).astype(np.float64).T
     # one rounding to the storage type (half an ulp) plus the f32 sums in another order (k 2^-24 of the summed magnitudes)
     half_ulp = 2.0 ** (-9 if dtype == BF16 else -12)
     mags = np.abs(to_f32(x, dtype)).astype(np.float64) @ np.abs(to_f32(w, dtype)).astype(np.float64).T
     assert np.all(np.abs(got - want) <= 2 * half_ulp * np.abs(want) + k * 2.0 ** -24 * mags + 1e-7)
+
+
+def test_a_payload_that_names_the_reference_order_keeps_it(dev):
+    """Payloads written before the tensor-core form existed say variant 0: they are admitted and give the reference's bits."""
+    rows, k, n = 16, 256, 520
+    rng = np.random.default_rng(1)
+    x, w = (to_bits(rng.standard_normal(c).astype(np.float32), BF16) for c in (rows * k, n * k))
+    prog = api.linear_rows_no_bias_out_in_typed("x", "w", "out", rows, k, n, BF16)
+    sealed = vb.target_compile(vb.compile(prog)).to_bytes()
+    for at in range(len(sealed) - 36):
+        if sealed[at:at + 4] != (10).to_bytes(4, "little"):
+            continue
+        body = sealed[:at] + bytes(4) + sealed[at + 4:-32]
+        try:
+            old = api.TargetPayload.from_bytes(body + vb.blake3(body))
+        except vb.BackendError:
+            continue
+        if old.kernel_variant() == 0:
+            break
+    else:
+        raise AssertionError("no variant word found")
+    sess = api.ArtifactSession(prog, dev, old.to_bytes())
+    assert sess.kernel_variant() == 0
+    got = np.frombuffer(sess.run_host([x, w])[0], np.uint16)
+    assert np.array_equal(got, oracle.linear_rows(x, w, None, rows, k, n, dtype=oracle.DT_BF16, weight_out_in=True))
 
 
 @pytest.mark.parametrize("rows,k,n,dtype,out_in", [(1, 1030, 321, F32, True), (5, 517, 129, F32, True), (16, 256, 65, F32, False), (19, 100, 300, BF16, False),

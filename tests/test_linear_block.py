@@ -52,7 +52,7 @@ def test_builder_slots_and_errors():
     (1, 14336, True, False, 1),     # ... the norm of a long row does not
     (1, 14336, True, True, 9),
     (5, 8192, False, True, 1),
-    (1, 3072, True, True, 1),       # other k: the tensor-memory kernel
+    (1, 3072, True, True, 1),       # other k: the kernels of the plain projection
     (256, 4096, True, True, 2),     # prefill
     (1, 96, True, True, 0),
 ])
@@ -139,3 +139,11 @@ def test_graph_pass_keeps_a_norm_that_something_else_reads():
                [("output", "z", vb.value_contract(bf16, [r, h], outl, ffi.ACCESS_READ_WRITE))])
     f, taken = g.fuse_linear_blocks()
     assert taken == 0 and f.digest() == g.digest()
+
+
+# 16-bit [out, in] weights at size sum on the tensor cores, and the payload says so; everything else keeps the reference's order
+@pytest.mark.parametrize("rows,k,n,dtype,out_in,want", [(16, 256, 512, ffi.DT_BF16, True, 10), (16, 256, 512, ffi.DT_F16, True, 10), (16, 256, 511, ffi.DT_BF16, True, 0),
+                                                        (16, 260, 512, ffi.DT_BF16, True, 0), (16, 256, 512, ffi.DT_F32, True, 0), (16, 256, 512, ffi.DT_BF16, False, 0)])
+def test_target_compiler_names_the_linear_rows_form(rows, k, n, dtype, out_in, want):
+    make = vb.api.linear_rows_no_bias_out_in_typed if out_in else vb.api.linear_rows_no_bias_typed
+    assert variant(make("x", "w", "out", rows, k, n, dtype)) == want

@@ -689,8 +689,7 @@ class ArtifactSession:
         return self.payload.to_bytes()
 
     def kernel_variant(self) -> int:
-        """The hand-written kernel the target compiler chose for this program (0: the reference's own operators in its
-        evaluation order, except 16-bit linear_rows at size, whose sums run on the tensor cores)."""
+        """The hand-written kernel the target compiler chose for this program (0: reference evaluation order)."""
         return self.payload.kernel_variant()
 
     def rematerialize(self) -> None:

@@ -80,7 +80,7 @@ uint32_t select_kernel_variant(const Program& p) {
     switch (p.kind) {
         case OpKind::LinearInt4GroupedRowmajor: {
             const uint32_t batch = p.params.u[0], in_dim = p.params.u[1], group = p.params.u[3];
-            // decode batches stream the weights once per 8 rows; from 65 rows on the contraction is dense enough
+            // decode batches read the weights once (f32 outputs: once per 8 rows); from 65 rows on the contraction is dense enough
             // for the tensor-core path with in-kernel dequantisation
             const bool gemv_ok = group == 128 && in_dim % 1024 == 0;
             const bool prefill_ok = in_dim % 64 == 0 && group % 64 == 0 && in_dim % group == 0;
@@ -108,6 +108,14 @@ uint32_t select_kernel_variant(const Program& p) {
             const uint64_t in_dim = p.params.u[0], out_dim = p.params.u[1], group = p.params.u[2], batch = p.params.u[3];
             const bool big = in_dim * out_dim * batch >= (1ull << 24);
             return big && in_dim % 8 == 0 && group % 8 == 0 && in_dim % group == 0 ? KV_AFFINE_GROUPED_OUTPUT_MAJOR : KV_GENERIC;
+        }
+        case OpKind::LinearRows: {
+            // 16-bit [out, in] weights without a bias, k rows of whole 16 bytes (tensor-map strides). From 2^21 multiply-adds on: below that
+            // the call is one launch latency either way, and the reference's fixtures (compared bit for bit) keep its order.
+            const uint64_t rows = p.params.u[0], in_dim = p.params.u[1], out_dim = p.params.u[2];
+            const bool half = p.params.u[3] == VYB_DT_BF16 || p.params.u[3] == VYB_DT_F16, out_in = p.params.u[4] != 0, bias = p.params.u[5] != 0;
+            const bool tensor = half && out_in && !bias && in_dim % 8 == 0 && rows <= 65535ull * 256 && rows * in_dim * out_dim >= (1ull << 21);
+            return tensor ? KV_LINEAR_ROWS_TCGEN05 : KV_GENERIC;
         }
         case OpKind::I4BatchedMatvec: {
             const uint64_t batch = p.params.u[0], rows = p.params.u[1], cols = p.params.u[2];

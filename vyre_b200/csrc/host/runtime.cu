@@ -318,7 +318,7 @@ cudaError_t dispatch(vyb_instance* inst, void* const* b, cudaStream_t s) {
         case OpKind::Int8Pack: return launch_int8_pack((const uint32_t*)b[0], (uint32_t*)b[1], u[0], s);
         case OpKind::LinearRows: {
             const bool has_bias = u[5] != 0;
-            if (u[4] && !has_bias && rt_dtype(u[3]) != 0 && dense_rows_supported(b[0], b[1], u[0], u[1], u[2]))
+            if (inst->variant == KV_LINEAR_ROWS_TCGEN05 && dense_rows_supported(b[0], b[1], u[1]))
                 return launch_dense_rows(b[0], b[1], b[2], u[0], u[1], u[2], rt_dtype(u[3]) == 2,
                                          inst->dev->prop.multiProcessorCount, s, inst->status_dev);
             return launch_linear_rows(b[0], b[1], has_bias ? b[2] : nullptr, has_bias ? b[3] : b[2], u[0], u[1], u[2],
@@ -700,7 +700,8 @@ int32_t vyb_materialize(vyb_device* d, const vyb_artifact* artifact, const vyb_p
     if (prog.fingerprint() != artifact->a.program.fingerprint())
         return invalid_module("target module group/stage/node identity must match the neutral selected plan");
     if (prog.trap) return fail_invalid_program(prog.trap_message);
-    if (m.kernel_variant != select_kernel_variant(prog))
+    // linear_rows has the reference's order (variant 0) at every size, for payloads that were written before it had another
+    if (m.kernel_variant != select_kernel_variant(prog) && !(prog.kind == OpKind::LinearRows && m.kernel_variant == KV_GENERIC))
         return invalid_module("target module kernel variant disagrees with the op spec");
     {
         std::string why;

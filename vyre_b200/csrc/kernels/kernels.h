@@ -206,7 +206,7 @@ cudaError_t launch_moe_skinny(const void* x_sorted, const void* w, const void* s
                               uint32_t n, uint32_t k, uint32_t group, uint32_t experts, bool glu, bool wide, int sm_count, cudaStream_t stream,
                               uint32_t* status);
 // linear_rows at size with 16-bit [out, in] weights (dense_rows_tcgen05.cu): tensor cores, f32 sums in another order
-bool dense_rows_supported(const void* x, const void* w, uint32_t rows, uint32_t in_dim, uint32_t out_dim);
+bool dense_rows_supported(const void* x, const void* w, uint32_t in_dim);
 cudaError_t launch_dense_rows(const void* x, const void* w, void* out, uint32_t rows, uint32_t in_dim, uint32_t out_dim, bool f16,
                               int sm_count, cudaStream_t stream, uint32_t* status);
 cudaError_t launch_matmul_u32(const uint32_t* a, const uint32_t* b, const uint32_t* bias, uint32_t* out, uint32_t m,
