@@ -112,14 +112,14 @@ def test_one_sm_is_left_free_on_request(m, n, k):
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph, stream=stream):
         launch(ys[1], ffi.LAUNCH_LEAVE_ONE_SM)
-    rt = pytest.importorskip("cuda.bindings.runtime")
-    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
-    err, _, count = rt.cudaGraphGetNodes(raw, 0)
-    err, nodes, count = rt.cudaGraphGetNodes(raw, count)
+    cu = pytest.importorskip("cuda.bindings.driver")
+    raw = cu.CUgraph(graph.raw_cuda_graph())
+    err, _, count = cu.cuGraphGetNodes(raw, 0)
+    err, nodes, count = cu.cuGraphGetNodes(raw, count)
     assert int(err) == 0 and count >= 1
     for node in nodes[:count]:
-        err, params = rt.cudaGraphKernelNodeGetParams(node)
-        assert int(err) == 0 and params.gridDim.x * params.gridDim.y <= 2 * (sms - 1)
+        err, params = cu.cuGraphKernelNodeGetParams(node)
+        assert int(err) == 0 and params.gridDimX * params.gridDimY <= 2 * (sms - 1)
     graph.instantiate()
     graph.replay()
     torch.cuda.synchronize()
