@@ -15,9 +15,9 @@
 // A lane loads 4 (2) neighbouring outputs of a word row, a warp four rows of 128 (64) bytes, four steps ahead.
 // Measured: see launch_affine_grouped_mma.
 //
-// An output that does not come out finite is computed again by the definition in f32: a group sum meets its scale late, so that it
-// can overflow (activations from about 1e35 on, or not finite) where the definition, which scales every weight first, does not.
-// A scale of 2^95 and more, whose product with a zero point of 32 bits can overflow in the definition alone, counts as one.
+// An output that does not come out below 2^64 is computed again by the definition in f32: a group sum meets its scale late, so that it
+// can overflow (activations from about 1e35 on, or not finite) where the definition, which scales every weight first, does not;
+// and where the definition's own product of scale and zero point overflows, the sum here is at least that large.
 // Replaces, at size, the generated kernel of vyre-libs/src/nn/linear/inner/linear_4bit.rs:399-775.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -62,7 +62,24 @@ __device__ __forceinline__ float add_keep(float a, float b) {
     asm("add.rn.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
     return d;
 }
-__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7F800000u) != 0x7F800000u; }
+__device__ __forceinline__ float fma_keep(float a, float b, float c) {
+    float d;
+    asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ bool ordinary(float v) { return fabsf(v) < 0x1p64f; }  // false for NaN
+
+// One output by the definition, without its bias. Out of line: next to nothing takes it, and its loop stays off the main path's registers.
+__device__ __noinline__ float by_definition(const float* __restrict__ x, const uint32_t* __restrict__ w, const float* __restrict__ scale,
+                                            const uint32_t* __restrict__ zp, uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t row, uint32_t n) {
+    float v = 0.0f;
+    for (uint32_t k = 0; k < in_dim; ++k) {
+        const size_t at = size_t(k / group) * out_dim + n;
+        const float q = float((__ldg(w + size_t(k / 8) * out_dim + n) >> (4 * (k % 8))) & 15u), s = scale[at];
+        v = fmaf(x[size_t(row) * in_dim + k], fmaf(q, s, -__fmul_rn(float(zp[at]), s)), v);
+    }
+    return v;
+}
 
 // R: 16-output MMA tiles per warp (4: a lane loads 16 bytes of a word row, 2: 8 bytes).
 // NB: blocks of eight batch rows; the three parts of a block are an 8-column tile each, so a lane holds all parts of its rows.
@@ -173,16 +190,6 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
             *reinterpret_cast<uint2*>(&v) = __ldg(reinterpret_cast<const uint2*>(p));
         }
     };
-    auto by_definition = [&](uint32_t r, uint32_t n) {
-        float v = 0.0f;
-        for (uint32_t k = 0; k < in_dim; ++k) {
-            const size_t at = size_t(k / group) * out_dim + n;
-            const float q = float((__ldg(w + size_t(k / 8) * out_dim + n) >> (4 * (k % 8))) & 15u), s = scale[at];
-            v = fmaf(x[size_t(b0 + r) * in_dim + k], fmaf(q, s, -__fmul_rn(float(zp[at]), s)), v);
-        }
-        return v;
-    };
-
     if (one_chunk && blockIdx.x < tiles) {
         aim(blockIdx.x, 0);  // the first weights are under way while the activations are staged
         stage(0, in_dim);
@@ -193,7 +200,6 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
         for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int c = 0; c < int(AC); ++c) acc[i][c][0] = acc[i][c][1] = acc[i][c][2] = acc[i][c][3] = 0.0f;
-        float top[2] = {0.0f, 0.0f};  // largest scale of this lane's outputs (NaN takes no part; it makes the sum NaN)
         for (uint32_t k0 = 0; k0 < in_dim; k0 += chunk) {
             if (!one_chunk) {
                 aim(tile, k0);
@@ -226,11 +232,6 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                             columns4(scale + at + nz, sz);
                             columns4(zp + at + nz, zz);
                         }
-#pragma unroll
-                        for (int i = 0; i < R; ++i) {
-                            top[0] = fmaxf(top[0], fabsf(sa[i]));
-                            top[1] = fmaxf(top[1], fabsf(sz[i]));
-                        }
                     }
                     const uint32_t kw = kw_first + st * 4;
                     uint4 xb[NT];
@@ -259,11 +260,11 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                                 float s4[4];
 #pragma unroll
                                 for (int j = 0; j < 4; ++j)
-                                    s4[j] = NB == 0 ? d[i][0][j] : (d[i][(3 * c) % NT][j] + d[i][(3 * c + 1) % NT][j]) + d[i][(3 * c + 2) % NT][j];
-                                acc[i][c][0] = fmaf(sa[i], fmaf(fa, x0, s4[0]), acc[i][c][0]);
-                                acc[i][c][1] = fmaf(sa[i], fmaf(fa, x1, s4[1]), acc[i][c][1]);
-                                acc[i][c][2] = fmaf(sz[i], fmaf(fz, x0, s4[2]), acc[i][c][2]);
-                                acc[i][c][3] = fmaf(sz[i], fmaf(fz, x1, s4[3]), acc[i][c][3]);
+                                    s4[j] = NB == 0 ? d[i][0][j] : add_keep(add_keep(d[i][(3 * c) % NT][j], d[i][(3 * c + 1) % NT][j]), d[i][(3 * c + 2) % NT][j]);
+                                acc[i][c][0] = fma_keep(sa[i], fma_keep(fa, x0, s4[0]), acc[i][c][0]);
+                                acc[i][c][1] = fma_keep(sa[i], fma_keep(fa, x1, s4[1]), acc[i][c][1]);
+                                acc[i][c][2] = fma_keep(sz[i], fma_keep(fz, x0, s4[2]), acc[i][c][2]);
+                                acc[i][c][3] = fma_keep(sz[i], fma_keep(fz, x1, s4[3]), acc[i][c][3]);
                             }
                         }
                         ++grp;
@@ -271,18 +272,12 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                 }
             }
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (top[h] >= 0x1p95f)
-#pragma unroll
-                for (int i = 0; i < R; ++i)
-#pragma unroll
-                    for (int c = 0; c < int(AC); ++c) acc[i][c][2 * h] = acc[i][c][2 * h + 1] = __uint_as_float(0x7FC00000u);
         const uint32_t oa = na, oz = nz;
         const bool have_a = in_a, have_z = in_z;
         if (one_chunk && tile + gridDim.x < tiles) aim(tile + gridDim.x, 0);  // the next tile's first weights, under this one's stores
         if constexpr (WK == 1 && NB > 0) {
             // a lane holds whole sums: outputs oa + i and oz + i of rows 2 t, 2 t + 1 of every block of eight
+            bool good = true;
 #pragma unroll
             for (int c = 0; c < int(AC); ++c)
 #pragma unroll
@@ -290,8 +285,16 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     const uint32_t r = c * 8 + 2 * t + (j & 1), n = j < 2 ? oa : oz;
                     if (r >= nb || !(j < 2 ? have_a : have_z)) continue;
 #pragma unroll
-                    for (int i = 0; i < R; ++i)
-                        out[size_t(b0 + r) * out_dim + n + i] = bias[n + i] + (finite(acc[i][c][j]) ? acc[i][c][j] : by_definition(r, n + i));
+                    for (int i = 0; i < R; ++i) {
+                        out[size_t(b0 + r) * out_dim + n + i] = bias[n + i] + acc[i][c][j];
+                        good = good && ordinary(acc[i][c][j]);
+                    }
+                }
+            if (!good)  // this lane's outputs once more
+                for (uint32_t e = 0; e < 4 * R * AC; ++e) {
+                    const uint32_t r = e / (4 * R) * 8 + 2 * t + (e & 1), n = (e & 2 ? oz : oa) + e / 4 % R;
+                    if (r < nb && (e & 2 ? have_z : have_a))
+                        out[size_t(b0 + r) * out_dim + n] = bias[n] + by_definition(x, w, scale, zp, in_dim, out_dim, group, b0 + r, n);
                 }
         } else {
             // sum the k slices (and, with NB = 0, the parts) in a fixed order
@@ -317,7 +320,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     const float* p = red + (((j / TILE) * WK + q) * TILE + j % TILE) * PITCH;
                     v += NB == 0 ? (p[3 * r] + p[3 * r + 1]) + p[3 * r + 2] : p[r];
                 }
-                if (!finite(v)) v = by_definition(r, n);
+                if (!ordinary(v)) v = by_definition(x, w, scale, zp, in_dim, out_dim, group, b0 + r, n);
                 out[size_t(b0 + r) * out_dim + n] = bias[n] + v;
             }
             __syncthreads();
