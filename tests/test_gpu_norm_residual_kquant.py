@@ -180,10 +180,11 @@ def test_k_quant_construction_errors():
         vb.q4_k_linear("x", "p", "s", "m", "b", "o", 1 << 17, 1 << 17)
 
 
-# one and two word columns a thread (from 12.8 k outputs for four bits, 25.6 k for two: two scales a thread), clusters of 16 and 8 and none,
-# a ragged last block and last k part
+# eight and sixteen warps a block, one and two word columns a thread (from 12.8 k outputs for four bits, 25.6 k for two: two scales a
+# thread), clusters of many sizes and none, a ragged last block and last k part
 @pytest.mark.parametrize("bits,in_dim,out_dim", [(4, 4096, 4096), (2, 4096, 4096), (4, 1100, 1056), (2, 2048, 576), (4, 14336, 4096), (2, 14336, 4096), (4, 28672, 512),
-                                                 (4, 1100, 4128), (2, 40, 28736), (4, 1030, 14368), (2, 1030, 28736), (4, 100, 151936), (2, 70, 151936)])
+                                                 (4, 1100, 4128), (2, 40, 28736), (4, 1030, 14368), (2, 1030, 28736), (4, 100, 151936), (2, 70, 151936), (4, 2050, 9216), (2, 2050, 9216),
+                                                 (4, 5000, 2080), (2, 5000, 8256), (4, 2050, 9248)])
 def test_k_quant_linear_large_shapes_take_the_word_column_kernel(dev, bits, in_dim, out_dim):
     rng = np.random.default_rng(bits + in_dim)
     block, wpb = (32, 4) if bits == 4 else (16, 1)

@@ -397,7 +397,7 @@ cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float
 // out[i] = b[i] + sum_k x[k] * (q * scale + min): scale and minimum belong to one k and 32 (16 for Q2_K) neighbouring outputs, so
 // a thread multiplies x[k] with both once per word row and spends a byte permutation, a subtraction and an FMA on a weight. The
 // weight stream is k-major with neighbouring outputs in neighbouring fields: a thread owns W neighbouring packed word columns (a
-// warp reads 128 W contiguous bytes of a k row); the eight warps of a block and the blocks of a cluster split k, and a set of
+// warp reads 128 W contiguous bytes of a k row); the eight or sixteen warps of a block and the blocks of a cluster split k, and a set of
 // word rows is under way while the one before is summed. Slices are folded through shared memory in warp order and then over the
 // cluster in rank order (distributed shared memory; deterministic, no scratch, one launch).
 // What bounds it: those instructions (about four per weight) and the latency of the next set; HBM alone would take 6.7 us at
@@ -414,11 +414,11 @@ __device__ __forceinline__ float peer_f32(const float* p, uint32_t rank) {
     return v;
 }
 
-constexpr int KQ_WARPS = 8, KQ_MAX_SPLIT = 16;
+constexpr int KQ_MAX_SPLIT = 16;  // blocks of a cluster
 
 // grid x = column blocks * split, cluster = split
-template <int BITS, int W>
-__global__ void __launch_bounds__(32 * KQ_WARPS, 2) k_quant_linear_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ packed,
+template <int BITS, int W, int KQ_WARPS>
+__global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ packed,
                                                                               const float* __restrict__ scales, const float* __restrict__ mins,
                                                                               const float* __restrict__ b, float* __restrict__ out,
                                                                               uint32_t in_dim, uint32_t out_dim, uint32_t split) {
@@ -545,7 +545,7 @@ bool k_quant_linear_fast_supported(uint32_t in_dim, uint32_t out_dim, uint32_t b
 }
 
 namespace {
-template <int BITS, int W>
+template <int BITS, int W, int KQ_WARPS>
 cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b, float* out,
                                uint32_t in_dim, uint32_t out_dim, uint32_t split, cudaStream_t s) {
     constexpr uint32_t OPT = W * (32 / BITS);
@@ -556,45 +556,68 @@ cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const flo
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W, KQ_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_quant_linear_fast_kernel<BITS, W, KQ_WARPS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_release);
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((out_dim / OPT + 31) / 32 * split);
     cfg.blockDim = dim3(32 * KQ_WARPS);
     cfg.dynamicSmemBytes = SMEM;
     cfg.stream = s;
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = split;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_quant_linear_fast_kernel<BITS, W>, x, packed, scales, mins, b, out, in_dim, out_dim, split);
+    const uint32_t blocks = (out_dim / OPT + 31) / 32;
+    if (split == 0) {  // the largest cluster of which all column blocks' are resident at once
+        static std::atomic<int> resident[64][KQ_MAX_SPLIT + 1];  // clusters + 1; 0: not asked yet
+        const uint32_t rows = KQ_WARPS * 6, most = (in_dim + rows - 1) / rows;  // every warp has rows
+        for (split = most < uint32_t(KQ_MAX_SPLIT) ? most : uint32_t(KQ_MAX_SPLIT); split > 1; --split) {
+            int n = resident[dev & 63][split].load(std::memory_order_relaxed) - 1;
+            if (n < 0) {
+                attr.val.clusterDim.x = split;
+                cfg.gridDim = dim3(split);
+                e = cudaOccupancyMaxActiveClusters(&n, k_quant_linear_fast_kernel<BITS, W, KQ_WARPS>, &cfg);
+                if (e != cudaSuccess) return e;
+                resident[dev & 63][split].store(n + 1, std::memory_order_relaxed);
+            }
+            if (uint32_t(n) >= blocks) break;
+        }
+    }
+    attr.val.clusterDim.x = split;
+    cfg.gridDim = dim3(blocks * split);
+    return cudaLaunchKernelEx(&cfg, k_quant_linear_fast_kernel<BITS, W, KQ_WARPS>, x, packed, scales, mins, b, out, in_dim, out_dim, split);
 }
 }  // namespace
 
 cudaError_t launch_k_quant_linear_fast(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b,
                                        float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, int sm_count, cudaStream_t s) {
-    // one word column per thread unless that fills a third of the SMs by itself; then two. Two blocks share an SM; clusters do not
-    // pack every SM of a GPC, so nine tenths of the slots are counted on. Sixteen parts where all clusters of sixteen are at work at
-    // once, else eight at most (clusters of 9 to 15 leave too many SMs of a GPC empty): with eight, few outputs and a long k took
-    // longer than in the two launches before (us, those / eight parts: Q4_K 14336 x 4096 34 / 43, 28672 x 512 35 / 44, Q2_K 28672 x 512 46 / 60).
+    // one word column per thread unless that fills a third of the SMs by itself; then two. Two blocks of eight warps share an SM;
+    // clusters do not pack every SM of a GPC, so nine tenths of the slots are counted on.
     const uint32_t vpw = 32 / bits, blocks1 = (out_dim / vpw + 31) / 32;
     const bool pair = blocks1 > uint32_t(sm_count) / 3;
     const uint32_t blocks = pair ? (out_dim / (2 * vpw) + 31) / 32 : blocks1;
     uint32_t split = uint32_t(sm_count) * 9 / 5 / blocks;
+    if (split > 8) split = 8;
     if (split > (in_dim + 63) / 64) split = (in_dim + 63) / 64;  // every warp has rows
-    if (split >= uint32_t(KQ_MAX_SPLIT)) split = KQ_MAX_SPLIT;
-    else if (split > 8) split = 8;
     if (split < 1) split = 1;
+    // Few outputs with a long k. The clusters above come two blocks to an SM, so that sixteen of eight parts work on 64 SMs (half of the time
+    // of an SM was idle: 14336 x 4096 Q4_K 44 us). A block of sixteen warps has an SM to itself, and its clusters are as large as lets
+    // all of them run at once: one part too many is a second wave. Before (two launches) / eight parts / now, us: Q4_K 14336 x 4096
+    // 34 / 43 / 29, 8192 x 4096 26 / 29 / 21, 28672 x 512 35 / 45 / 26, Q2_K 14336 x 8192 52 / 60 / 44, 14336 x 4096 31 / 36 / 30.
+    const uint32_t blocks16 = (out_dim / 16 + 31) / 32;
+    if (in_dim >= 2048 && blocks16 <= 18) {
+        if (bits == 2) return launch_k_quant_cfg<2, 1, 16>(x, packed, scales, mins, b, out, in_dim, out_dim, 0, s);
+        return blocks1 <= 4 ? launch_k_quant_cfg<4, 1, 16>(x, packed, scales, mins, b, out, in_dim, out_dim, 0, s)
+                            : launch_k_quant_cfg<4, 2, 16>(x, packed, scales, mins, b, out, in_dim, out_dim, 0, s);
+    }
     if (bits == 4)
-        return pair ? launch_k_quant_cfg<4, 2>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
-                    : launch_k_quant_cfg<4, 1>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
-    return pair ? launch_k_quant_cfg<2, 2>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
-                : launch_k_quant_cfg<2, 1>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
+        return pair ? launch_k_quant_cfg<4, 2, 8>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
+                    : launch_k_quant_cfg<4, 1, 8>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
+    return pair ? launch_k_quant_cfg<2, 2, 8>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s)
+                : launch_k_quant_cfg<2, 1, 8>(x, packed, scales, mins, b, out, in_dim, out_dim, split, s);
 }
 
 }  // namespace vybk
