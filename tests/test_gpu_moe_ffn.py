@@ -114,6 +114,28 @@ def test_moe_ffn_few_rows_per_expert(tokens, hidden, inter, experts, topk, group
     check_against_oracle(*got, *want, x, wr)
 
 
+# experts of several chunks of 32 and 64 rows, all tokens on the same ones and spread
+@pytest.mark.parametrize("tokens,experts,topk,crowded", [(256, 8, 2, True), (256, 8, 2, False), (200, 16, 1, True)])
+def test_moe_ffn_few_rows_form_with_many_chunks(tokens, experts, topk, crowded):
+    test_moe_ffn_few_rows_per_expert(tokens, 512, 256, experts, topk, 128, crowded)
+
+
+# several items per CTA of the few-rows GEMMs (the accumulator sets and every ring wrap and flip their parity: 8 and 32 stages an item), narrow and wide
+@pytest.mark.parametrize("tokens,experts", [(60, 8), (128, 8)])
+def test_moe_ffn_few_rows_many_items_per_cta(tokens, experts):
+    hidden, inter, topk = 2048, 8192, 2
+    x, wr, w13, s13, w2, s2 = synth.moe_ffn_inputs(tokens, hidden, inter, experts, seed=tokens)
+    wr = synth.f32_to_bf16_bits(synth.bf16_bits_to_f32(wr) * np.float32(25.0))
+    got = run_kernel_level(x, wr, w13, s13, w2, s2, tokens, hidden, inter, experts, topk)
+    again = run_kernel_level(x, wr, w13, s13, w2, s2, tokens, hidden, inter, experts, topk)
+    for u, v in zip(got, again):
+        assert np.array_equal(u, v)
+    sel = np.arange(0, tokens, 5)
+    want = oracle.moe_ffn_int4(x, wr, w13, s13, w2, s2, sel, hidden, inter, experts, topk, mode=1)
+    # the down projection sums 8192 terms in another order than the oracle: single-ulp flips as in the full-size test below, whose share they get
+    check_against_oracle(got[0][sel], got[1][sel], got[2][sel], *want, x[sel], wr, max_tie_frac=0.05, min_identical=0.93)
+
+
 def test_moe_ffn_contract_path_matches_kernel_level_and_is_deterministic():
     tokens, hidden, inter, experts, topk = 200, 256, 512, 8, 2
     x, wr, w13, s13, w2, s2 = synth.moe_ffn_inputs(tokens, hidden, inter, experts, seed=9)
