@@ -18,7 +18,7 @@
 // results agree with it within f32 rounding before the cast. Small shapes stay on the reference-order kernel, and the
 // payload records which of the two a program got.
 //
-// Every wait is bounded; on expiry a status word is raised, the CTA drains and frees its TMEM. No multicast.
+// Every wait is bounded; on expiry a status word is raised, the CTA waits for what it has started and frees its TMEM. No multicast.
 //
 // Replaces, at size, the generated kernel of vyre-libs/src/nn/linear/inner/linear_rows.rs (typed, [out, in] weights).
 #include <cuda_bf16.h>
@@ -42,7 +42,7 @@ constexpr int CTRL_BYTES = 256, ALIGN_SLACK = 1024;
 constexpr int HALF_SM = 112 * 1024, FULL_SM = 224 * 1024;
 
 struct Bars {
-    unsigned long long full[MAX_STAGES], empty[MAX_STAGES], acc_full;
+    unsigned long long full[MAX_STAGES], empty[MAX_STAGES], acc_full, drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -84,6 +84,7 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             mbar_init(smem_u32(&bars->empty[s]), 1);
         }
         mbar_init(smem_u32(&bars->acc_full), 1);
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_w);
@@ -101,13 +102,15 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     bool ok = true;
     if (warp == 0) {
         if (elect_one()) {
-            for (uint32_t i = 0; i < kbs; ++i) {
+            uint32_t i = 0;
+            for (; i < kbs; ++i) {
                 const uint32_t s = i % p.stages, bar = smem_u32(&bars->full[s]), dst = smem_u32(tiles + s * stage_bytes);
                 if (i >= p.stages && !mbar_wait(smem_u32(&bars->empty[s]), ((i / p.stages) - 1) & 1, abort_flag)) break;
                 mbar_arrive_expect_tx(bar, stage_bytes);
                 tma_load_2d(dst, &map_w, int((kb0 + i) * BK), int(n0), bar);
                 tma_load_2d(dst + A_BYTES, &map_x, int((kb0 + i) * BK), int(r0), bar);
             }
+            settle_copies(bars->full, p.stages, i);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -125,6 +128,7 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 tc_commit(smem_u32(&bars->empty[s]));
                 if (i + 1 == kbs) tc_commit(smem_u32(&bars->acc_full));
             }
+            if (*abort_flag != 0) settle_mma(smem_u32(&bars->drained));
         }
         __syncwarp();
     }

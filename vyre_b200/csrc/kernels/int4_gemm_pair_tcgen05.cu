@@ -77,7 +77,7 @@ constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
 
 struct Bars {
     unsigned long long a_full[STAGES], b_full[STAGES], empty[STAGES], raw_full[RAW_STAGES], raw_empty[RAW_STAGES];
-    unsigned long long acc_full[2], acc_empty[2];
+    unsigned long long acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -158,6 +158,7 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             mbar_init(smem_u32(&bars->acc_full[a]), 1);
             mbar_init(smem_u32(&bars->acc_empty[a]), 8);  // leader: 4 epilogue warps of each CTA
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_x);
@@ -215,6 +216,9 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     }
                 }
             }
+            settle_copies(bars->raw_full, RAW_STAGES, r_it);
+            // the leader's barriers count both CTAs' activation boxes, and the pair leaves together (cluster_sync below)
+            if (rank == 0) settle_copies(bars->a_full, A_STAGES, a_it);
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
@@ -254,6 +258,10 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     tc_commit_pair(af);
                     tc_commit_pair(mapa(af, 1));
                 }
+            }
+            if (*abort_flag != 0) {
+                tc_commit_pair(smem_u32(&bars->drained));
+                mbar_settle(smem_u32(&bars->drained), 0);
             }
         }
         __syncwarp();

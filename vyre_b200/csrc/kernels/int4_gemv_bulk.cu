@@ -240,12 +240,20 @@ __global__ void __launch_bounds__(THREADS, 1) int4_gemv_kernel(const Params p) {
         // tell the consumers the barriers exist (they wait on named barrier 2) and start streaming at once
         asm volatile("bar.arrive 2, %0;" ::"n"(THREADS) : "memory");
         bool ok = true;
-        for (uint32_t u = 0; u < units; ++u) {
+        uint32_t u = 0;
+        for (; u < units; ++u) {
             if (u >= STAGES) ok = mbar_wait(smem_u32(&ctrl->empty[u % STAGES]), ((u / STAGES) - 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             produce(u);
         }
+        // the shared memory outlives its copies, also when a wait ran out: the last `STAGES` phases complete, with the same limit
+        if (lane == 0)
+            for (uint32_t v = u > STAGES ? u - STAGES : 0; v < u; ++v) {
+                const long long t0 = clock64();
+                for (uint32_t it = 0; it < WAIT_LIMIT && !mbar_try_wait(smem_u32(&ctrl->full[v % STAGES]), (v / STAGES) & 1); ++it)
+                    if ((it & 255u) == 255u && clock64() - t0 > WAIT_CLOCKS) break;
+            }
         if (!ok && lane == 0 && p.status) atomicOr(p.status, 2u);
         return;
     }

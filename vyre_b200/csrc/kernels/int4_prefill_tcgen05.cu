@@ -53,7 +53,7 @@ constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
 
 struct Bars {
     unsigned long long a_full[A_STAGES], a_empty[A_STAGES], raw_full[RAW_STAGES], raw_empty[RAW_STAGES];
-    unsigned long long b_full[B_STAGES], b_empty[B_STAGES], acc_full[2], acc_empty[2];
+    unsigned long long b_full[B_STAGES], b_empty[B_STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -100,6 +100,7 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             mbar_init(smem_u32(&bars->acc_full[a]), 1);
             mbar_init(smem_u32(&bars->acc_empty[a]), 4);
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_x);
@@ -154,6 +155,11 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 __syncwarp();
             }
         }
+        if (lane == 0) {
+            settle_copies(bars->raw_full, RAW_STAGES, r_it);
+            settle_copies(bars->a_full, A_STAGES, a_it);
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------ MMA issuer ---------------------------------------
         constexpr uint32_t idesc = idesc_bf16_f32(BM, BN);
@@ -188,6 +194,8 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             if (ok && lane == 0) tc_commit(smem_u32(&bars->acc_full[acc]));
             __syncwarp();
         }
+        if (*abort_flag != 0 && lane == 0) settle_mma(smem_u32(&bars->drained));
+        __syncwarp();
     } else if (warp < 6) {
         // ------------------------------------ epilogue warps ------------------------------------
         const uint32_t quad = warp & 3;

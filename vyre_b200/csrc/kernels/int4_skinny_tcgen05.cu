@@ -27,7 +27,7 @@
 // at 64 rows 17.2 us, at 16 rows 14.4 us; 4096 x 14336 at 8 rows 13.7 us (two launches of the four-row k-block form: 26.6 us).
 // At 3 to 8 rows of 4096 k the 8-row kernel (10.8 us) is the faster one and stays.
 //
-// Every wait is bounded; on expiry a status word is raised, the CTA drains and frees its TMEM. No multicast.
+// Every wait is bounded; on expiry a status word is raised, the CTA waits for what it has started and frees its TMEM. No multicast.
 //
 // Replaces the generated scalar kernel of vyre-libs/src/nn/linear/inner/linear_4bit.rs:399-775 for the row-major layout of
 // vyre-primitives/src/math/quantized/programs.rs:186-300 at decode batches.
@@ -69,7 +69,7 @@ struct Cfg {
 };
 
 struct Bars {
-    unsigned long long full[8], empty[8], a_full[4], a_empty[4], d_full[2], d_empty[2];
+    unsigned long long full[8], empty[8], a_full[4], a_empty[4], d_full[2], d_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -115,6 +115,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             mbar_init(smem_u32(&bars->d_full[s]), 1);
             mbar_init(smem_u32(&bars->d_empty[s]), 4);
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_w);
@@ -150,11 +151,13 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             for (uint32_t i = 0; i < ahead; ++i) load_raw(i);
             asm volatile("griddepcontrol.wait;" ::: "memory");
             for (uint32_t i = 0; i < ahead; ++i) load_x(i);
-            for (uint32_t i = ahead; i < kbs; ++i) {
+            uint32_t i = ahead;
+            for (; i < kbs; ++i) {
                 if (!mbar_wait(smem_u32(&bars->empty[i % C::STAGES]), ((i / C::STAGES) - 1) & 1, abort_flag)) break;
                 load_raw(i);
                 load_x(i);
             }
+            settle_copies(bars->full, C::STAGES, i);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -189,6 +192,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     a_parity ^= 1;
                 }
             }
+            if (*abort_flag != 0) settle_mma(smem_u32(&bars->drained));
         }
         __syncwarp();
     } else if (warp >= 4 && warp < 12) {

@@ -35,7 +35,7 @@ constexpr int GSTAGE_BYTES = 4 * 32 * GSTAGE_PITCH * 4;  // one 32 x 32 block pe
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + GSTAGE_BYTES;
 
 struct Bars {
-    unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+    unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -66,6 +66,7 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             mbar_init(smem_u32(&bars->acc_full[a]), 1);
             mbar_init(smem_u32(&bars->acc_empty[a]), 8);  // leader: 4 epilogue warps of each CTA
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_a);
@@ -83,7 +84,7 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
     if (warp == TMA_WARP) {
         if (elect_one()) {
-            uint32_t s = 0, parity = 1;  // of the stage's previous release; the first round finds the stages free
+            uint32_t s = 0, parity = 1, issued = 0;  // parity: of the stage's previous release; the first round finds the stages free
             bool ok = true, first = true;
             for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
                 const int m0 = int((tile % m_tiles) * 2 * BM + rank * BM);
@@ -98,6 +99,7 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     uint8_t* st = tiles + size_t(s) * STAGE_BYTES;
                     tma_load_2d_pair(smem_u32(st), &map_a, int(kb * BK), m0, leader_bar);
                     tma_load_2d_pair(smem_u32(st + A_BYTES), &map_w, int(kb * BK), n0, leader_bar);
+                    ++issued;
                     if (++s == uint32_t(STAGES)) {
                         s = 0;
                         first = false;
@@ -105,6 +107,8 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     }
                 }
             }
+            // the leader's barriers count both CTAs' boxes, and the pair leaves together (cluster_sync below)
+            if (rank == 0) settle_copies(bars->full, STAGES, issued);
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
@@ -143,6 +147,10 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     tc_commit_pair(af);
                     tc_commit_pair(mapa(af, 1));
                 }
+            }
+            if (*abort_flag != 0) {
+                tc_commit_pair(smem_u32(&bars->drained));
+                mbar_settle(smem_u32(&bars->drained), 0);
             }
         }
         __syncwarp();

@@ -60,7 +60,7 @@ constexpr int TMEM_COLS = 512;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct Bars {
-    unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
+    unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
 };
@@ -85,6 +85,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             mbar_init(smem_u32(&bars->acc_full[a]), 1);
             mbar_init(smem_u32(&bars->acc_empty[a]), 4);
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_a);
@@ -121,6 +122,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 __syncwarp();
             }
         }
+        if (lane == 0) settle_copies(bars->full, STAGES, it);
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------ MMA issuer ---------------------------------------
         constexpr uint32_t idesc = idesc_s8_s32(BM, BN);
@@ -154,6 +157,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if (ok && lane == 0) tc_commit(smem_u32(&bars->acc_full[acc]));
             __syncwarp();
         }
+        if (*abort_flag != 0 && lane == 0) settle_mma(smem_u32(&bars->drained));
+        __syncwarp();
     } else {
         // ------------------------------------ epilogue warps ------------------------------------
         const uint32_t quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32) belong to this warp

@@ -19,7 +19,7 @@
 // is the order in which a shift and a mask unpack a word, 15 instructions per eight weights instead of 17, 7 of them on the
 // half-rate logic pipe instead of 9. Values and rounding points are the pair GEMM's.
 //
-// Every wait is bounded; on expiry a status word is raised, the CTA drains and frees its TMEM. No multicast.
+// Every wait is bounded; on expiry a status word is raised, the CTA waits for what it has started and frees its TMEM. No multicast.
 //
 // Replaces the per-token expert_mlp of vyre-libs/src/nn/moe/expert_mlp.rs:18-150 for decode batches.
 #include <cuda_bf16.h>
@@ -43,7 +43,7 @@ constexpr uint32_t MAX_EXPERTS = 64;
 constexpr uint32_t ROW_TILE = 256;                // rows that an expert's segment is padded to
 
 struct Bars {
-    unsigned long long full[4], empty[4], a_full[4], a_empty[4], d_full[2], d_empty[2];
+    unsigned long long full[4], empty[4], a_full[4], a_empty[4], d_full[2], d_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
     uint32_t seg_row[MAX_EXPERTS], seg_count[MAX_EXPERTS];
@@ -111,6 +111,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             mbar_init(smem_u32(&bars->d_full[s]), 1);
             mbar_init(smem_u32(&bars->d_empty[s]), 4);
         }
+        mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_w);
@@ -151,7 +152,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     bool ok = true;
     if (warp == 0) {
         if (elect_one()) {
-            uint32_t s = 0, parity = 1;
+            uint32_t s = 0, parity = 1, issued = 0;
             bool first = true;
             for (uint32_t i = blockIdx.x; i < total && ok; i += gridDim.x) {
                 const Item it = decode(i);
@@ -169,6 +170,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
                     for (int j = 0; j < KB / 64; ++j)
                         tma_load_2d(dst + 2 * RAW_BYTES + j * BN * 128, &map_x, int(kb * KB + j * 64), x_row, bar);
+                    ++issued;
                     if (++s == uint32_t(C::STAGES)) {
                         s = 0;
                         first = false;
@@ -176,6 +178,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     }
                 }
             }
+            settle_copies(bars->full, C::STAGES, issued);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -213,6 +216,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 }
                 if (ok) tc_commit(smem_u32(&bars->d_full[set]));
             }
+            if (*abort_flag != 0) settle_mma(smem_u32(&bars->drained));
         }
         __syncwarp();
     } else if (warp >= 4 && warp < uint32_t(EPI_WARP)) {
