@@ -1,4 +1,4 @@
-"""The int4 linear at 5 to 64 rows on the tensor cores with weights unpacked into tensor memory: exact weights, f32 sums."""
+"""The int4 linear at 1 to 64 rows around the kernel that unpacks weights into tensor memory (bf16 outputs) and the ones that keep f32 outputs."""
 import ctypes as C
 
 import numpy as np
@@ -124,3 +124,45 @@ def test_one_sm_is_left_free_on_request(m, n, k):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(ys[0].view(torch.int16), ys[1].view(torch.int16))
+
+
+@pytest.mark.parametrize("m", [1, 4, 8])
+def test_dependent_launches_wait_for_their_activations(m):
+    """Seven projections in a row, each reading what the one before it wrote, launched with overlapping weight prefetch: tensor-memory, bulk-copy,
+    k-block and whole-row launches in turn. Replayed as a graph with new activations each time, the bits are those of the plain chain."""
+    dims = [(5120, 5120), (5120, 3072), (3072, 6144), (6144, 5120), (5120, 1024), (1024, 2048), (2048, 4096)]  # (k, n) of each
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    ws = [torch.randint(0, 256, (n, k // 2), generator=g, device="cuda", dtype=torch.uint8) for k, n in dims]
+    ss = [(torch.rand(n, k // 128, generator=g, device="cuda") * 0.4 + 0.8).mul_(0.22 / k ** 0.5).to(torch.bfloat16) for k, n in dims]
+    x = torch.empty(m, dims[0][0], dtype=torch.bfloat16, device="cuda")
+    chains = [[torch.zeros(m, n, dtype=torch.bfloat16, device="cuda") for _, n in dims] for _ in range(2)]
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+
+    def launch(ys, flags):
+        src = x
+        for (k, n), w, s, y in zip(dims, ws, ss, ys):
+            ffi.check(ffi.lib().vyb_k_int4_gemv_ex(src.data_ptr(), w.data_ptr(), s.data_ptr(), y.data_ptr(), m, n, k, 128, ffi.DT_BF16, flags,
+                                                   C.c_void_p(stream.cuda_stream), status.data_ptr()))
+            src = y
+
+    x.normal_(generator=g)
+    torch.cuda.synchronize()
+    launch(chains[0], ffi.LAUNCH_CONSTANT_WEIGHTS)  # first use of every kernel and workspace
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        launch(chains[0], ffi.LAUNCH_CONSTANT_WEIGHTS)
+    for _ in range(8):
+        x.normal_(generator=g)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        stream.synchronize()
+        launch(chains[1], 0)
+        stream.synchronize()
+        assert status.tolist() == [0] * 4
+        assert torch.isfinite(chains[1][-1].float()).all() and chains[1][-1].float().abs().mean() > 1e-3
+        for a, b in zip(*chains):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))

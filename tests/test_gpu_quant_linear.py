@@ -127,8 +127,8 @@ def test_decode_gemv_outlier_activations(dev, m, log2_ratio, outlier_nibble):
 @pytest.mark.parametrize("m", [1, 2, 4, 8])
 @pytest.mark.parametrize("n,k", [(4096, 14336), (300, 8192), (70, 6144)])
 def test_decode_gemv_long_rows_run_k_block_by_k_block(dev, m, n, k):
-    # rows of 6144, 8192, 14336 (multiples of 2048 beyond 4096): one launch of the half-SM kernel per block of 4096 / 2048
-    # columns, the sums carried in f32 from launch to launch
+    # rows of 6144, 8192, 14336 (multiples of 2048 beyond 4096): the half-SM kernel's k-block form, up to four bf16 rows a launch, f32 rows
+    # one a launch; more bf16 rows take the tensor-memory kernel
     x, w, s = synth.int4_linear_inputs(m, n, k, seed=k + m)
     got = run_int4(dev, x, w, s, m, n, k)
     want = oracle.int4_rowmajor_linear(x, w, s, m, n, k)
@@ -147,8 +147,8 @@ def test_decode_gemv_long_rows_run_k_block_by_k_block(dev, m, n, k):
 
 
 def test_decode_gemv_other_row_lengths_with_outliers(dev):
-    # k that is not 2048 or 4096 takes the bulk-copy kernel, which keeps 22 bits per group: exact for elements within
-    # 2^-14 of their group's maximum
+    # f32 outputs of odd multiples of 1024 take the bulk-copy kernel, which keeps 30 bits per group for them: exact for elements within
+    # 2^-22 of their group's maximum
     m, n, k = 3, 320, 3072
     x, w, s = _outlier_inputs(m, n, k, 10, 8, seed=77)
     got32 = run_int4(dev, x, w, s, m, n, k, out_dtype=ffi.DT_F32)
@@ -157,7 +157,7 @@ def test_decode_gemv_other_row_lengths_with_outliers(dev):
 
 
 def test_decode_gemv_larger_batches_and_generic_fallback(dev):
-    # batch > 8 loops the skinny kernel; group != 128 or k % 1024 != 0 takes the plain-load kernel
+    # f32 batches beyond 8 loop the eight-row kernels; group != 128 or k % 1024 != 0 takes the plain-load kernel
     for (m, n, k, g) in [(13, 96, 1024, 128), (20, 40, 2048, 128), (3, 50, 512, 64), (2, 33, 1280, 128), (4, 20, 256, 32)]:
         x, w, s = synth.int4_linear_inputs(m, n, k, group=g, seed=m * 7 + n)
         got = run_int4(dev, x, w, s, m, n, k, group=g, out_dtype=ffi.DT_F32)

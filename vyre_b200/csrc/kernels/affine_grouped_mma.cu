@@ -26,6 +26,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "tcgen05_common.cuh"
 
 namespace vybk {
 namespace {
@@ -33,15 +34,10 @@ namespace {
 constexpr int WARPS = 8, THREADS = WARPS * 32;
 constexpr uint32_t XS_BYTES = 64 * 1024;  // staged activations of one k chunk
 
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t bits) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(mask), "r"(bits));
-    return d;
-}
 // nibbles i and i + 4 of a word -> bf16 pair q - 8 (0x43nn is 128 + nn, the subtraction is exact)
 __device__ __forceinline__ uint32_t unpack_pair(uint32_t w, int i) {
     uint32_t d;
-    asm("sub.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(and_or(w >> (4 * i), 0x000F000Fu, 0x43004300u)), "r"(0x43084308u));
+    asm("sub.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(tc::and_or(w >> (4 * i), 0x000F000Fu, 0x43004300u)), "r"(0x43084308u));
     return d;
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {

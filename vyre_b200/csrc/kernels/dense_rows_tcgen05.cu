@@ -57,12 +57,6 @@ struct Params {
     uint32_t f16;
 };
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 // grid: x = weight tiles * split (a cluster spans the k parts of one tile), y = tiles of bn rows
 __global__ void __launch_bounds__(THREADS, 2)
 dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {

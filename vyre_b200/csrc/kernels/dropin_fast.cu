@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "tcgen05_common.cuh"
 
 namespace vybk {
 namespace {
@@ -403,17 +404,6 @@ cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float
 // What bounds it: those instructions (about four per weight) and the latency of the next set; HBM alone would take 6.7 us at
 // 4096 x 14336 Q4_K. Measured per linear in a chain of submissions, before (k chunks to scratch, a second launch that folds them)
 // and now: Q4_K 4096 -> 14336 48 / 29 us, Q2_K 4096 -> 14336 53 / 30 us; rule and figures for long k: launch_k_quant_linear_fast.
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float peer_f32(const float* p, uint32_t rank) {
-    uint32_t a = uint32_t(__cvta_generic_to_shared(p));
-    float v;
-    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}" : "=f"(v) : "r"(a), "r"(rank) : "memory");
-    return v;
-}
-
 constexpr int KQ_MAX_SPLIT = 16;  // blocks of a cluster
 
 // grid x = column blocks * split, cluster = split
@@ -523,21 +513,21 @@ __global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_f
         for (int s = 0; s < KQ_WARPS; ++s) sum += red[s * PITCH + (o / OPT) * (OPT + 1) + o % OPT];
         sums[o] = sum;
     }
-    cluster_barrier();
+    tc::cluster_sync();
     for (uint32_t o = rank * 32 + lane + warp * 32 * split; o < 32 * OPT; o += 32 * split * KQ_WARPS) {
         const uint32_t i = xb * 32 * OPT + o;
         if (i >= out_dim) continue;
         float part[KQ_MAX_SPLIT];
 #pragma unroll
         for (uint32_t q = 0; q < KQ_MAX_SPLIT; ++q)
-            if (q < split) part[q] = peer_f32(sums + o, q);
+            if (q < split) part[q] = tc::ld_cluster_f32(tc::mapa(tc::smem_u32(sums + o), q));
         float sum = part[0];
 #pragma unroll
         for (uint32_t q = 1; q < KQ_MAX_SPLIT; ++q)
             if (q < split) sum += part[q];
         out[i] = sum + b[i];
     }
-    cluster_barrier();  // no block leaves while another still reads its sums
+    tc::cluster_sync();  // no block leaves while another still reads its sums
 }
 
 bool k_quant_linear_fast_supported(uint32_t in_dim, uint32_t out_dim, uint32_t bits) {

@@ -83,12 +83,6 @@ struct Params {
     uint32_t tile0;          // first weight tile of this launch
 };
 
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 template <int BN>
 __global__ void __launch_bounds__(THREADS, Cfg<BN>::HALF ? 2 : 1)
 int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
