@@ -61,7 +61,7 @@ def test_long_rows_beyond_four_at_kernel_level_in_a_chain(m, n, k, f32):
 
 
 # f32 outputs: the sum of a 128-k group is exact, so large activations that cancel inside their group leave no trace in its small ones.
-# (Whole rows of 2048 and 4096 beyond one row run on the f16 tensor path, whose group sums are f32.)
+# (Whole rows of 2048 and 4096 beyond one row run on the tensor cores, whose group sums are f32.)
 @pytest.mark.parametrize("m,n,k", [(1, 300, 1024), (3, 64, 3072), (8, 200, 5120), (2, 140, 6144), (5, 72, 14336), (12, 96, 3072), (33, 40, 8192)])
 def test_f32_outputs_have_exact_group_sums(dev, m, n, k):
     rng = np.random.default_rng(m + k)

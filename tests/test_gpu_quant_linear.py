@@ -157,7 +157,7 @@ def test_decode_gemv_other_row_lengths_with_outliers(dev):
 
 
 def test_decode_gemv_larger_batches_and_generic_fallback(dev):
-    # f32 batches beyond 8 loop the eight-row kernels; group != 128 or k % 1024 != 0 takes the plain-load kernel
+    # f32 batches beyond 8 loop the eight-row kernels (k 2048 and 4096: one launch); group != 128 or k % 1024 != 0 takes the plain-load kernel
     for (m, n, k, g) in [(13, 96, 1024, 128), (20, 40, 2048, 128), (3, 50, 512, 64), (2, 33, 1280, 128), (4, 20, 256, 32)]:
         x, w, s = synth.int4_linear_inputs(m, n, k, group=g, seed=m * 7 + n)
         got = run_int4(dev, x, w, s, m, n, k, group=g, out_dtype=ffi.DT_F32)

@@ -67,7 +67,7 @@ cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const voi
     // not (activations of widely different size, relative error against 64-bit sums: 0.8e-7 against 1.4 to 2.0e-7).
     if (int4_gemv_kblocks_supported(1, n, k, 128)) {
         if (!out_f32 && m > 4 && int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
-            return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, sm_count, stream, status, constant_weights);
+            return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, 0, sm_count, stream, status, constant_weights);
         for (uint32_t b0 = 0; b0 < m; b0 += step) {
             const uint32_t mb = m - b0 < step ? m - b0 : step;
             cudaError_t e = launch_int4_gemv_kblocks(static_cast<const uint16_t*>(x_bf16) + size_t(b0) * k, w_packed, scale_bf16,
@@ -99,7 +99,7 @@ cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const voi
     // group sums (activations of widely different size: error 0.6 to 1.0e-7 against 1.1 to 2.9e-7).
     const bool small = n <= 16 * uint32_t(sm_count) && (k == 1024 || (k == 3072 && m <= 2));
     if (!out_f32 && !small && int4_skinny_supported(x_bf16, w_packed, scale_bf16, m, n, k, 128))
-        return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, sm_count, stream, status, constant_weights);
+        return launch_int4_skinny(x_bf16, w_packed, scale_bf16, y, m, n, k, 0, sm_count, stream, status, constant_weights);
     return launch_int4_gemv_bulk(x_bf16, w_packed, scale_bf16, y, m, n, k, out_f32, sm_count, stream, status, constant_weights);
 }
 

@@ -1,6 +1,6 @@
-// Group-quantized int4 linear for up to 64 activation rows on the tensor cores (tcgen05, sm_100a), weights exact, bf16 outputs:
+// Group-quantized int4 linear for up to 64 activation rows on the tensor cores (tcgen05, sm_100a), weights exact:
 //
-//   y[m, n] = bf16( sum_g s[n, g] * sum_{k in g} x[m, k] * (q[n, k] - 8) )        group 128
+//   y[m, n] = cast( sum_g s[n, g] * sum_{k in g} x[m, k] * (q[n, k] - 8) )        group 128
 //
 // What bounds it: the packed weights' bytes (each is read once for all rows) and, close behind, the instructions that turn
 // nibbles into tensor-core operands. So the WEIGHT rows are the M = 128 side of the MMA and the activation rows its N side
@@ -20,8 +20,9 @@
 // its weights while this one drains. Few weight tiles: the k range of a tile is split over a cluster, the partial sums are
 // added in rank order over distributed shared memory (deterministic, no workspace).
 //
-// f32 outputs keep the integer kernels, whose group sums are exact (launch_int4_gemv); next to the one rounding to bf16 the difference
-// does not show (relative error 1.65e-3 on both).
+// f32 outputs run here only where the kernel they had sums in f32 as well (beyond eight rows of 2048 and 4096 k); the others keep the
+// integer kernels, whose group sums are exact (launch_int4_gemv). Next to the rounding to bf16 the difference does not show (relative
+// error 1.65e-3 on both).
 //
 // Measured (64-launch graphs over rotating weights): 14336 x 4096 at 48 rows 15.1 us (six launches of the 8-row kernel: 91 us),
 // at 64 rows 17.2 us, at 16 rows 14.4 us; 4096 x 14336 at 8 rows 13.7 us (two launches of the four-row k-block form: 26.6 us).
@@ -77,13 +78,13 @@ static_assert(sizeof(Bars) <= CTRL_BYTES, "control block");
 
 struct Params {
     const uint16_t* scales;  // bf16 [n][k / 128]
-    __nv_bfloat16* y;
+    void* y;
     uint32_t* status;
     uint32_t m, n, k, split;
     uint32_t tile0;          // first weight tile of this launch
 };
 
-template <int BN>
+template <int BN, bool OUT_F32>
 __global__ void __launch_bounds__(THREADS, Cfg<BN>::HALF ? 2 : 1)
 int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
     using C = Cfg<BN>;
@@ -94,6 +95,10 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t part = blockIdx.x % p.split, n0 = (p.tile0 + blockIdx.x / p.split) * BM;
     const uint32_t blocks = p.k / KB, base = blocks / p.split, rem = blocks % p.split;
+    auto store = [&](size_t at, float v) {
+        if constexpr (OUT_F32) static_cast<float*>(p.y)[at] = v;
+        else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
+    };
     const uint32_t kb0 = part * base + min(part, rem), kbs = base + (part < rem ? 1u : 0u);
 
     if (threadIdx.x == 0) {
@@ -273,7 +278,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (p.split == 1) {
 #pragma unroll
                 for (int c = 0; c < BN; ++c)
-                    if (uint32_t(c) < p.m && row < p.n) p.y[size_t(c) * p.n + row] = __float2bfloat16_rn(acc[c]);
+                    if (uint32_t(c) < p.m && row < p.n) store(size_t(c) * p.n + row, acc[c]);
             } else {
                 // the last group sum is complete, so every load and MMA of this CTA is: the stages are free
                 float* partial = reinterpret_cast<float*>(tiles);  // [BN][128]
@@ -297,7 +302,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
             for (uint32_t q = 1; q < MAX_SPLIT; ++q)
                 if (q < p.split) sum += v[q];
-            p.y[size_t(c) * p.n + n0 + o] = __float2bfloat16_rn(sum);
+            store(size_t(c) * p.n + n0 + o, sum);
         }
         cluster_sync();  // no CTA leaves while another still reads its shared memory
     } else {
@@ -311,18 +316,22 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 template <int BN>
-cudaError_t launch_bn(const void* x, const void* w, const Params& p0, int sm_count, cudaStream_t stream, bool constant_weights) {
+cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t out_f32, int sm_count, cudaStream_t stream, bool constant_weights) {
     using C = Cfg<BN>;
+    using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const Params);
+    static const Kernel kernels[2] = {int4_skinny_kernel<BN, false>, int4_skinny_kernel<BN, true>};
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        e = cudaFuncSetAttribute(int4_skinny_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(int4_skinny_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
+        for (const Kernel f : kernels) {
+            e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return e;
+        }
         configured.fetch_or(bit, std::memory_order_release);
     }
     Params p = p0;
@@ -357,7 +366,7 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, int sm_cou
     const uint32_t step = sm_count < sms && tiles > slots ? slots : tiles;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split);
-        e = cudaLaunchKernelEx(&cfg, int4_skinny_kernel<BN>, mw, mx, p);
+        e = cudaLaunchKernelEx(&cfg, kernels[out_f32 ? 1 : 0], mw, mx, p);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -370,19 +379,19 @@ bool int4_skinny_supported(const void* x, const void* w, const void* scale, uint
            ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0 && (reinterpret_cast<uintptr_t>(scale) & 3u) == 0;
 }
 
-cudaError_t launch_int4_skinny(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y_bf16, uint32_t m, uint32_t n,
-                               uint32_t k, int sm_count, cudaStream_t stream, uint32_t* status, bool constant_weights) {
+cudaError_t launch_int4_skinny(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n,
+                               uint32_t k, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status, bool constant_weights) {
     Params p = {};
     p.scales = static_cast<const uint16_t*>(scale_bf16);
-    p.y = static_cast<__nv_bfloat16*>(y_bf16);
+    p.y = y;
     p.status = status;
     p.m = m;
     p.n = n;
     p.k = k;
     // 17..32 rows take the 48-column form: a 32-column form with two CTAs per SM measured 18.7 us at 14336 x 4096, 48 columns 15.7
-    if (m <= 16) return launch_bn<16>(x_bf16, w_packed, p, sm_count, stream, constant_weights);
-    if (m <= 48) return launch_bn<48>(x_bf16, w_packed, p, sm_count, stream, constant_weights);
-    return launch_bn<64>(x_bf16, w_packed, p, sm_count, stream, constant_weights);
+    if (m <= 16) return launch_bn<16>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
+    if (m <= 48) return launch_bn<48>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
+    return launch_bn<64>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
 }
 
 }  // namespace vybk

@@ -26,10 +26,10 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
                                      uint32_t n, uint32_t k, uint32_t out_f32, int sm_count, cudaStream_t stream,
                                      bool constant_weights, const void* resid = nullptr, const void* gate = nullptr,
                                      bool* stores_fused = nullptr);
-// tcgen05 form with unpacked weights in tensor memory (int4_skinny_tcgen05.cu): up to 64 rows in one launch, k a multiple of 256, bf16 outputs
+// tcgen05 form with unpacked weights in tensor memory (int4_skinny_tcgen05.cu): up to 64 rows in one launch, k a multiple of 256
 bool int4_skinny_supported(const void* x, const void* w, const void* scale, uint32_t m, uint32_t n, uint32_t k, uint32_t group);
-cudaError_t launch_int4_skinny(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y_bf16, uint32_t m, uint32_t n,
-                               uint32_t k, int sm_count, cudaStream_t stream, uint32_t* status, bool constant_weights);
+cudaError_t launch_int4_skinny(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n,
+                               uint32_t k, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status, bool constant_weights);
 // bulk-copy form (int4_gemv_bulk.cu): up to eight rows, k a multiple of 1024, integer sums
 cudaError_t launch_int4_gemv_bulk(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n,
                                   uint32_t k, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status,
