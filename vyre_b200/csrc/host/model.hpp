@@ -142,8 +142,8 @@ enum KernelVariant : uint32_t {
     KV_I4_MATVEC_WARP_ROWS = 6,          // i4x8 matvec, warp per row
     KV_K_QUANT_WORD_COLUMNS = 7,         // K-quant linear: packed word columns per thread, k slices folded in fixed order
     KV_RMS_NORM_TREE = 8,                // RMSNorm rows of 2048 elements and more: sum of squares as a tree, not a chain
-    KV_LINEAR_ROWS_TCGEN05 = 10,         // 16-bit linear_rows at size: sums on the tensor cores
     KV_INT4_BLOCK_GEMV = 9,              // decode GEMV with the norm in its prologue and / or the residual add in its stores
+    KV_LINEAR_ROWS_TCGEN05 = 10,         // 16-bit linear_rows at size: sums on the tensor cores
 };
 
 uint32_t select_kernel_variant(const Program& p);
