@@ -138,7 +138,7 @@ enum KernelVariant : uint32_t {
     KV_INT4_PREFILL_TCGEN05 = 2,
     KV_INT8_GEMM_TCGEN05 = 3,
     KV_MOE_FUSED = 4,
-    KV_AFFINE_GROUPED_OUTPUT_MAJOR = 5,  // the reference's own 4-bit layout at size: neighbouring outputs per lane, a weight unpacked once for all rows
+    KV_AFFINE_GROUPED_OUTPUT_MAJOR = 5,  // the reference's own 4-bit layout at size: f32 or tensor-core sums by group, outputs and rows (contract buffers are always aligned)
     KV_I4_MATVEC_WARP_ROWS = 6,          // i4x8 matvec, warp per row
     KV_K_QUANT_WORD_COLUMNS = 7,         // K-quant linear: packed word columns per thread, k slices folded in fixed order
     KV_RMS_NORM_TREE = 8,                // RMSNorm rows of 2048 elements and more: sum of squares as a tree, not a chain

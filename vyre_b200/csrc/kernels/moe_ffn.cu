@@ -385,9 +385,10 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
     if (e != cudaSuccess) return e;
     // Few rows per expert: weight rows on the M side, unpacked into tensor memory (8 experts, 4096 / 14336, top-2: 270 against
     // 784 us at 64 tokens, 644 against 795 us at 512 = 128 rows per expert; at 192 rows both take about 700 us: the pair GEMM's 256-row
-    // tiles are filled there). The line is the average, which the host knows: with all tokens on one or two experts this form is up to 13 %
-    // slower than the pair GEMM (512 tokens on two experts 500 against 449 us). A choice by the plan kernel, both forms launched and
-    // one returning at once, cost every balanced layer 9 us (3 to 10 %).
+    // tiles are filled there). The line is the average, which the host knows: with all tokens on one or two experts this form can be
+    // slower than the pair GEMM (wide: 512 tokens on two of 8 experts 500 against 449 us; narrow: 160 tokens on two of 16 experts, 4096 / 4096,
+    // 160 against 130 us, balanced 193 against 459). A choice by the plan kernel, both forms launched and one returning at once,
+    // cost every balanced layer 9 us (3 to 10 %); 64 columns from 129 tokens on whatever the average, 1 to 7 %.
     if (skinny) {
         const bool wide = uint64_t(tokens) * topk > uint64_t(experts) * 20;  // at 20 rows on average the fullest of balanced experts still fits 32
         e = launch_moe_skinny(xg, w13, s13, h, plan, L.max_rows, inter, hidden, group, experts, true, wide, sm_count, stream, status);
