@@ -81,10 +81,11 @@ def test_tiled_rows_keep_the_reference_order_bits(dev, rows, k, n, dtype, out_in
     assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
 
 
-# the tiled kernel's range: from 2^14 outputs (f32 [out, in]), 2^16 (16 bits), 2^18 and 2^19 ([in, out]), one and four rows a warp, with and
-# without a bias, tails in rows, outputs and k
+# the tiled kernel's range: f32 from 2^14 outputs ([out, in]) and 2^18 ([in, out]) or from 2^22 and 2^23 weights, 16 bits [out, in] from 5 x 2^15
+# outputs, one and four rows a warp, with and without a bias, tails in rows, outputs and k
 @pytest.mark.parametrize("rows,k,n,dtype,out_in,bias", [(5, 33, 3300, F32, True, False), (4, 35, 4100, F32, True, False), (4, 5, 65600, F32, False, True),
-                                                        (17, 100, 3900, BF16, True, False), (66, 9, 4100, F32, False, True), (129, 5, 4100, F16, False, False),
+                                                        (43, 100, 3900, BF16, True, False), (66, 9, 4100, F32, False, True), (42, 33, 3910, F16, True, False),
+                                                        (1, 2055, 2049, F32, True, False), (3, 4099, 2050, F32, False, True),
                                                         (70, 37, 3800, F32, False, False)])
 def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
     rng = np.random.default_rng(rows + k)

@@ -361,9 +361,9 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t o
     // A caller that wants an SM left free (sm_count below the device's, VYB_LAUNCH_LEAVE_ONE_SM) gets launches that fit the other SMs at once:
     // a second wave of one launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
     int sms = 0;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (tiles > slots) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    const uint32_t step = sm_count < sms && tiles > slots ? slots : tiles;
+    const uint32_t step = sm_count < sms ? slots : tiles;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split);
         e = cudaLaunchKernelEx(&cfg, kernels[out_f32 ? 1 : 0], mw, mx, p);

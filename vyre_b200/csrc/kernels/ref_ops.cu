@@ -620,16 +620,18 @@ cudaError_t launch_int8_pack(const uint32_t* in, uint32_t* out, uint32_t n, cuda
 }
 cudaError_t launch_linear_rows(const void* x, const void* w, const void* bias, void* out, uint32_t rows,
                                uint32_t in_dim, uint32_t out_dim, uint32_t dtype, uint32_t out_in, cudaStream_t s) {
-    // The tiled form (same bits) where the plain kernel is bound by its throughput and not by its chain of dependent additions, which is
-    // the shorter one. Plain: 280 products a ns with [out, in] weights (neighbouring lanes a row apart), 2900 with [in, out], 33 to
-    // 52 ns a step of the chain; tiled: 55 to 66 ns a step, 140 with 16-bit operands. Measured, plain / tiled, us: f32 [out, in]
-    // 64 x 4096 x 64 203 / 269, 16 x 512 x 512 38 / 40, 4 x 4096 x 4096 317 / 222, 16 x 2048 x 2048 285 / 140, 64 x 4096 x 4096 3870 / 316;
-    // 16 bits [out, in] (without tensor cores) 16 x 100 x 3000 17 / 21, 64 x 100 x 3000 38 / 21; f32 [in, out] 16 x 4096 x 4096
-    // 200 / 271, 64 x 4096 x 4096 369 / 315; 16 bits [in, out] 64 x 4096 x 4096 418 / 638, 256 x 2048 x 2048 401 / 348.
-    const uint64_t outputs = uint64_t(rows) * out_dim;
+    // The tiled form (same bits) where it is the faster one. The plain kernel is bound by its chain of dependent additions (33 to 52 ns a step)
+    // as long as its operands come from L2, by their latency (about 88 ns a step) when they do not, and with many outputs by its
+    // throughput (280 products a ns with [out, in] weights, whose neighbouring lanes read a row apart, 2900 with [in, out]). The tiled one
+    // takes 54 to 66 ns a step from either, 145 to 230 with 16-bit operands. So f32 weights too large to be in L2 from one call to the next, or many
+    // outputs. Plain / tiled, us: f32 [out, in] 1 x 8188 x 4096 from HBM 724 / 488, 16 x 2048 x 2048 285 / 140, 64 x 4096 x 4096 3870 / 316; from
+    // L2 5 x 3000 x 1000 125 / 199; f32 [in, out] 1 x 4092 x 8192 from HBM 351 / 245, from L2 4 x 2048 x 2048 67 / 114; 16 bits [out, in] (odd
+    // k) 16 x 4092 x 4096 from HBM 422 / 948, 64 x 4092 x 4096 1492 / 904; 16 bits [in, out] never (64 x 4096 x 4096 from L2 418 / 638).
+    const uint64_t outputs = uint64_t(rows) * out_dim, weights = uint64_t(in_dim) * out_dim;
     const int rt = rows <= 4 ? 1 : 4;
-    const uint64_t from = out_in ? (dtype == 0 ? 1u << 14 : 1u << 16) : dtype == 0 ? 1u << 18 : 1u << 19;
-    if (outputs >= from && outputs * in_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
+    const bool tiled = dtype == 0 ? weights >= (out_in ? 1ull << 22 : 1ull << 23) || outputs >= (out_in ? 1ull << 14 : 1ull << 18)
+                                  : out_in && outputs >= (5ull << 15);
+    if (tiled && outputs * in_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
         const dim3 grid((out_dim + 63) / 64, (rows + 4 * rt - 1) / (4 * rt));
         if (rt == 1) linear_rows_tiled_kernel<1><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
         else linear_rows_tiled_kernel<4><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
