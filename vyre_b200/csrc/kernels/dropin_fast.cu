@@ -339,17 +339,12 @@ cudaError_t launch_affine_cfg(const float* x, const uint32_t* w, const float* sc
 cudaError_t launch_affine_grouped_fast(const float* x, const uint32_t* w, const float* scale, const uint32_t* zp,
                                        const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                        uint32_t batch, int sm_count, cudaStream_t s) {
-    constexpr int DKS = 8;
-    // Groups of whole 32-k steps and aligned rows: tensor-core sums (figures there). The f32 kernels below keep the other groups (8, 24 ...),
-    // outputs that are no multiple of four and unaligned buffers, and three or four rows with few groups and outputs, where the tensor-core
-    // blocks stage activations for eight rows and have little else to do (4 rows, group 128, us, f32 / tensor cores: 4096 x 4096 24 / 27,
-    // 8192 x 4096 39 / 44, 4096 x 8192 31 / 33; 4096 x 11008 40 / 40, 8192 x 8192 71 / 54; group 64 4096 x 4096 30 / 27): all blocks
-    // of the f32 kernel resident at once, two an SM at most.
-    const uint32_t blocks32 = (out_dim + 31) / 32, sms = uint32_t(sm_count);
-    const bool few = batch >= 3 && batch <= 4 && group == 128 && (in_dim <= 4096 ? blocks32 <= 2 * sms : in_dim <= 8192 && blocks32 <= sms);
-    if (!few && affine_grouped_mma_supported(x, w, scale, zp, in_dim, out_dim, group))
+    // Groups of whole 32-k steps and aligned rows: tensor-core sums, faster at every batch (figures there). The f32 kernels below
+    // keep the other groups (8, 24 ...), outputs that are no multiple of four and unaligned buffers.
+    if (affine_grouped_mma_supported(x, w, scale, zp, in_dim, out_dim, group))
         return launch_affine_grouped_mma(x, w, scale, zp, b, out, in_dim, out_dim, group, batch, sm_count, s);
     // decode batches: whole activation rows in shared memory, scale and zero point applied per group
+    constexpr int DKS = 8;
     if (batch <= 4 && (group == 64 || group == 128) && in_dim <= 8192) {
         const int dbt = batch == 1 ? 1 : batch == 2 ? 2 : 4;
         const size_t smem = (size_t(dbt) * in_dim + size_t(dbt) * (in_dim / group) * DKS + size_t(DKS) * dbt * 32) * sizeof(float);
