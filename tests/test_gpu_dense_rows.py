@@ -99,7 +99,7 @@ def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
     assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
 
 
-@pytest.mark.parametrize("m,k", [(2, 512), (2, 520), (4097, 896), (4097, 904), (1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
+@pytest.mark.parametrize("m,k", [(2, 512), (513, 512), (513, 520), (4097, 896), (4097, 904), (1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
 def test_wide_quantiser_equals_the_rule(m, k):
     import torch
     rng = np.random.default_rng(k)
@@ -114,7 +114,7 @@ def test_wide_quantiser_equals_the_rule(m, k):
 
 # the register forms (16 and 32 elements a thread) and the loop: one summation order, restated here
 @pytest.mark.parametrize("rows,hidden,dtype", [(3, 2048, BF16), (2, 4100, F32), (1, 4096, F16), (5, 8192, BF16), (2, 8200, F32),
-                                               (296, 2052, BF16), (297, 2052, BF16)])
+                                               (592, 2052, BF16), (593, 2052, BF16), (297, 4100, BF16)])
 def test_long_row_norm_in_registers_has_the_tree_bits(dev, rows, hidden, dtype):
     rng = np.random.default_rng(hidden)
     x = to_bits(rng.standard_normal((rows, hidden)).astype(np.float32), dtype)

@@ -339,8 +339,9 @@ cudaError_t launch_affine_cfg(const float* x, const uint32_t* w, const float* sc
 cudaError_t launch_affine_grouped_fast(const float* x, const uint32_t* w, const float* scale, const uint32_t* zp,
                                        const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                        uint32_t batch, int sm_count, cudaStream_t s) {
-    // Groups of whole 32-k steps and aligned rows: tensor-core sums, faster at every batch (figures there). The f32 kernels below
-    // keep the other groups (8, 24 ...), outputs that are no multiple of four and unaligned buffers.
+    // Groups of whole 32-k steps and aligned rows: tensor-core sums, faster at every batch (figures there; three and four rows at group 128 with
+    // weights in L2 are the exception, 4 x 4096 x 4096 28 against 24 us, with weights from HBM 32 against 39). The f32 kernels below keep
+    // the other groups (8, 24 ...), outputs that are no multiple of four and unaligned buffers.
     if (affine_grouped_mma_supported(x, w, scale, zp, in_dim, out_dim, group))
         return launch_affine_grouped_mma(x, w, scale, zp, b, out, in_dim, out_dim, group, batch, sm_count, s);
     // decode batches: whole activation rows in shared memory, scale and zero point applied per group

@@ -673,10 +673,10 @@ cudaError_t launch_residual_add(const void* residual, const void* branch, void* 
 }
 cudaError_t launch_rms_norm(const void* input, const void* weight, const void* gate, void* out, uint32_t rows, uint32_t hidden,
                             float eps, uint32_t dtype, uint32_t weight_dtype, bool tree, cudaStream_t s) {
-    // In registers while all rows fit the SMs at once (two blocks of 108 registers on each of 148: its latency is shorter); more rows: the
-    // loop, whose 27 registers hold eight blocks on an SM (us, loop / registers: 64 x 8192 10.4 / 8.3, 296 x 4096 8.3 / 6.3, 296 x 8192
-    // 10.9 / 10.4; 600 x 6144 10.4 / 12.4, 1024 x 2048 6.3 / 8.3, 8192 x 4096 41 / 48, 8192 x 6144 60 / 94)
-    const bool few = rows <= 296;
+    // In registers while all rows fit the SMs at once (four blocks of 60 registers, two of 108, on each of 148: its latency is shorter);
+    // more rows: the loop, whose 27 registers hold eight blocks on an SM (us, loop / registers: 64 x 8192 10.4 / 8.3, 400 x 4096 8.3 / 6.3,
+    // 296 x 8192 10.9 / 10.4; 600 x 6144 10.4 / 12.4, 1024 x 2048 6.3 / 8.3, 8192 x 4096 41 / 48, 8192 x 6144 60 / 94)
+    const bool few = rows <= (hidden <= 4096 ? 592u : 296u);
     if (tree && !gate && few && hidden <= 4096)
         rms_norm_tree_regs_kernel<16><<<rows, 256, 0, s>>>(input, weight, out, hidden, eps, dtype, weight_dtype);
     else if (tree && !gate && few && hidden <= 8192)
