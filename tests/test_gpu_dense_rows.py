@@ -82,9 +82,9 @@ def test_tiled_rows_keep_the_reference_order_bits(dev, rows, k, n, dtype, out_in
 
 
 # the tiled kernel's range: f32 from 2^14 outputs ([out, in]) and 2^18 ([in, out]) or from 2^22 and 2^23 weights, 16 bits [out, in] from 5 x 2^15
-# outputs, one and four rows a warp, with and without a bias, tails in rows, outputs and k
+# outputs and [in, out] from 2^21, one and four rows a warp, with and without a bias, tails in rows, outputs and k
 @pytest.mark.parametrize("rows,k,n,dtype,out_in,bias", [(5, 33, 3300, F32, True, False), (4, 35, 4100, F32, True, False), (4, 5, 65600, F32, False, True),
-                                                        (43, 100, 3900, BF16, True, False), (66, 9, 4100, F32, False, True), (42, 33, 3910, F16, True, False),
+                                                        (43, 100, 3900, BF16, True, False), (66, 9, 4100, F32, False, True), (42, 33, 3910, F16, True, False), (513, 5, 4100, F16, False, False),
                                                         (1, 2055, 2049, F32, True, False), (3, 4099, 2050, F32, False, True),
                                                         (70, 37, 3800, F32, False, False)])
 def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
@@ -99,7 +99,7 @@ def test_tiled_rows_where_they_are_chosen(dev, rows, k, n, dtype, out_in, bias):
     assert np.array_equal(got.view(np.uint8), np.ascontiguousarray(want).reshape(-1).view(np.uint8))
 
 
-@pytest.mark.parametrize("m,k", [(2, 512), (513, 512), (513, 520), (4097, 896), (4097, 904), (1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
+@pytest.mark.parametrize("m,k", [(2, 512), (1184, 512), (1185, 512), (1185, 520), (4097, 896), (4097, 904), (1, 16), (3, 2048), (5, 2064), (2, 8192), (3, 16384), (2, 16400)])
 def test_wide_quantiser_equals_the_rule(m, k):
     import torch
     rng = np.random.default_rng(k)

@@ -275,9 +275,9 @@ cudaError_t launch_quantize_per_token_int8(const void* x_bf16, int8_t* q, float*
                                            cudaStream_t stream) {
     // rows of whole 16-byte chunks that fit 256 threads' registers; other rows and unaligned buffers keep the element kernel, and so do many
     // short rows, which leave most of a block idle (element / this one, us: 4096 x 512 6.3 / 8.3, 4096 x 768 9.7 / 8.3, 16384 x 640 16.5 / 20.6,
-    // 16384 x 1024 24.7 / 22.7; 256 x 512 4.2 / 4.2 from L2 and 8.2 / 6.2 from HBM)
+    // 16384 x 1024 24.7 / 22.7; 513 x 512 4.4 / 4.4 from L2 and 8.2 / 7.5 from HBM: up to eight blocks an SM)
     const bool aligned = ((reinterpret_cast<uintptr_t>(x_bf16) & 15u) | (reinterpret_cast<uintptr_t>(q) & 7u)) == 0;
-    if (aligned && k % 8 == 0 && k > (m <= 512 ? 0u : m <= 4096 ? 512u : 896u) && k <= 16384) {
+    if (aligned && k % 8 == 0 && k > (m <= 1184 ? 0u : m <= 4096 ? 512u : 896u) && k <= 16384) {
         const uint4* x = static_cast<const uint4*>(x_bf16);
         uint2* out = reinterpret_cast<uint2*>(q);
         const uint32_t chunks = k / 8;

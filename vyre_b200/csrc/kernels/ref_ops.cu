@@ -626,11 +626,12 @@ cudaError_t launch_linear_rows(const void* x, const void* w, const void* bias, v
     // takes 54 to 66 ns a step from either, 145 to 230 with 16-bit operands. So f32 weights too large to be in L2 from one call to the next, or many
     // outputs. Plain / tiled, us: f32 [out, in] 1 x 8188 x 4096 from HBM 724 / 488, 16 x 2048 x 2048 285 / 140, 64 x 4096 x 4096 3870 / 316; from
     // L2 5 x 3000 x 1000 125 / 199; f32 [in, out] 1 x 4092 x 8192 from HBM 351 / 245, from L2 4 x 2048 x 2048 67 / 114; 16 bits [out, in] (odd
-    // k) 16 x 4092 x 4096 from HBM 422 / 948, 64 x 4092 x 4096 1492 / 904; 16 bits [in, out] never (64 x 4096 x 4096 from L2 418 / 638).
+    // k) 16 x 4092 x 4096 from HBM 422 / 948, 64 x 4092 x 4096 1492 / 904; 16 bits [in, out]
+    // from HBM 256 x 4092 x 4096 1527 / 1785, 512 x 4092 x 4096 2951 / 2501.
     const uint64_t outputs = uint64_t(rows) * out_dim, weights = uint64_t(in_dim) * out_dim;
     const int rt = rows <= 4 ? 1 : 4;
     const bool tiled = dtype == 0 ? weights >= (out_in ? 1ull << 22 : 1ull << 23) || outputs >= (out_in ? 1ull << 14 : 1ull << 18)
-                                  : out_in && outputs >= (5ull << 15);
+                                  : outputs >= (out_in ? 5ull << 15 : 1ull << 21);
     if (tiled && outputs * in_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
         const dim3 grid((out_dim + 63) / 64, (rows + 4 * rt - 1) / (4 * rt));
         if (rt == 1) linear_rows_tiled_kernel<1><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
