@@ -28,3 +28,6 @@ def test_copies_and_mmas_are_settled(f):
     assert rings == barriers - {"acc_full", "b_full", "d_full"} - ({"a_full"} if "skinny" in f else set())
     assert re.search(r"if \(\*abort_flag != 0[^\n]*\)\s*(\{\s*tc_commit_pair\(smem_u32\(&bars->drained\)\)|settle_mma\(smem_u32\(&bars->drained\)\))", s)
     assert "mbar_init(smem_u32(&bars->drained), 1)" in s
+    # when all roles have met, and with the counts that the TMA role left
+    assert s.index("settle_copies(") > s.rindex("issued = ") and s.index("settle_copies(") > s.index("tmem_ld_wait()")
+    assert len(re.findall(r"settle_copies\(bars->\w+, [\w.:]+, bars->\w*issued\);", s)) == len(rings)

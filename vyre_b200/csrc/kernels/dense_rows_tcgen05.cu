@@ -45,6 +45,7 @@ struct Bars {
     unsigned long long full[MAX_STAGES], empty[MAX_STAGES], acc_full, drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t issued;  // copies of the TMA role
 };
 
 struct Params {
@@ -104,7 +105,7 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                 tma_load_2d(dst, &map_w, int((kb0 + i) * BK), int(n0), bar);
                 tma_load_2d(dst + A_BYTES, &map_x, int((kb0 + i) * BK), int(r0), bar);
             }
-            settle_copies(bars->full, p.stages, i);
+            bars->issued = i;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -182,7 +183,10 @@ dense_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         tc_fence_after();
         tmem_dealloc(tmem, p.tmem_cols);
     }
-    if (threadIdx.x == 0 && bars->abort_flag != 0 && p.status) atomicOr(p.status, 32u);
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->full, p.stages, bars->issued);
+        if (p.status) atomicOr(p.status, 32u);
+    }
 }
 
 }  // namespace

@@ -80,6 +80,7 @@ struct Bars {
     unsigned long long acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t a_issued, raw_issued;  // copies of the TMA role
 };
 
 struct Params {
@@ -216,9 +217,8 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     }
                 }
             }
-            settle_copies(bars->raw_full, RAW_STAGES, r_it);
-            // the leader's barriers count both CTAs' activation boxes, and the pair leaves together (cluster_sync below)
-            if (rank == 0) settle_copies(bars->a_full, A_STAGES, a_it);
+            bars->raw_issued = r_it;
+            bars->a_issued = a_it;
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
@@ -411,6 +411,11 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->raw_full, RAW_STAGES, bars->raw_issued);
+        if (rank == 0) settle_copies(bars->a_full, A_STAGES, bars->a_issued);  // the leader's count both CTAs' boxes; the pair leaves together
+    }
+    __syncwarp();
     cluster_sync();  // the peer may still be reading this CTA's shared memory / TMEM through the pair MMA until here
     if (warp == MMA_WARP) {
         tc_fence_after();

@@ -56,6 +56,7 @@ struct Bars {
     unsigned long long b_full[B_STAGES], b_empty[B_STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t a_issued, raw_issued;  // copies of the TMA role
 };
 
 __device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
@@ -156,8 +157,8 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             }
         }
         if (lane == 0) {
-            settle_copies(bars->raw_full, RAW_STAGES, r_it);
-            settle_copies(bars->a_full, A_STAGES, a_it);
+            bars->raw_issued = r_it;
+            bars->a_issued = a_it;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -322,7 +323,11 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
-    if (threadIdx.x == 0 && bars->abort_flag != 0 && status) atomicOr(status, 8u);
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->raw_full, RAW_STAGES, bars->raw_issued);
+        settle_copies(bars->a_full, A_STAGES, bars->a_issued);
+        if (status) atomicOr(status, 8u);
+    }
 }
 
 }  // namespace

@@ -73,6 +73,7 @@ struct Bars {
     unsigned long long full[8], empty[8], a_full[4], a_empty[4], d_full[2], d_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t issued;  // copies of the TMA role
 };
 static_assert(sizeof(Bars) <= CTRL_BYTES, "control block");
 
@@ -156,7 +157,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 load_raw(i);
                 load_x(i);
             }
-            settle_copies(bars->full, C::STAGES, i);
+            bars->issued = i;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -312,7 +313,10 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
     }
-    if (threadIdx.x == 0 && bars->abort_flag != 0 && p.status) atomicOr(p.status, 64u);
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->full, C::STAGES, bars->issued);
+        if (p.status) atomicOr(p.status, 64u);
+    }
 }
 
 template <int BN>

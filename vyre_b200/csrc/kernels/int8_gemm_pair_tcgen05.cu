@@ -38,6 +38,7 @@ struct Bars {
     unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t issued;  // copies of the TMA role
 };
 
 __device__ __forceinline__ bool is_epilogue_warp(int w) { return w == 8 || (w >= 1 && w <= 3); }
@@ -107,8 +108,7 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     }
                 }
             }
-            // the leader's barriers count both CTAs' boxes, and the pair leaves together (cluster_sync below)
-            if (rank == 0) settle_copies(bars->full, STAGES, issued);
+            bars->issued = issued;
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
@@ -218,6 +218,9 @@ int8_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
     tc_fence_before();
     __syncthreads();
+    // the leader's barriers count both CTAs' boxes, and the pair leaves together
+    if (threadIdx.x == 0 && rank == 0 && bars->abort_flag != 0) settle_copies(bars->full, STAGES, bars->issued);
+    __syncwarp();
     cluster_sync();  // the peer may still be reading this CTA's shared memory / TMEM through the pair MMA until here
     if (warp == MMA_WARP) {
         tc_fence_after();

@@ -63,6 +63,7 @@ struct Bars {
     unsigned long long full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t issued;  // copies of the TMA role
 };
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -122,7 +123,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 __syncwarp();
             }
         }
-        if (lane == 0) settle_copies(bars->full, STAGES, it);
+        if (lane == 0) bars->issued = it;
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------ MMA issuer ---------------------------------------
@@ -204,7 +205,10 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
-    if (threadIdx.x == 0 && bars->abort_flag != 0 && status) atomicOr(status, 4u);
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->full, STAGES, bars->issued);
+        if (status) atomicOr(status, 4u);
+    }
 }
 
 // Per-token symmetric int8 quantisation: s_t = max|x| / 127, q = clamp(rint(x / s_t), -127, 127); one warp per row.

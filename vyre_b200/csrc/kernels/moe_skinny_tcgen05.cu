@@ -46,6 +46,7 @@ struct Bars {
     unsigned long long full[4], empty[4], a_full[4], a_empty[4], d_full[2], d_empty[2], drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
+    uint32_t issued;  // copies of the TMA role
     uint32_t seg_row[MAX_EXPERTS], seg_count[MAX_EXPERTS];
 };
 
@@ -178,7 +179,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     }
                 }
             }
-            settle_copies(bars->full, C::STAGES, issued);
+            bars->issued = issued;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -323,7 +324,10 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);
     }
-    if (threadIdx.x == 0 && bars->abort_flag != 0 && p.status) atomicOr(p.status, 512u);
+    if (threadIdx.x == 0 && bars->abort_flag != 0) {
+        settle_copies(bars->full, C::STAGES, bars->issued);
+        if (p.status) atomicOr(p.status, 512u);
+    }
 }
 
 template <int BN, bool GLU>
