@@ -153,3 +153,40 @@ def test_prepared_outputs_direct_or_copied_equal_ordinary_submissions(dev, m, n,
     prep.free()
     dev.free_resident(hw)
     dev.free_resident(hs)
+
+
+def test_queued_submissions_have_times_and_outputs_of_their_own(dev):
+    """Submissions queued behind a pending one take their times beside the stream; waits may come in any order, a completion keeps its
+    times while later submissions run, and outputs that are copied out, or a replay in between, start the times anew."""
+    m, n, k = 1, 512, 4096
+    x, w, s = synth.int4_linear_inputs(m, n, k, seed=14)
+    sess = gemv_session(dev, m, n, k)
+    host = sess.host_bindings([x, w.view(np.uint32), s])
+    want = sess.submit(host).wait().output(3)
+    handles = [dev.resident_from(v) for v in (x, w.view(np.uint32), s)]
+    outs = [dev.allocate_resident(2 * m * n) for _ in range(6)]
+    chain = []
+    for h in outs:
+        bs = vb.BindingSet(sess.artifact.digest())
+        for slot, v in enumerate(handles + [h]):
+            bs.insert_resident(slot, v)
+        chain.append(bs)
+    kept = []
+    for order in ([0, 1, 2, 3, 4, 5], [5, 3, 4, 0, 2, 1]):
+        subs = [sess.submit(bs, leave_resident=True) for bs in chain]
+        done = [subs[i].wait() for i in order]
+        kept += done
+        assert all(0 < c.device_ns < 5_000_000 for c in done)
+    first = [c.device_ns for c in kept]
+    a, b, c = sess.submit(chain[0], leave_resident=True), sess.submit(host), sess.submit(chain[1], leave_resident=True)
+    prep = sess.prepare(chain[2])
+    d, e = prep.submit(), sess.submit(chain[3], leave_resident=True)
+    done = [v.wait() for v in (e, d, c, b, a)]
+    assert done[3].output(3) == want and all(v.device_ns > 0 for v in done[:1] + done[2:]) and done[1].device_ns is None
+    assert [c.device_ns for c in kept] == first  # read again: their events were not recycled under them
+    for h in outs:
+        assert dev.download_resident(h, 2 * m * n).tobytes() == want
+    del kept, done
+    prep.free()
+    for h in handles + outs:
+        dev.free_resident(h)
