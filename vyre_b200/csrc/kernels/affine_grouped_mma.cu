@@ -25,6 +25,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -92,6 +93,8 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
     constexpr uint32_t PITCH = SUMS + 1;
     constexpr int AHEAD = NB == 2 ? 2 : 4;                    // steps of weights in flight (registers: sixteen rows leave room for two)
     extern __shared__ __align__(16) uint8_t smem[];
+    lets_next_start();
+    waits_for_previous();
     uint4* xs = reinterpret_cast<uint4*>(smem);               // [chunk / 8][COLS]: (k0,k4) (k1,k5) (k2,k6) (k3,k7) of a column
     float* xsum = reinterpret_cast<float*>(smem + XS_BYTES);  // [groups of the chunk][SUMS]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -345,8 +348,8 @@ cudaError_t launch_cfg(const float* x, const uint32_t* w, const float* scale, co
     if (rows > 65535u) return cudaErrorInvalidValue;
     // two blocks per SM walk the tiles, so that activations are staged once
     const uint32_t fit = (2u * uint32_t(sm_count) + rows - 1) / rows, grid = tiles < fit ? tiles : fit;
-    affine_grouped_mma_kernel<R, NB, WK><<<dim3(grid, rows), THREADS, smem, s>>>(x, w, scale, zp, b, out, in_dim, out_dim, group, batch, chunk);
-    return cudaGetLastError();
+    return launch_dependent(affine_grouped_mma_kernel<R, NB, WK>, dim3(grid, rows), dim3(THREADS), smem, s, x, w, scale, zp, b, out, in_dim, out_dim,
+                            group, batch, chunk);
 }
 
 }  // namespace

@@ -24,6 +24,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -45,6 +46,7 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
                                                                       const float* __restrict__ bias, float* __restrict__ out,
                                                                       uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                                                       int group_shift, uint32_t batch) {
+    dependent_start();
     constexpr int WPT = (KCHUNK / 8) / KS;
     constexpr int XS = BT * KCHUNK, RED = KS * BT * OT * TX;
     __shared__ __align__(16) float smem[XS > RED ? XS : RED];
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const fl
                                                                         const float* __restrict__ scale, const uint32_t* __restrict__ zp,
                                                                         const float* __restrict__ bias, float* __restrict__ out,
                                                                         uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t batch) {
+    dependent_start();
     extern __shared__ __align__(16) float dsm[];
     const uint32_t groups = in_dim / group, wpg = group / 8;  // words per group; WPT = wpg / KS of them are this thread's
     constexpr uint32_t wpt = WPT;
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const fl
 __global__ void __launch_bounds__(256) i4_matvec_fast_kernel(const uint32_t* __restrict__ w, const float* __restrict__ x,
                                                              const float* __restrict__ scales, float* __restrict__ out,
                                                              uint32_t batch, uint32_t rows, uint32_t cols) {
+    dependent_start();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t b0 = blockIdx.y * MV_BT;
     const uint32_t nb = min(uint32_t(MV_BT), batch - b0);
@@ -331,8 +335,8 @@ cudaError_t launch_affine_cfg(const float* x, const uint32_t* w, const float* sc
     const int shift = (group & (group - 1)) == 0 ? __builtin_ctz(group) : -1;
     const dim3 grid((out_dim + TX * OT - 1) / (TX * OT), (batch + BT - 1) / BT);
     if (grid.y > 65535u) return cudaErrorInvalidValue;
-    affine_grouped_fast_kernel<TX, OT, KS, BT, KCHUNK><<<grid, dim3(TX, KS), 0, s>>>(x, w, scale, zp, b, out, in_dim, out_dim, group, shift, batch);
-    return cudaGetLastError();
+    return launch_dependent(affine_grouped_fast_kernel<TX, OT, KS, BT, KCHUNK>, grid, dim3(TX, KS), 0, s, x, w, scale, zp, b, out, in_dim, out_dim, group,
+                            shift, batch);
 }
 }  // namespace
 
@@ -367,9 +371,8 @@ cudaError_t launch_affine_grouped_fast(const float* x, const uint32_t* w, const 
             if (e != cudaSuccess) return e;
             configured.fetch_or(bit, std::memory_order_release);
         }
-        kernels[group == 128 ? 1 : 0][dbt == 1 ? 0 : dbt == 2 ? 1 : 2]<<<grid, block, smem, s>>>(x, w, scale, zp, b, out, in_dim, out_dim,
-                                                                                             group, batch);
-        return cudaGetLastError();
+        return launch_dependent(kernels[group == 128 ? 1 : 0][dbt == 1 ? 0 : dbt == 2 ? 1 : 2], grid, block, smem, s, x, w, scale, zp, b, out, in_dim,
+                                out_dim, group, batch);
     }
     // batch rows per block: every row beyond the batch is wasted arithmetic, every row within it reuses the dequantised weight
     const int bt = batch >= 12 ? 16 : batch >= 3 ? 8 : 2;
@@ -385,8 +388,7 @@ cudaError_t launch_affine_grouped_fast(const float* x, const uint32_t* w, const 
 
 cudaError_t launch_i4_matvec_fast(const uint32_t* w, const float* x, const float* scales, float* out, uint32_t batch,
                                   uint32_t rows, uint32_t cols, cudaStream_t s) {
-    i4_matvec_fast_kernel<<<dim3((rows + 7) / 8, (batch + MV_BT - 1) / MV_BT), 256, 0, s>>>(w, x, scales, out, batch, rows, cols);
-    return cudaGetLastError();
+    return launch_dependent(i4_matvec_fast_kernel, dim3((rows + 7) / 8, (batch + MV_BT - 1) / MV_BT), dim3(256), 0, s, w, x, scales, out, batch, rows, cols);
 }
 
 
@@ -414,6 +416,8 @@ __global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_f
     constexpr int OPS = OPT / SPT;                        // outputs per scale
     constexpr int ROWS = OPT == 8 ? 8 : OPT == 16 ? 6 : 3;              // word rows fetched together, one set ahead of the one that is summed
     constexpr uint32_t FIELD = (1u << BITS) - 1u, SPREAD = FIELD * 0x01010101u;
+    lets_next_start();
+    waits_for_previous();
     extern __shared__ float red[];                        // [KQ_WARPS][32][OPT + 1], then [32 * OPT] sums of this block
     constexpr uint32_t PITCH = 32 * (OPT + 1);
     float* sums = red + KQ_WARPS * PITCH;
@@ -551,10 +555,11 @@ cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const flo
     cfg.blockDim = dim3(32 * KQ_WARPS);
     cfg.dynamicSmemBytes = SMEM;
     cfg.stream = s;
-    cudaLaunchAttribute attr = {};
+    cudaLaunchAttribute attrs[2] = {}, &attr = attrs[0];
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
+    dependent(attrs[1]);
+    cfg.attrs = attrs;
     cfg.numAttrs = 1;
     const uint32_t blocks = (out_dim / OPT + 31) / 32;
     if (split == 0) {  // the largest cluster of which all column blocks' are resident at once
@@ -574,6 +579,7 @@ cudaError_t launch_k_quant_cfg(const float* x, const uint32_t* packed, const flo
     }
     attr.val.clusterDim.x = split;
     cfg.gridDim = dim3(blocks * split);
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k_quant_linear_fast_kernel<BITS, W, KQ_WARPS>, x, packed, scales, mins, b, out, in_dim, out_dim, split);
 }
 }  // namespace

@@ -7,6 +7,7 @@
 // vyre-primitives/src/math/quantized/programs.rs:186-300.
 #include <cuda_bf16.h>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -18,6 +19,7 @@ __global__ void __launch_bounds__(256) int4_linear_generic_kernel(const uint16_t
                                                                  const uint16_t* __restrict__ scales, void* y,
                                                                  uint32_t m, uint32_t n, uint32_t k, uint32_t group,
                                                                  uint32_t out_f32) {
+    dependent_start();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
     if (row >= n) return;
@@ -106,10 +108,8 @@ cudaError_t launch_int4_gemv(const void* x_bf16, const void* w_packed, const voi
 cudaError_t launch_int4_linear_generic(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y,
                                        uint32_t m, uint32_t n, uint32_t k, uint32_t group, uint32_t out_f32,
                                        cudaStream_t stream) {
-    int4_linear_generic_kernel<<<(n + 7) / 8, 256, 0, stream>>>(
-        static_cast<const uint16_t*>(x_bf16), static_cast<const uint32_t*>(w_packed),
-        static_cast<const uint16_t*>(scale_bf16), y, m, n, k, group, out_f32);
-    return cudaGetLastError();
+    return launch_dependent(int4_linear_generic_kernel, dim3((n + 7) / 8), dim3(256), 0, stream, static_cast<const uint16_t*>(x_bf16),
+                            static_cast<const uint32_t*>(w_packed), static_cast<const uint16_t*>(scale_bf16), y, m, n, k, group, out_f32);
 }
 
 }  // namespace vybk

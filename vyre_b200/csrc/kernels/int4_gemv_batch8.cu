@@ -34,6 +34,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_batch8_kernel(const __gri
     extern __shared__ __align__(128) uint8_t smem[];
     // let the next launch of the stream become resident beside this one at once; it waits (griddepcontrol.wait)
     // before it reads activations or writes outputs. A no-op for plain launches.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    lets_next_start();
     constexpr uint32_t K = 128u * GPW * W;
     constexpr uint32_t ROW_BYTES = K / 2;            // packed bytes of one row of W
     constexpr uint32_t PITCH = GPW * 64;             // of which this warp owns (= row pitch of its stages)
@@ -161,8 +162,16 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_batch8_kernel(const __gri
         }
         cp_async_commit();
     };
-    // Weights are constants: prefetched before the dependency wait, paced so that the predecessor's activation loads on
+    // Weights that are constants are prefetched before the dependency wait, paced so that the predecessor's activation loads on
     // the same SM do not queue behind a 96 KB burst.
+    // Without that promise (no pause either) they come after it, and the first tiles are brought into L2 meanwhile.
+    if (p.pace_ns == 0) {
+        for (uint32_t u = 0; u < STAGES; ++u)
+#pragma unroll
+            for (uint32_t i = 0; i < NCP; ++i)
+                if (cp_chunk % 8 == 0 && u * TILE_ROWS + i * RPI + cp_row < nrows) prefetch_l2(cp_src + (u * TILE_ROWS + i * RPI) * size_t(ROW_BYTES));
+        waits_for_previous();
+    }
 #pragma unroll
     for (int u = 0; u < STAGES; ++u) {
         if (u > 0 && p.pace_ns) __nanosleep(p.pace_ns);
@@ -173,7 +182,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_batch8_kernel(const __gri
     const uint32_t t = lane & 3;
 
     // ---- activations: everything below reads x, so the previous launch of the stream must be complete ----
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waits_for_previous();
     // This lane's B fragments: batch row g, k = 128 c + 32 t + 8 u + (0..7) of the warp's slice, i.e. the elements under
     // the lane's 16-byte weight chunk 4c + t. Word u of that chunk feeds two MMAs: nibbles (0,4) and (1,5), then (2,6)
     // and (3,7); the activations are paired the same way.
@@ -362,10 +371,9 @@ cudaError_t launch_int4_gemv_batch8(const void* x_bf16, const void* w_packed, co
     cfg.dynamicSmemBytes = SMEM_TOTAL;
     cfg.stream = stream;
     cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights ? 1 : 0;
+    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernels[k == 4096 ? 0 : 1][out_f32 ? 1 : 0], p);
 }
 

@@ -41,6 +41,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -144,6 +145,7 @@ struct Params {
     void* y;
     uint32_t m, n, k, groups;  // groups = k / 128
     uint32_t* status;
+    uint32_t constant;  // weights and scales may be read before the launches before this one are complete
 };
 
 template <int LIMBS, bool OUT_F32>
@@ -158,7 +160,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_gemv_kernel(const Params p) {
     const int lane = threadIdx.x & 31;
     // Programmatic dependent launch: let the next kernel in the stream begin its own launch and weight prefetch
     // now; it still waits (griddepcontrol.wait) before touching activations or outputs. No-ops for plain launches.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    lets_next_start();
     const uint32_t rows_base = p.n / gridDim.x, rows_rem = p.n % gridDim.x;
     const uint32_t r0 = blockIdx.x * rows_base + min(blockIdx.x, rows_rem);
     const uint32_t r1 = r0 + rows_base + (blockIdx.x < rows_rem ? 1u : 0u);
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_gemv_kernel(const Params p) {
     uint4 xv[8];
     // activations may come from the preceding kernel: everything that reads x or writes y runs after this point,
     // only the (constant) weight stream of the producer warp starts before it
-    if (warp != WARPS) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp != WARPS || !p.constant) waits_for_previous();
     if (coop) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -529,6 +531,7 @@ cudaError_t launch_int4_gemv_bulk(const void* x_bf16, const void* w_packed, cons
     p.k = k;
     p.groups = k / 128;
     p.status = status;
+    p.constant = constant_weights;
     const uint32_t tiles = (n + TILE_ROWS - 1) / TILE_ROWS;
     const uint32_t grid = tiles < uint32_t(sm_count) ? tiles : uint32_t(sm_count);
     cudaLaunchConfig_t cfg = {};
@@ -537,11 +540,9 @@ cudaError_t launch_int4_gemv_bulk(const void* x_bf16, const void* w_packed, cons
     cfg.dynamicSmemBytes = SMEM_TOTAL;
     cfg.stream = stream;
     cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    // with constant weights the launch may overlap the tail of the preceding kernel of the stream
+    dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights ? 1 : 0;
+    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
     if (out_f32) return cudaLaunchKernelEx(&cfg, int4_gemv_kernel<4, true>, p);
     return cudaLaunchKernelEx(&cfg, int4_gemv_kernel<3, false>, p);
 }

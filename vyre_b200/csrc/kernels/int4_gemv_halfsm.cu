@@ -57,6 +57,7 @@
 #include <mutex>
 #include <utility>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "peer_gather.cuh"
 
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_halfsm_kernel(const __gri
     extern __shared__ __align__(128) uint8_t smem[];
     // let the next launch of the stream become resident beside this one at once; it waits (griddepcontrol.wait)
     // before it reads activations or writes outputs. A no-op for plain launches.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    lets_next_start();
     constexpr uint32_t K = 128u * GPW * W;
     constexpr uint32_t ROW_BYTES_DENSE = K / 2;      // packed bytes of one row of W when the launch covers whole rows
     constexpr uint32_t PITCH = GPW * 64;             // of which this warp owns (= row pitch of its stages)
@@ -329,10 +330,18 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_halfsm_kernel(const __gri
         }
         cp_async_commit();
     };
-    // Weights are constants: prefetched before the dependency wait. Under programmatic dependent launch this CTA arrives
+    // Weights that are constants are prefetched before the dependency wait. Under programmatic dependent launch this CTA arrives
     // on its SM just when its predecessor is about to be released and load its activations through the same load/store
     // queue, so the prefetch is paced (about PACE_NS between tiles) rather than issued as one 96 KB burst that the
     // predecessor's few activation loads would have to queue behind. This CTA has microseconds to spare here.
+    // Without that promise (no pause either) they come after it, and the first tiles are brought into L2 meanwhile.
+    if (p.pace_ns == 0) {
+        for (uint32_t u = 0; u < ST; ++u)
+#pragma unroll
+            for (uint32_t i = 0; i < NCP; ++i)
+                if (cp_chunk % 8 == 0 && u * TILE_ROWS + i * RPI + cp_row < nrows) prefetch_l2(cp_src + (u * TILE_ROWS + i * RPI) * size_t(ROW_BYTES));
+        waits_for_previous();
+    }
 #pragma unroll
     for (int u = 0; u < ST; ++u) {
         if (u > 0 && p.pace_ns) __nanosleep(DEEP ? p.pace_ns / 2 : p.pace_ns);  // the same bytes per pause
@@ -343,7 +352,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_halfsm_kernel(const __gri
     const uint32_t t = lane & 3;
 
     // ---- activations: everything below reads x, so the previous launch of the stream must be complete ----
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    waits_for_previous();
     uint32_t launch_index = 0;  // GATHER: how many gathering launches this rank has completed before this one
     if constexpr (GATHER) {
         launch_index = *(reinterpret_cast<const volatile uint32_t*>(p.ag.epoch) + EPOCH_INDEX + p.half);
@@ -923,10 +932,9 @@ cudaError_t launch_int4_gemv_halfsm(const void* x_bf16, const void* w_packed, co
     cfg.dynamicSmemBytes = SMEM_TOTAL;
     cfg.stream = stream;
     cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights ? 1 : 0;
+    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, block ? fused[k == 4096 ? 0 : 1] : kernels[variant][gather ? 2 : out_f32 ? 1 : 0], p);
 }
 
@@ -1042,10 +1050,9 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
                 cfg.dynamicSmemBytes = SMEM_TOTAL;
                 cfg.stream = stream;
                 cudaLaunchAttribute attr = {};
-                attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr.val.programmaticStreamSerializationAllowed = 1;
+                dependent(attr);
                 cfg.attrs = &attr;
-                cfg.numAttrs = constant_weights ? 1 : 0;
+                cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
                 return cudaLaunchKernelEx(&cfg, kernels[m <= 2 ? 0 : 1][blk == 4096 ? 0 : 1][out_f32 ? 1 : 0], p);
             }
         }
@@ -1080,10 +1087,9 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
         cfg.dynamicSmemBytes = SMEM_TOTAL;
         cfg.stream = stream;
         cudaLaunchAttribute attr = {};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
+        dependent(attr);
         cfg.attrs = &attr;
-        cfg.numAttrs = constant_weights ? 1 : 0;
+        cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
         e = cudaLaunchKernelEx(&cfg, kernels[m <= 2 ? 0 : 1][blk == 4096 ? 0 : 1][(last ? out_f32 != 0 : true) ? 1 : 0], p);
         kb += blk;
     }

@@ -36,6 +36,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -83,6 +84,7 @@ struct Params {
     uint32_t* status;
     uint32_t m, n, k, split;
     uint32_t tile0;          // first weight tile of this launch
+    uint32_t constant;       // weights and scales may be read before the launches before this one are complete
 };
 
 template <int BN, bool OUT_F32>
@@ -130,7 +132,8 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     // only now, with this CTA's tensor memory in hand, may the next launch's CTA take the rest of it
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    lets_next_start();
+    if (!p.constant && warp != 0) waits_for_previous();
 
     bool ok = true;
     if (warp == 0) {
@@ -148,8 +151,12 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         };
         const uint32_t ahead = min(kbs, uint32_t(C::STAGES));
         if (elect_one()) {
+            if (!p.constant) {
+                for (uint32_t i = 0; i < ahead; ++i) tma_prefetch_2d(&map_w, int((kb0 + i) * (KB / 2)), int(n0));
+                waits_for_previous();
+            }
             for (uint32_t i = 0; i < ahead; ++i) load_raw(i);
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            waits_for_previous();
             for (uint32_t i = 0; i < ahead; ++i) load_x(i);
             uint32_t i = ahead;
             for (; i < kbs; ++i) {
@@ -347,6 +354,7 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t o
     if (p.split > blocks / 2) p.split = blocks / 2;
     if (p.split > uint32_t(MAX_SPLIT)) p.split = MAX_SPLIT;
     if (p.split < 1) p.split = 1;
+    const bool all_sms = whole_device(dev, sm_count);
     CUtensorMap mw, mx;
     if (!encode_tensor_map_2d(&mw, w, p.n, p.k / 2, 1, BM, KB / 2, true) || !encode_tensor_map_2d(&mx, x, p.m, p.k, 2, BN, 64, true))
         return cudaErrorInvalidValue;
@@ -358,16 +366,13 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t o
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = p.split;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    dependent(attr[1]);
     cfg.attrs = attr;
-    cfg.numAttrs = constant_weights ? 2 : 1;
+    cfg.numAttrs = constant_weights || all_sms ? 2 : 1;
+    p.constant = constant_weights;
     // A caller that wants an SM left free (sm_count below the device's, VYB_LAUNCH_LEAVE_ONE_SM) gets launches that fit the other SMs at once:
     // a second wave of one launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
-    int sms = 0;
-    if (tiles > slots) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    const uint32_t step = sm_count < sms ? slots : tiles;
+    const uint32_t step = all_sms ? tiles : slots;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split);
         e = cudaLaunchKernelEx(&cfg, kernels[out_f32 ? 1 : 0], mw, mx, p);

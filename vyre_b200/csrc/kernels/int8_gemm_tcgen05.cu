@@ -16,6 +16,7 @@
 // word, the CTA drains, frees its TMEM and returns.
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -214,6 +215,7 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // Per-token symmetric int8 quantisation: s_t = max|x| / 127, q = clamp(rint(x / s_t), -127, 127); one warp per row.
 __global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t* __restrict__ x, int8_t* __restrict__ q,
                                                                 float* __restrict__ scales, uint32_t M, uint32_t K) {
+    dependent_start();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= M) return;
     const uint16_t* xr = x + size_t(row) * K;
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t*
 template <int V>
 __global__ void __launch_bounds__(256) quantize_per_token_wide_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
                                                                      float* __restrict__ scales, uint32_t chunks) {
+    dependent_start();
     __shared__ float warp_max[8];
     const size_t row = blockIdx.x;
     const uint4* xr = x + row * chunks;
@@ -285,14 +288,12 @@ cudaError_t launch_quantize_per_token_int8(const void* x_bf16, int8_t* q, float*
         const uint4* x = static_cast<const uint4*>(x_bf16);
         uint2* out = reinterpret_cast<uint2*>(q);
         const uint32_t chunks = k / 8;
-        if (chunks <= 256) quantize_per_token_wide_kernel<1><<<m, 256, 0, stream>>>(x, out, scales, chunks);
-        else if (chunks <= 512) quantize_per_token_wide_kernel<2><<<m, 256, 0, stream>>>(x, out, scales, chunks);
-        else if (chunks <= 1024) quantize_per_token_wide_kernel<4><<<m, 256, 0, stream>>>(x, out, scales, chunks);
-        else quantize_per_token_wide_kernel<8><<<m, 256, 0, stream>>>(x, out, scales, chunks);
-        return cudaGetLastError();
+        if (chunks <= 256) return launch_dependent(quantize_per_token_wide_kernel<1>, dim3(m), dim3(256), 0, stream, x, out, scales, chunks);
+        if (chunks <= 512) return launch_dependent(quantize_per_token_wide_kernel<2>, dim3(m), dim3(256), 0, stream, x, out, scales, chunks);
+        if (chunks <= 1024) return launch_dependent(quantize_per_token_wide_kernel<4>, dim3(m), dim3(256), 0, stream, x, out, scales, chunks);
+        return launch_dependent(quantize_per_token_wide_kernel<8>, dim3(m), dim3(256), 0, stream, x, out, scales, chunks);
     }
-    quantize_per_token_kernel<<<(m + 7) / 8, 256, 0, stream>>>(static_cast<const uint16_t*>(x_bf16), q, scales, m, k);
-    return cudaGetLastError();
+    return launch_dependent(quantize_per_token_kernel, dim3((m + 7) / 8), dim3(256), 0, stream, static_cast<const uint16_t*>(x_bf16), q, scales, m, k);
 }
 
 bool int8_gemm_supported(uint32_t m, uint32_t n, uint32_t k) {

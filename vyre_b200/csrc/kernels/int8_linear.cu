@@ -10,6 +10,7 @@
 // (linear_rows_no_bias_out_in, f32 accumulate).
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* __re
                                                               const int8_t* __restrict__ w,
                                                               const float* __restrict__ scale, float* __restrict__ y,
                                                               uint32_t m, uint32_t n, uint32_t k) {
+    dependent_start();
     const uint32_t col = blockIdx.x * 8 + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
     if (col >= n) return;
@@ -84,6 +86,7 @@ constexpr int WPB = 4;     // warps per block
 __global__ void __launch_bounds__(WPB * 32, 3) int8_weight_only_tiled_kernel(const float* __restrict__ x, const int8_t* __restrict__ w,
                                                                           const float* __restrict__ scale, float* __restrict__ y,
                                                                           uint32_t m, uint32_t n, uint32_t k) {
+    dependent_start();
     extern __shared__ __align__(16) float xs[];  // [MB][KC]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t col0 = (blockIdx.x * WPB + warp) * CPW;
@@ -173,11 +176,9 @@ cudaError_t launch_int8_weight_only_linear(const float* x, const int8_t* w, cons
             configured.fetch_or(bit, std::memory_order_release);
         }
         const uint32_t per_block = WPB * CPW;
-        int8_weight_only_tiled_kernel<<<(n + per_block - 1) / per_block, WPB * 32, SMEM, stream>>>(x, w, scale, y, m, n, k);
-        return cudaGetLastError();
+        return launch_dependent(int8_weight_only_tiled_kernel, dim3((n + per_block - 1) / per_block), dim3(WPB * 32), SMEM, stream, x, w, scale, y, m, n, k);
     }
-    int8_weight_only_kernel<<<(n + 7) / 8, 256, 0, stream>>>(x, w, scale, y, m, n, k);
-    return cudaGetLastError();
+    return launch_dependent(int8_weight_only_kernel, dim3((n + 7) / 8), dim3(256), 0, stream, x, w, scale, y, m, n, k);
 }
 
 }  // namespace vybk

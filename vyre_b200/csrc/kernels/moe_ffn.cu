@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <float.h>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -37,6 +38,7 @@ template <bool WR_IN_SMEM>
 __global__ void __launch_bounds__(256, 2)
 moe_router_gate_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w_router, uint32_t* __restrict__ idx,
                        float* __restrict__ wts, uint32_t tokens, uint32_t hidden, uint32_t experts, uint32_t topk) {
+    dependent_start();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     __shared__ float s_logits[8][MAX_EXPERTS];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -162,11 +164,9 @@ cudaError_t launch_router_gate(const uint16_t* x, const uint16_t* w_router, uint
         }
         const uint32_t per_sm = uint32_t(std::max<size_t>(1, std::min<size_t>(2, (200 * 1024) / std::max<size_t>(wr_bytes, 1))));
         const uint32_t grid = min(want_blocks, uint32_t(sm_count) * per_sm);
-        moe_router_gate_kernel<true><<<grid, 256, wr_bytes, stream>>>(x, w_router, idx, wts, tokens, hidden, experts, topk);
-    } else {
-        moe_router_gate_kernel<false><<<want_blocks, 256, 0, stream>>>(x, w_router, idx, wts, tokens, hidden, experts, topk);
+        return launch_dependent(moe_router_gate_kernel<true>, dim3(grid), dim3(256), wr_bytes, stream, x, w_router, idx, wts, tokens, hidden, experts, topk);
     }
-    return cudaGetLastError();
+    return launch_dependent(moe_router_gate_kernel<false>, dim3(want_blocks), dim3(256), 0, stream, x, w_router, idx, wts, tokens, hidden, experts, topk);
 }
 
 // ---- plan: expert segments, tile table, deterministic row positions (single CTA) -------------------------------------
@@ -175,6 +175,7 @@ cudaError_t launch_router_gate(const uint16_t* x, const uint16_t* w_router, uint
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, uint32_t* __restrict__ pos,
                 uint32_t* __restrict__ row_token, uint32_t tokens, uint32_t experts, uint32_t topk, uint32_t max_rows) {
+    dependent_start();
     __shared__ uint32_t s_count[MAX_EXPERTS], s_start[MAX_EXPERTS + 1], s_cursor[MAX_EXPERTS];
     __shared__ uint32_t s_warp_cnt[MAX_EXPERTS][32];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -243,6 +244,7 @@ moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, u
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ row_token, const uint32_t* __restrict__ plan,
                   uint16_t* __restrict__ xg, uint32_t hidden, uint32_t experts, bool skinny) {
+    dependent_start();
     const uint32_t rows = plan[1 + experts];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t p = blockIdx.x * 8 + warp; p < rows; p += gridDim.x * 8) {
@@ -273,6 +275,7 @@ constexpr uint32_t SEG = 64;  // two chunks per lane
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const uint16_t* __restrict__ y, const uint32_t* __restrict__ pos, const float* __restrict__ wts,
                    uint16_t* __restrict__ out, uint32_t tokens, uint32_t hidden, uint32_t topk) {
+    dependent_start();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t chunks = hidden / 8, segs = (chunks + SEG - 1) / SEG;
     for (uint64_t unit = blockIdx.x * 8 + warp; unit < uint64_t(tokens) * segs; unit += gridDim.x * 8) {
@@ -377,11 +380,11 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
     cudaError_t e = launch_router_gate(static_cast<const uint16_t*>(x_bf16), static_cast<const uint16_t*>(w_router_bf16),
                                        routing_idx, routing_w, tokens, hidden, experts, topk, sm_count, stream);
     if (e != cudaSuccess) return e;
-    moe_plan_kernel<<<1, 1024, 0, stream>>>(routing_idx, plan, pos, row_token, tokens, experts, topk, L.max_rows);
+    e = launch_dependent(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, routing_idx, plan, pos, row_token, tokens, experts, topk, L.max_rows);
+    if (e != cudaSuccess) return e;
     const bool skinny = uint64_t(tokens) * topk <= uint64_t(experts) * SKINNY_ROWS;
-    moe_gather_kernel<<<sm_count * 4, 256, 0, stream>>>(static_cast<const uint16_t*>(x_bf16), row_token, plan, xg, hidden,
-                                                        experts, skinny);
-    e = cudaGetLastError();
+    e = launch_dependent(moe_gather_kernel, dim3(sm_count * 4), dim3(256), 0, stream, static_cast<const uint16_t*>(x_bf16), row_token, plan, xg, hidden,
+                         experts, skinny);
     if (e != cudaSuccess) return e;
     // Few rows per expert: weight rows on the M side, unpacked into tensor memory (8 experts, 4096 / 14336, top-2: 270 against
     // 784 us at 64 tokens, 644 against 795 us at 512 = 128 rows per expert; at 192 rows both take about 700 us: the pair GEMM's 256-row
@@ -395,8 +398,8 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
         if (e == cudaSuccess)
             e = launch_moe_skinny(h, w2, s2, y, plan, L.max_rows, hidden, inter, group, experts, false, wide, sm_count, stream, status);
         if (e != cudaSuccess) return e;
-        moe_combine_kernel<<<sm_count * 4, 256, 0, stream>>>(y, pos, routing_w, static_cast<uint16_t*>(out_bf16), tokens, hidden, topk);
-        return cudaGetLastError();
+        return launch_dependent(moe_combine_kernel, dim3(sm_count * 4), dim3(256), 0, stream, y, pos, routing_w, static_cast<uint16_t*>(out_bf16), tokens,
+                                hidden, topk);
     }
     // h = swiglu(xg . W1^T, xg . W3^T) per expert
     e = launch_int4_gemm_pair(xg, w13, s13, h, L.max_rows, inter, hidden, group, 0, 1, experts, tile_expert, plan, inter,
@@ -406,9 +409,8 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
     e = launch_int4_gemm_pair(h, w2, s2, y, L.max_rows, hidden, inter, group, 0, 0, experts, tile_expert, plan, hidden,
                               sm_count, stream, status);
     if (e != cudaSuccess) return e;
-    moe_combine_kernel<<<sm_count * 4, 256, 0, stream>>>(y, pos, routing_w, static_cast<uint16_t*>(out_bf16), tokens,
-                                                         hidden, topk);
-    return cudaGetLastError();
+    return launch_dependent(moe_combine_kernel, dim3(sm_count * 4), dim3(256), 0, stream, y, pos, routing_w, static_cast<uint16_t*>(out_bf16), tokens,
+                                hidden, topk);
 }
 
 // ---- the stages on their own, for expert-parallel runs where an exchange sits between them ---------------------------
@@ -452,9 +454,8 @@ cudaError_t launch_moe_combine(const void* y_rows, const uint32_t* pos, const fl
                                uint32_t tokens, uint32_t hidden, uint32_t topk, int sm_count, cudaStream_t stream) {
     if (hidden % 8 || topk == 0 || topk > MAX_TOPK) return cudaErrorNotSupported;
     if (tokens == 0) return cudaSuccess;
-    moe_combine_kernel<<<sm_count * 4, 256, 0, stream>>>(static_cast<const uint16_t*>(y_rows), pos, routing_w,
-                                                         static_cast<uint16_t*>(out_bf16), tokens, hidden, topk);
-    return cudaGetLastError();
+    return launch_dependent(moe_combine_kernel, dim3(sm_count * 4), dim3(256), 0, stream, static_cast<const uint16_t*>(y_rows), pos, routing_w,
+                            static_cast<uint16_t*>(out_bf16), tokens, hidden, topk);
 }
 
 }  // namespace vybk

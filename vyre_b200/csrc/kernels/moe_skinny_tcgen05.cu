@@ -26,6 +26,7 @@
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -118,15 +119,17 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         tma_prefetch_desc(&map_w);
         tma_prefetch_desc(&map_x);
     }
+    lets_next_start();
+    if (warp == 1) {
+        tmem_alloc(smem_u32(&bars->tmem_base), TMEM_COLS);
+        tmem_relinquish();
+    }
+    waits_for_previous();
     for (uint32_t e = threadIdx.x; e < p.experts; e += THREADS) {
         const uint32_t here = p.plan[1 + e], next = p.plan[2 + e];
         const uint32_t row = here & ~(ROW_TILE - 1);
         bars->seg_row[e] = row;
         bars->seg_count[e] = (next & ~(ROW_TILE - 1)) - row - (here & (ROW_TILE - 1));
-    }
-    if (warp == 1) {
-        tmem_alloc(smem_u32(&bars->tmem_base), TMEM_COLS);
-        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
@@ -345,8 +348,7 @@ cudaError_t launch_cfg(const CUtensorMap& mw, const void* x, uint32_t max_rows, 
     }
     CUtensorMap mx;
     if (!encode_tensor_map_2d(&mx, x, max_rows, p.k, 2, BN, 64, true)) return cudaErrorInvalidValue;
-    moe_skinny_kernel<BN, GLU><<<sm_count, THREADS, C::SMEM_BYTES, stream>>>(mw, mx, p);
-    return cudaGetLastError();
+    return launch_dependent(moe_skinny_kernel<BN, GLU>, dim3(sm_count), dim3(THREADS), C::SMEM_BYTES, stream, mw, mx, p);
 }
 
 }  // namespace

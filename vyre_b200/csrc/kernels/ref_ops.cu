@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <float.h>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 
 namespace vybk {
@@ -39,6 +40,7 @@ __device__ __forceinline__ void store_typed(void* p, size_t i, uint32_t dt, floa
 // vyre-libs/src/nn/linear/inner/linear_4bit.rs:255-335: thread per output, sequential k, mul then add.
 __global__ void linear_4bit_kernel(const float* x, const uint32_t* w, const float* b, float* out, uint32_t in_dim,
                                    uint32_t out_dim) {
+    dependent_start();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= out_dim) return;
     float acc = b[i];
@@ -54,6 +56,7 @@ __global__ void linear_4bit_kernel(const float* x, const uint32_t* w, const floa
 __global__ void affine_grouped_kernel(const float* x, const uint32_t* w, const float* scale, const uint32_t* zp,
                                       const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                       uint32_t total) {
+    dependent_start();
     const uint32_t o = blockIdx.x * 8 + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
     if (o >= total) return;
@@ -154,6 +157,7 @@ __global__ void int8_pack_kernel(const uint32_t* in, uint32_t* out, uint32_t n) 
 // vyre-libs/src/nn/linear/inner/builder.rs:287-344
 __global__ void linear_rows_kernel(const void* x, const void* w, const void* bias, void* out, uint32_t rows,
                                    uint32_t in_dim, uint32_t out_dim, uint32_t dt, uint32_t out_in) {
+    dependent_start();
     const uint32_t index = blockIdx.x * blockDim.x + threadIdx.x;
     if (index >= rows * out_dim) return;
     const uint32_t row = index / out_dim, col = index % out_dim;
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(128) linear_rows_tiled_kernel(const void* __re
                                                                 const void* __restrict__ bias, void* __restrict__ out,
                                                                 uint32_t rows, uint32_t in_dim, uint32_t out_dim, uint32_t dt,
                                                                 uint32_t out_in) {
+    dependent_start();
     constexpr uint32_t CB = 64, KC = 32, RB = 4 * RT;
     __shared__ float ws[KC][CB + 1];
     __shared__ __align__(16) float xs[RB][KC];
@@ -369,18 +374,23 @@ __global__ void top_k_kernel(const float* in, uint32_t* out_idx, float* vals, ui
 
 // vyre-libs/src/nn/activation/unary.rs:79-100: gate * (up * (1/(1+exp(-gate))))
 __global__ void swiglu_kernel(const void* gate, const void* up, void* out, uint32_t n, uint32_t dt) {
+    waits_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float g = load_typed(gate, i, dt), u = load_typed(up, i, dt);
+    lets_next_start();
     const float sig = fdiv(1.0f, fadd(1.0f, expf(-g)));
     store_typed(out, i, dt, fmul(g, fmul(u, sig)));
 }
 
 // vyre-libs/src/nn/activation/residual_add.rs:40-52: cast(dtype, f32(residual) + f32(branch))
 __global__ void residual_add_kernel(const void* residual, const void* branch, void* out, uint32_t n, uint32_t dt) {
+    waits_for_previous();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    store_typed(out, i, dt, fadd(load_typed(residual, i, dt), load_typed(branch, i, dt)));
+    const float r = load_typed(residual, i, dt), b = load_typed(branch, i, dt);
+    lets_next_start();
+    store_typed(out, i, dt, fadd(r, b));
 }
 
 // vyre-libs/src/nn/norm/gated_rms_norm.rs:123-247. The reference recomputes the row's sum of squares in every
@@ -389,6 +399,7 @@ __global__ void residual_add_kernel(const void* residual, const void* branch, vo
 // eps)), rounded to dtype, times f32(weight), times gate / (1 + exp(-gate)) with a gate, one cast). Same values.
 __global__ void rms_norm_kernel(const void* input, const void* weight, const void* gate, void* out, uint32_t hidden, float eps,
                                 uint32_t dt, uint32_t wdt) {
+    waits_for_previous();
     __shared__ float tile[1024];
     __shared__ float inv_shared;
     const size_t base = size_t(blockIdx.x) * hidden;
@@ -426,6 +437,7 @@ __global__ void rms_norm_kernel(const void* input, const void* weight, const voi
 // (about 1e-7 relative), everything after the sum is the code above.
 __global__ void __launch_bounds__(256) rms_norm_tree_kernel(const void* input, const void* weight, const void* gate, void* out,
                                                             uint32_t hidden, float eps, uint32_t dt, uint32_t wdt) {
+    waits_for_previous();
     __shared__ float warp_sum[8];
     __shared__ float inv_shared;
     const size_t base = size_t(blockIdx.x) * hidden;
@@ -464,6 +476,7 @@ __global__ void __launch_bounds__(256) rms_norm_tree_kernel(const void* input, c
 template <int V>
 __global__ void __launch_bounds__(256) rms_norm_tree_regs_kernel(const void* input, const void* weight, void* out, uint32_t hidden, float eps,
                                                                  uint32_t dt, uint32_t wdt) {
+    waits_for_previous();
     __shared__ float warp_sum[8];
     const size_t base = size_t(blockIdx.x) * hidden;
     float x[V], w[V];
@@ -484,6 +497,7 @@ __global__ void __launch_bounds__(256) rms_norm_tree_regs_kernel(const void* inp
     for (int o = 16; o > 0; o >>= 1) sum = fadd(sum, __shfl_xor_sync(0xffffffffu, sum, o));
     if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = sum;
     __syncthreads();
+    lets_next_start();  // not before the loads: a projection's prefetch would keep them waiting (10 us a decode block at 8 rows)
     float total = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) total = fadd(total, warp_sum[i]);
@@ -520,6 +534,7 @@ __global__ void k_quant_unpack_kernel(const uint32_t* packed, const float* scale
 // nibbles of the k-major weight stream, so a warp reads 16 (Q4_K) or 8 (Q2_K) contiguous bytes per k.
 __global__ void k_quant_linear_kernel(const float* x, const uint32_t* packed, const float* scales, const float* mins,
                                       const float* b, float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits) {
+    dependent_start();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= out_dim) return;
     float acc = b[i];
@@ -571,15 +586,13 @@ inline uint32_t blocks(uint64_t n, uint32_t per) { return uint32_t((n + per - 1)
 
 cudaError_t launch_linear_4bit(const float* x, const uint32_t* w, const float* b, float* out, uint32_t in_dim,
                                uint32_t out_dim, cudaStream_t s) {
-    linear_4bit_kernel<<<blocks(out_dim, 256), 256, 0, s>>>(x, w, b, out, in_dim, out_dim);
-    return cudaGetLastError();
+    return launch_dependent(linear_4bit_kernel, dim3(blocks(out_dim, 256)), dim3(256), 0, s, x, w, b, out, in_dim, out_dim);
 }
 cudaError_t launch_linear_4bit_affine_grouped(const float* x, const uint32_t* w, const float* scale,
                                               const uint32_t* zp, const float* b, float* out, uint32_t in_dim,
                                               uint32_t out_dim, uint32_t group, uint32_t batch, cudaStream_t s) {
     const uint32_t total = batch * out_dim;
-    affine_grouped_kernel<<<blocks(total, 8), 256, 0, s>>>(x, w, scale, zp, b, out, in_dim, out_dim, group, total);
-    return cudaGetLastError();
+    return launch_dependent(affine_grouped_kernel, dim3(blocks(total, 8)), dim3(256), 0, s, x, w, scale, zp, b, out, in_dim, out_dim, group, total);
 }
 cudaError_t launch_i4_unpack(const uint32_t* packed, int32_t* out, uint32_t lanes, cudaStream_t s) {
     i4_unpack_kernel<<<blocks(lanes, 256), 256, 0, s>>>(packed, out, lanes);
@@ -634,13 +647,10 @@ cudaError_t launch_linear_rows(const void* x, const void* w, const void* bias, v
                                   : outputs >= (out_in ? 5ull << 15 : 1ull << 21);
     if (tiled && outputs * in_dim >= (1ull << 18) && (rows + 4 * rt - 1) / (4 * rt) <= 65535u) {
         const dim3 grid((out_dim + 63) / 64, (rows + 4 * rt - 1) / (4 * rt));
-        if (rt == 1) linear_rows_tiled_kernel<1><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
-        else linear_rows_tiled_kernel<4><<<grid, 128, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
-        return cudaGetLastError();
+        if (rt == 1) return launch_dependent(linear_rows_tiled_kernel<1>, grid, dim3(128), 0, s, x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
+        return launch_dependent(linear_rows_tiled_kernel<4>, grid, dim3(128), 0, s, x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
     }
-    linear_rows_kernel<<<blocks(uint64_t(rows) * out_dim, 64), 64, 0, s>>>(x, w, bias, out, rows, in_dim, out_dim,
-                                                                           dtype, out_in);
-    return cudaGetLastError();
+    return launch_dependent(linear_rows_kernel, dim3(blocks(uint64_t(rows) * out_dim, 64)), dim3(64), 0, s, x, w, bias, out, rows, in_dim, out_dim, dtype, out_in);
 }
 cudaError_t launch_matmul_u32(const uint32_t* a, const uint32_t* b, const uint32_t* bias, uint32_t* out, uint32_t m,
                               uint32_t k, uint32_t n, cudaStream_t s) {
@@ -669,8 +679,7 @@ cudaError_t launch_top_k(const float* in, uint32_t* out_idx, float* best_vals, u
     return cudaGetLastError();
 }
 cudaError_t launch_residual_add(const void* residual, const void* branch, void* out, uint32_t n, uint32_t dtype, cudaStream_t s) {
-    residual_add_kernel<<<blocks(n, 256), 256, 0, s>>>(residual, branch, out, n, dtype);
-    return cudaGetLastError();
+    return launch_between<residual_add_kernel>(dim3(blocks(n, 256)), dim3(256), 0, s, residual, branch, out, n, dtype);
 }
 cudaError_t launch_rms_norm(const void* input, const void* weight, const void* gate, void* out, uint32_t rows, uint32_t hidden,
                             float eps, uint32_t dtype, uint32_t weight_dtype, bool tree, cudaStream_t s) {
@@ -679,12 +688,11 @@ cudaError_t launch_rms_norm(const void* input, const void* weight, const void* g
     // 296 x 8192 10.9 / 10.4; 600 x 6144 10.4 / 12.4, 1024 x 2048 6.3 / 8.3, 8192 x 4096 41 / 48, 8192 x 6144 60 / 94)
     const bool few = rows <= (hidden <= 4096 ? 592u : 296u);
     if (tree && !gate && few && hidden <= 4096)
-        rms_norm_tree_regs_kernel<16><<<rows, 256, 0, s>>>(input, weight, out, hidden, eps, dtype, weight_dtype);
-    else if (tree && !gate && few && hidden <= 8192)
-        rms_norm_tree_regs_kernel<32><<<rows, 256, 0, s>>>(input, weight, out, hidden, eps, dtype, weight_dtype);
-    else if (tree) rms_norm_tree_kernel<<<rows, 256, 0, s>>>(input, weight, gate, out, hidden, eps, dtype, weight_dtype);
-    else rms_norm_kernel<<<rows, 256, 0, s>>>(input, weight, gate, out, hidden, eps, dtype, weight_dtype);
-    return cudaGetLastError();
+        return launch_between<rms_norm_tree_regs_kernel<16>>(dim3(rows), dim3(256), 0, s, input, weight, out, hidden, eps, dtype, weight_dtype);
+    if (tree && !gate && few && hidden <= 8192)
+        return launch_between<rms_norm_tree_regs_kernel<32>>(dim3(rows), dim3(256), 0, s, input, weight, out, hidden, eps, dtype, weight_dtype);
+    if (tree) return launch_between<rms_norm_tree_kernel>(dim3(rows), dim3(256), 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
+    return launch_between<rms_norm_kernel>(dim3(rows), dim3(256), 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
 }
 cudaError_t launch_k_quant_unpack(const uint32_t* packed, const float* scales, const float* mins, float* out, uint32_t n,
                                   uint32_t bits, cudaStream_t s) {
@@ -693,12 +701,10 @@ cudaError_t launch_k_quant_unpack(const uint32_t* packed, const float* scales, c
 }
 cudaError_t launch_k_quant_linear(const float* x, const uint32_t* packed, const float* scales, const float* mins, const float* b,
                                   float* out, uint32_t in_dim, uint32_t out_dim, uint32_t bits, cudaStream_t s) {
-    k_quant_linear_kernel<<<blocks(out_dim, 64), 64, 0, s>>>(x, packed, scales, mins, b, out, in_dim, out_dim, bits);
-    return cudaGetLastError();
+    return launch_dependent(k_quant_linear_kernel, dim3(blocks(out_dim, 64)), dim3(64), 0, s, x, packed, scales, mins, b, out, in_dim, out_dim, bits);
 }
 cudaError_t launch_swiglu(const void* gate, const void* up, void* out, uint32_t n, uint32_t dtype, cudaStream_t s) {
-    swiglu_kernel<<<blocks(n, 256), 256, 0, s>>>(gate, up, out, n, dtype);
-    return cudaGetLastError();
+    return launch_between<swiglu_kernel>(dim3(blocks(n, 256)), dim3(256), 0, s, gate, up, out, n, dtype);
 }
 cudaError_t launch_expert_mlp(const float* x, const float* wg, const float* bg, const float* wu, const float* bu,
                               const float* wd, const float* bd, float* out, float* hidden_scratch, uint32_t in_dim,
