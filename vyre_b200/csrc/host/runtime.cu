@@ -320,6 +320,10 @@ cudaError_t run_int4_linear(vyb_instance* inst, uint32_t variant, const void* x,
         // One launch that reads the weights once for all rows. f32 outputs: where the eight-row kernel's group sums are f32 as well (error
         // against 64-bit sums, eight-row launches / one, mean of 40 inputs each: N(0, 1) activations 6.5 / 5.9e-8 at k 2048 and 7.0 / 7.0e-8 at
         // 4096, log-normal ones over four decades 1.50 / 1.47 and 1.58 / 1.59e-7); other k keep their exact ones.
+        // Up to 16 rows the form with one CTA to an SM, as nothing of the next submission is under way under this one's (8 rows, us: 4096 -> 14336 15.8 / 13.5,
+        // 4096 -> 4096 7.9 / 7.1, 1024 -> 14336 7.1 / 5.4).
+        if (batch > 8 && batch <= 16 && (!out_f32 || k == 2048 || k == 4096) && int4_few_rows_supported(x, w, scale, batch, n, k, group))
+            return launch_int4_few_rows(x, w, scale, y, batch, n, k, group, out_f32, inst->dev->prop.multiProcessorCount, s, inst->status_dev);
         if (batch > 8 && (!out_f32 || k == 2048 || k == 4096) && int4_skinny_supported(x, w, scale, batch, n, k, group))
             return launch_int4_skinny(x, w, scale, y, batch, n, k, out_f32, inst->dev->prop.multiProcessorCount, s, inst->status_dev, false);
         for (uint32_t b0 = 0; b0 < batch; b0 += 8) {
@@ -330,6 +334,14 @@ cudaError_t run_int4_linear(vyb_instance* inst, uint32_t variant, const void* x,
         }
         return cudaSuccess;
     }
+    // Up to eight rows of other groups and row lengths. Weights through tensor memory too, whose f32 group sums are as good here (error against
+    // 64-bit sums, generic / that kernel, N(0, 1) and log-normal activations: group 64 7.0 / 6.1e-8 and 1.16 / 1.17e-7 at k 1024, 1.2 / 0.9 and
+    // 2.6 / 1.3e-7 at 6400), except f32 outputs of groups of 128 (0.7 / 0.5 and 1.1 / 1.9e-7 at k 1280). Small calls of up to four rows stay on
+    // the warp-per-row kernel, which has no pipeline to fill (us: 1 x 512 -> 1024 2.7 / 3.5, 1 x 256 -> 4096 3.3 / 2.8, 1 x 1600 -> 64 6.2 / 4.5,
+    // 1 x 4096 -> 8192 58 / 10, 8 x 6400 -> 14336 371 / 21).
+    if (batch <= 8 && (!out_f32 || group == 64) && (batch > 4 || k >= 1024 || uint64_t(n) * k >= (1u << 20)) &&
+        int4_few_rows_supported(x, w, scale, batch, n, k, group))
+        return launch_int4_few_rows(x, w, scale, y, batch, n, k, group, out_f32, inst->dev->prop.multiProcessorCount, s, inst->status_dev);
     return launch_int4_linear_generic(x, w, scale, y, batch, n, k, group, out_f32, s);
 }
 

@@ -8,7 +8,7 @@
 // holds its own 128 activation rows and HALF of the weight rows of the tile, and the leader CTA issues
 // tcgen05.mma.cta_group::2 (M = 256). Compared with one CTA per 128 x 256 tile this halves, per SM, the packed
 // weights that are dequantised, the bf16 tile bytes written to shared memory and the operand bytes the tensor
-// core reads from it - the three things that bound the single-CTA kernel.
+// core reads from it - the three things that bound such a kernel on single CTAs.
 //
 // Roles per CTA (20 warps, placed by SM sub-partition = warp id % 4): warp 0 TMA producer (activation box -> the
 // LEADER's barrier with the pair form of the tensor load; packed-weight box -> a local barrier), warp 4 TMEM owner
@@ -375,8 +375,8 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 const uint32_t c0 = (kb % RAW_KB) * 2;
                 uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
                 if (r < half_rows) {
-                    w0 = *reinterpret_cast<const uint4*>(raw_row + ((c0 ^ (r & 7u)) << 4));
-                    w1 = *reinterpret_cast<const uint4*>(raw_row + (((c0 + 1) ^ (r & 7u)) << 4));
+                    w0 = lds_128(raw_row + ((c0 ^ (r & 7u)) << 4));
+                    w1 = lds_128(raw_row + (((c0 + 1) ^ (r & 7u)) << 4));
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[rs]));  // the packed bytes now live in registers

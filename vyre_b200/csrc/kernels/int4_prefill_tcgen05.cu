@@ -1,32 +1,32 @@
-// Prefill GEMM for group-quantized int4 weights on the 5th-generation tensor cores (tcgen05, sm_100a):
+// Group-quantized int4 linear with the weights in tensor memory (tcgen05, sm_100a): prefill batches, and few rows of any row length.
 //
-//   y[m, n] = bf16|f32( sum_k x[m, k] * bf16((q[n, k] - 8) * s[n, k / group]) )      f32 accumulate in TMEM
+//   rounded (prefill):  y[m, n] = cast( sum_k x[m, k] * bf16((q[n, k] - 8) * s[n, g(k)]) )          any group of whole 64 k, f32 sums
+//   exact (few rows):   y[m, n] = cast( sum_g s[n, g] * sum_{k in g} x[m, k] * (q[n, k] - 8) )      groups of 64 or 128, up to 16 rows
 //
-// With hundreds of activation rows the op is a dense contraction, so it runs on the tensor cores; the weights
-// stay packed in HBM and L2 and are dequantised to bf16 tiles on the fly, inside the kernel, straight into
-// the swizzled shared-memory layout the MMA reads.
+// The WEIGHT rows are the M = 128 side of the MMA and the activation rows its N side (16 to 128 columns); a thread unpacks a weight row's
+// nibbles in registers and stores them to tensor memory, where the MMA reads its A operand: no unpacked byte goes through shared memory.
+// A CTA per 128 x BN tile; k is split over a cluster where tiles leave SMs idle (partial tiles meet in distributed shared memory, added
+// in rank order). Per CTA: warp 0 packed weights by TMA (256 k a stage), warp 2 activations, warp 1 MMAs, warp 3 prefetches scales, sixteen
+// warps unpack (two sets of eight take the stages in turn), the last warps drain the sums: exact weights have an accumulator per
+// group, which meets its scale in f32 registers; rounded ones one accumulator for the whole row.
 //
-// One persistent CTA per SM walks 128 (rows of x) x 256 (rows of W) output tiles, M fastest. Per 64-k stage:
-//   * warp 0 issues two TMA tensor loads: the bf16 activation box (128 x 64, 128-byte swizzle) and the raw
-//     packed-weight box (256 rows x 32 bytes);
-//   * 16 dequant warps (two threads per weight row) read their 16 raw bytes, turn each nibble pair into bf16 with
-//     the (w & 0x000F000F) | 0x43004300 magic (= 128+q exactly), subtract 136 and multiply by the group scale
-//     with packed bf16 arithmetic (one rounding: bf16((q-8)*s)), and store 4 x 16 B into the 128-byte-swizzled
-//     K-major tile (chunk j of row r goes to chunk j ^ (r & 7), which is also bank-conflict free), then fence the
-//     generic-proxy writes towards the async proxy and arrive on the stage barrier;
-//   * one thread of warp 1 issues 4 x tcgen05.mma.kind::f16 (M=128, N=256, K=16) per stage from shared-memory
-//     descriptors; tcgen05.commit releases the stage;
-//   * 4 epilogue warps drain the 128 x 256 f32 accumulator from TMEM (tcgen05.ld) and store bf16 (or f32) rows.
-// Two accumulators (512 TMEM columns) overlap the epilogue of tile i with the main loop of tile i+1.
-// Every mbarrier wait is bounded; a wait that runs out raises a status word, the CTA drains and frees its TMEM.
+// What bounds it: a chain per stage (unpack 700 to 1500 cycles, MMA thread 400 + 430, waits of about 150 each), 1100 cycles with three unpacked
+// stages in flight, where the logic pipe needs 512 and, at 128 columns, the MMAs 1024. Packed bytes at HBM speed would take 5 us of the
+// 14 at 16 x 4096 -> 14336. Measured (nothing promised about the weights, HBM-cold, us, before / now): prefill kernels 16 x 4096 -> 14336 49 / 14,
+// 64 x 3072 -> 2658 52 / 7.5, 128 x 7168 -> 1024 81 / 11; generic kernel at groups of 64 8 x 6400 -> 14336 371 / 21, 1 x 4096 -> 8192 58 / 10; the other
+// tensor-memory kernel (int4_skinny_tcgen05.cu) 8 x 4096 -> 14336 15.8 / 13.5, 8 x 1024 -> 14336 7.1 / 5.4: that one keeps the decode launches,
+// since two of its CTAs share an SM and with constant weights the next launch's are on their way under this one's (four decode blocks of
+// 2048 / 6144 at 6 rows 92 us with it, 109 with this).
 //
-// Replaces, for large batches, the generated scalar kernel of
-// vyre-libs/src/nn/linear/inner/linear_4bit.rs:399-775; the tile layout is the row-major primitive layout of
-// vyre-primitives/src/math/quantized/programs.rs:181.
+// Every wait is bounded; on expiry a status word is raised, the CTA waits for what it has started and frees its TMEM. No multicast.
+//
+// Replaces the generated scalar kernel of vyre-libs/src/nn/linear/inner/linear_4bit.rs:399-775 for the row-major layout of
+// vyre-primitives/src/math/quantized/programs.rs:186-300 at prefill batches.
 #include <cuda_bf16.h>
 
 #include <atomic>
 
+#include "dependent_launch.cuh"
 #include "kernels.h"
 #include "tcgen05_common.cuh"
 
@@ -35,77 +35,99 @@ namespace {
 
 using namespace tc;
 
-constexpr int BM = 128, BN = 256, BK = 64;  // BK in bf16 elements (128 bytes per row)
-constexpr int UMMA_K = 16;
-// Three independent rings: the packed weights are prefetched deepest (they are small and come from HBM/L2), the
-// activation boxes next, and the dequantised tiles (the large ones) only need to cover dequant + MMA latency.
-constexpr int A_STAGES = 4, RAW_STAGES = 8, B_STAGES = 3;
-constexpr int RAW_AHEAD = 4;              // raw loads run this many stages ahead of the activation loads
-constexpr int A_BYTES = BM * BK * 2;      // 16 KB activations
-constexpr int B_BYTES = BN * BK * 2;      // 32 KB dequantised weights
-constexpr int RAW_BYTES = BN * (BK / 2);  // 8 KB packed weights
-constexpr int B_RING = 0, A_RING = B_STAGES * B_BYTES, RAW_RING = A_RING + A_STAGES * A_BYTES;
-constexpr int RING_BYTES = RAW_RING + RAW_STAGES * RAW_BYTES;
-constexpr int DEQ_WARPS = 16;                 // two threads per weight row (32 k each)
-constexpr int THREADS = (6 + DEQ_WARPS) * 32;  // TMA, MMA, 4 epilogue, 16 dequant
+constexpr int BM = 128, UMMA_K = 16;
+constexpr int KB = 256;                           // k per stage
+constexpr int RAW_BYTES = BM * KB / 2;            // 16 KB of packed weights
+constexpr int MAX_SPLIT = 8;
+constexpr int UNPACK_WARPS = 16, EPI_WARP = 4 + UNPACK_WARPS;
+constexpr int READY = 4, DONE = 8;                // barriers of stages that are ready and that are done: who follows them is never further behind
 constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
+constexpr int CTRL_BYTES = 512, ALIGN_SLACK = 1024;
+constexpr uint32_t PREFETCH_STAGES = 24;
+
+// BN: activation rows of a tile. G: scale groups of 128 k (group 128: 1, group 64: 2), an accumulator each and exact weights; 0: rounded
+// weights, one accumulator for the whole row.
+template <int BN, int G>
+struct Cfg {
+    static constexpr int X_BYTES = BN * KB * 2;
+    // Weights and activations have rings of their own: a stage of weights is free as soon as it is unpacked, one of activations when its MMAs
+    // are complete.
+    static constexpr int STAGES = BN == 16 ? 10 : BN == 32 ? 9 : BN == 64 ? 6 : 5, X_STAGES = BN == 16 ? 6 : BN <= 64 ? 4 : 2;
+    static constexpr int RING_BYTES = STAGES * RAW_BYTES + X_STAGES * X_BYTES;
+    static constexpr int SMEM_BYTES = RING_BYTES + CTRL_BYTES + ALIGN_SLACK;
+    static constexpr int SETS = G == 0 ? 1 : 2 * G;            // accumulators of a stage
+    static constexpr int A_COL = G == 0 ? BN : 2 * SETS * BN;  // accumulators (of two stages) come first
+    static constexpr int A_SLOTS = 3;                          // unpacked stages (8 x 4096 -> 14336: 13.4 us with two, 12.1 with three)
+    static_assert(A_COL + A_SLOTS * 128 <= TMEM_COLS && X_STAGES <= DONE && STAGES <= 10, "tensor memory, barriers");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
+    static_assert(BN * BM * 4 <= RING_BYTES, "the partial tile reuses the stages");
+};
+constexpr int EPI_WARPS = 4, THREADS = (EPI_WARP + EPI_WARPS) * 32;
 
 struct Bars {
-    unsigned long long a_full[A_STAGES], a_empty[A_STAGES], raw_full[RAW_STAGES], raw_empty[RAW_STAGES];
-    unsigned long long b_full[B_STAGES], b_empty[B_STAGES], acc_full[2], acc_empty[2], drained;
+    unsigned long long full[10], empty[10], x_full[6], b_full[READY], done[DONE], acc_full, drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
-    uint32_t a_issued, raw_issued;  // copies of the TMA role
+    uint32_t issued, x_issued;  // copies of the TMA roles
+};
+static_assert(sizeof(Bars) <= CTRL_BYTES, "control block");
+
+struct Params {
+    const uint16_t* scales;  // bf16 [n][k / group]
+    void* y;
+    uint32_t* status;
+    uint32_t m, n, k, split;
+    uint32_t group_inv;      // G = 0: group / 64 > 1: (i * group_inv) >> 32 = i / (group / 64) for the 64-k blocks i of a row; else 0
+    uint32_t groups;         // of a row
+    uint32_t tile0;          // first weight tile of this launch
+    // unpack_word's, from here so that they stay in registers: an instruction takes one immediate, and the compiler makes a second one
+    // anew before every use (three instructions a word)
+    uint32_t mask, mul, add;
 };
 
-__device__ __forceinline__ uint32_t bf16x2_sub(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("sub.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
-__device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
+// A packed word of eight nibbles -> four bf16 pairs (k, k + 1) = (q - 8) / 64. A byte in both halves of a register, masked to its low nibble
+// below and to its high one above, is a pair of subnormal bf16 numbers n 2^-133 and 16 n 2^-133; one exact fused multiply-add makes n / 64 - 1 / 8.
+__device__ __forceinline__ void unpack_word(uint32_t w, uint32_t* out, uint32_t mask, uint32_t mul, uint32_t add) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __byte_perm(w, 0u, 0x4040 | i | i << 8) & mask;
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(out[i]) : "r"(t), "r"(mul), "r"(add));
+    }
 }
 
-template <bool OUT_F32>
-__global__ void __launch_bounds__(THREADS, 1)
-int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                    const uint16_t* __restrict__ scales, void* __restrict__ y, uint32_t M, uint32_t N, uint32_t K,
-                    uint32_t group, uint32_t* status) {
+template <int BN, int G, bool OUT_F32>
+__global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
+    using C = Cfg<BN, G>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    Bars* bars = reinterpret_cast<Bars*>(tiles + RING_BYTES);
+    uint8_t* x_tiles = tiles + C::STAGES * RAW_BYTES;
+    Bars* bars = reinterpret_cast<Bars*>(tiles + C::RING_BYTES);
     volatile unsigned int* abort_flag = &bars->abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t m_tiles = (M + BM - 1) / BM, n_tiles = (N + BN - 1) / BN;
-    const uint32_t total_tiles = m_tiles * n_tiles, k_blocks = (K + BK - 1) / BK;
-    const uint32_t groups = K / group;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t part = blockIdx.x % p.split, n0 = (p.tile0 + blockIdx.x / p.split) * BM, m0 = blockIdx.y * BN;
+    const uint32_t blocks = (p.k + KB - 1) / KB, base = blocks / p.split, rem = blocks % p.split;
+    const uint32_t kb0 = part * base + min(part, rem), kbs = base + (part < rem ? 1u : 0u);  // stages of this part
+    auto store = [&](uint32_t c, uint32_t row, float v) {
+        if (m0 + c >= p.m || row >= p.n) return;
+        const size_t at = size_t(m0 + c) * p.n + row;
+        if constexpr (OUT_F32) static_cast<float*>(p.y)[at] = v;
+        else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
+    };
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < A_STAGES; ++s) {
-            mbar_init(smem_u32(&bars->a_full[s]), 1);
-            mbar_init(smem_u32(&bars->a_empty[s]), 1);
+        for (int s = 0; s < C::STAGES; ++s) {
+            mbar_init(smem_u32(&bars->full[s]), 1);
+            mbar_init(smem_u32(&bars->empty[s]), UNPACK_WARPS / 2);
         }
-        for (int s = 0; s < RAW_STAGES; ++s) {
-            mbar_init(smem_u32(&bars->raw_full[s]), 1);
-            mbar_init(smem_u32(&bars->raw_empty[s]), DEQ_WARPS);
-        }
-        for (int s = 0; s < B_STAGES; ++s) {
-            mbar_init(smem_u32(&bars->b_full[s]), DEQ_WARPS);
-            mbar_init(smem_u32(&bars->b_empty[s]), 1);
-        }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(smem_u32(&bars->acc_full[a]), 1);
-            mbar_init(smem_u32(&bars->acc_empty[a]), 4);
-        }
+        for (int s = 0; s < C::X_STAGES; ++s) mbar_init(smem_u32(&bars->x_full[s]), 1);
+        for (int s = 0; s < READY; ++s) mbar_init(smem_u32(&bars->b_full[s]), UNPACK_WARPS / 2 + (G == 0 ? 0 : EPI_WARPS));  // unpacked, and its accumulators free
+        for (int s = 0; s < DONE; ++s) mbar_init(smem_u32(&bars->done[s]), 1);
+        mbar_init(smem_u32(&bars->acc_full), 1);
         mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&map_x);
         tma_prefetch_desc(&map_w);
+        tma_prefetch_desc(&map_x);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(&bars->tmem_base), TMEM_COLS);
@@ -114,261 +136,351 @@ int4_prefill_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = bars->tmem_base;
+    const uint32_t tmem = bars->tmem_base;
+    lets_next_start();
+    auto done_wait = [&](uint32_t i) { return mbar_wait(smem_u32(&bars->done[i % DONE]), (i / DONE) & 1, abort_flag); };
 
+    bool ok = true;
     if (warp == 0) {
-        // ------------------------------------ TMA producer ------------------------------------
-        // two cursors over the same (tile, k-block) sequence: the raw-weight cursor leads the activation cursor
-        uint32_t a_it = 0, r_it = 0, r_tile = blockIdx.x, r_kb = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            const int m0 = int(tile % m_tiles) * BM;
-            for (uint32_t kb = 0; kb < k_blocks && ok; ++kb, ++a_it) {
-                while (ok && r_tile < total_tiles && r_it <= a_it + RAW_AHEAD) {
-                    const uint32_t rs = r_it % RAW_STAGES;
-                    if (r_it >= RAW_STAGES)
-                        ok = mbar_wait(smem_u32(&bars->raw_empty[rs]), ((r_it / RAW_STAGES) - 1) & 1, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    if (lane == 0) {
-                        const uint32_t bar = smem_u32(&bars->raw_full[rs]);
-                        mbar_arrive_expect_tx(bar, RAW_BYTES);
-                        tma_load_2d(smem_u32(tiles + RAW_RING + rs * RAW_BYTES), &map_w, int(r_kb * (BK / 2)),
-                                    int(r_tile / m_tiles) * BN, bar);
-                    }
-                    __syncwarp();
-                    ++r_it;
-                    if (++r_kb == k_blocks) {
-                        r_kb = 0;
-                        r_tile += gridDim.x;
-                    }
-                }
-                if (!ok) break;
-                const uint32_t as = a_it % A_STAGES;
-                if (a_it >= A_STAGES) ok = mbar_wait(smem_u32(&bars->a_empty[as]), ((a_it / A_STAGES) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (lane == 0) {
-                    const uint32_t bar = smem_u32(&bars->a_full[as]);
-                    mbar_arrive_expect_tx(bar, A_BYTES);
-                    tma_load_2d(smem_u32(tiles + A_RING + as * A_BYTES), &map_x, int(kb * BK), m0, bar);
-                }
-                __syncwarp();
+        // ---- packed weights: into L2 while the launches before this one run, from there when they are complete ----
+        if (elect_one()) {
+            for (uint32_t i = 0; i < min(kbs, PREFETCH_STAGES); ++i) tma_prefetch_2d(&map_w, int((kb0 + i) * (KB / 2)), int(n0));
+            waits_for_previous();
+            uint32_t i = 0;
+            for (; i < kbs; ++i) {
+                const uint32_t s = i % C::STAGES, bar = smem_u32(&bars->full[s]);
+                if (i >= uint32_t(C::STAGES) && !mbar_wait(smem_u32(&bars->empty[s]), ((i / C::STAGES) - 1) & 1, abort_flag)) break;
+                mbar_arrive_expect_tx(bar, RAW_BYTES);
+                tma_load_2d(smem_u32(tiles + s * RAW_BYTES), &map_w, int((kb0 + i) * (KB / 2)), int(n0), bar);
             }
-        }
-        if (lane == 0) {
-            bars->raw_issued = r_it;
-            bars->a_issued = a_it;
+            bars->issued = i;
         }
         __syncwarp();
+    } else if (warp == 2) {
+        // ---- activations ----
+        if (elect_one()) {
+            waits_for_previous();
+            uint32_t i = 0;
+            for (; i < kbs; ++i) {
+                const uint32_t s = i % C::X_STAGES, bar = smem_u32(&bars->x_full[s]), dst = smem_u32(x_tiles + s * C::X_BYTES);
+                if (i >= uint32_t(C::X_STAGES) && !done_wait(i - C::X_STAGES)) break;
+                mbar_arrive_expect_tx(bar, C::X_BYTES);
+#pragma unroll
+                for (int j = 0; j < KB / 64; ++j) tma_load_2d(dst + j * BN * 128, &map_x, int((kb0 + i) * KB + j * 64), int(m0), bar);
+            }
+            bars->x_issued = i;
+        }
+        __syncwarp();
+    } else if (warp == 3) {
+        // ---- scales into L2: a row's share is a few sectors, read two bytes at a time ----
+        const uint32_t row_bytes = p.groups * 2, per = G == 0 ? 8 : 4 * G, first = kb0 * per, last = min(row_bytes, first + kbs * per);
+        for (uint32_t r = lane; r < BM && n0 + r < p.n; r += 32)
+            for (uint32_t at = first; at < last; at += 32)
+                prefetch_l2(reinterpret_cast<const uint8_t*>(p.scales) + size_t(n0 + r) * row_bytes + at);
     } else if (warp == 1) {
-        // ------------------------------------ MMA issuer ---------------------------------------
+        // ---- MMA: one commit per stage frees the unpacked weights and the activations and hands the sums on ----
         constexpr uint32_t idesc = idesc_bf16_f32(BM, BN);
-        uint32_t it = 0, local = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++local) {
-            const uint32_t acc = local & 1;
-            if (local >= 2) ok = mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag);
+        if (elect_one()) {
+            uint32_t xs = 0, x_parity = 0, slot = 0;
+#pragma unroll 1
+            for (uint32_t i = 0; i < kbs; ++i) {
+                // One round trip for all that a stage waits for: a wait takes this thread 150 cycles although the barrier is complete, a commit
+                // 60 to 100, an MMA 20 (with waits and commits of their own for activations, accumulators and slots 830 cycles per 128 k).
+                if (!mbar_wait2(smem_u32(&bars->x_full[xs]), x_parity, smem_u32(&bars->b_full[i % READY]), (i / READY) & 1, abort_flag)) break;
+                tc_fence_after();
+                const uint32_t b = smem_u32(x_tiles + xs * C::X_BYTES), d = G == 0 ? tmem : tmem + (i & 1) * C::SETS * BN, a = tmem + C::A_COL + slot * 128;
+                const uint64_t db = smem_desc_sw128(b);
+#pragma unroll
+                for (int k = 0; k < KB / UMMA_K; ++k)
+                    mma_f16_ts(d + k / (16 / C::SETS) * BN, a + k * (UMMA_K / 2), smem_desc_advance(db, k / 4 * BN * 128 + (k & 3) * UMMA_K * 2), idesc,
+                               k % (16 / C::SETS) != 0 || (G == 0 && i != 0));
+                tc_commit(smem_u32(&bars->done[i % DONE]));
+                slot = slot + 1 == uint32_t(C::A_SLOTS) ? 0u : slot + 1;
+                if (++xs == uint32_t(C::X_STAGES)) {
+                    xs = 0;
+                    x_parity ^= 1;
+                }
+            }
+            if (G == 0 && *abort_flag == 0) tc_commit(smem_u32(&bars->acc_full));
+            if (*abort_flag != 0) settle_mma(smem_u32(&bars->drained));
+        }
+        __syncwarp();
+    } else if (warp < uint32_t(EPI_WARP)) {
+        // ---- unpack: a thread per weight row, eight warps a stage, two sets of eight in turn: what one set waits for lies under the work of the other ----
+        const uint32_t unit = (warp >> 2) - 1, half = unit & 1, quad = warp & 3, r = quad * 32 + lane;
+        const uint32_t mask = p.mask, mul = p.mul, add = p.add;
+        uint32_t s = unit >> 1, parity = 0;
+        // G = 0: the scales of this thread's two 64-k blocks, a stage of its own ahead
+        if (G == 0) waits_for_previous();
+        const uint16_t* sp = p.scales + size_t(min(n0 + r, p.n - 1)) * p.groups;
+        auto scale = [&](uint32_t i, uint32_t b) {
+            const uint32_t at = (kb0 + i) * 4 + half * 2 + b, g = p.group_inv ? __umulhi(at, p.group_inv) : at;
+            return g < p.groups ? uint32_t(__ldg(sp + g)) * 0x10001u : 0u;  // past the row's last group the activations are zeros
+        };
+        uint32_t next0 = G == 0 ? scale(s, 0) : 0, next1 = G == 0 ? scale(s, 1) : 0;
+#pragma unroll 1
+        for (uint32_t i = s; i < kbs; i += 2) {
+            const uint32_t s0 = next0, s1 = next1;
+            if constexpr (G == 0) {
+                next0 = scale(i + 2, 0);
+                next1 = scale(i + 2, 1);
+            }
+            ok = mbar_wait(smem_u32(&bars->full[s]), parity, abort_flag);
+            if (i >= uint32_t(C::A_SLOTS)) ok = ok && done_wait(i - C::A_SLOTS);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + acc * BN;
-            for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-                const uint32_t as = it % A_STAGES, bs = it % B_STAGES;
-                ok = mbar_wait(smem_u32(&bars->a_full[as]), (it / A_STAGES) & 1, abort_flag) &&
-                     mbar_wait(smem_u32(&bars->b_full[bs]), (it / B_STAGES) & 1, abort_flag);
+            const uint8_t* row = tiles + s * RAW_BYTES + r * 128;
+            const uint32_t dst = tmem + ((quad * 32) << 16) + C::A_COL + i % C::A_SLOTS * 128 + half * 64;
+            uint4 v[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4*>(row + (((half * 4 + j) ^ (r & 7u)) << 4));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t a[16];
+                const uint32_t words[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if constexpr (G != 0) {
+                        unpack_word(words[u], a + 4 * u, mask, mul, add);
+                    } else {
+                        uint32_t q[4];
+                        unpack_int4_bf16(words[u], q);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) asm("mul.bf16x2 %0, %1, %2;" : "=r"(a[4 * u + e]) : "r"(q[e]), "r"(j < 2 ? s0 : s1));
+                    }
+                }
+                tmem_st_32x16(dst + j * 16, a);
+            }
+            // The packed bytes have been used, not only loaded: the compiler may move loads below an arrival that only follows them in the
+            // source, and the next copy then lands under them (wrong rows in half of a few hundred launches).
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->empty[s]));
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->b_full[i % READY]));
+            s += 2;
+            if (s >= uint32_t(C::STAGES)) {
+                s -= C::STAGES;
+                parity ^= 1;
+            }
+        }
+    } else if constexpr (G == 0) {
+        // ---- epilogue: the sums as they are ----
+        const uint32_t quad = warp & 3, o = quad * 32 + lane, row = n0 + o;
+        ok = mbar_wait(smem_u32(&bars->acc_full), 0, abort_flag);  // of its own: this role does not follow `done` stage by stage
+        ok = __all_sync(0xffffffffu, ok);
+        if (ok) {
+            tc_fence_after();
+            float* partial = reinterpret_cast<float*>(tiles);  // every load and MMA of this CTA is complete: the stages are free
+#pragma unroll 1
+            for (uint32_t c = 0; c < BN && m0 + c < p.m; c += 16) {
+                uint32_t v[16];
+                tmem_ld_32x16(tmem + ((quad * 32) << 16) + c, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (p.split == 1) store(c + j, row, __uint_as_float(v[j]));
+                    else partial[(c + j) * BM + o] = __uint_as_float(v[j]);
+                }
+            }
+        }
+    } else {
+        // ---- epilogue: acc += scale * group sum ----
+        waits_for_previous();  // scales
+        const uint32_t quad = warp & 3, o = quad * 32 + lane, row = n0 + o;
+        const uint32_t groups = p.groups, g0 = kb0 * C::SETS;
+        const uint16_t* sp = p.scales + size_t(min(row, p.n - 1)) * groups;
+        float acc[BN];
+#pragma unroll
+        for (int c = 0; c < BN; ++c) acc[c] = 0.0f;
+        if (lane == 0) {  // both stages' accumulators are free
+            mbar_arrive(smem_u32(&bars->b_full[0]));
+            mbar_arrive(smem_u32(&bars->b_full[1]));
+        }
+        constexpr uint32_t AHEAD = 2;  // stages whose scales are in flight
+        uint32_t queue[AHEAD][G];
+        auto load_scales = [&](uint32_t i, uint32_t (&q)[G]) {
+#pragma unroll
+            for (int h = 0; h < G; ++h) {  // past the row's last group the activations are zeros
+                const uint32_t g = g0 + i * C::SETS + 2 * h;
+                q[h] = (g < groups ? uint32_t(__ldg(sp + g)) : 0u) | (g + 1 < groups ? uint32_t(__ldg(sp + g + 1)) << 16 : 0u);
+            }
+        };
+#pragma unroll
+        for (uint32_t d = 0; d < AHEAD; ++d) load_scales(d, queue[d]);
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < kbs && ok; i0 += AHEAD) {
+#pragma unroll
+            for (uint32_t d = 0; d < AHEAD; ++d) {
+                const uint32_t i = i0 + d;
+                if (i >= kbs || !ok) break;
+                uint32_t bits[G];
+#pragma unroll
+                for (int h = 0; h < G; ++h) bits[h] = queue[d][h];
+                load_scales(i + AHEAD, queue[d]);
+                ok = done_wait(i);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
-                    const uint64_t da = smem_desc_sw128(smem_u32(tiles + A_RING + as * A_BYTES));
-                    const uint64_t db = smem_desc_sw128(smem_u32(tiles + B_RING + bs * B_BYTES));
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        mma_f16(d_tmem, smem_desc_advance(da, k * UMMA_K * 2), smem_desc_advance(db, k * UMMA_K * 2), idesc,
-                                (kb | uint32_t(k)) != 0);
-                    tc_commit(smem_u32(&bars->a_empty[as]));
-                    tc_commit(smem_u32(&bars->b_empty[bs]));
-                }
-                __syncwarp();
-            }
-            if (ok && lane == 0) tc_commit(smem_u32(&bars->acc_full[acc]));
-            __syncwarp();
-        }
-        if (*abort_flag != 0 && lane == 0) settle_mma(smem_u32(&bars->drained));
-        __syncwarp();
-    } else if (warp < 6) {
-        // ------------------------------------ epilogue warps ------------------------------------
-        const uint32_t quad = warp & 3;
-        uint32_t local = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++local) {
-            const uint32_t acc = local & 1;
-            const uint32_t m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
-            ok = mbar_wait(smem_u32(&bars->acc_full[acc]), (local >> 1) & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t row = m0 + quad * 32 + lane;
-            const uint32_t taddr = tmem_base + ((quad * 32) << 16) + acc * BN;
-#pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t r[32];
-                tmem_ld_32x32(taddr + c * 32, r);
-                tmem_ld_wait();
-                const uint32_t col0 = n0 + c * 32;
-                if (row < M && col0 < N) {
-                    if constexpr (OUT_F32) {
-                        float* dst = static_cast<float*>(y) + size_t(row) * N + col0;
-                        if (col0 + 32 <= N && (N & 3u) == 0) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                reinterpret_cast<uint4*>(dst)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-                        } else {
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) dst[j] = __uint_as_float(r[j]);
-                        }
-                    } else {
-                        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(y) + size_t(row) * N + col0;
-                        if (col0 + 32 <= N && (N & 7u) == 0) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                uint32_t pk[4];
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-                                    const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 2 * q]),
-                                                                                   __uint_as_float(r[8 * j + 2 * q + 1]));
-                                    pk[q] = *reinterpret_cast<const uint32_t*>(&h);
-                                }
-                                reinterpret_cast<uint4*>(dst)[j] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                            }
-                        } else {
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
-                        }
+                for (int h = 0; h < C::SETS; ++h) {
+                    const float s = __uint_as_float(h & 1 ? bits[h / 2] & 0xFFFF0000u : bits[h / 2] << 16) * 64.0f;  // tensor memory holds (q - 8) / 64
+                    uint32_t v[BN];
+                    tmem_ld_32x16(tmem + ((quad * 32) << 16) + (d * C::SETS + h) * BN, v);
+                    tmem_ld_wait();
+                    if (h == C::SETS - 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&bars->b_full[(i + 2) % READY]));  // for the stage after the next
                     }
+#pragma unroll
+                    for (int c = 0; c < BN; ++c) acc[c] = fmaf(s, __uint_as_float(v[c]), acc[c]);
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[acc]));
         }
-    } else {
-        // ------------------------------------ dequant warps ------------------------------------
-        const uint32_t tid = (warp - 6) * 32 + lane;
-        const uint32_t r = tid >> 1;     // weight row inside the tile
-        const uint32_t half = tid & 1u;  // which 32-k half of the 64-k stage row
-        uint32_t it = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            const uint32_t n0 = (tile / m_tiles) * BN;
-            const bool row_valid = n0 + r < N;
-            const uint16_t* srow = scales + size_t(row_valid ? n0 + r : 0) * groups;
-            // scales are read one group ahead: the load issued at a group change is consumed at the next one,
-            // so its latency hides behind a whole group of dequantisation instead of stalling every other stage
-            uint32_t cur_group = 0xFFFFFFFFu, s2 = 0;
-            uint32_t s_next = row_valid ? uint32_t(srow[0]) : 0u;
-            for (uint32_t kb = 0; kb < k_blocks; ++kb, ++it) {
-                const uint32_t rs = it % RAW_STAGES, bs = it % B_STAGES;
-                const uint32_t g = (kb * BK) / group;
-                if (g != cur_group) {
-                    cur_group = g;
-                    s2 = s_next | (s_next << 16);  // this group's scale in both bf16 halves
-                    s_next = (row_valid && g + 1 < groups) ? uint32_t(srow[g + 1]) : 0u;
-                }
-                ok = mbar_wait(smem_u32(&bars->raw_full[rs]), (it / RAW_STAGES) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const uint4 w0 = *reinterpret_cast<const uint4*>(tiles + RAW_RING + rs * RAW_BYTES + r * (BK / 2) + half * 16);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[rs]));  // the packed bytes now live in registers
-                const uint32_t words[4] = {w0.x, w0.y, w0.z, w0.w};
-                uint4 o[4];
+        if (ok) {
+            if (p.split == 1) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t w = words[j];
-                    uint32_t t0 = and_or(w, 0x000F000Fu, 0x43004300u);          // (k0, k4) as 128+q
-                    uint32_t t1 = and_or(w >> 4, 0x000F000Fu, 0x43004300u);   // (k1, k5)
-                    uint32_t t2 = and_or(w >> 8, 0x000F000Fu, 0x43004300u);   // (k2, k6)
-                    uint32_t t3 = and_or(w >> 12, 0x000F000Fu, 0x43004300u);  // (k3, k7)
-                    t0 = bf16x2_mul(bf16x2_sub(t0, 0x43084308u), s2);       // exact q-8, then one rounding of (q-8)*s
-                    t1 = bf16x2_mul(bf16x2_sub(t1, 0x43084308u), s2);
-                    t2 = bf16x2_mul(bf16x2_sub(t2, 0x43084308u), s2);
-                    t3 = bf16x2_mul(bf16x2_sub(t3, 0x43084308u), s2);
-                    o[j].x = __byte_perm(t0, t1, 0x5410);  // (k0, k1)
-                    o[j].y = __byte_perm(t2, t3, 0x5410);  // (k2, k3)
-                    o[j].z = __byte_perm(t0, t1, 0x7632);  // (k4, k5)
-                    o[j].w = __byte_perm(t2, t3, 0x7632);  // (k6, k7)
-                }
-                // the dequantised tile slot must have been consumed by the MMAs of its previous use
-                if (it >= B_STAGES) ok = mbar_wait(smem_u32(&bars->b_empty[bs]), ((it / B_STAGES) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                uint8_t* brow = tiles + B_RING + bs * B_BYTES + r * 128;
+                for (int c = 0; c < BN; ++c) store(c, row, acc[c]);
+            } else {
+                // the last group sum is complete, so every load and MMA of this CTA is: the stages are free
+                float* partial = reinterpret_cast<float*>(tiles);  // [BN][128]
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t chunk = half * 4 + uint32_t(j);
-                    *reinterpret_cast<uint4*>(brow + ((chunk ^ (r & 7u)) << 4)) = o[j];
-                }
-                fence_proxy_async();  // make the generic-proxy stores visible to the tensor core's operand reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->b_full[bs]));
+                for (int c = 0; c < BN; ++c) partial[c * BM + o] = acc[c];
             }
         }
     }
-
     tc_fence_before();
-    __syncthreads();
+    if (p.split > 1) {
+        cluster_sync();  // every part's partial tile is in its shared memory
+        for (uint32_t idx = threadIdx.x; idx < ((BN + p.split - 1 - part) / p.split) * BM; idx += THREADS) {
+            const uint32_t c = (idx / BM) * p.split + part, o = idx % BM;
+            if (m0 + c >= p.m || n0 + o >= p.n) continue;
+            const uint32_t addr = smem_u32(reinterpret_cast<float*>(tiles) + c * BM + o);
+            float v[MAX_SPLIT];
+#pragma unroll
+            for (uint32_t q = 0; q < MAX_SPLIT; ++q)
+                if (q < p.split) v[q] = ld_cluster_f32(mapa(addr, q));
+            float sum = v[0];
+#pragma unroll
+            for (uint32_t q = 1; q < MAX_SPLIT; ++q)
+                if (q < p.split) sum += v[q];
+            store(c, n0 + o, sum);
+        }
+        cluster_sync();  // no CTA leaves while another still reads its shared memory
+    } else {
+        __syncthreads();
+    }
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem, TMEM_COLS);
     }
     if (threadIdx.x == 0 && bars->abort_flag != 0) {
-        settle_copies(bars->raw_full, RAW_STAGES, bars->raw_issued);
-        settle_copies(bars->a_full, A_STAGES, bars->a_issued);
-        if (status) atomicOr(status, 8u);
+        settle_copies(bars->full, C::STAGES, bars->issued);
+        settle_copies(bars->x_full, C::X_STAGES, bars->x_issued);
+        if (p.status) atomicOr(p.status, 8u);
     }
 }
 
-}  // namespace
-
-bool int4_prefill_supported(uint32_t m, uint32_t n, uint32_t k, uint32_t group) {
-    // 64-k stages must not straddle a scale group; tensor-map strides need 16-byte multiples
-    return m >= 1 && n >= 1 && k >= 64 && k % 64 == 0 && group >= 64 && group % 64 == 0 && k % group == 0;
-}
-
-cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m,
-                                uint32_t n, uint32_t k, uint32_t group, uint32_t out_f32, int sm_count,
-                                cudaStream_t stream, uint32_t* status) {
-    // above 128 rows the CTA-pair kernel (256-row tiles, half the dequantisation per SM) takes over
-    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2)
-        return launch_int4_gemm_pair(x_bf16, w_packed, scale_bf16, y, m, n, k, group, out_f32, 0, 1, nullptr, nullptr, n,
-                                     sm_count, stream, status);
+template <int BN, int G, bool OUT_F32>
+cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cudaStream_t stream) {
+    using C = Cfg<BN, G>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured.load() & bit)) {
-        e = cudaFuncSetAttribute(int4_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(int4_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        const void* f = (const void*)int4_tmem_kernel<BN, G, OUT_F32>;
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
-        configured.fetch_or(bit);
+        configured.fetch_or(bit, std::memory_order_release);
     }
-    CUtensorMap mx, mw;
-    if (!encode_tensor_map_2d(&mx, x_bf16, m, k, 2, BM, BK, true) ||
-        !encode_tensor_map_2d(&mw, w_packed, n, k / 2, 1, BN, BK / 2, false))
+    const uint32_t tiles = (p.n + BM - 1) / BM, rows = (p.m + BN - 1) / BN, slots = uint32_t(sm_count) / rows > 0 ? uint32_t(sm_count) / rows : 1u;
+    // as many parts of the k range as fit at once, two stages each at least
+    const uint32_t blocks = (p.k + KB - 1) / KB;
+    p.split = slots / tiles;
+    if (p.split > blocks / 2) p.split = blocks / 2;
+    if (p.split > uint32_t(MAX_SPLIT)) p.split = MAX_SPLIT;
+    if (p.split < 1) p.split = 1;
+    const bool all_sms = whole_device(dev, sm_count);
+    CUtensorMap mw, mx;
+    if (!encode_tensor_map_2d(&mw, w, p.n, p.k / 2, 1, BM, KB / 2, true) || !encode_tensor_map_2d(&mx, x, p.m, p.k, 2, BN, 64, true))
         return cudaErrorInvalidValue;
-    const uint32_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
-    const uint32_t grid = tiles < uint32_t(sm_count) ? tiles : uint32_t(sm_count);
-    if (out_f32)
-        int4_prefill_kernel<true><<<grid, THREADS, SMEM_BYTES, stream>>>(mx, mw, static_cast<const uint16_t*>(scale_bf16),
-                                                                         y, m, n, k, group, status);
-    else
-        int4_prefill_kernel<false><<<grid, THREADS, SMEM_BYTES, stream>>>(mx, mw, static_cast<const uint16_t*>(scale_bf16),
-                                                                          y, m, n, k, group, status);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    dependent(attr[1]);
+    cfg.attrs = attr;
+    cfg.numAttrs = all_sms ? 2 : 1;
+    // A caller that wants an SM left free (sm_count below the device's) gets launches that fit the other SMs at once: a second wave of one
+    // launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
+    const uint32_t step = all_sms ? tiles : slots;
+    for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
+        cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split, rows);
+        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, OUT_F32>, mw, mx, p);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+Params make_params(const void* scale, void* y, uint32_t m, uint32_t n, uint32_t k, uint32_t group, uint32_t* status) {
+    Params p = {};
+    p.scales = static_cast<const uint16_t*>(scale);
+    p.y = y;
+    p.status = status;
+    p.m = m;
+    p.n = n;
+    p.k = k;
+    p.groups = k / group;
+    p.mask = 0x00F0000Fu;
+    p.mul = 0x7D007F00u;  // 2^123 | 2^127
+    p.add = 0xBE00BE00u;  // -1/8
+    return p;
+}
+
+}  // namespace
+
+bool int4_prefill_supported(uint32_t m, uint32_t n, uint32_t k, uint32_t group) {
+    // 64-k blocks must not straddle a scale group; tensor-map strides need 16-byte multiples
+    return m >= 1 && n >= 1 && k >= 64 && k % 64 == 0 && group >= 64 && group % 64 == 0 && k % group == 0;
+}
+bool int4_few_rows_supported(const void* x, const void* w, const void* scale, uint32_t m, uint32_t n, uint32_t k, uint32_t group) {
+    return m >= 1 && m <= 16 && n >= 1 && (group == 128 || group == 64) && k >= 64 && k % group == 0 &&
+           ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0 && (reinterpret_cast<uintptr_t>(scale) & 1u) == 0;
+}
+
+cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
+                                 uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
+    const Params p = make_params(scale_bf16, y, m, n, k, group, status);
+    const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
+    return group == 64 ? launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
+}
+
+cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
+                                uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
+    // The CTA-pair GEMM (256-row tiles, half of the dequantisation per SM) from 129 rows on, except where this kernel's 128 x 128 tiles fit
+    // the SMs at once or rows are long (pair / this, us: 160 x 4096 -> 4096 25 / 14, 512 x 7168 -> 1024 40 / 14, 1024 x 4096 -> 14336 153 / 126,
+    // but 256 x 1024 -> 14336 18 / 23 and 1024 x 2048 -> 8192 49 / 60; beyond 1024 rows not measured).
+    const uint64_t items = uint64_t((n + 127) / 128) * ((m + 127) / 128);
+    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > uint64_t(sm_count) && (k < 3072 || m > 1024))
+        return launch_int4_gemm_pair(x_bf16, w_packed, scale_bf16, y, m, n, k, group, out_f32, 0, 1, nullptr, nullptr, n, sm_count, stream, status);
+    if (m > 65535u * 128u) return cudaErrorInvalidValue;
+    Params p = make_params(scale_bf16, y, m, n, k, group, status);
+    const uint32_t per = group / 64;
+    if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
+    const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
+    if (m <= 16) return launch(launch_cfg<16, 0, true>, launch_cfg<16, 0, false>);
+    if (m <= 32) return launch(launch_cfg<32, 0, true>, launch_cfg<32, 0, false>);
+    return m <= 64 ? launch(launch_cfg<64, 0, true>, launch_cfg<64, 0, false>) : launch(launch_cfg<128, 0, true>, launch_cfg<128, 0, false>);
 }
 
 }  // namespace vybk
