@@ -52,5 +52,6 @@ def test_rounded_weights(m, n, k, group):
                                                 C.c_void_p(torch.cuda.current_stream().cuda_stream), C.c_void_p(status.data_ptr())))
     torch.cuda.synchronize()
     assert status.tolist() == [0] * 4 and (y[m] == 7.0).all()
-    # the tensor core drops the bits of an addend below its sum's f32 mantissa (about 1e-6 of an output's typical size)
-    assert rel(y[:m].cpu().numpy(), want.reshape(m, n), 0.1) <= 1e-4
+    # Each of the k / 16 additions to a running sum may drop what lies below its f32 mantissa: at most 2^-23 of it, and running sums reach five
+    # times the outputs' RMS, of which the window's floor is a tenth (the prefill kernels before had the same sums).
+    assert rel(y[:m].cpu().numpy(), want.reshape(m, n), 0.1) <= max(1e-4, k / 16 * 2.0**-23 * 5 / 0.1)
