@@ -39,9 +39,10 @@ def test_few_rows_of_other_groups(m, n, k, group):
 
 
 # rounded weights: every tile width, one row past it, several tiles of rows, long rows beyond 128 rows, groups that are no power of two, 16 and
-# 17 stages in one CTA
+# 17 stages in one CTA; CTA pairs: two passes a tile for four sets of warps, six, a last tile of few rows, ragged outputs
 @pytest.mark.parametrize("m,n,k,group", [(16, 129, 448, 64), (17, 128, 1344, 192), (33, 1000, 4096, 128), (65, 260, 1024, 512), (128, 127, 64, 64),
-                                         (129, 300, 3072, 128), (300, 257, 512, 256), (33, 9601, 4096, 128), (17, 9600, 4352, 64), (66, 9600, 4352, 64)])
+                                         (129, 300, 3072, 128), (300, 257, 512, 256), (33, 9601, 4096, 128), (17, 9600, 4352, 64), (66, 9600, 4352, 64),
+                                         (129, 9700, 256, 64), (260, 9601, 768, 128), (385, 5000, 512, 256)])
 def test_rounded_weights(m, n, k, group):
     x, w, s = synth.int4_linear_inputs(m, n, k, group=group, seed=m + n + k)
     want = oracle.int4_rowmajor_linear(x, w, s, m, n, k, group=group, out_dtype=oracle.DT_F32, mode=1)

@@ -4,31 +4,23 @@
 //   plain:  y[m, n]  = bf16|f32( sum_k x[m, k] * bf16((q[e(m), n, k] - 8) * s[e(m), n, k / group]) )
 //   glu:    h[m, j]  = bf16( g * (u * sigmoid(g)) ),  g = bf16(x[m,:] . W1[e(m), j, :]),  u = bf16(x[m,:] . W3[e(m), j, :])
 //
-// Two CTAs of a cluster (one TPC) share every MMA: the pair owns a 256-row x BN-column accumulator tile, each CTA
-// holds its own 128 activation rows and HALF of the weight rows of the tile, and the leader CTA issues
-// tcgen05.mma.cta_group::2 (M = 256). Compared with one CTA per 128 x 256 tile this halves, per SM, the packed
-// weights that are dequantised, the bf16 tile bytes written to shared memory and the operand bytes the tensor
-// core reads from it - the three things that bound such a kernel on single CTAs.
+// Two CTAs of a cluster (one TPC) share every MMA: M = 256 WEIGHT rows, 128 in each CTA's tensor memory, N = up to 256 activation rows, half
+// of them in each CTA's shared memory. The unpacked weights go from registers to tensor memory, where the MMA reads its A operand, so that
+// shared memory carries the activations alone (with weights unpacked into shared memory its writes and operand reads bound this kernel).
 //
-// Roles per CTA (20 warps, placed by SM sub-partition = warp id % 4): warp 0 TMA producer (activation box -> the
-// LEADER's barrier with the pair form of the tensor load; packed-weight box -> a local barrier), warp 4 TMEM owner
-// (+ MMA issuer in the leader); warps 8, 1, 2, 3 epilogue (tcgen05.ld -> global); the twelve warps >= 5 outside
-// sub-partition 0 dequantise in three groups of four: group g takes the stages with stage % 3 == g, one weight row
-// per thread, so three stages are always in flight (one group per stage could not keep up with the MMAs).
-// Activation and dequantised tiles share a 6-stage ring of 64 k with one "consumed" barrier per CTA (two
-// tcgen05.commit per stage); packed weights arrive 256 k at a time as 128-byte swizzled rows (2 slots) - 32-byte
-// rows cost four times the TMA requests and starved the pipeline. Group scales are prefetched four stages ahead
-// into registers (an L2 hit takes longer than a stage).
-// In glu mode the leader dequantises the gate rows and the peer the up rows of the same 128 output columns, so the
-// epilogue finds g in accumulator columns [0, BN/2) and u in [BN/2, BN) of its own TMEM.
-// BN is 256 unless the problem is narrower (a multiple of 32, or 64 for glu).
+// Roles per CTA (28 warps): warp 0 packed weights by TMA (256 k a stage), warp 2 activations (128 k a pass, completion counted on the LEADER's
+// barrier), warp 1 tensor memory and, in the leader, the MMAs (one commit a pass to each CTA); four sets of four warps unpack, a thread per
+// weight row, each set a pass in four; eight warps drain the one accumulator, half of its columns each (the unpacking of the next tile's first
+// four passes lies under it).
+// bf16 results pass through 64 KB of shared memory, so that the accumulator is free as soon as it is read (about 1200 cycles): with SwiGLU and 2-byte
+// stores between its read and its release 4096 tokens of eight experts took 3220 us a layer, now 2733 (2992 with the weights through shared memory).
+// In glu mode lanes 0-63 of a CTA hold gate rows and lanes 64-127 the same up rows; they meet where the results pass through shared memory.
+// The activation rows of a plain tile are chosen so that the tiles fill whole waves of pairs (choose_bn).
 //
-// A packed word is unpacked through its bytes (two masks, two byte interleavings, four byte permutations that set 0x43 beside
-// each nibble, four exact subtractions, four products): 17 instructions per eight weights; one multiplication per byte to spread
-// its nibbles took 24. With that and the roles in one elected lane 2048 x 14336 x 4096 went from 238 to 223 us in a stream.
-//
-// Remote mbarrier arrives use the default semantics: an explicit cluster-scope release made every arrive wait for
-// a cluster-wide fence (~2000 cycles each, measured).
+// What bounds it: at 2048 and more rows of wide projections the power cap (cuBLAS sustains 1.40 PFLOP/s there, this 1.37); below, the MMAs (1024
+// cycles a pass; unpacking takes 830 to 1500, four passes at once) and the last wave. Measured, us in a stream, with the weights unpacked into shared
+// memory / into tensor memory: 2048 x 4096 -> 14336 187 / 175, 1024 x 4096 -> 14336 152 / 94, 512 x 4096 -> 14336 90 / 51, 2048 x 4096 -> 4096 89 / 53,
+// 2048 x 3072 -> 2658 118 / 30, 4096 x 4096 -> 14336 394 / 364.
 //
 // Every wait is clock-bounded; on expiry the CTA raises a status word, drains and frees its TMEM. No multicast.
 //
@@ -47,41 +39,28 @@ namespace {
 
 using namespace tc;
 
-constexpr int BM = 128;  // activation rows per CTA (256 per pair)
-constexpr int BK = 64;   // bf16 elements per stage row (128 bytes)
-constexpr int UMMA_K = 16;
-constexpr int MAX_BN = 256;
-constexpr int STAGES = 6;  // activation and dequantised tiles share one ring index and one 'consumed' barrier
-constexpr int A_STAGES = STAGES, B_STAGES = STAGES, RAW_STAGES = 2, RAW_AHEAD = 1;
-constexpr int RAW_KB = 4;  // k-blocks per packed-weight load: 128-byte rows, a quarter of the TMA requests of 32-byte rows
-constexpr int A_BYTES = BM * BK * 2;                 // 16 KB
-constexpr int B_BYTES = (MAX_BN / 2) * BK * 2;       // 16 KB: this CTA's half of the dequantised tile
-constexpr int RAW_BYTES = (MAX_BN / 2) * RAW_KB * (BK / 2);  // 16 KB: 128 rows x 128 bytes (256 k), 128-byte swizzle
-constexpr int B_RING = 0, A_RING = B_STAGES * B_BYTES, RAW_RING = A_RING + A_STAGES * A_BYTES;
-constexpr int RING_BYTES = RAW_RING + RAW_STAGES * RAW_BYTES;
-constexpr int DEQ_GROUPS = 3, DEQ_GROUP_WARPS = 4;
-// Warp roles are laid out by scheduler (warp id % 4 selects the SM sub-partition): the two single-thread roles that
-// pace the pipeline, TMA (warp 0) and MMA (warp 4), share sub-partition 0 with only one epilogue warp, so the
-// instruction-heavy dequantisation warps (sub-partitions 1-3) never compete with them for issue slots.
-constexpr int TMA_WARP = 0, MMA_WARP = 4;
-constexpr int NUM_WARPS = 20;
-constexpr int THREADS = NUM_WARPS * 32;
-// epilogue: warps 8 (TMEM lanes 0-31), 1, 2, 3; dequant: the twelve warps >= 5 off sub-partition 0; warps 12, 16 idle
-__device__ __forceinline__ bool is_epilogue_warp(int w) { return w == 8 || (w >= 1 && w <= 3); }
-__device__ __forceinline__ int dequant_index(int w) {  // 0..11, or -1
-    if ((w & 3) == 0 || w < 5) return -1;
-    return (w - 5) - ((w - 4) >> 2);  // skip the warps of sub-partition 0 (8, 12, 16)
-}
-constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
+constexpr int BM = 128;        // weight rows per CTA (256 per pair)
+constexpr int MAX_BN = 256;    // activation rows per pair
+constexpr int PASS = 128, KB = 256, UMMA_K = 16;
+constexpr int RAW_STAGES = 4, X_STAGES = 3, SLOTS = 4, DONE = 8;
+constexpr int RAW_BYTES = BM * KB / 2;               // 16 KB: two boxes of 64 rows, 128-byte swizzle
+constexpr int X_BYTES = (MAX_BN / 2) * PASS * 2;     // 32 KB: this CTA's half, two boxes of 64 k
+constexpr int X_RING = RAW_STAGES * RAW_BYTES, OUT = X_RING + X_STAGES * X_BYTES;
+constexpr int OUT_BYTES = MAX_BN * BM * 2;           // 64 KB: a tile's sums as bf16 [activation row][weight row]
+constexpr int RING_BYTES = OUT + OUT_BYTES;
+constexpr int UNPACK_WARP = 4, EPI_WARP = 20, EPI_WARPS = 8, THREADS = (EPI_WARP + EPI_WARPS) * 32, MMA_WARP = 1;
+constexpr int TMEM_COLS = 512, A_COL = MAX_BN;       // the accumulator, then four slots of 64 columns
+constexpr int SMEM_BYTES = RING_BYTES + 1024 + 1024;
+static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 
 struct Bars {
-    unsigned long long a_full[STAGES], b_full[STAGES], empty[STAGES], raw_full[RAW_STAGES], raw_empty[RAW_STAGES];
-    unsigned long long acc_full[2], acc_empty[2], drained;
+    unsigned long long raw_full[RAW_STAGES], raw_empty[RAW_STAGES], a_full[X_STAGES], b_full[SLOTS], done[DONE];
+    unsigned long long acc_full, acc_empty, dumped, stored, drained;
     uint32_t tmem_base;
     unsigned int abort_flag;
-    uint32_t a_issued, raw_issued;  // copies of the TMA role
+    uint32_t a_issued, raw_issued;  // copies of the TMA roles
 };
+static_assert(sizeof(Bars) <= 1024, "control block");
 
 struct Params {
     const uint16_t* scales;     // bf16 [weight rows][K / group]
@@ -90,12 +69,13 @@ struct Params {
     const uint32_t* tile_expert;  // optional: expert of each 256-row tile
     uint32_t* status;
     uint32_t M, N, K, group;    // M: activation/output rows; N: output columns
-    uint32_t bn;                // accumulator columns per tile
+    uint32_t bn;                // activation rows per tile
     uint32_t m_tiles, n_tiles;
     uint32_t expert_rows;       // weight rows per expert in the stacked weight tensor
     uint32_t glu_stride;        // glu: rows between W1[j] and W3[j] of one expert
     uint32_t ldy;               // output row stride in elements
     uint32_t out_f32;           // plain mode only: store f32 instead of bf16
+    uint32_t group_inv;         // group / 64 > 1: (i * group_inv) >> 32 = i / (group / 64) for the 64-k blocks i of a row; else 0
 };
 
 __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
@@ -103,7 +83,6 @@ __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
     asm("mul.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
-__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 struct TileCoord {
     uint32_t mt, nt, expert;
@@ -116,16 +95,12 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     Bars* bars = reinterpret_cast<Bars*>(tiles + RING_BYTES);
     volatile unsigned int* abort_flag = &bars->abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();  // 0 = leader
     const uint32_t pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const uint32_t m_tiles = p.m_tiles_dev ? min(*p.m_tiles_dev, p.m_tiles) : p.m_tiles;
-    const uint32_t total_tiles = m_tiles * p.n_tiles, k_blocks = p.K / BK;
-    const uint32_t groups = p.K / p.group;
-    const uint32_t half_rows = p.bn >> 1;           // weight rows this CTA dequantises per tile
-    const uint32_t raw_bytes = half_rows * RAW_KB * (BK / 2);
-    const uint32_t raw_blocks = k_blocks / RAW_KB;  // packed-weight loads per tile
-    const uint32_t out_cols = GLU ? half_rows : p.bn;  // output columns per tile
+    const uint32_t total_tiles = m_tiles * p.n_tiles, passes = p.K / PASS, stages = p.K / KB;
+    const uint32_t half_bn = p.bn >> 1;          // activation rows in this CTA's shared memory
 
     auto coord = [&](uint32_t tile) {
         TileCoord c;
@@ -134,38 +109,28 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
         c.expert = p.tile_expert ? p.tile_expert[c.mt] : 0u;
         return c;
     };
-    // first weight row (in the stacked tensor) of this CTA's half of a tile
-    auto weight_row0 = [&](const TileCoord& c) {
-        return GLU ? c.expert * p.expert_rows + rank * p.glu_stride + c.nt * half_rows
-                   : c.expert * p.expert_rows + c.nt * p.bn + rank * half_rows;
-    };
-    // how many of this CTA's weight rows exist (tail tiles in N)
-    auto weight_rows_valid = [&](const TileCoord& c) {
-        const uint32_t first = GLU ? c.nt * half_rows : c.nt * p.bn + rank * half_rows;
-        return first >= p.N ? 0u : min(half_rows, p.N - first);
-    };
+    // first output column of this CTA's weight rows (glu: of its 64 gate and 64 up rows)
+    auto column0 = [&](const TileCoord& c) { return GLU ? c.nt * BM + rank * (BM / 2) : c.nt * 2 * BM + rank * BM; };
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&bars->a_full[s]), 1);                    // leader: one expect_tx arrival, bytes from both CTAs
-            mbar_init(smem_u32(&bars->b_full[s]), 2 * DEQ_GROUP_WARPS);  // leader: dequant warps of both CTAs
-            mbar_init(smem_u32(&bars->empty[s]), 1);                     // one tcgen05.commit per CTA
-        }
         for (int s = 0; s < RAW_STAGES; ++s) {
             mbar_init(smem_u32(&bars->raw_full[s]), 1);
-            mbar_init(smem_u32(&bars->raw_empty[s]), RAW_KB * DEQ_GROUP_WARPS);  // each stage: the four warps of one group
+            mbar_init(smem_u32(&bars->raw_empty[s]), 8);  // the warps of a stage's two passes
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(smem_u32(&bars->acc_full[a]), 1);
-            mbar_init(smem_u32(&bars->acc_empty[a]), 8);  // leader: 4 epilogue warps of each CTA
-        }
+        for (int s = 0; s < X_STAGES; ++s) mbar_init(smem_u32(&bars->a_full[s]), 1);  // leader: one expect_tx arrival, bytes from both CTAs
+        for (int s = 0; s < SLOTS; ++s) mbar_init(smem_u32(&bars->b_full[s]), 8);     // leader: four warps of each CTA
+        for (int s = 0; s < DONE; ++s) mbar_init(smem_u32(&bars->done[s]), 1);        // a commit to each CTA
+        mbar_init(smem_u32(&bars->acc_full), 1);
+        mbar_init(smem_u32(&bars->acc_empty), 2 * EPI_WARPS);  // leader: both CTAs' epilogue warps
+        mbar_init(smem_u32(&bars->dumped), EPI_WARPS);
+        mbar_init(smem_u32(&bars->stored), EPI_WARPS);
         mbar_init(smem_u32(&bars->drained), 1);
         bars->abort_flag = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_x);
         tma_prefetch_desc(&map_w);
     }
-    if (warp == MMA_WARP) {
+    if (warp == uint32_t(MMA_WARP)) {
         tmem_alloc_pair(smem_u32(&bars->tmem_base), TMEM_COLS);
         tmem_relinquish_pair();
     }
@@ -174,87 +139,82 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     cluster_sync();  // both CTAs' barriers exist before any remote arrive, commit or TMA completion can target them
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
+    // passes are numbered through all tiles; nobody is further behind than the eight barriers of completed ones
+    auto done_wait = [&](uint32_t gp) { return mbar_wait(smem_u32(&bars->done[gp % DONE]), (gp / DONE) & 1, abort_flag); };
 
-    const int deq_idx = dequant_index(warp);
-    if (warp == TMA_WARP) {
-        // ------------------------------------ TMA producer ------------------------------------
+    bool ok = true;
+    if (warp == 0) {
+        // ---- packed weights ----
         if (elect_one()) {
-            uint32_t a_it = 0, r_it = 0, r_tile = pair, r_blk = 0;
-            uint32_t as = 0, a_parity = 1;
-            bool ok = true;
+            uint32_t gi = 0;
             for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
                 const TileCoord c = coord(tile);
-                const int m0 = int(c.mt * 2 * BM + rank * BM);
-                for (uint32_t kb = 0; kb < k_blocks; ++kb, ++a_it) {
-                    while (r_tile < total_tiles && r_it <= a_it / RAW_KB + RAW_AHEAD) {
-                        const uint32_t rs = r_it % RAW_STAGES;
-                        if (r_it >= RAW_STAGES && !mbar_wait(smem_u32(&bars->raw_empty[rs]), ((r_it / RAW_STAGES) - 1) & 1, abort_flag)) {
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t bar = smem_u32(&bars->raw_full[rs]);
-                        mbar_arrive_expect_tx(bar, raw_bytes);
-                        tma_load_2d(smem_u32(tiles + RAW_RING + rs * RAW_BYTES), &map_w, int(r_blk * RAW_KB * (BK / 2)),
-                                    int(weight_row0(coord(r_tile))), bar);
-                        ++r_it;
-                        if (++r_blk == raw_blocks) {
-                            r_blk = 0;
-                            r_tile += pairs;
-                        }
-                    }
-                    if (!ok) break;
-                    if (a_it >= A_STAGES && !mbar_wait(smem_u32(&bars->empty[as]), a_parity, abort_flag)) {
+                const int row0 = int(c.expert * p.expert_rows + column0(c)), row1 = row0 + int(GLU ? p.glu_stride : BM / 2);
+                for (uint32_t i = 0; i < stages; ++i, ++gi) {
+                    const uint32_t s = gi % RAW_STAGES, bar = smem_u32(&bars->raw_full[s]), dst = smem_u32(tiles + s * RAW_BYTES);
+                    if (gi >= uint32_t(RAW_STAGES) && !mbar_wait(smem_u32(&bars->raw_empty[s]), ((gi / RAW_STAGES) - 1) & 1, abort_flag)) {
                         ok = false;
                         break;
                     }
-                    // both CTAs' activation boxes count on the leader's barrier; the leader posts the expectation
-                    const uint32_t leader_bar = mapa(smem_u32(&bars->a_full[as]), 0);
-                    if (rank == 0) mbar_arrive_expect_tx(smem_u32(&bars->a_full[as]), 2 * A_BYTES);
-                    tma_load_2d_pair(smem_u32(tiles + A_RING + as * A_BYTES), &map_x, int(kb * BK), m0, leader_bar);
-                    if (++as == uint32_t(A_STAGES)) {
-                        as = 0;
-                        a_parity ^= 1;
-                    }
+                    mbar_arrive_expect_tx(bar, RAW_BYTES);
+                    tma_load_2d(dst, &map_w, int(i * (KB / 2)), row0, bar);
+                    tma_load_2d(dst + RAW_BYTES / 2, &map_w, int(i * (KB / 2)), row1, bar);
                 }
             }
-            bars->raw_issued = r_it;
-            bars->a_issued = a_it;
+            bars->raw_issued = gi;
         }
         __syncwarp();
-    } else if (warp == MMA_WARP) {
-        // ------------------------------------ MMA issuer (leader CTA only) ------------------------------------
+    } else if (warp == 2) {
+        // ---- activations: both CTAs' boxes count on the leader's barrier; the leader posts the expectation ----
+        if (elect_one()) {
+            uint32_t gp = 0;
+            for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs) {
+                const int m0 = int((tile % m_tiles) * p.bn + rank * half_bn);
+                for (uint32_t i = 0; i < passes; ++i, ++gp) {
+                    const uint32_t s = gp % X_STAGES, dst = smem_u32(tiles + X_RING + s * X_BYTES);
+                    if (gp >= uint32_t(X_STAGES) && !done_wait(gp - X_STAGES)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t leader_bar = mapa(smem_u32(&bars->a_full[s]), 0);
+                    if (rank == 0) mbar_arrive_expect_tx(smem_u32(&bars->a_full[s]), 2 * half_bn * PASS * 2);
+#pragma unroll
+                    for (int j = 0; j < PASS / 64; ++j) tma_load_2d_pair(dst + j * half_bn * 128, &map_x, int(i * PASS + j * 64), m0, leader_bar);
+                }
+            }
+            bars->a_issued = gp;
+        }
+        __syncwarp();
+    } else if (warp == uint32_t(MMA_WARP)) {
+        // ---- MMA issuer (leader CTA only) ----
         if (rank == 0 && elect_one()) {
             const uint32_t idesc = idesc_bf16_f32(2 * BM, p.bn);
-            uint32_t s = 0, parity = 0, local = 0;
-            bool ok = true;
+            uint32_t gp = 0, local = 0, xs = 0, x_parity = 0;
             for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
-                const uint32_t acc = local & 1;
-                if (local >= 2 && !mbar_wait(smem_u32(&bars->acc_empty[acc]), ((local >> 1) - 1) & 1, abort_flag)) break;
-                tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * MAX_BN;
-                for (uint32_t kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait2(smem_u32(&bars->a_full[s]), parity, smem_u32(&bars->b_full[s]), parity, abort_flag)) {
+                if (local >= 1 && !mbar_wait(smem_u32(&bars->acc_empty), (local - 1) & 1, abort_flag)) break;
+                for (uint32_t i = 0; i < passes; ++i, ++gp) {
+                    const uint32_t s = gp % SLOTS, parity = (gp / SLOTS) & 1;
+                    if (!mbar_wait2(smem_u32(&bars->a_full[xs]), x_parity, smem_u32(&bars->b_full[s]), parity, abort_flag)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t da = smem_desc_sw128(smem_u32(tiles + A_RING + s * A_BYTES));
-                    const uint64_t db = smem_desc_sw128(smem_u32(tiles + B_RING + s * B_BYTES));
+                    const uint32_t a = tmem_base + A_COL + s * 64, b = smem_u32(tiles + X_RING + xs * X_BYTES);
+                    const uint64_t db0 = smem_desc_sw128(b), db1 = smem_desc_sw128(b + half_bn * 128);
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k)
-                        mma_f16_pair(d_tmem, smem_desc_advance(da, k * UMMA_K * 2), smem_desc_advance(db, k * UMMA_K * 2),
-                                     idesc, (kb | uint32_t(k)) != 0);
-                    // free the stage in both CTAs
-                    const uint32_t em = smem_u32(&bars->empty[s]);
-                    tc_commit_pair(em);
-                    tc_commit_pair(mapa(em, 1));
-                    if (++s == uint32_t(STAGES)) {
-                        s = 0;
-                        parity ^= 1;
+                    for (int k = 0; k < PASS / UMMA_K; ++k)
+                        mma_f16_ts_pair(tmem_base, a + k * (UMMA_K / 2), smem_desc_advance(k < 4 ? db0 : db1, (k & 3) * UMMA_K * 2), idesc,
+                                        (i | uint32_t(k)) != 0);
+                    const uint32_t dn = smem_u32(&bars->done[gp % DONE]);
+                    tc_commit_pair(dn);
+                    tc_commit_pair(mapa(dn, 1));
+                    if (++xs == uint32_t(X_STAGES)) {
+                        xs = 0;
+                        x_parity ^= 1;
                     }
                 }
                 if (ok) {
-                    const uint32_t af = smem_u32(&bars->acc_full[acc]);
+                    const uint32_t af = smem_u32(&bars->acc_full);
                     tc_commit_pair(af);
                     tc_commit_pair(mapa(af, 1));
                 }
@@ -265,147 +225,144 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             }
         }
         __syncwarp();
-    } else if (is_epilogue_warp(warp)) {
-        // ------------------------------------ epilogue warps ------------------------------------
-        const uint32_t quad = warp & 3;  // TMEM lane quarter this warp may read
-        uint32_t local = 0;
-        bool ok = true;
-        for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
-            const uint32_t acc = local & 1;
+    } else if (warp >= uint32_t(UNPACK_WARP) && warp < uint32_t(EPI_WARP)) {
+        // ---- unpack: a thread per weight row, every fourth pass ----
+        const uint32_t unit = (warp - UNPACK_WARP) >> 2, quad = warp & 3, r = quad * 32 + lane, half = unit & 1;
+        const uint32_t groups = p.K / p.group, dst = tmem_base + ((quad * 32) << 16) + A_COL + unit * 64;
+        const uint32_t ready = mapa(smem_u32(&bars->b_full[unit]), 0);
+        uint32_t tile = pair, pass = unit;
+        const uint16_t* srow = nullptr;
+        bool valid = false;
+        auto settle_tile = [&]() {  // the tile that `pass` falls into, and this row's scales
+            bool moved = srow == nullptr;
+            while (pass >= passes && tile < total_tiles) {
+                pass -= passes;
+                tile += pairs;
+                moved = true;
+            }
+            if (!moved || tile >= total_tiles) return;
             const TileCoord c = coord(tile);
-            ok = mbar_wait(smem_u32(&bars->acc_full[acc]), (local >> 1) & 1, abort_flag);
+            const uint32_t col = column0(c) + (GLU ? r % (BM / 2) : r);
+            valid = col < p.N;
+            srow = p.scales + size_t(c.expert * p.expert_rows + (valid ? col : 0u) + (GLU && r >= BM / 2 ? p.glu_stride : 0u)) * groups;
+        };
+        auto scale = [&](uint32_t b) {
+            const uint32_t at = pass * 2 + b;
+            return valid ? uint32_t(__ldg(srow + (p.group_inv ? __umulhi(at, p.group_inv) : at))) * 0x10001u : 0u;
+        };
+        settle_tile();
+        bool more = tile < total_tiles;
+        uint32_t s0 = more ? scale(0) : 0, s1 = more ? scale(1) : 0;
+#pragma unroll 1
+        for (uint32_t gp = unit; more; gp += 4) {
+            const uint32_t c0 = s0, c1 = s1, gi = gp >> 1, s = gi % RAW_STAGES;
+            pass += 4;
+            settle_tile();
+            more = tile < total_tiles;
+            if (more) {
+                s0 = scale(0);
+                s1 = scale(1);
+            }
+            ok = mbar_wait(smem_u32(&bars->raw_full[s]), (gi / RAW_STAGES) & 1, abort_flag);
+            if (gp >= uint32_t(SLOTS)) ok = ok && done_wait(gp - SLOTS);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t row = c.mt * 2 * BM + rank * BM + quad * 32 + lane;
-            const uint32_t taddr = tmem_base + ((quad * 32) << 16) + acc * MAX_BN;
-            const uint32_t n0 = c.nt * out_cols;
-            for (uint32_t cc = 0; cc < out_cols / 32; ++cc) {
-                uint32_t r[32];
-                tmem_ld_32x32(taddr + cc * 32, r);
-                if constexpr (GLU) {
-                    uint32_t ru[32];
-                    tmem_ld_32x32(taddr + half_rows + cc * 32, ru);
-                    tmem_ld_wait();
+            const uint8_t* row = tiles + s * RAW_BYTES + r * 128;
+            uint4 v[4];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        // same rounding points as the single-token reference ops: g and u are bf16 values, the
-                        // activation is evaluated in f32 as g * (u * (1 / (1 + exp(-g)))) and stored as bf16
-                        const float g = bf16_round(__uint_as_float(r[j])), u = bf16_round(__uint_as_float(ru[j]));
-                        const float sig = 1.0f / (1.0f + expf(-g));
-                        r[j] = __float_as_uint(g * (u * sig));
-                    }
-                } else {
-                    tmem_ld_wait();
+            for (uint32_t j = 0; j < 4; ++j) v[j] = lds_128(row + (((half * 4 + j) ^ (r & 7u)) << 4));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                uint32_t a[16];
+                const uint32_t words[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    uint32_t q[4];
+                    unpack_int4_bf16(words[u], q);  // exact q - 8, natural order; one rounding of the product
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a[4 * u + e] = bf16x2_mul(q[e], j < 2 ? c0 : c1);
                 }
-                const uint32_t col0 = n0 + cc * 32;
-                if (row < p.M && col0 < p.N) {
-                    const bool f32_out = !GLU && p.out_f32 != 0;
-                    if (f32_out) {
-                        float* dst = static_cast<float*>(p.y) + size_t(row) * p.ldy + col0;
-                        if (col0 + 32 <= p.N && (p.ldy & 3u) == 0) {
+                tmem_st_32x16(dst + j * 16, a);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[s]));  // the packed bytes have been used
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(ready);
+        }
+    } else if (warp >= uint32_t(EPI_WARP)) {
+        // ---- epilogue: a thread per weight row (output column), 16 activation rows at a time. bf16 results go to shared memory first: the accumulator
+        // is free after 1200 cycles, and rounding points, SwiGLU and 128- or 256-byte stores lie under the next tile's MMAs ----
+        const uint32_t quad = warp & 3, ew = warp - EPI_WARP, set = ew >> 2, taddr = tmem_base + ((quad * 32) << 16);
+        const uint32_t chunks = p.bn / 16, first = set * (chunks / 2), last = first + chunks / 2;
+        const uint32_t empty = mapa(smem_u32(&bars->acc_empty), 0), dumped = smem_u32(&bars->dumped), stored = smem_u32(&bars->stored);
+        const bool staged = GLU || p.out_f32 == 0;
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(tiles + OUT);
+        uint32_t local = 0;
+        for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, ++local) {
+            const uint32_t mt = tile % m_tiles, m0 = mt * p.bn;
+            const TileCoord c{mt, tile / m_tiles, 0};
+            ok = mbar_wait(smem_u32(&bars->acc_full), local & 1, abort_flag);
+            if (staged && local >= 1) ok = ok && mbar_wait(stored, (local - 1) & 1, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t col = column0(c) + quad * 32 + lane;
+            for (uint32_t cc = first; cc < last; ++cc) {
+                uint32_t v[16];
+                tmem_ld_32x16(taddr + cc * 16, v);
+                tmem_ld_wait();
+                if (staged) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                reinterpret_cast<uint4*>(dst)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-                        } else {
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < p.N) dst[j] = __uint_as_float(r[j]);
-                        }
-                    } else {
-                        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.y) + size_t(row) * p.ldy + col0;
-                        if (col0 + 32 <= p.N && (p.ldy & 7u) == 0) {
+                    for (int j = 0; j < 16; ++j) out[(cc * 16 + j) * BM + quad * 32 + lane] = __float2bfloat16_rn(__uint_as_float(v[j]));
+                } else if (col < p.N) {
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                uint32_t pk[4];
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-                                    const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[8 * j + 2 * q]),
-                                                                                   __uint_as_float(r[8 * j + 2 * q + 1]));
-                                    pk[q] = *reinterpret_cast<const uint32_t*>(&h);
-                                }
-                                reinterpret_cast<uint4*>(dst)[j] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                            }
-                        } else {
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < p.N) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
-                        }
-                    }
+                    for (int j = 0; j < 16; ++j)
+                        if (m0 + cc * 16 + j < p.M) static_cast<float*>(p.y)[size_t(m0 + cc * 16 + j) * p.ldy + col] = __uint_as_float(v[j]);
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&bars->acc_empty[acc]), 0));
-        }
-    } else if (deq_idx >= 0) {
-        // ------------------------------------ dequant warps ------------------------------------
-        const uint32_t dgroup = uint32_t(deq_idx) / DEQ_GROUP_WARPS;  // takes the stages with stage % DEQ_GROUPS == dgroup
-        const uint32_t r = (uint32_t(deq_idx) % DEQ_GROUP_WARPS) * 32 + lane;  // weight row of this thread
-        const uint32_t gdiv = p.group / BK;            // stages per scale group
-        uint32_t it_base = 0, raw_base = 0;
-        bool ok = true;
-        for (uint32_t tile = pair; tile < total_tiles && ok; tile += pairs, raw_base += raw_blocks, it_base += k_blocks) {
-            const TileCoord c = coord(tile);
-            const bool row_valid = r < weight_rows_valid(c);
-            const uint16_t* srow = p.scales + size_t(row_valid ? weight_row0(c) + r : 0) * groups;
-            // Each stage needs one group scale per row. The loads run four of this warp's stages ahead (a queue of
-            // four registers): one stage ahead is not enough, an L2 hit costs more than a stage takes.
-            // this group's stages of the tile: global stage numbers congruent to dgroup modulo DEQ_GROUPS
-            const uint32_t kb_first = (dgroup + DEQ_GROUPS - it_base % DEQ_GROUPS) % DEQ_GROUPS;
-            const uint32_t n_own = kb_first < k_blocks ? (k_blocks - kb_first + DEQ_GROUPS - 1) / DEQ_GROUPS : 0u;
-            uint32_t q[4];
+            if (lane == 0) mbar_arrive_cluster(empty);
+            if (!staged) continue;
+            if (lane == 0) mbar_arrive(dumped);
+            ok = mbar_wait(dumped, local & 1, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            __nv_bfloat16* y = static_cast<__nv_bfloat16*>(p.y);
+            for (uint32_t t = ew; t < p.bn && m0 + t < p.M; t += EPI_WARPS) {
+                const size_t row = size_t(m0 + t) * p.ldy;
+                if constexpr (GLU) {  // a lane: two neighbouring outputs
+                    const uint32_t j = column0(c) + 2 * lane;
+                    const __nv_bfloat162 g2 = *reinterpret_cast<const __nv_bfloat162*>(out + t * BM + 2 * lane);
+                    const __nv_bfloat162 u2 = *reinterpret_cast<const __nv_bfloat162*>(out + t * BM + BM / 2 + 2 * lane);
+                    // same rounding points as the single-token reference ops: g and u are bf16 values, the
+                    // activation is evaluated in f32 as g * (u * (1 / (1 + exp(-g)))) and stored as bf16
+                    const float g0 = __low2float(g2), g1 = __high2float(g2);
+                    const float h0 = g0 * (__low2float(u2) * (1.0f / (1.0f + expf(-g0)))), h1 = g1 * (__high2float(u2) * (1.0f / (1.0f + expf(-g1))));
+                    if (j + 1 < p.N && (p.ldy & 1u) == 0) {
+                        *reinterpret_cast<__nv_bfloat162*>(y + row + j) = __floats2bfloat162_rn(h0, h1);
+                    } else {
+                        if (j < p.N) y[row + j] = __float2bfloat16_rn(h0);
+                        if (j + 1 < p.N) y[row + j + 1] = __float2bfloat16_rn(h1);
+                    }
+                } else {  // four
+                    const uint32_t j = column0(c) + 4 * lane;
+                    const uint2 v = *reinterpret_cast<const uint2*>(out + t * BM + 4 * lane);
+                    if (j + 3 < p.N && (p.ldy & 3u) == 0) {
+                        *reinterpret_cast<uint2*>(y + row + j) = v;
+                    } else {
+                        const uint32_t e[4] = {v.x & 0xFFFFu, v.x >> 16, v.y & 0xFFFFu, v.y >> 16};
 #pragma unroll
-            for (uint32_t d = 0; d < 4; ++d)
-                q[d] = (row_valid && d < n_own) ? uint32_t(srow[(kb_first + DEQ_GROUPS * d) / gdiv]) : 0u;
-            for (uint32_t j0 = 0; j0 < n_own && ok; j0 += 4) {
-#pragma unroll
-              for (uint32_t u = 0; u < 4; ++u) {
-                const uint32_t j = j0 + u;
-                if (j >= n_own || !ok) break;
-                const uint32_t kb = DEQ_GROUPS * j + kb_first, it = it_base + kb;
-                const uint32_t r_it = raw_base + kb / RAW_KB, rs = r_it % RAW_STAGES, bs = it % B_STAGES;
-                const uint32_t sv = q[u];
-                const uint32_t s2 = sv | (sv << 16);  // this stage's group scale in both bf16 halves
-                if (row_valid && j + 4 < n_own) q[u] = uint32_t(srow[(kb + 4 * DEQ_GROUPS) / gdiv]);
-                ok = mbar_wait(smem_u32(&bars->raw_full[rs]), (r_it / RAW_STAGES) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                // the packed slot holds 128-byte rows (4 k-blocks) with the 128-byte swizzle: 16-byte chunk c of row r
-                // sits at chunk c ^ (r & 7), which also keeps a quarter warp's reads in distinct bank groups
-                const uint8_t* raw_row = tiles + RAW_RING + rs * RAW_BYTES + r * 128;
-                const uint32_t c0 = (kb % RAW_KB) * 2;
-                uint4 w0 = make_uint4(0, 0, 0, 0), w1 = w0;
-                if (r < half_rows) {
-                    w0 = lds_128(raw_row + ((c0 ^ (r & 7u)) << 4));
-                    w1 = lds_128(raw_row + (((c0 + 1) ^ (r & 7u)) << 4));
+                        for (uint32_t q = 0; q < 4; ++q)
+                            if (j + q < p.N) reinterpret_cast<uint16_t*>(y)[row + j + q] = uint16_t(e[q]);
+                    }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&bars->raw_empty[rs]));  // the packed bytes now live in registers
-                const uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                uint4 o[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const uint32_t w = words[j];
-                    uint32_t q8[4];
-                    unpack_int4_bf16(w, q8);  // exact q - 8, natural order; one rounding of the product
-                    o[j].x = bf16x2_mul(q8[0], s2);
-                    o[j].y = bf16x2_mul(q8[1], s2);
-                    o[j].z = bf16x2_mul(q8[2], s2);
-                    o[j].w = bf16x2_mul(q8[3], s2);
-                }
-                // the dequantised slot must have been consumed by the MMAs of its previous use
-                if (it >= B_STAGES) ok = mbar_wait(smem_u32(&bars->empty[bs]), ((it / B_STAGES) - 1) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                if (r < half_rows) {
-                    uint8_t* brow = tiles + B_RING + bs * B_BYTES + r * 128;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(brow + ((uint32_t(j) ^ (r & 7u)) << 4)) = o[j];
-                }
-                fence_proxy_async();  // generic-proxy stores -> visible to the tensor core's operand reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(mapa(smem_u32(&bars->b_full[bs]), 0));
-              }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(stored);
         }
     }
 
@@ -413,11 +370,11 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     __syncthreads();
     if (threadIdx.x == 0 && bars->abort_flag != 0) {
         settle_copies(bars->raw_full, RAW_STAGES, bars->raw_issued);
-        if (rank == 0) settle_copies(bars->a_full, A_STAGES, bars->a_issued);  // the leader's count both CTAs' boxes; the pair leaves together
+        if (rank == 0) settle_copies(bars->a_full, X_STAGES, bars->a_issued);  // the leader's count both CTAs' boxes; the pair leaves together
     }
     __syncwarp();
     cluster_sync();  // the peer may still be reading this CTA's shared memory / TMEM through the pair MMA until here
-    if (warp == MMA_WARP) {
+    if (warp == uint32_t(MMA_WARP)) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, TMEM_COLS);
     }
@@ -427,23 +384,24 @@ int4_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 }  // namespace
 
 bool int4_gemm_pair_supported(uint32_t m, uint32_t n, uint32_t k, uint32_t group) {
-    // 64-k stages must not straddle a scale group; packed weights are fetched 256 k at a time; one CTA pair per
-    // 256 activation rows only pays above 128 rows
+    // 64-k blocks must not straddle a scale group; packed weights are fetched 256 k at a time
     return m > 128 && n >= 1 && k >= 256 && k % 256 == 0 && group >= 64 && group % 64 == 0 && k % group == 0;
 }
 
 namespace {
 
-// accumulator columns per tile
-uint32_t choose_bn(uint32_t n, bool glu) {
-    // 256 accumulator columns amortise the activation operand best (measured: 224-wide tiles are slower even when
-    // they save a tail wave); narrower tiles only when the problem itself is narrow
-    const uint32_t cols = glu ? 2 * n : n;
-    const uint32_t step = glu ? 64 : 32;
-    uint32_t bn = ((cols + step - 1) / step) * step;
-    if (bn < 128) bn = 128;
-    if (bn > 256) bn = 256;
-    return bn;
+// Activation rows of a plain tile: what makes the waves of pairs shortest, a tile's time being its rows and about 24 rows' worth of epilogue
+uint32_t choose_bn(uint32_t m, uint32_t n_tiles, uint32_t pairs) {
+    uint32_t best = MAX_BN;
+    uint64_t cost = ~0ull;
+    for (uint32_t bn = MAX_BN; bn >= 128; bn -= 32) {
+        const uint64_t t = uint64_t((m + bn - 1) / bn) * n_tiles, c = (t + pairs - 1) / pairs * (bn + 24);
+        if (c < cost) {
+            cost = c;
+            best = bn;
+        }
+    }
+    return best;
 }
 
 }  // namespace
@@ -468,15 +426,10 @@ cudaError_t launch_int4_gemm_pair(const void* x_bf16, const void* w_packed, cons
     const uint32_t pairs_avail = uint32_t(sm_count) / 2;
     if (pairs_avail == 0) return cudaErrorInvalidConfiguration;
     Params p{};
-    p.m_tiles = (m + 2 * BM - 1) / (2 * BM);
-    p.bn = choose_bn(n, glu != 0);
-    // Few tiles (a decode-sized batch, or one expert's rows on an expert-parallel rank): with 256-wide tiles a handful of
-    // tiles beyond one wave of CTA pairs costs a whole second wave (5 row tiles x 16 column tiles = 80 tiles on 74 pairs
-    // is two waves). 128-wide tiles halve that granularity; they amortise the activation operand less well, which only
-    // matters once there are many waves.
-    if (!glu && p.bn == 256 && uint64_t(p.m_tiles) * ((n + 255) / 256) < 4ull * pairs_avail) p.bn = 128;
-    const uint32_t cols = glu ? p.bn / 2 : p.bn;
+    const uint32_t cols = glu ? BM : 2 * BM;
     p.n_tiles = (n + cols - 1) / cols;
+    p.bn = tile_expert || glu ? uint32_t(MAX_BN) : choose_bn(m, p.n_tiles, pairs_avail);  // grouped: the segments' 256-row tiles
+    p.m_tiles = (m + p.bn - 1) / p.bn;
     p.scales = static_cast<const uint16_t*>(scale_bf16);
     p.y = y;
     p.m_tiles_dev = m_tiles_dev;
@@ -490,13 +443,15 @@ cudaError_t launch_int4_gemm_pair(const void* x_bf16, const void* w_packed, cons
     p.glu_stride = n;
     p.ldy = ldy;
     p.out_f32 = out_f32;
+    const uint32_t per = group / 64;
+    p.group_inv = per > 1 ? uint32_t((0x100000000ull + per - 1) / per) : 0u;
     const uint64_t weight_rows = uint64_t(experts) * p.expert_rows;
     CUtensorMap mx, mw;
-    if (!encode_tensor_map_2d(&mx, x_bf16, m, k, 2, BM, BK, true) ||
-        !encode_tensor_map_2d(&mw, w_packed, weight_rows, k / 2, 1, p.bn / 2, RAW_KB * (BK / 2), true))
+    if (!encode_tensor_map_2d(&mx, x_bf16, m, k, 2, p.bn / 2, 64, true) ||
+        !encode_tensor_map_2d(&mw, w_packed, weight_rows, k / 2, 1, BM / 2, KB / 2, true))
         return cudaErrorInvalidValue;
-    const uint32_t tiles = p.m_tiles * p.n_tiles;
-    const uint32_t pairs = tiles < pairs_avail ? tiles : pairs_avail;
+    const uint64_t tiles = uint64_t(p.m_tiles) * p.n_tiles;
+    const uint32_t pairs = tiles < pairs_avail ? uint32_t(tiles) : pairs_avail;
 
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * pairs);
@@ -518,4 +473,3 @@ cudaError_t launch_int4_gemm_pair(const void* x_bf16, const void* w_packed, cons
 }
 
 }  // namespace vybk
-

@@ -467,11 +467,10 @@ cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const
 
 cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
                                 uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
-    // The CTA-pair GEMM (256-row tiles, half of the dequantisation per SM) from 129 rows on, except where this kernel's 128 x 128 tiles fit
-    // the SMs at once or rows are long (pair / this, us: 160 x 4096 -> 4096 25 / 14, 512 x 7168 -> 1024 40 / 14, 1024 x 4096 -> 14336 153 / 126,
-    // but 256 x 1024 -> 14336 18 / 23 and 1024 x 2048 -> 8192 49 / 60; beyond 1024 rows not measured).
+    // The CTA-pair GEMM from 129 rows on, except where tiles are so few that this kernel splits the k range over idle SMs (pair / this, us:
+    // 256 x 4096 -> 4096 18.1 / 16.0, 256 x 3072 -> 2658 14.7 / 11.9; 256 x 3072 -> 8192 16.1 / 18.6, 512 x 3072 -> 2658 15.5 / 18.2)
     const uint64_t items = uint64_t((n + 127) / 128) * ((m + 127) / 128);
-    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > uint64_t(sm_count) && (k < 3072 || m > 1024))
+    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > uint64_t(sm_count) / 2)
         return launch_int4_gemm_pair(x_bf16, w_packed, scale_bf16, y, m, n, k, group, out_f32, 0, 1, nullptr, nullptr, n, sm_count, stream, status);
     if (m > 65535u * 128u) return cudaErrorInvalidValue;
     Params p = make_params(scale_bf16, y, m, n, k, group, status);
