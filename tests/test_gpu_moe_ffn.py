@@ -120,6 +120,12 @@ def test_moe_ffn_few_rows_form_with_many_chunks(tokens, experts, topk, crowded):
     test_moe_ffn_few_rows_per_expert(tokens, 512, 256, experts, topk, 128, crowded)
 
 
+# either side of the line between the few-rows and the pair form (96 rows per expert; 96 pair tiles, which fill the device)
+@pytest.mark.parametrize("tokens", [384, 388])
+def test_moe_ffn_at_the_line_between_the_forms(tokens):
+    test_moe_ffn_few_rows_per_expert(tokens, 256, 768, 16, 4, 128, False)
+
+
 # several items per CTA of the few-rows GEMMs (the accumulator sets and every ring wrap and flip their parity: 8 and 32 stages an item), narrow and wide
 @pytest.mark.parametrize("tokens,experts", [(60, 8), (128, 8)])
 def test_moe_ffn_few_rows_many_items_per_cta(tokens, experts):

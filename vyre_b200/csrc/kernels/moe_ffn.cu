@@ -26,7 +26,8 @@ namespace vybk {
 namespace {
 
 constexpr uint32_t ROW_TILE = 256;       // rows per CTA-pair tile of the grouped GEMM
-constexpr uint32_t SKINNY_ROWS = 128;    // average rows per expert up to which the skinny expert GEMMs run
+constexpr uint32_t SKINNY_ROWS = 96;     // average rows per expert up to which the skinny expert GEMMs run
+constexpr uint32_t SKINNY_ROWS_FEW = 128;  // and where the pair GEMM's tiles would not fill the device
 constexpr uint32_t MAX_EXPERTS = 64;
 constexpr uint32_t MAX_TOPK = 8;
 constexpr uint32_t PAD_TOKEN = 0xFFFFFFFFu;
@@ -382,13 +383,17 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
     if (e != cudaSuccess) return e;
     e = launch_dependent(moe_plan_kernel, dim3(1), dim3(1024), 0, stream, routing_idx, plan, pos, row_token, tokens, experts, topk, L.max_rows);
     if (e != cudaSuccess) return e;
-    const bool skinny = uint64_t(tokens) * topk <= uint64_t(experts) * SKINNY_ROWS;
+    const uint64_t rows = uint64_t(tokens) * topk;
+    const bool skinny = rows <= uint64_t(experts) * SKINNY_ROWS ||
+                        (rows <= uint64_t(experts) * SKINNY_ROWS_FEW && uint64_t(experts) * ((inter + 127) / 128) < uint64_t(sm_count) / 2);
     e = launch_dependent(moe_gather_kernel, dim3(sm_count * 4), dim3(256), 0, stream, static_cast<const uint16_t*>(x_bf16), row_token, plan, xg, hidden,
                          experts, skinny);
     if (e != cudaSuccess) return e;
-    // Few rows per expert: weight rows on the M side, unpacked into tensor memory (8 experts, 4096 / 14336, top-2: 270 against
-    // 784 us at 64 tokens, 644 against 795 us at 512 = 128 rows per expert; at 192 rows both take about 700 us: the pair GEMM's 256-row
-    // tiles are filled there). The line is the average, which the host knows: with all tokens on one or two experts this form can be
+    // Few rows per expert: weight rows on the M side of single CTAs, 32 or 64 activation rows a chunk. This / the pair GEMM, us a layer, at 64, 96, 112
+    // and 128 rows per expert: 8 experts of 4096 / 14336 401 / 464, 490 / 475, 492 / 490, 628 / 497; 16 of 2048 / 4096 173 / 198, 190 / 215, 205 / 210,
+    // 240 / 211; 16 of 3328 / 2816 190 / 221, 234 / 240, 256 / 243, 274 / 248; 32 of 2048 / 2048 180 / 228, 227 / 234, 244 / 239, 275 / 245; four of
+    // 1280 / 1536, whose 48 pair tiles leave 26 of 74 pairs idle, 51 / 65 at all four.
+    // The line is the average, which the host knows: with all tokens on one or two experts this form can be
     // slower than the pair GEMM (wide: 512 tokens on two of 8 experts 500 against 449 us; narrow: 160 tokens on two of 16 experts, 4096 / 4096,
     // 160 against 130 us, balanced 193 against 459). A choice by the plan kernel, both forms launched and one returning at once,
     // cost every balanced layer 9 us (3 to 10 %); 64 columns from 129 tokens on whatever the average, 1 to 7 %.
