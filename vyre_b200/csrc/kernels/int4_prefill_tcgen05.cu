@@ -472,7 +472,17 @@ cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const 
     const uint64_t items = uint64_t((n + 127) / 128) * ((m + 127) / 128);
     if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > uint64_t(sm_count) / 2)
         return launch_int4_gemm_pair(x_bf16, w_packed, scale_bf16, y, m, n, k, group, out_f32, 0, 1, nullptr, nullptr, n, sm_count, stream, status);
-    if (m > 65535u * 128u) return cudaErrorInvalidValue;
+    // Rows are the grid's y dimension, which ends at 65535 tiles: more rows are further launches
+    constexpr uint32_t MAX_ROWS = 65535u * 128u;
+    if (m > MAX_ROWS) {
+        for (uint64_t r0 = 0; r0 < m; r0 += MAX_ROWS) {
+            const cudaError_t e = launch_int4_prefill(static_cast<const uint16_t*>(x_bf16) + r0 * k, w_packed, scale_bf16,
+                                                      static_cast<uint8_t*>(y) + r0 * n * (out_f32 ? 4 : 2), uint32_t(m - r0 < MAX_ROWS ? m - r0 : MAX_ROWS), n,
+                                                      k, group, out_f32, sm_count, stream, status);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     Params p = make_params(scale_bf16, y, m, n, k, group, status);
     const uint32_t per = group / 64;
     if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
