@@ -73,6 +73,8 @@ struct Bars {
 static_assert(sizeof(Bars) <= CTRL_BYTES, "control block");
 
 struct Params {
+    const uint16_t* x;       // bf16 [m][k] and packed weights [n][k / 8], for by_definition
+    const uint32_t* w;
     const uint16_t* scales;  // bf16 [n][k / group]
     void* y;
     uint32_t* status;
@@ -95,6 +97,30 @@ __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t* out, uint32_t 
     }
 }
 
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.40282347e38f; }  // false for NaN
+
+// One output of exact weights by the definition, as int4_linear_generic_kernel computes it (a lane's words in ascending order, then the lanes
+// as the shuffles add them): a group's sum, or a scale times 64, can leave f32's range where no term does. An output that does not come out
+// finite is computed anew, so that an infinity or NaN stands only where the definition has one. Out of line: next to nothing takes it.
+__device__ __noinline__ float by_definition(const uint16_t* x, const uint32_t* w, const uint16_t* scales, uint32_t k, uint32_t group) {
+    float part[32];
+#pragma unroll 1
+    for (uint32_t lane = 0; lane < 32; ++lane) {
+        float acc = 0.0f;
+#pragma unroll 1
+        for (uint32_t wi = lane; wi < k / 8; wi += 32) {
+            const float s = __uint_as_float(uint32_t(scales[wi * 8 / group]) << 16);
+            for (uint32_t i = 0; i < 8; ++i)
+                acc = fmaf(__uint_as_float(uint32_t(x[wi * 8 + i]) << 16), float(int(w[wi] >> (4 * i) & 15u) - 8) * s, acc);
+        }
+        part[lane] = acc;
+    }
+#pragma unroll 1
+    for (uint32_t o = 16; o > 0; o >>= 1)
+        for (uint32_t lane = 0; lane < o; ++lane) part[lane] += part[lane + o];
+    return part[0];
+}
+
 template <int BN, int G, bool OUT_F32>
 __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
     using C = Cfg<BN, G>;
@@ -112,6 +138,9 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
         const size_t at = size_t(m0 + c) * p.n + row;
         if constexpr (OUT_F32) static_cast<float*>(p.y)[at] = v;
         else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
+    };
+    auto definition = [&](uint32_t c, uint32_t row) {
+        return by_definition(p.x + size_t(m0 + c) * p.k, p.w + size_t(row) * (p.k / 8), p.scales + size_t(row) * p.groups, p.k, p.k / p.groups);
     };
 
     if (threadIdx.x == 0) {
@@ -342,8 +371,14 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
         }
         if (ok) {
             if (p.split == 1) {
+                bool good = true;
 #pragma unroll
-                for (int c = 0; c < BN; ++c) store(c, row, acc[c]);
+                for (int c = 0; c < BN; ++c) {
+                    store(c, row, acc[c]);
+                    good = good && finite(acc[c]);
+                }
+                if (!good && row < p.n)  // this thread's outputs once more
+                    for (uint32_t c = 0; c < BN && m0 + c < p.m; ++c) store(c, row, definition(c, row));
             } else {
                 // the last group sum is complete, so every load and MMA of this CTA is: the stages are free
                 float* partial = reinterpret_cast<float*>(tiles);  // [BN][128]
@@ -367,6 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
 #pragma unroll
             for (uint32_t q = 1; q < MAX_SPLIT; ++q)
                 if (q < p.split) sum += v[q];
+            if (G != 0 && !finite(sum)) sum = definition(c, n0 + o);
             store(c, n0 + o, sum);
         }
         cluster_sync();  // no CTA leaves while another still reads its shared memory
@@ -432,8 +468,10 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     return cudaSuccess;
 }
 
-Params make_params(const void* scale, void* y, uint32_t m, uint32_t n, uint32_t k, uint32_t group, uint32_t* status) {
+Params make_params(const void* x, const void* w, const void* scale, void* y, uint32_t m, uint32_t n, uint32_t k, uint32_t group, uint32_t* status) {
     Params p = {};
+    p.x = static_cast<const uint16_t*>(x);
+    p.w = static_cast<const uint32_t*>(w);
     p.scales = static_cast<const uint16_t*>(scale);
     p.y = y;
     p.status = status;
@@ -460,7 +498,7 @@ bool int4_few_rows_supported(const void* x, const void* w, const void* scale, ui
 
 cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
                                  uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
-    const Params p = make_params(scale_bf16, y, m, n, k, group, status);
+    const Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
     return group == 64 ? launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
 }
@@ -483,7 +521,7 @@ cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const 
         }
         return cudaSuccess;
     }
-    Params p = make_params(scale_bf16, y, m, n, k, group, status);
+    Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
     const uint32_t per = group / 64;
     if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
