@@ -334,11 +334,12 @@ cudaError_t run_int4_linear(vyb_instance* inst, uint32_t variant, const void* x,
         }
         return cudaSuccess;
     }
-    // Up to eight rows of other groups and row lengths. Weights through tensor memory too, whose f32 group sums are as good here (error against
-    // 64-bit sums, generic / that kernel, N(0, 1) and log-normal activations: group 64 7.0 / 6.1e-8 and 1.16 / 1.17e-7 at k 1024, 1.2 / 0.9 and
-    // 2.6 / 1.3e-7 at 6400), except f32 outputs of groups of 128 (0.7 / 0.5 and 1.1 / 1.9e-7 at k 1280). Small calls of up to four rows stay on
-    // the warp-per-row kernel, which has no pipeline to fill (us: 1 x 512 -> 1024 2.7 / 3.5, 1 x 256 -> 4096 3.3 / 2.8, 1 x 1600 -> 64 6.2 / 4.5,
-    // 1 x 4096 -> 8192 58 / 10, 8 x 6400 -> 14336 371 / 21).
+    // Up to eight rows of other groups and row lengths. Weights through tensor memory too, with f32 sums over 64 k at most, whose error against
+    // 64-bit sums is below the warp-per-row kernel's (RMS of the outputs' f32 bits, warp-per-row / that kernel, N(0, 1) activations and ones over four
+    // decades: groups of 64 3.4 / 2.4 and 6.0 / 4.2e-8 at k 64, 7.0 / 6.1 and 9.8 / 7.0e-8 at 1024, 1.2 / 0.9 and 2.0 / 0.9e-7 at 6400; groups of 128 4.3 /
+    // 3.1 and 6.7 / 4.8e-8 at k 128, 7.3 / 6.8 and 10.6 / 7.5e-8 at 1280, 1.2 / 0.9 and 2.1 / 0.9e-7 at 6400; sums over 128 k had 8.1e-8 at k 128). f32
+    // outputs of groups of 128 stay where they were. Small calls of up to four rows stay on the warp-per-row kernel, which has no pipeline to
+    // fill (us: 1 x 512 -> 1024 2.7 / 3.5, 1 x 256 -> 4096 3.3 / 2.8, 1 x 1600 -> 64 6.2 / 4.5, 1 x 4096 -> 8192 58 / 10, 8 x 6400 -> 14336 371 / 21).
     if (batch <= 8 && (!out_f32 || group == 64) && (batch > 4 || k >= 1024 || uint64_t(n) * k >= (1u << 20)) &&
         int4_few_rows_supported(x, w, scale, batch, n, k, group))
         return launch_int4_few_rows(x, w, scale, y, batch, n, k, group, out_f32, inst->dev->prop.multiProcessorCount, s, inst->status_dev);

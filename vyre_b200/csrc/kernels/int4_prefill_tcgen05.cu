@@ -8,7 +8,7 @@
 // A CTA per 128 x BN tile; k is split over a cluster where tiles leave SMs idle (partial tiles meet in distributed shared memory, added
 // in rank order). Per CTA: warp 0 packed weights by TMA (256 k a stage), warp 2 activations, warp 1 MMAs, warp 3 prefetches scales, sixteen
 // warps unpack (two sets of eight take the stages in turn), the last warps drain the sums: exact weights have an accumulator per
-// group, which meets its scale in f32 registers; rounded ones one accumulator for the whole row.
+// group (up to eight rows: per 64 k), which meets its scale in f32 registers; rounded ones one accumulator for the whole row.
 //
 // What bounds it: a chain per stage (unpack 700 to 1500 cycles, MMA thread 400 + 430, waits of about 150 each), 1100 cycles with three unpacked
 // stages in flight, where the logic pipe needs 512 and, at 128 columns, the MMAs 1024. Packed bytes at HBM speed would take 5 us of the
@@ -45,9 +45,9 @@ constexpr int TMEM_COLS = 512;
 constexpr int CTRL_BYTES = 512, ALIGN_SLACK = 1024;
 constexpr uint32_t PREFETCH_STAGES = 24;
 
-// BN: activation rows of a tile. G: scale groups of 128 k (group 128: 1, group 64: 2), an accumulator each and exact weights; 0: rounded
-// weights, one accumulator for the whole row.
-template <int BN, int G>
+// BN: activation rows of a tile. G: exact weights, pairs of scales in a stage (group 128: 1, group 64: 2); 0: rounded weights, one accumulator
+// for the whole row. SETS: accumulators of a stage, one per group or, with twice as many, per half of a group.
+template <int BN, int G, int SETS_>
 struct Cfg {
     static constexpr int X_BYTES = BN * KB * 2;
     // Weights and activations have rings of their own: a stage of weights is free as soon as it is unpacked, one of activations when its MMAs
@@ -55,7 +55,7 @@ struct Cfg {
     static constexpr int STAGES = BN == 16 ? 10 : BN == 32 ? 9 : BN == 64 ? 6 : 5, X_STAGES = BN == 16 ? 6 : BN <= 64 ? 4 : 2;
     static constexpr int RING_BYTES = STAGES * RAW_BYTES + X_STAGES * X_BYTES;
     static constexpr int SMEM_BYTES = RING_BYTES + CTRL_BYTES + ALIGN_SLACK;
-    static constexpr int SETS = G == 0 ? 1 : 2 * G;            // accumulators of a stage
+    static constexpr int SETS = SETS_;
     static constexpr int A_COL = G == 0 ? BN : 2 * SETS * BN;  // accumulators (of two stages) come first
     static constexpr int A_SLOTS = 3;                          // unpacked stages (8 x 4096 -> 14336: 13.4 us with two, 12.1 with three)
     static_assert(A_COL + A_SLOTS * 128 <= TMEM_COLS && X_STAGES <= DONE && STAGES <= 10, "tensor memory, barriers");
@@ -102,7 +102,11 @@ __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.40282347e
 // One output of exact weights by the definition, as int4_linear_generic_kernel computes it (a lane's words in ascending order, then the lanes
 // as the shuffles add them): a group's sum, or a scale times 64, can leave f32's range where no term does. An output that does not come out
 // finite is computed anew, so that an infinity or NaN stands only where the definition has one. Out of line: next to nothing takes it.
-__device__ __noinline__ float by_definition(const uint16_t* x, const uint32_t* w, const uint16_t* scales, uint32_t k, uint32_t group) {
+__device__ __noinline__ float by_definition(const Params& p, uint32_t m, uint32_t n) {
+    const uint16_t* x = p.x + size_t(m) * p.k;
+    const uint32_t* w = p.w + size_t(n) * (p.k / 8);
+    const uint16_t* scales = p.scales + size_t(n) * p.groups;
+    const uint32_t k = p.k, group = k / p.groups;
     float part[32];
 #pragma unroll 1
     for (uint32_t lane = 0; lane < 32; ++lane) {
@@ -121,9 +125,10 @@ __device__ __noinline__ float by_definition(const uint16_t* x, const uint32_t* w
     return part[0];
 }
 
-template <int BN, int G, bool OUT_F32>
-__global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
-    using C = Cfg<BN, G>;
+template <int BN, int G, int SETS, bool OUT_F32>
+__global__ void __launch_bounds__(THREADS, 1)
+int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ Params p) {
+    using C = Cfg<BN, G, SETS>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_tiles = tiles + C::STAGES * RAW_BYTES;
@@ -138,9 +143,6 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
         const size_t at = size_t(m0 + c) * p.n + row;
         if constexpr (OUT_F32) static_cast<float*>(p.y)[at] = v;
         else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
-    };
-    auto definition = [&](uint32_t c, uint32_t row) {
-        return by_definition(p.x + size_t(m0 + c) * p.k, p.w + size_t(row) * (p.k / 8), p.scales + size_t(row) * p.groups, p.k, p.k / p.groups);
     };
 
     if (threadIdx.x == 0) {
@@ -319,7 +321,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
         // ---- epilogue: acc += scale * group sum ----
         waits_for_previous();  // scales
         const uint32_t quad = warp & 3, o = quad * 32 + lane, row = n0 + o;
-        const uint32_t groups = p.groups, g0 = kb0 * C::SETS;
+        const uint32_t groups = p.groups, g0 = kb0 * 2 * G;
         const uint16_t* sp = p.scales + size_t(min(row, p.n - 1)) * groups;
         float acc[BN];
 #pragma unroll
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
         auto load_scales = [&](uint32_t i, uint32_t (&q)[G]) {
 #pragma unroll
             for (int h = 0; h < G; ++h) {  // past the row's last group the activations are zeros
-                const uint32_t g = g0 + i * C::SETS + 2 * h;
+                const uint32_t g = g0 + (i * G + h) * 2;
                 q[h] = (g < groups ? uint32_t(__ldg(sp + g)) : 0u) | (g + 1 < groups ? uint32_t(__ldg(sp + g + 1)) << 16 : 0u);
             }
         };
@@ -355,7 +357,8 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
                 tc_fence_after();
 #pragma unroll
                 for (int h = 0; h < C::SETS; ++h) {
-                    const float s = __uint_as_float(h & 1 ? bits[h / 2] & 0xFFFF0000u : bits[h / 2] << 16) * 64.0f;  // tensor memory holds (q - 8) / 64
+                    const int g = h * 2 * G / C::SETS;
+                    const float s = __uint_as_float(g & 1 ? bits[g / 2] & 0xFFFF0000u : bits[g / 2] << 16) * 64.0f;  // tensor memory holds (q - 8) / 64
                     uint32_t v[BN];
                     tmem_ld_32x16(tmem + ((quad * 32) << 16) + (d * C::SETS + h) * BN, v);
                     tmem_ld_wait();
@@ -378,7 +381,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
                     good = good && finite(acc[c]);
                 }
                 if (!good && row < p.n)  // this thread's outputs once more
-                    for (uint32_t c = 0; c < BN && m0 + c < p.m; ++c) store(c, row, definition(c, row));
+                    for (uint32_t c = 0; c < BN && m0 + c < p.m; ++c) store(c, row, by_definition(p, m0 + c, row));
             } else {
                 // the last group sum is complete, so every load and MMA of this CTA is: the stages are free
                 float* partial = reinterpret_cast<float*>(tiles);  // [BN][128]
@@ -402,7 +405,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
 #pragma unroll
             for (uint32_t q = 1; q < MAX_SPLIT; ++q)
                 if (q < p.split) sum += v[q];
-            if (G != 0 && !finite(sum)) sum = definition(c, n0 + o);
+            if (G != 0 && !finite(sum)) sum = by_definition(p, m0 + c, n0 + o);
             store(c, n0 + o, sum);
         }
         cluster_sync();  // no CTA leaves while another still reads its shared memory
@@ -420,16 +423,16 @@ __global__ void __launch_bounds__(THREADS, 1) int4_tmem_kernel(const __grid_cons
     }
 }
 
-template <int BN, int G, bool OUT_F32>
+template <int BN, int G, int SETS, bool OUT_F32>
 cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cudaStream_t stream) {
-    using C = Cfg<BN, G>;
+    using C = Cfg<BN, G, SETS>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        const void* f = (const void*)int4_tmem_kernel<BN, G, OUT_F32>;
+        const void* f = (const void*)int4_tmem_kernel<BN, G, SETS, OUT_F32>;
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
@@ -462,7 +465,7 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     const uint32_t step = all_sms ? tiles : slots;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split, rows);
-        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, OUT_F32>, mw, mx, p);
+        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, SETS, OUT_F32>, mw, mx, p);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -500,7 +503,11 @@ cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const
                                  uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
     const Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
-    return group == 64 ? launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
+    if (group == 64) return launch(launch_cfg<16, 2, 4, true>, launch_cfg<16, 2, 4, false>);
+    // Up to eight rows of groups of 128: sums in the tensor core over 64 k (run_int4_linear, which sends bf16 outputs alone, has the errors). More
+    // rows: over a whole group, as the kernel has them that takes 17 rows on.
+    if (m <= 8 && !out_f32) return launch_cfg<16, 1, 4, false>(x_bf16, w_packed, p, sm_count, stream);
+    return launch(launch_cfg<16, 1, 2, true>, launch_cfg<16, 1, 2, false>);
 }
 
 cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
@@ -525,9 +532,9 @@ cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const 
     const uint32_t per = group / 64;
     if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
-    if (m <= 16) return launch(launch_cfg<16, 0, true>, launch_cfg<16, 0, false>);
-    if (m <= 32) return launch(launch_cfg<32, 0, true>, launch_cfg<32, 0, false>);
-    return m <= 64 ? launch(launch_cfg<64, 0, true>, launch_cfg<64, 0, false>) : launch(launch_cfg<128, 0, true>, launch_cfg<128, 0, false>);
+    if (m <= 16) return launch(launch_cfg<16, 0, 1, true>, launch_cfg<16, 0, 1, false>);
+    if (m <= 32) return launch(launch_cfg<32, 0, 1, true>, launch_cfg<32, 0, 1, false>);
+    return m <= 64 ? launch(launch_cfg<64, 0, 1, true>, launch_cfg<64, 0, 1, false>) : launch(launch_cfg<128, 0, 1, true>, launch_cfg<128, 0, 1, false>);
 }
 
 }  // namespace vybk
