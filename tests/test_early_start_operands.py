@@ -1,0 +1,49 @@
+"""Kernels that start before the launches before them are complete (dependent_launch.cuh) read operands that those may still be writing, until the
+wait. So nothing may promise the compiler or the read-only cache path that the operands do not change while the kernel lives. What such a
+promise leaves to chance cannot be provoked, so this reads the sources."""
+import os
+import re
+
+import pytest
+
+KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vyre_b200", "csrc", "kernels")
+SOURCES = {f: open(os.path.join(KERNELS, f), encoding="utf-8").read() for f in sorted(os.listdir(KERNELS)) if f.endswith(".cu")}
+
+
+def functions(source):
+    """(name, signature, body) of the device functions of a file."""
+    source = re.sub(r"//[^\n]*", "", source)
+    for m in re.finditer(r"\b__(?:global|device)__\b", source):
+        end = source.find("{", m.end())
+        head = source[m.start() : end]
+        if end < 0 or ";" in head:
+            continue
+        depth, i = 1, end + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(source[i], 0)
+            i += 1
+        names = [n for n in re.findall(r"(\w+)\s*\(", head) if n != "__launch_bounds__"]
+        yield names[0], head, source[end:i]
+
+
+FUNCTIONS = {f: list(functions(s)) for f, s in SOURCES.items()}
+EARLY = [(f, name) for f, fs in FUNCTIONS.items() for name, head, body in fs
+         if "__global__" in head and re.search(r"\b(waits_for_previous|dependent_start)\(\)", body)]
+
+
+def test_the_early_kernels_are_found():
+    assert len(EARLY) >= 28 and ("int4_prefill_tcgen05.cu", "int4_tmem_kernel") in EARLY and ("moe_ffn.cu", "moe_combine_kernel") in EARLY
+
+
+@pytest.mark.parametrize("f,name", EARLY)
+def test_no_operand_is_promised_read_only(f, name):
+    known = {n: (head, body) for n, head, body in FUNCTIONS[f]}
+    todo, seen = [name], set()
+    while todo:  # the kernel and the functions of its file that it calls
+        n = todo.pop()
+        if n in seen:
+            continue
+        seen.add(n)
+        head, body = known[n]
+        assert "__restrict__" not in head + body and "__ldg(" not in body, f"{n} ({f})"
+        todo += [c for c in set(re.findall(r"\b(\w+)\s*(?:<[^;(){}]*>)?\(", body)) if c in known]

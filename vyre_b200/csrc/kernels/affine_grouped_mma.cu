@@ -67,12 +67,12 @@ __device__ __forceinline__ float fma_keep(float a, float b, float c) {
 __device__ __forceinline__ bool ordinary(float v) { return fabsf(v) < 0x1p64f; }  // false for NaN
 
 // One output by the definition, without its bias. Out of line: next to nothing takes it, and its loop stays off the main path's registers.
-__device__ __noinline__ float by_definition(const float* __restrict__ x, const uint32_t* __restrict__ w, const float* __restrict__ scale,
-                                            const uint32_t* __restrict__ zp, uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t row, uint32_t n) {
+__device__ __noinline__ float by_definition(const float* x, const uint32_t* w, const float* scale,
+                                            const uint32_t* zp, uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t row, uint32_t n) {
     float v = 0.0f;
     for (uint32_t k = 0; k < in_dim; ++k) {
         const size_t at = size_t(k / group) * out_dim + n;
-        const float q = float((__ldg(w + size_t(k / 8) * out_dim + n) >> (4 * (k % 8))) & 15u), s = scale[at];
+        const float q = float((w[size_t(k / 8) * out_dim + n] >> (4 * (k % 8))) & 15u), s = scale[at];
         v = fmaf(x[size_t(row) * in_dim + k], fmaf(q, s, -__fmul_rn(float(zp[at]), s)), v);
     }
     return v;
@@ -84,8 +84,8 @@ __device__ __noinline__ float by_definition(const float* __restrict__ x, const u
 // WK: warps of the block that share a tile of outputs and split its groups; the other WARPS / WK factors are further outputs.
 template <int R, int NB, int WK>
 __global__ void __launch_bounds__(THREADS, 2)
-affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restrict__ w, const float* __restrict__ scale,
-                          const uint32_t* __restrict__ zp, const float* __restrict__ bias, float* __restrict__ out, uint32_t in_dim,
+affine_grouped_mma_kernel(const float* x, const uint32_t* w, const float* scale,
+                          const uint32_t* zp, const float* bias, float* out, uint32_t in_dim,
                           uint32_t out_dim, uint32_t group, uint32_t batch, uint32_t chunk) {
     constexpr uint32_t NT = NB == 0 ? 1 : 3 * NB, COLS = 8 * NT, ROWS = NB == 0 ? 2 : 8 * NB;
     constexpr uint32_t AC = NB == 0 ? 1 : NB, SUMS = 8 * AC;  // accumulators per output: columns (NB = 0) or rows
@@ -115,7 +115,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
             uint32_t part[3][4] = {};
             if (r < nb) {
                 const float4* src = reinterpret_cast<const float4*>(x + size_t(b0 + r) * in_dim + k0 + kw * 8);
-                const float4 lo = __ldg(src), hi = __ldg(src + 1);
+                const float4 lo = src[0], hi = src[1];
                 const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -156,13 +156,13 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
     auto load = [&](uint32_t st, uint32_t (&a)[R], uint32_t (&z)[R]) {
         const uint32_t* row = wp + size_t(st) * 4 * out_dim;
         if constexpr (R == 4) {
-            const uint4 va = st < steps && in_a ? __ldg(reinterpret_cast<const uint4*>(row + na)) : make_uint4(0, 0, 0, 0);
-            const uint4 vz = st < steps && in_z ? __ldg(reinterpret_cast<const uint4*>(row + nz)) : make_uint4(0, 0, 0, 0);
+            const uint4 va = st < steps && in_a ? *reinterpret_cast<const uint4*>(row + na) : make_uint4(0, 0, 0, 0);
+            const uint4 vz = st < steps && in_z ? *reinterpret_cast<const uint4*>(row + nz) : make_uint4(0, 0, 0, 0);
             a[0] = va.x; a[1] = va.y; a[2] = va.z; a[3] = va.w;
             z[0] = vz.x; z[1] = vz.y; z[2] = vz.z; z[3] = vz.w;
         } else {
-            const uint2 va = st < steps && in_a ? __ldg(reinterpret_cast<const uint2*>(row + na)) : make_uint2(0, 0);
-            const uint2 vz = st < steps && in_z ? __ldg(reinterpret_cast<const uint2*>(row + nz)) : make_uint2(0, 0);
+            const uint2 va = st < steps && in_a ? *reinterpret_cast<const uint2*>(row + na) : make_uint2(0, 0);
+            const uint2 vz = st < steps && in_z ? *reinterpret_cast<const uint2*>(row + nz) : make_uint2(0, 0);
             a[0] = va.x; a[1] = va.y;
             z[0] = vz.x; z[1] = vz.y;
         }
@@ -183,10 +183,10 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
     };
     auto columns4 = [&](const auto* p, auto (&v)[R]) {  // R neighbouring words of a sidecar row
         if constexpr (R == 4) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+            const uint4 q = *reinterpret_cast<const uint4*>(p);
             *reinterpret_cast<uint4*>(&v) = q;
         } else {
-            *reinterpret_cast<uint2*>(&v) = __ldg(reinterpret_cast<const uint2*>(p));
+            *reinterpret_cast<uint2*>(&v) = *reinterpret_cast<const uint2*>(p);
         }
     };
     if (one_chunk && blockIdx.x < tiles) {
@@ -277,6 +277,12 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
         if constexpr (WK == 1 && NB > 0) {
             // a lane holds whole sums: outputs oa + i and oz + i of rows 2 t, 2 t + 1 of every block of eight
             bool good = true;
+            float ba[R], bz[R];  // before the stores, past which no load may move
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                ba[i] = have_a ? bias[oa + i] : 0.0f;
+                bz[i] = have_z ? bias[oz + i] : 0.0f;
+            }
 #pragma unroll
             for (int c = 0; c < int(AC); ++c)
 #pragma unroll
@@ -285,7 +291,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     if (r >= nb || !(j < 2 ? have_a : have_z)) continue;
 #pragma unroll
                     for (int i = 0; i < R; ++i) {
-                        out[size_t(b0 + r) * out_dim + n + i] = bias[n + i] + acc[i][c][j];
+                        out[size_t(b0 + r) * out_dim + n + i] = (j < 2 ? ba[i] : bz[i]) + acc[i][c][j];
                         good = good && ordinary(acc[i][c][j]);
                     }
                 }
@@ -310,8 +316,15 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     rz[1] = acc[i][c][3];
                 }
             __syncthreads();
+            auto bias_of = [&](uint32_t e) {
+                const uint32_t n = tile * WN * TILE + e % (WN * TILE);
+                return e < WN * TILE * nb && n < out_dim ? bias[n] : 0.0f;
+            };
+            float next = bias_of(threadIdx.x);  // one ahead: no load moves up past a store
             for (uint32_t e = threadIdx.x; e < WN * TILE * nb; e += THREADS) {
                 const uint32_t j = e % (WN * TILE), r = e / (WN * TILE), n = tile * WN * TILE + j;
+                const float bn = next;
+                next = bias_of(e + THREADS);
                 if (n >= out_dim) continue;
                 float v = 0.0f;
 #pragma unroll
@@ -320,7 +333,7 @@ affine_grouped_mma_kernel(const float* __restrict__ x, const uint32_t* __restric
                     v += NB == 0 ? (p[3 * r] + p[3 * r + 1]) + p[3 * r + 2] : p[r];
                 }
                 if (!ordinary(v)) v = by_definition(x, w, scale, zp, in_dim, out_dim, group, b0 + r, n);
-                out[size_t(b0 + r) * out_dim + n] = bias[n] + v;
+                out[size_t(b0 + r) * out_dim + n] = bn + v;
             }
             __syncthreads();
         }

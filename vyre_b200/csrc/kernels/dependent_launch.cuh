@@ -2,7 +2,9 @@
 // of its blocks have started, and that launch has its own start (1 to 3 us of launch latency, barriers, tensor memory, descriptors)
 // behind it when it comes to waits_for_previous(), which returns when everything before it in the stream is complete and visible.
 // Both are no-ops in a plain launch. A kernel that is launched this way calls waits_for_previous() in every thread that reads or
-// writes global memory, before it does, since the launch before it may still be waiting for the one before that.
+// writes global memory, before it does, since the launch before it may still be waiting for the one before that. What earlier launches may
+// still be writing when it starts is no read-only data: neither `__restrict__` nor `__ldg` on its operands, whose loads the compiler may
+// move up past the wait, or the hardware serve from lines that nobody invalidates.
 // Where a kernel calls lets_next_start(): at its start if what follows does little before its wait; behind its own loads if it is short
 // and a projection's prefetch of weights may follow (RMSNorm at 8 rows in front of a projection: 10 us a decode block lost otherwise).
 // Measured, us a call in chains of submissions, plain / dependent: int4 linear at 48 rows 20.6 / 18.6, published affine-grouped row

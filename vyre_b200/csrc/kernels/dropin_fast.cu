@@ -40,10 +40,10 @@ constexpr int MV_BT = 8;     // batch rows per block of the matvec kernel
 // before this chunk's barrier, so the global loads overlap the staging of x and the arithmetic.
 // grid (ceil(N / (TX * OT)), ceil(B / BT)).
 template <int TX, int OT, int KS, int BT, int KCHUNK>
-__global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ w,
-                                                                      const float* __restrict__ scale,
-                                                                      const uint32_t* __restrict__ zp,
-                                                                      const float* __restrict__ bias, float* __restrict__ out,
+__global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float* x, const uint32_t* w,
+                                                                      const float* scale,
+                                                                      const uint32_t* zp,
+                                                                      const float* bias, float* out,
                                                                       uint32_t in_dim, uint32_t out_dim, uint32_t group,
                                                                       int group_shift, uint32_t batch) {
     dependent_start();
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
 #pragma unroll
             for (int o = 0; o < OT; ++o) {
                 const uint32_t i = i0 + o * TX;
-                dst[j][o] = (kw < words && i < out_dim) ? __ldg(w + size_t(kw) * out_dim + i) : 0u;
+                dst[j][o] = (kw < words && i < out_dim) ? w[size_t(kw) * out_dim + i] : 0u;
             }
         }
     };
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
         for (uint32_t e = ty * TX + tx; e < BT * (KCHUNK / 4); e += TX * KS) {  // float4 per thread; in_dim % 8 == 0
             const uint32_t b = e / (KCHUNK / 4), k = (e % (KCHUNK / 4)) * 4;
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (b < nb && k < kc) v = __ldg(reinterpret_cast<const float4*>(x + size_t(b0 + b) * in_dim + k0 + k));
+            if (b < nb && k < kc) v = *reinterpret_cast<const float4*>(x + size_t(b0 + b) * in_dim + k0 + k);
             *reinterpret_cast<float4*>(&xs[b][k]) = v;
         }
         __syncthreads();
@@ -149,6 +149,9 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
     for (int b = 0; b < BT; ++b)
 #pragma unroll
         for (int o = 0; o < OT; ++o) red[(ty * BT + b) * (OT * TX) + o * TX + tx] = acc[b][o];
+    float bias_of[OT];  // before the stores, past which no load may move
+#pragma unroll
+    for (int o = 0; o < OT; ++o) bias_of[o] = i0 + o * TX < out_dim ? bias[i0 + o * TX] : 0.0f;
     __syncthreads();
     for (uint32_t b = ty; b < nb; b += KS) {
 #pragma unroll
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
             float v = red[b * (OT * TX) + o * TX + tx];
 #pragma unroll
             for (int y = 1; y < KS; ++y) v += red[(y * BT + b) * (OT * TX) + o * TX + tx];
-            out[size_t(b0 + b) * out_dim + i] = bias[i] + v;
+            out[size_t(b0 + b) * out_dim + i] = bias_of[o] + v;
         }
     }
 }
@@ -172,9 +175,9 @@ __global__ void __launch_bounds__(TX* KS) affine_grouped_fast_kernel(const float
 // batch 1). Same values as the operator's definition up to f32 summation order; exact whenever every partial sum is.
 // grid (ceil(N / 32), ceil(B / BT)), block 32 x KS; needs (group / 8) % KS == 0.
 template <int KS, int BT, int WPT>
-__global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const float* __restrict__ x, const uint32_t* __restrict__ w,
-                                                                        const float* __restrict__ scale, const uint32_t* __restrict__ zp,
-                                                                        const float* __restrict__ bias, float* __restrict__ out,
+__global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const float* x, const uint32_t* w,
+                                                                        const float* scale, const uint32_t* zp,
+                                                                        const float* bias, float* out,
                                                                         uint32_t in_dim, uint32_t out_dim, uint32_t group, uint32_t batch) {
     dependent_start();
     extern __shared__ __align__(16) float dsm[];
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const fl
     for (uint32_t e = tid; e < BT * (in_dim / 4); e += 32 * KS) {
         const uint32_t b = e / (in_dim / 4), k = (e % (in_dim / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (b < nb) v = __ldg(reinterpret_cast<const float4*>(x + size_t(b0 + b) * in_dim + k));
+        if (b < nb) v = *reinterpret_cast<const float4*>(x + size_t(b0 + b) * in_dim + k);
         *reinterpret_cast<float4*>(xs + size_t(b) * in_dim + k) = v;
     }
     __syncthreads();
@@ -215,9 +218,9 @@ __global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const fl
         for (int gg = 0; gg < GB; ++gg) {
             const uint32_t g = min(g0 + gg, groups - 1);  // past the end: reloaded, not used
 #pragma unroll
-            for (int j = 0; j < WPT; ++j) words[gg][j] = __ldg(w + size_t(g * wpg + j * KS + ty) * out_dim + ic);
-            sc[gg] = __ldg(scale + size_t(g) * out_dim + ic);
-            z[gg] = float(__ldg(zp + size_t(g) * out_dim + ic));
+            for (int j = 0; j < WPT; ++j) words[gg][j] = w[size_t(g * wpg + j * KS + ty) * out_dim + ic];
+            sc[gg] = scale[size_t(g) * out_dim + ic];
+            z[gg] = float(zp[size_t(g) * out_dim + ic]);
         }
 #pragma unroll
         for (int gg = 0; gg < GB; ++gg) {
@@ -256,18 +259,19 @@ __global__ void __launch_bounds__(32 * KS) affine_grouped_decode_kernel(const fl
     // fold the k slices in slice order (deterministic)
 #pragma unroll
     for (int b = 0; b < BT; ++b) red[(ty * BT + b) * 32 + tx] = acc[b];
+    const float bias_i = bias[ic];
     __syncthreads();
     for (uint32_t b = ty; b < nb; b += KS) {
         if (i >= out_dim) continue;
         float v = red[b * 32 + tx];
         for (uint32_t y = 1; y < KS; ++y) v += red[(y * BT + b) * 32 + tx];
-        out[size_t(b0 + b) * out_dim + i] = bias[i] + v;
+        out[size_t(b0 + b) * out_dim + i] = bias_i + v;
     }
 }
 
 // one warp per row, 8 rows per block; grid (ceil(rows / 8), ceil(batch / MV_BT))
-__global__ void __launch_bounds__(256) i4_matvec_fast_kernel(const uint32_t* __restrict__ w, const float* __restrict__ x,
-                                                             const float* __restrict__ scales, float* __restrict__ out,
+__global__ void __launch_bounds__(256) i4_matvec_fast_kernel(const uint32_t* w, const float* x,
+                                                             const float* scales, float* out,
                                                              uint32_t batch, uint32_t rows, uint32_t cols) {
     dependent_start();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -289,8 +293,8 @@ __global__ void __launch_bounds__(256) i4_matvec_fast_kernel(const uint32_t* __r
 #pragma unroll
             for (int b = 0; b < MV_BT; ++b) {
                 if (uint32_t(b) < nb) {
-                    const float4 xa = __ldg(reinterpret_cast<const float4*>(x + size_t(b0 + b) * cols + c0));
-                    const float4 xb = __ldg(reinterpret_cast<const float4*>(x + size_t(b0 + b) * cols + c0 + 4));
+                    const float4 xa = *reinterpret_cast<const float4*>(x + size_t(b0 + b) * cols + c0);
+                    const float4 xb = *reinterpret_cast<const float4*>(x + size_t(b0 + b) * cols + c0 + 4);
                     float a = acc[b];
                     a = __fmaf_rn(wv[0], xa.x, a);
                     a = __fmaf_rn(wv[1], xa.y, a);
@@ -406,9 +410,9 @@ constexpr int KQ_MAX_SPLIT = 16;  // blocks of a cluster
 
 // grid x = column blocks * split, cluster = split
 template <int BITS, int W, int KQ_WARPS>
-__global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_fast_kernel(const float* __restrict__ x, const uint32_t* __restrict__ packed,
-                                                                              const float* __restrict__ scales, const float* __restrict__ mins,
-                                                                              const float* __restrict__ b, float* __restrict__ out,
+__global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_fast_kernel(const float* x, const uint32_t* packed,
+                                                                              const float* scales, const float* mins,
+                                                                              const float* b, float* out,
                                                                               uint32_t in_dim, uint32_t out_dim, uint32_t split) {
     constexpr int VPW = 32 / BITS, OPT = W * VPW;         // outputs per packed word, per thread
     constexpr uint32_t BLOCK = BITS == 4 ? 32 : 16;       // weights per scale / min
@@ -442,16 +446,16 @@ __global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_f
             const uint32_t k = min(k0 + r, in_dim - 1);  // past this block's range: reloaded, times zero
             const uint32_t* src = wp + size_t(k) * row_words;
             if constexpr (W == 2) {
-                const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+                const uint2 v = *reinterpret_cast<const uint2*>(src);
                 t.words[r][0] = v.x; t.words[r][1] = v.y;
             } else {
-                t.words[r][0] = __ldg(src);
+                t.words[r][0] = *src;
             }
-            t.xk[r] = k0 + r < k_end ? __ldg(x + k) : 0.0f;
+            t.xk[r] = k0 + r < k_end ? x[k] : 0.0f;
 #pragma unroll
             for (int j = 0; j < SPT; ++j) {
-                t.sc[r][j] = __ldg(scales + size_t(k) * row_scales + s0 + j);
-                t.mn[r][j] = __ldg(mins + size_t(k) * row_scales + s0 + j);
+                t.sc[r][j] = scales[size_t(k) * row_scales + s0 + j];
+                t.mn[r][j] = mins[size_t(k) * row_scales + s0 + j];
             }
         }
     };
@@ -518,6 +522,7 @@ __global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_f
         const uint32_t i = xb * 32 * OPT + o;
         if (i >= out_dim) continue;
         float part[KQ_MAX_SPLIT];
+        const float bias = b[i];
 #pragma unroll
         for (uint32_t q = 0; q < KQ_MAX_SPLIT; ++q)
             if (q < split) part[q] = tc::ld_cluster_f32(tc::mapa(tc::smem_u32(sums + o), q));
@@ -525,7 +530,7 @@ __global__ void __launch_bounds__(32 * KQ_WARPS, 16 / KQ_WARPS) k_quant_linear_f
 #pragma unroll
         for (uint32_t q = 1; q < KQ_MAX_SPLIT; ++q)
             if (q < split) sum += part[q];
-        out[i] = sum + b[i];
+        out[i] = sum + bias;
     }
     tc::cluster_sync();  // no block leaves while another still reads its sums
 }

@@ -14,9 +14,9 @@ namespace vybk {
 namespace {
 
 // ---- fallback: any group size dividing k, any batch; warp per output row, plain 32-bit loads -------------------
-__global__ void __launch_bounds__(256) int4_linear_generic_kernel(const uint16_t* __restrict__ x,
-                                                                 const uint32_t* __restrict__ w,
-                                                                 const uint16_t* __restrict__ scales, void* y,
+__global__ void __launch_bounds__(256) int4_linear_generic_kernel(const uint16_t* x,
+                                                                 const uint32_t* w,
+                                                                 const uint16_t* scales, void* y,
                                                                  uint32_t m, uint32_t n, uint32_t k, uint32_t group,
                                                                  uint32_t out_f32) {
     dependent_start();

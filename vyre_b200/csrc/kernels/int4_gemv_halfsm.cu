@@ -384,8 +384,8 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_halfsm_kernel(const __gri
             pre_w[0] = pre_w[1] = make_uint4(0, 0, 0, 0);
             if (mine) {
                 const uint4* wsrc = reinterpret_cast<const uint4*>(p.norm_w + warp * (GPW * 128) + lane * 16);
-                pre_w[0] = __ldg(wsrc);
-                pre_w[1] = __ldg(wsrc + 1);
+                pre_w[0] = __ldcg(wsrc);
+                pre_w[1] = __ldcg(wsrc + 1);
             }
 #pragma unroll
             for (int j = 0; j < 2 * NM; ++j) {

@@ -246,7 +246,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const uint16_t* sp = p.scales + size_t(min(n0 + r, p.n - 1)) * p.groups;
         auto scale = [&](uint32_t i, uint32_t b) {
             const uint32_t at = (kb0 + i) * 4 + half * 2 + b, g = p.group_inv ? __umulhi(at, p.group_inv) : at;
-            return g < p.groups ? uint32_t(__ldg(sp + g)) * 0x10001u : 0u;  // past the row's last group the activations are zeros
+            return g < p.groups ? uint32_t(sp[g]) * 0x10001u : 0u;  // past the row's last group the activations are zeros
         };
         uint32_t next0 = G == 0 ? scale(s, 0) : 0, next1 = G == 0 ? scale(s, 1) : 0;
 #pragma unroll 1
@@ -336,7 +336,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
             for (int h = 0; h < G; ++h) {  // past the row's last group the activations are zeros
                 const uint32_t g = g0 + (i * G + h) * 2;
-                q[h] = (g < groups ? uint32_t(__ldg(sp + g)) : 0u) | (g + 1 < groups ? uint32_t(__ldg(sp + g + 1)) << 16 : 0u);
+                q[h] = (g < groups ? uint32_t(sp[g]) : 0u) | (g + 1 < groups ? uint32_t(sp[g + 1]) << 16 : 0u);
             }
         };
 #pragma unroll

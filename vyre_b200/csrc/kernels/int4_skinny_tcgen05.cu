@@ -248,14 +248,14 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         constexpr uint32_t AHEAD = 4;  // scale pairs in flight: an L2 round trip is several stages long
         uint32_t queue[AHEAD];
 #pragma unroll
-        for (uint32_t d = 0; d < AHEAD; ++d) queue[d] = d < kbs ? __ldg(sp + d) : 0u;
+        for (uint32_t d = 0; d < AHEAD; ++d) queue[d] = d < kbs ? sp[d] : 0u;
         for (uint32_t i0 = 0; i0 < kbs && ok; i0 += AHEAD) {
 #pragma unroll
             for (uint32_t d = 0; d < AHEAD; ++d) {
                 const uint32_t i = i0 + d;
                 if (i >= kbs || !ok) break;
                 const uint32_t pair = queue[d];
-                if (i + AHEAD < kbs) queue[d] = __ldg(sp + i + AHEAD);
+                if (i + AHEAD < kbs) queue[d] = sp[i + AHEAD];
 #pragma unroll
                 for (uint32_t buf = 0; buf < 2; ++buf) {
                     // PASS = 1: one accumulator per group, set = group parity; PASS = 2: both groups' accumulators, set = stage parity

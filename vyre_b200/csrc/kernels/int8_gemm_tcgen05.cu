@@ -213,8 +213,8 @@ int8_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 }
 
 // Per-token symmetric int8 quantisation: s_t = max|x| / 127, q = clamp(rint(x / s_t), -127, 127); one warp per row.
-__global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t* __restrict__ x, int8_t* __restrict__ q,
-                                                                float* __restrict__ scales, uint32_t M, uint32_t K) {
+__global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t* x, int8_t* q,
+                                                                float* scales, uint32_t M, uint32_t K) {
     dependent_start();
     const uint32_t row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= M) return;
@@ -224,9 +224,13 @@ __global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t*
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float s = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
     if (lane == 0) scales[row] = s;
-    for (uint32_t k = lane; k < K; k += 32) {
-        const float v = __fdiv_rn(__uint_as_float(uint32_t(xr[k]) << 16), s);
-        q[size_t(row) * K + k] = int8_t(fminf(127.0f, fmaxf(-127.0f, rintf(v))));
+    for (uint32_t k0 = lane; k0 < K; k0 += 128) {  // four loads before their stores, past which none may move
+        uint32_t e[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) e[j] = k0 + 32 * j < K ? uint32_t(xr[k0 + 32 * j]) : 0u;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            if (k0 + 32 * j < K) q[size_t(row) * K + k0 + 32 * j] = int8_t(fminf(127.0f, fmaxf(-127.0f, rintf(__fdiv_rn(__uint_as_float(e[j] << 16), s)))));
     }
 }
 
@@ -235,8 +239,8 @@ __global__ void __launch_bounds__(256) quantize_per_token_kernel(const uint16_t*
 // with the exact division that the rounding rule asks for. Measured at 4096 x 8192: the kernel above 94 us (2-byte loads,
 // the second pass over x from L2, 512 blocks of serial rows), this one 37 us.
 template <int V>
-__global__ void __launch_bounds__(256) quantize_per_token_wide_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
-                                                                     float* __restrict__ scales, uint32_t chunks) {
+__global__ void __launch_bounds__(256) quantize_per_token_wide_kernel(const uint4* x, uint2* q,
+                                                                     float* scales, uint32_t chunks) {
     dependent_start();
     __shared__ float warp_max[8];
     const size_t row = blockIdx.x;
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(256) quantize_per_token_wide_kernel(const uint
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         const uint32_t c = threadIdx.x + 256 * i;
-        v[i] = c < chunks ? __ldg(xr + c) : make_uint4(0, 0, 0, 0);
+        v[i] = c < chunks ? xr[c] : make_uint4(0, 0, 0, 0);
     }
     float amax = 0.0f;
 #pragma unroll

@@ -18,9 +18,9 @@ namespace {
 
 constexpr int MB = 16;  // batch rows held in registers
 
-__global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* __restrict__ x,
-                                                              const int8_t* __restrict__ w,
-                                                              const float* __restrict__ scale, float* __restrict__ y,
+__global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* x,
+                                                              const int8_t* w,
+                                                              const float* scale, float* y,
                                                               uint32_t m, uint32_t n, uint32_t k) {
     dependent_start();
     const uint32_t col = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* __re
 constexpr int KC = 1024;   // k per shared-memory tile
 constexpr int CPW = 2;     // output channels per warp
 constexpr int WPB = 4;     // warps per block
-__global__ void __launch_bounds__(WPB * 32, 3) int8_weight_only_tiled_kernel(const float* __restrict__ x, const int8_t* __restrict__ w,
-                                                                          const float* __restrict__ scale, float* __restrict__ y,
+__global__ void __launch_bounds__(WPB * 32, 3) int8_weight_only_tiled_kernel(const float* x, const int8_t* w,
+                                                                          const float* scale, float* y,
                                                                           uint32_t m, uint32_t n, uint32_t k) {
     dependent_start();
     extern __shared__ __align__(16) float xs[];  // [MB][KC]

@@ -37,8 +37,8 @@ __device__ __forceinline__ float bf16_bits_to_float(uint32_t b) { return __uint_
 // ---- router + gate: one warp per token; a CTA keeps the router weights in shared memory and walks many tokens -------
 template <bool WR_IN_SMEM>
 __global__ void __launch_bounds__(256, 2)
-moe_router_gate_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w_router, uint32_t* __restrict__ idx,
-                       float* __restrict__ wts, uint32_t tokens, uint32_t hidden, uint32_t experts, uint32_t topk) {
+moe_router_gate_kernel(const uint16_t* x, const uint16_t* w_router, uint32_t* idx,
+                       float* wts, uint32_t tokens, uint32_t hidden, uint32_t experts, uint32_t topk) {
     dependent_start();
     extern __shared__ __align__(16) uint8_t s_dyn[];
     __shared__ float s_logits[8][MAX_EXPERTS];
@@ -63,7 +63,7 @@ moe_router_gate_kernel(const uint16_t* __restrict__ x, const uint16_t* __restric
 #pragma unroll
         for (uint32_t c = 0; c < XCHUNKS; ++c) {
             const uint32_t k = c * 256 + lane * 8;
-            xrow[c] = k < hidden ? __ldg(reinterpret_cast<const uint4*>(xr + k)) : make_uint4(0, 0, 0, 0);
+            xrow[c] = k < hidden ? *reinterpret_cast<const uint4*>(xr + k) : make_uint4(0, 0, 0, 0);
         }
     }
     for (uint32_t e0 = 0; e0 < experts; e0 += 8) {
@@ -174,8 +174,8 @@ cudaError_t launch_router_gate(const uint16_t* x, const uint16_t* w_router, uint
 // plan words: [0] number of 256-row tiles, [1 .. E] segment starts (rows; the low eight bits hold the padding rows at the
 // segment's end), [1+E] end of the last segment, then tile_expert[max_tiles].
 __global__ void __launch_bounds__(1024)
-moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, uint32_t* __restrict__ pos,
-                uint32_t* __restrict__ row_token, uint32_t tokens, uint32_t experts, uint32_t topk, uint32_t max_rows) {
+moe_plan_kernel(const uint32_t* idx, uint32_t* plan, uint32_t* pos,
+                uint32_t* row_token, uint32_t tokens, uint32_t experts, uint32_t topk, uint32_t max_rows) {
     dependent_start();
     __shared__ uint32_t s_count[MAX_EXPERTS], s_start[MAX_EXPERTS + 1], s_cursor[MAX_EXPERTS];
     __shared__ uint32_t s_warp_cnt[MAX_EXPERTS][32];
@@ -243,8 +243,8 @@ moe_plan_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ plan, u
 
 // ---- gather: expert-sorted activation rows ---------------------------------------------------
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ row_token, const uint32_t* __restrict__ plan,
-                  uint16_t* __restrict__ xg, uint32_t hidden, uint32_t experts, bool skinny) {
+moe_gather_kernel(const uint16_t* x, const uint32_t* row_token, const uint32_t* plan,
+                  uint16_t* xg, uint32_t hidden, uint32_t experts, bool skinny) {
     dependent_start();
     const uint32_t rows = plan[1 + experts];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -257,12 +257,20 @@ moe_gather_kernel(const uint16_t* __restrict__ x, const uint32_t* __restrict__ r
                 for (uint32_t c = lane; c < hidden / 8; c += 32) dst[c] = make_uint4(0, 0, 0, 0);
         } else {
             const uint4* src = reinterpret_cast<const uint4*>(x + size_t(t) * hidden);
-            for (uint32_t c = lane; c < hidden / 8; c += 32) {
-                uint4 v = src[c];
-                if (skinny)  // k order 0 4 1 5 2 6 3 7, in which the skinny GEMMs unpack weights
-                    v = make_uint4(__byte_perm(v.x, v.z, 0x5410), __byte_perm(v.x, v.z, 0x7632), __byte_perm(v.y, v.w, 0x5410),
-                                   __byte_perm(v.y, v.w, 0x7632));
-                dst[c] = v;
+            constexpr uint32_t AHEAD = 8;  // loads before their stores, past which none may move
+            for (uint32_t c0 = lane; c0 < hidden / 8; c0 += 32 * AHEAD) {
+                uint4 v[AHEAD];
+#pragma unroll
+                for (uint32_t i = 0; i < AHEAD; ++i)
+                    if (c0 + 32 * i < hidden / 8) v[i] = src[c0 + 32 * i];
+#pragma unroll
+                for (uint32_t i = 0; i < AHEAD; ++i) {
+                    if (c0 + 32 * i >= hidden / 8) break;
+                    if (skinny)  // k order 0 4 1 5 2 6 3 7, in which the skinny GEMMs unpack weights
+                        v[i] = make_uint4(__byte_perm(v[i].x, v[i].z, 0x5410), __byte_perm(v[i].x, v[i].z, 0x7632), __byte_perm(v[i].y, v[i].w, 0x5410),
+                                          __byte_perm(v[i].y, v[i].w, 0x7632));
+                    dst[c0 + 32 * i] = v[i];
+                }
             }
         }
     }
@@ -274,32 +282,41 @@ constexpr uint32_t SEG = 64;  // two chunks per lane
 
 // ---- combine: out[t] = bf16( sum_j w[t,j] * y[pos[t,j]] ), slots in selection order, separate multiply and add -------
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const uint16_t* __restrict__ y, const uint32_t* __restrict__ pos, const float* __restrict__ wts,
-                   uint16_t* __restrict__ out, uint32_t tokens, uint32_t hidden, uint32_t topk) {
+moe_combine_kernel(const uint16_t* y, const uint32_t* pos, const float* wts,
+                   uint16_t* out, uint32_t tokens, uint32_t hidden, uint32_t topk) {
     dependent_start();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t chunks = hidden / 8, segs = (chunks + SEG - 1) / SEG;
     for (uint64_t unit = blockIdx.x * 8 + warp; unit < uint64_t(tokens) * segs; unit += gridDim.x * 8) {
         const uint32_t t = uint32_t(unit / segs), seg = uint32_t(unit % segs), c1 = min(chunks, (seg + 1) * SEG);
-        for (uint32_t c = seg * SEG + lane; c < c1; c += 32) {
-            float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (uint32_t j = 0; j < topk; ++j) {
-                const float w = wts[size_t(t) * topk + j];
-                const uint4 v = reinterpret_cast<const uint4*>(y + size_t(pos[size_t(t) * topk + j]) * hidden)[c];
-                const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+        const uint32_t c0 = seg * SEG + lane;  // this lane's chunks: c0 and c0 + 32, loaded before either is stored
+        float acc[SEG / 32][8] = {};
+        for (uint32_t j = 0; j < topk; ++j) {
+            const float w = wts[size_t(t) * topk + j];
+            const uint4* src = reinterpret_cast<const uint4*>(y + size_t(pos[size_t(t) * topk + j]) * hidden);
+            uint4 v[SEG / 32];
+#pragma unroll
+            for (uint32_t i = 0; i < SEG / 32; ++i) v[i] = c0 + 32 * i < c1 ? src[c0 + 32 * i] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (uint32_t i = 0; i < SEG / 32; ++i) {
+                const uint32_t vw[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    acc[2 * q] = __fadd_rn(acc[2 * q], __fmul_rn(w, bf16_bits_to_float(vw[q] & 0xFFFFu)));
-                    acc[2 * q + 1] = __fadd_rn(acc[2 * q + 1], __fmul_rn(w, bf16_bits_to_float(vw[q] >> 16)));
+                    acc[i][2 * q] = __fadd_rn(acc[i][2 * q], __fmul_rn(w, bf16_bits_to_float(vw[q] & 0xFFFFu)));
+                    acc[i][2 * q + 1] = __fadd_rn(acc[i][2 * q + 1], __fmul_rn(w, bf16_bits_to_float(vw[q] >> 16)));
                 }
             }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < SEG / 32; ++i) {
+            if (c0 + 32 * i >= c1) break;
             uint32_t pk[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(acc[i][2 * q], acc[i][2 * q + 1]);
                 pk[q] = *reinterpret_cast<const uint32_t*>(&h2);
             }
-            reinterpret_cast<uint4*>(out + size_t(t) * hidden)[c] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            reinterpret_cast<uint4*>(out + size_t(t) * hidden)[c0 + 32 * i] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
     }
 }

@@ -235,8 +235,8 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             // the scales of the step's two 64-k blocks, two stages ahead
             auto fetch = [&](uint32_t kb) {
                 const uint32_t b0 = kb * 4 + part * 2, b1 = b0 + 1;
-                return kb < stages_per_item ? make_uint2(__ldg(srow + (p.group_inv ? __umulhi(b0, p.group_inv) : b0)),
-                                                         __ldg(srow + (p.group_inv ? __umulhi(b1, p.group_inv) : b1)))
+                return kb < stages_per_item ? make_uint2(srow[p.group_inv ? __umulhi(b0, p.group_inv) : b0],
+                                                         srow[p.group_inv ? __umulhi(b1, p.group_inv) : b1])
                                             : make_uint2(0, 0);
             };
             uint2 sc = fetch(0), sc1 = fetch(1);

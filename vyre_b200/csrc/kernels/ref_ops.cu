@@ -175,8 +175,8 @@ __global__ void linear_rows_kernel(const void* x, const void* w, const void* bia
 // staged weight serves RT rows. What bounds it is the order itself: in_dim dependent additions, 4 cycles each, and two
 // f32 instructions per product. Where it is the faster one: launch_linear_rows.
 template <int RT>
-__global__ void __launch_bounds__(128) linear_rows_tiled_kernel(const void* __restrict__ x, const void* __restrict__ w,
-                                                                const void* __restrict__ bias, void* __restrict__ out,
+__global__ void __launch_bounds__(128) linear_rows_tiled_kernel(const void* x, const void* w,
+                                                                const void* bias, void* out,
                                                                 uint32_t rows, uint32_t in_dim, uint32_t out_dim, uint32_t dt,
                                                                 uint32_t out_in) {
     dependent_start();
