@@ -47,3 +47,15 @@ def test_no_operand_is_promised_read_only(f, name):
         head, body = known[n]
         assert "__restrict__" not in head + body and "__ldg(" not in body, f"{n} ({f})"
         todo += [c for c in set(re.findall(r"\b(\w+)\s*(?:<[^;(){}]*>)?\(", body)) if c in known]
+
+
+WITH_TENSOR_MEMORY = [(f, name) for f, name in EARLY if any(n == name and "tmem_alloc" in body for n, _, body in FUNCTIONS[f])]
+
+
+@pytest.mark.parametrize("f,name", WITH_TENSOR_MEMORY)
+def test_tensor_memory_is_held_before_the_next_launch_may_start(f, name):
+    """A block of the next launch on the same SM could otherwise allocate first and wait for this one, which waits for the allocation."""
+    assert len(WITH_TENSOR_MEMORY) >= 3
+    body = next(body for n, _, body in FUNCTIONS[f] if n == name)
+    alloc, meet, start = body.index("tmem_alloc("), body.index("__syncthreads()", body.index("tmem_alloc(")), body.index("lets_next_start()")
+    assert alloc < meet < start and body.count("lets_next_start()") == 1 and "dependent_start()" not in body

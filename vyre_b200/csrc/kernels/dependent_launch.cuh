@@ -7,6 +7,8 @@
 // move up past the wait, or the hardware serve from lines that nobody invalidates.
 // Where a kernel calls lets_next_start(): at its start if what follows does little before its wait; behind its own loads if it is short
 // and a projection's prefetch of weights may follow (RMSNorm at 8 rows in front of a projection: 10 us a decode block lost otherwise).
+// A kernel with tensor memory calls it when the block has allocated its share: a block of the next launch beside it may take what is left, keeps
+// it while it waits for this launch, and an allocation waits without a limit.
 // Measured, us a call in chains of submissions, plain / dependent: int4 linear at 48 rows 20.6 / 18.6, published affine-grouped row
 // 16.0 / 14.5, affine-grouped decode 36.0 / 35.3, Q4_K linear 24.8 / 23.8; a MoE layer of 64 tokens (six launches) 268 / 257.
 #pragma once

@@ -119,11 +119,15 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         tma_prefetch_desc(&map_w);
         tma_prefetch_desc(&map_x);
     }
-    lets_next_start();
     if (warp == 1) {
         tmem_alloc(smem_u32(&bars->tmem_base), TMEM_COLS);
         tmem_relinquish();
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    lets_next_start();
     waits_for_previous();
     for (uint32_t e = threadIdx.x; e < p.experts; e += THREADS) {
         const uint32_t here = p.plan[1 + e], next = p.plan[2 + e];
@@ -131,10 +135,7 @@ moe_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         bars->seg_row[e] = row;
         bars->seg_count[e] = (next & ~(ROW_TILE - 1)) - row - (here & (ROW_TILE - 1));
     }
-    tc_fence_before();
     __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = bars->tmem_base;
 
     uint32_t total = 0;
     for (uint32_t e = 0; e < p.experts; ++e) total += (bars->seg_count[e] + BN - 1) / BN * p.n_tiles;
