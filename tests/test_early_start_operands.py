@@ -59,3 +59,32 @@ def test_tensor_memory_is_held_before_the_next_launch_may_start(f, name):
     body = next(body for n, _, body in FUNCTIONS[f] if n == name)
     alloc, meet, start = body.index("tmem_alloc("), body.index("__syncthreads()", body.index("tmem_alloc(")), body.index("lets_next_start()")
     assert alloc < meet < start and body.count("lets_next_start()") == 1 and "dependent_start()" not in body
+
+
+def roles(body):
+    """The branches of a kernel's chain of roles: (condition, text)."""
+    at = [m for m in re.finditer(r"\n    (?:\} else )?(?:if constexpr|if|else if)? ?\((warp[^\n]*|G == 0)\) \{|\n    \} else \{", body)]
+    return [(m.group(1), body[m.end() : n.start() if n else len(body)]) for m, n in zip(at, at[1:] + [None])]
+
+
+WITH_LIMITS = [(f, name) for f, name in EARLY if any(n == name and re.search(r"\bmbar_wait2?\(", body) for n, _, body in FUNCTIONS[f])]
+
+
+@pytest.mark.parametrize("f,name", WITH_LIMITS)
+def test_waits_with_a_limit_begin_behind_the_wait_for_earlier_launches(f, name):
+    """The time that earlier launches still take (a peer that is late, a kernel of seconds) would count against the limit."""
+    assert {x[0] for x in WITH_LIMITS} == {"int4_gemv_bulk.cu", "int4_prefill_tcgen05.cu", "int4_skinny_tcgen05.cu", "moe_skinny_tcgen05.cu"}
+    body = next(body for n, _, body in FUNCTIONS[f] if n == name)
+    if f == "int4_gemv_bulk.cu":  # consumers: before anything of theirs; the producer: before the first stage that it has to wait for
+        assert "if (warp != WARPS || !p.constant) waits_for_previous();" in body
+        assert re.search(r"if \(u == STAGES\) waits_for_previous\(\);\s*if \(u >= STAGES\) ok = mbar_wait\(", body)
+        return
+    chain = body.index("bool ok = true;")
+    guard = re.search(r"(if \(([^;]*)\) )?waits_for_previous\(\);", body[body.index("lets_next_start()") : chain])
+    # roles that are left out there, for what they may read or prefetch before, wait before their own first wait with a limit
+    late = {None: [], "warp != 0 && warp != 3": ["warp == 0", "warp == 3"], "warp != 0 && !(p.constant && warp >= 12)": ["warp == 0", "warp >= 12"]}[guard.group(2)]
+    found = dict(roles(body[chain:]))
+    for role in late:
+        text = found[role]
+        limit = re.search(r"\b(mbar_wait2?|done_wait)\(", text)
+        assert "waits_for_previous();" in text and (not limit or text.index("waits_for_previous();") < limit.start()), role

@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_gemv_kernel(const Params p) {
         bool ok = true;
         uint32_t u = 0;
         for (; u < units; ++u) {
+            if (u == STAGES) waits_for_previous();  // whose time is not the wait's, which has a limit
             if (u >= STAGES) ok = mbar_wait(smem_u32(&ctrl->empty[u % STAGES]), ((u / STAGES) - 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;

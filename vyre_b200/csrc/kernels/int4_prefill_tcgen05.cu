@@ -169,14 +169,18 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     lets_next_start();
+    // Before any wait with a limit: the time that the launches before this one still take is not this one's. Prefetches come first.
+    if (warp != 0 && warp != 3) waits_for_previous();
     auto done_wait = [&](uint32_t i) { return mbar_wait(smem_u32(&bars->done[i % DONE]), (i / DONE) & 1, abort_flag); };
 
     bool ok = true;
     if (warp == 0) {
         // ---- packed weights: into L2 while the launches before this one run, from there when they are complete ----
-        if (elect_one()) {
+        if (elect_one())
             for (uint32_t i = 0; i < min(kbs, PREFETCH_STAGES); ++i) tma_prefetch_2d(&map_w, int((kb0 + i) * (KB / 2)), int(n0));
-            waits_for_previous();
+        __syncwarp();
+        waits_for_previous();
+        if (elect_one()) {
             uint32_t i = 0;
             for (; i < kbs; ++i) {
                 const uint32_t s = i % C::STAGES, bar = smem_u32(&bars->full[s]);
@@ -190,7 +194,6 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     } else if (warp == 2) {
         // ---- activations ----
         if (elect_one()) {
-            waits_for_previous();
             uint32_t i = 0;
             for (; i < kbs; ++i) {
                 const uint32_t s = i % C::X_STAGES, bar = smem_u32(&bars->x_full[s]), dst = smem_u32(x_tiles + s * C::X_BYTES);
@@ -208,6 +211,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         for (uint32_t r = lane; r < BM && n0 + r < p.n; r += 32)
             for (uint32_t at = first; at < last; at += 32)
                 prefetch_l2(reinterpret_cast<const uint8_t*>(p.scales) + size_t(n0 + r) * row_bytes + at);
+        waits_for_previous();
     } else if (warp == 1) {
         // ---- MMA: one commit per stage frees the unpacked weights and the activations and hands the sums on ----
         constexpr uint32_t idesc = idesc_bf16_f32(BM, BN);
@@ -242,7 +246,6 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const uint32_t mask = p.mask, mul = p.mul, add = p.add;
         uint32_t s = unit >> 1, parity = 0;
         // G = 0: the scales of this thread's two 64-k blocks, a stage of its own ahead
-        if (G == 0) waits_for_previous();
         const uint16_t* sp = p.scales + size_t(min(n0 + r, p.n - 1)) * p.groups;
         auto scale = [&](uint32_t i, uint32_t b) {
             const uint32_t at = (kb0 + i) * 4 + half * 2 + b, g = p.group_inv ? __umulhi(at, p.group_inv) : at;
@@ -319,7 +322,6 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         }
     } else {
         // ---- epilogue: acc += scale * group sum ----
-        waits_for_previous();  // scales
         const uint32_t quad = warp & 3, o = quad * 32 + lane, row = n0 + o;
         const uint32_t groups = p.groups, g0 = kb0 * 2 * G;
         const uint16_t* sp = p.scales + size_t(min(row, p.n - 1)) * groups;

@@ -133,7 +133,9 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const uint32_t tmem = bars->tmem_base;
     // only now, with this CTA's tensor memory in hand, may the next launch's CTA take the rest of it
     lets_next_start();
-    if (!p.constant && warp != 0) waits_for_previous();
+    // Before any wait with a limit: the time that the launches before this one still take is not this one's. Only constant weights (warp 0) and
+    // scales (from warp 12 on) are read before.
+    if (warp != 0 && !(p.constant && warp >= 12)) waits_for_previous();
 
     bool ok = true;
     if (warp == 0) {
@@ -249,6 +251,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         uint32_t queue[AHEAD];
 #pragma unroll
         for (uint32_t d = 0; d < AHEAD; ++d) queue[d] = d < kbs ? sp[d] : 0u;
+        waits_for_previous();
         for (uint32_t i0 = 0; i0 < kbs && ok; i0 += AHEAD) {
 #pragma unroll
             for (uint32_t d = 0; d < AHEAD; ++d) {
