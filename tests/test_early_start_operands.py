@@ -80,11 +80,12 @@ def test_waits_with_a_limit_begin_behind_the_wait_for_earlier_launches(f, name):
         assert re.search(r"if \(u == STAGES\) waits_for_previous\(\);\s*if \(u >= STAGES\) ok = mbar_wait\(", body)
         return
     chain = body.index("bool ok = true;")
-    guard = re.search(r"(if \(([^;]*)\) )?waits_for_previous\(\);", body[body.index("lets_next_start()") : chain])
-    # roles that are left out there, for what they may read or prefetch before, wait before their own first wait with a limit
-    late = {None: [], "warp != 0 && warp != 3": ["warp == 0", "warp == 3"], "warp != 0 && !(p.constant && warp >= 12)": ["warp == 0", "warp >= 12"]}[guard.group(2)]
-    found = dict(roles(body[chain:]))
-    for role in late:
-        text = found[role]
+    guard = re.search(r"\n    (if \(([^;]*)\) )?waits_for_previous\(\);", body[body.index("lets_next_start()") : chain])
+    left_out = {None: (), "warp != 0 && !(p.constant && warp >= 12)": ("warp == 0", "warp >= 12")}[guard.group(2)] if guard else None
+    found = roles(body[chain:])
+    assert len(found) >= 4
+    # without a wait of the whole block, or for the roles that it leaves out for what they may read or prefetch before: before their own first wait
+    for role, text in found:
         limit = re.search(r"\b(mbar_wait2?|done_wait)\(", text)
-        assert "waits_for_previous();" in text and (not limit or text.index("waits_for_previous();") < limit.start()), role
+        if limit and (left_out is None or role in left_out):
+            assert "waits_for_previous();" in text[: limit.start()], role
