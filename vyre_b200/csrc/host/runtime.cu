@@ -114,6 +114,7 @@ struct vyb_instance {
 
     // events are recycled: creating and destroying three per submission costs more than the launch itself
     std::vector<TimePoint*> time_points;
+    std::vector<TimePoint*> late_points;  // whose record may still be to come on the clock stream: not to be recorded again before
     std::vector<cudaEvent_t> plain_events;
     cudaEvent_t acquire_event() {
         cudaEvent_t e = nullptr;
@@ -130,6 +131,11 @@ struct vyb_instance {
     }
     TimePoint* acquire_time() {
         TimePoint* t;
+        for (size_t i = late_points.size(); time_points.empty() && i-- > 0;)
+            if (cudaEventQuery(late_points[i]->event) == cudaSuccess) {
+                time_points.push_back(late_points[i]);
+                late_points.erase(late_points.begin() + i);
+            }
         if (time_points.empty()) {
             t = new TimePoint;
             cudaEventCreate(&t->event);
@@ -140,8 +146,21 @@ struct vyb_instance {
         t->users = 1;
         return t;
     }
-    void release_time(TimePoint* t) {
-        if (t && --t->users == 0) time_points.push_back(t);
+    void release_time(TimePoint* t, bool there) {
+        if (t && --t->users == 0) (there ? time_points : late_points).push_back(t);
+    }
+    // Reads a submission's times and gives them back; false while its end is still to come
+    bool read_times(TimePoint*& start, TimePoint*& end, uint64_t* ns) {
+        float ms = 0.0f;
+        if (!start || cudaEventElapsedTime(&ms, start->event, end->event) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        release_time(start, true);
+        release_time(end, true);
+        start = end = nullptr;
+        *ns = uint64_t(double(ms) * 1.0e6);
+        return true;
     }
 
     // The newest vyb_submit while it has not been waited for. What is queued behind it takes its times on a stream beside the
@@ -223,10 +242,11 @@ void instance_unref(vyb_instance* i) {
         std::lock_guard<std::mutex> lk(i->dev->mu);
         i->dev->clock_streams.push_back(i->clock);
     }
-    for (TimePoint* t : i->time_points) {
-        cudaEventDestroy(t->event);
-        delete t;
-    }
+    for (auto* pool : {&i->time_points, &i->late_points})
+        for (TimePoint* t : *pool) {
+            cudaEventDestroy(t->event);
+            delete t;
+        }
     for (cudaEvent_t e : i->plain_events) cudaEventDestroy(e);
     for (auto& b : i->pinned) cudaFreeHost(b.ptr);
     for (auto& b : i->temps) cudaFree(b.ptr);
@@ -250,6 +270,7 @@ struct vyb_prepared;
 struct vyb_submission {
     vyb_instance* inst = nullptr;
     TimePoint *start = nullptr, *end = nullptr;  // of its kernels
+    bool beside = false;                         // its end is taken on the clock stream
     cudaEvent_t done = nullptr;
     std::vector<void*> temps;
     std::vector<void*> staged;  // pinned copies of the caller's host inputs (the BindingSet owns its bytes)
@@ -284,7 +305,9 @@ struct vyb_completion {
     vyb_instance* inst = nullptr;
     Digest artifact{};
     std::vector<OutputSlot> outputs;
-    TimePoint *start = nullptr, *end = nullptr;  // nullptr for a prepared submission
+    uint64_t device_ns = 0;
+    bool has_device_ns = false;
+    TimePoint *start = nullptr, *end = nullptr;  // while the end is still to come
 };
 
 namespace {
@@ -980,21 +1003,24 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         return fail_oom(16, 0);
     }
     std::memset(sub->status_host, 0, 16);
-    // Behind a submission that is still pending, and with nothing but kernels of its own, this one starts where that one ends, and
-    // its own end is taken beside the stream (vyb_instance::tail). inst->mu is held for the whole submission.
+    // Behind a submission that is still pending, and with nothing but kernels of its own, this one starts where that one ends, as an event that
+    // is recorded here would have it, and its own end is taken beside the stream (vyb_instance::tail). inst->mu is held for the whole
+    // submission.
     bool queued = sub->temps.empty() && inst->tail && cudaEventQuery(inst->tail->done) == cudaErrorNotReady;
     for (const OutputSlot& o : sub->outputs) queued = queued && !o.host;
     if (queued)  // that one's end is not the end of its copies
         for (const OutputSlot& o : inst->tail->outputs) queued = queued && !o.host;
     queued = queued && inst->clock_stream() != nullptr;
+    sub->beside = queued;
     sub->end = inst->acquire_time();
     sub->done = inst->acquire_event();
-    if (queued) {
+    if (queued && inst->tail->beside) {
         sub->start = inst->tail->end;
         ++sub->start->users;
-    } else {
+    } else {  // both times on one stream: the way from one to the other takes some microseconds
         sub->start = inst->acquire_time();
-        cudaEventRecord(sub->start->event, inst->stream);
+        if (queued) cudaStreamWaitEvent(inst->clock, inst->tail->done, 0);
+        cudaEventRecord(sub->start->event, queued ? inst->clock : inst->stream);
     }
     cudaGetLastError();  // a non-sticky error left by an unrelated earlier call must not be blamed on this launch
     uint32_t* const shared_status = inst->status_dev;
@@ -1008,8 +1034,8 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         cudaGetLastError();
         cudaStreamSynchronize(inst->stream);
         cleanup();
-        inst->release_time(sub->start);
-        inst->release_time(sub->end);
+        inst->release_time(sub->start, !queued);
+        inst->release_time(sub->end, true);
         inst->release_event(sub->done);
         if (e == cudaErrorNotSupported) return fail_unsupported("operator `" + p.op_id + "`");
         return fail_dispatch(int(e), "kernel launch failed: " + cuda_msg(e));
@@ -1051,6 +1077,8 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
     vyb_prepared* prep = s->prepared;
     cudaSetDevice(d->ordinal);
     cudaError_t e = cudaEventSynchronize(s->done);
+    uint64_t ns = 0;
+    bool timed = false;
     // the status words this submission itself read back (never another submission's)
     const uint32_t status = e == cudaSuccess && s->status_host ? s->status_host[0] : 0;
     {
@@ -1059,6 +1087,9 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
         for (void* t : s->staged) inst->release_pinned(t);
         if (!prep && s->status_host) inst->release_pinned(s->status_host);
         if (!prep) {
+            // An end that is taken beside the stream is there 6 us after the submission's own event. In a chain that is waited for in order only the
+            // last one's is still to come: the completion reads it when it is asked (waiting for it here: 149 / 156 us a chain of eight).
+            if (e == cudaSuccess && !(s->beside && inst->tail == s)) timed = inst->read_times(s->start, s->end, &ns);
             inst->release_event(s->done);
             if (inst->tail == s) inst->tail = nullptr;
         }
@@ -1077,8 +1108,8 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
             prep->busy = false;
             return;
         }
-        inst->release_time(s->start);
-        inst->release_time(s->end);
+        inst->release_time(s->start, false);
+        inst->release_time(s->end, false);
         for (auto& o : s->outputs)
             if (o.host) inst->release_pinned(o.host);
     };
@@ -1108,6 +1139,8 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
     c->prepared = prep;
     c->artifact = inst->artifact;
     c->outputs = prep ? prep->outputs : std::move(s->outputs);
+    c->has_device_ns = timed;
+    c->device_ns = ns;
     c->start = s->start;
     c->end = s->end;
     delete s;
@@ -1130,16 +1163,17 @@ int32_t vyb_completion_output(const vyb_completion* c, uint32_t value_id, const 
     return fail_invalid_program("Fix: value id " + std::to_string(value_id) + " is not an output of this artifact.");
 }
 uint32_t vyb_completion_output_count(const vyb_completion* c) { return c ? uint32_t(c->outputs.size()) : 0; }
-int32_t vyb_completion_device_ns(const vyb_completion* c, uint64_t* ns) {
-    if (!c || !ns) return fail_invalid_program("Fix: pass non-null completion and ns pointers.");
-    float ms = 0.0f;
-    // an end that was taken beside the instance's stream may be a little behind the submission's own event
-    if (c->start) cudaSetDevice(c->inst->dev->ordinal);
-    if (!c->start || cudaEventSynchronize(c->end->event) != cudaSuccess || cudaEventElapsedTime(&ms, c->start->event, c->end->event) != cudaSuccess) {
-        cudaGetLastError();
-        return fail_unsupported("device timestamps for this submission");
+int32_t vyb_completion_device_ns(const vyb_completion* completion, uint64_t* ns) {
+    if (!completion || !ns) return fail_invalid_program("Fix: pass non-null completion and ns pointers.");
+    vyb_completion* c = const_cast<vyb_completion*>(completion);
+    std::lock_guard<std::mutex> ilk(c->inst->mu);
+    if (!c->has_device_ns && c->start) {
+        cudaSetDevice(c->inst->dev->ordinal);
+        cudaEventSynchronize(c->end->event);
+        c->has_device_ns = c->inst->read_times(c->start, c->end, &c->device_ns);
     }
-    *ns = uint64_t(double(ms) * 1.0e6);
+    if (!c->has_device_ns) return fail_unsupported("device timestamps for this submission");
+    *ns = c->device_ns;
     clear_error();
     return VYB_OK;
 }
@@ -1150,8 +1184,8 @@ void vyb_completion_free(vyb_completion* c) {
         if (c->prepared) {
             c->prepared->busy = false;  // its buffers may be written by the next replay
         } else {
-            c->inst->release_time(c->start);
-            c->inst->release_time(c->end);
+            c->inst->release_time(c->start, false);
+            c->inst->release_time(c->end, false);
             for (auto& o : c->outputs)
                 if (o.host) c->inst->release_pinned(o.host);
         }
