@@ -35,6 +35,6 @@ def test_times_are_read_when_the_submission_is_waited_for():
 def test_an_event_is_not_recorded_again_before_its_record_is_there():
     assert "(there ? time_points : late_points).push_back(t)" in body("release_time")
     a = body("acquire_time")
-    assert "cudaEventQuery(late_points[i]->event) == cudaSuccess" in a
+    assert "query_event(late_points[i]->event) == cudaSuccess" in a
     # who gives back times without having read them does not know
     assert not re.search(r"release_time\((?!sub->end|start|end)[^,;]+, true\)", RUNTIME) and "c->inst->release_time(c->end, false);" in RUNTIME

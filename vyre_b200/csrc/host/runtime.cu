@@ -90,6 +90,17 @@ struct TimePoint {
     cudaEvent_t event = nullptr;
     int users = 0;
 };
+// Asking for an event while a stream is captured anywhere in the process (cudaStreamCaptureModeGlobal) is refused and ends that capture, unless
+// the thread says that the question has nothing to do with it.
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+cudaError_t query_event(cudaEvent_t e) {
+    BesideCaptures b;
+    return cudaEventQuery(e);
+}
 
 }  // namespace
 
@@ -132,7 +143,7 @@ struct vyb_instance {
     TimePoint* acquire_time() {
         TimePoint* t;
         for (size_t i = late_points.size(); time_points.empty() && i-- > 0;)
-            if (cudaEventQuery(late_points[i]->event) == cudaSuccess) {
+            if (query_event(late_points[i]->event) == cudaSuccess) {
                 time_points.push_back(late_points[i]);
                 late_points.erase(late_points.begin() + i);
             }
@@ -179,6 +190,7 @@ struct vyb_instance {
                 return clock;
             }
         }
+        BesideCaptures b;
         if (cudaStreamCreateWithFlags(&clock, cudaStreamNonBlocking) != cudaSuccess) {
             cudaGetLastError();
             clock = nullptr;
@@ -1006,7 +1018,7 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
     // Behind a submission that is still pending, and with nothing but kernels of its own, this one starts where that one ends, as an event that
     // is recorded here would have it, and its own end is taken beside the stream (vyb_instance::tail). inst->mu is held for the whole
     // submission.
-    bool queued = sub->temps.empty() && inst->tail && cudaEventQuery(inst->tail->done) == cudaErrorNotReady;
+    bool queued = sub->temps.empty() && inst->tail && query_event(inst->tail->done) == cudaErrorNotReady;
     for (const OutputSlot& o : sub->outputs) queued = queued && !o.host;
     if (queued)  // that one's end is not the end of its copies
         for (const OutputSlot& o : inst->tail->outputs) queued = queued && !o.host;
