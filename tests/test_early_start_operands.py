@@ -89,3 +89,14 @@ def test_waits_with_a_limit_begin_behind_the_wait_for_earlier_launches(f, name):
         limit = re.search(r"\b(mbar_wait2?|done_wait)\(", text)
         if limit and (left_out is None or role in left_out):
             assert "waits_for_previous();" in text[: limit.start()], role
+
+
+@pytest.mark.parametrize("f", ["int4_gemv_batch8.cu", "int4_gemv_bulk.cu", "int4_gemv_halfsm.cu", "int4_prefill_tcgen05.cu", "int4_skinny_tcgen05.cu"])
+def test_a_launch_that_leaves_an_sm_free_lets_nobody_start(f):
+    """The kernels that take a number of SMs: what starts early behind one that leaves SMs free would sit on them until it ends."""
+    s = SOURCES[f]
+    starts = re.findall(r"([^\n;{}]*)\blets_next_start\(\);", s)
+    assert [x.strip() for x in starts] == ["if (p.early)"]
+    launches, early = re.findall(r"cfg\.numAttrs = ([^;]*);", s), re.findall(r"p\.early = ([^;]*);", s)
+    assert launches and set(launches) <= {"p.early ? 1 : 0", "p.early ? 2 : 1"} and len(early) == len(launches)
+    assert set(early) <= {"all_sms", "constant_weights || all_sms", "constant_weights || whole_device(dev, sm_count)"}

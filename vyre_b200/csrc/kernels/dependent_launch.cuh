@@ -32,7 +32,9 @@ inline void dependent(cudaLaunchAttribute& a) {
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     a.val.programmaticStreamSerializationAllowed = 1;
 }
-// A caller that leaves SMs free for another kernel does not want the next launch on them early
+// A caller that leaves SMs free for another kernel does not want the next launch on them early: such a launch neither starts early nor lets the
+// next one start (small operators behind a projection would fill the free SM and sit there until it ends), except in chains of constant
+// weights, whose launches are meant to overlap.
 inline bool whole_device(int dev, int sm_count) {
     int sms = 0;
     return cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sm_count >= sms;

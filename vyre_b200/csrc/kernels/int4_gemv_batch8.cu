@@ -94,6 +94,7 @@ struct Params {
     uint32_t m, n;
     uint32_t tiles_per_cta, tiles_rem;  // whole 16-row tiles per CTA; the first tiles_rem CTAs own one more
     uint32_t pace_ns;                   // pause between the prefetched tiles (0: none)
+    uint32_t early;                     // the next launch may start beside this one
 };
 
 // W warps, each owning GPW 128-k groups of every row: k = 128 GPW W
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_batch8_kernel(const __gri
     extern __shared__ __align__(128) uint8_t smem[];
     // let the next launch of the stream become resident beside this one at once; it waits (griddepcontrol.wait)
     // before it reads activations or writes outputs. A no-op for plain launches.
-    lets_next_start();
+    if (p.early) lets_next_start();
     constexpr uint32_t K = 128u * GPW * W;
     constexpr uint32_t ROW_BYTES = K / 2;            // packed bytes of one row of W
     constexpr uint32_t PITCH = GPW * 64;             // of which this warp owns (= row pitch of its stages)
@@ -360,6 +361,7 @@ cudaError_t launch_int4_gemv_batch8(const void* x_bf16, const void* w_packed, co
     p.m = m;
     p.n = n;
     p.pace_ns = constant_weights ? PACE_NS : 0u;
+    p.early = constant_weights || whole_device(dev, sm_count);
     // one CTA per SM, whole 16-row tiles each, the remainder spread one tile per CTA
     const uint32_t tiles = (n + TILE_ROWS - 1) / TILE_ROWS;
     const uint32_t grid = tiles < uint32_t(sm_count) ? tiles : uint32_t(sm_count);
@@ -373,7 +375,7 @@ cudaError_t launch_int4_gemv_batch8(const void* x_bf16, const void* w_packed, co
     cudaLaunchAttribute attr = {};
     dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
+    cfg.numAttrs = p.early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernels[k == 4096 ? 0 : 1][out_f32 ? 1 : 0], p);
 }
 

@@ -146,6 +146,7 @@ struct Params {
     uint32_t m, n, k, groups;  // groups = k / 128
     uint32_t* status;
     uint32_t constant;  // weights and scales may be read before the launches before this one are complete
+    uint32_t early;     // the next launch may start beside this one
 };
 
 template <int LIMBS, bool OUT_F32>
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(THREADS, 1) int4_gemv_kernel(const Params p) {
     const int lane = threadIdx.x & 31;
     // Programmatic dependent launch: let the next kernel in the stream begin its own launch and weight prefetch
     // now; it still waits (griddepcontrol.wait) before touching activations or outputs. No-ops for plain launches.
-    lets_next_start();
+    if (p.early) lets_next_start();
     const uint32_t rows_base = p.n / gridDim.x, rows_rem = p.n % gridDim.x;
     const uint32_t r0 = blockIdx.x * rows_base + min(blockIdx.x, rows_rem);
     const uint32_t r1 = r0 + rows_base + (blockIdx.x < rows_rem ? 1u : 0u);
@@ -533,6 +534,7 @@ cudaError_t launch_int4_gemv_bulk(const void* x_bf16, const void* w_packed, cons
     p.groups = k / 128;
     p.status = status;
     p.constant = constant_weights;
+    p.early = constant_weights || whole_device(dev, sm_count);
     const uint32_t tiles = (n + TILE_ROWS - 1) / TILE_ROWS;
     const uint32_t grid = tiles < uint32_t(sm_count) ? tiles : uint32_t(sm_count);
     cudaLaunchConfig_t cfg = {};
@@ -543,7 +545,7 @@ cudaError_t launch_int4_gemv_bulk(const void* x_bf16, const void* w_packed, cons
     cudaLaunchAttribute attr = {};
     dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
+    cfg.numAttrs = p.early ? 1 : 0;
     if (out_f32) return cudaLaunchKernelEx(&cfg, int4_gemv_kernel<4, true>, p);
     return cudaLaunchKernelEx(&cfg, int4_gemv_kernel<3, false>, p);
 }

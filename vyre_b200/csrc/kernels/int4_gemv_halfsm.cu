@@ -104,6 +104,7 @@ struct Params {
     uint32_t m, n;
     uint32_t tiles_per_cta, tiles_rem;  // whole 16-row tiles per CTA; the first tiles_rem CTAs own one more
     uint32_t pace_ns;                   // pause between the prefetched tiles (0: none)
+    uint32_t early;                     // the next launch may start beside this one
     // the gathering form only: the outputs go to this rank's slice of buffer half `half` on EVERY rank
     PeerGather ag;
     uint32_t half;
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(W * 32, 2) int4_gemv_halfsm_kernel(const __gri
     extern __shared__ __align__(128) uint8_t smem[];
     // let the next launch of the stream become resident beside this one at once; it waits (griddepcontrol.wait)
     // before it reads activations or writes outputs. A no-op for plain launches.
-    lets_next_start();
+    if (p.early) lets_next_start();
     constexpr uint32_t K = 128u * GPW * W;
     constexpr uint32_t ROW_BYTES_DENSE = K / 2;      // packed bytes of one row of W when the launch covers whole rows
     constexpr uint32_t PITCH = GPW * 64;             // of which this warp owns (= row pitch of its stages)
@@ -914,6 +915,7 @@ cudaError_t launch_int4_gemv_halfsm(const void* x_bf16, const void* w_packed, co
     p.m = m;
     p.n = n;
     p.pace_ns = constant_weights ? PACE_NS : 0u;
+    p.early = constant_weights || whole_device(dev, sm_count);
     p.status = status;  // only the gathering form has a wait that can run out
     p.half = half & 1u;
     p.pipelined = pipelined ? 1u : 0u;
@@ -934,7 +936,7 @@ cudaError_t launch_int4_gemv_halfsm(const void* x_bf16, const void* w_packed, co
     cudaLaunchAttribute attr = {};
     dependent(attr);
     cfg.attrs = &attr;
-    cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
+    cfg.numAttrs = p.early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, block ? fused[k == 4096 ? 0 : 1] : kernels[variant][gather ? 2 : out_f32 ? 1 : 0], p);
 }
 
@@ -1032,6 +1034,7 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
                 p.m = m;
                 p.n = n;
                 p.pace_ns = constant_weights ? PACE_NS : 0u;
+                p.early = constant_weights || whole_device(dev, sm_count);
                 p.row_bytes = k / 2;
                 p.scale_stride = k / 128;
                 p.x_stride = k;
@@ -1052,7 +1055,7 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
                 cudaLaunchAttribute attr = {};
                 dependent(attr);
                 cfg.attrs = &attr;
-                cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
+                cfg.numAttrs = p.early ? 1 : 0;
                 return cudaLaunchKernelEx(&cfg, kernels[m <= 2 ? 0 : 1][blk == 4096 ? 0 : 1][out_f32 ? 1 : 0], p);
             }
         }
@@ -1075,6 +1078,7 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
         p.m = m;
         p.n = n;
         p.pace_ns = constant_weights ? PACE_NS : 0u;
+        p.early = constant_weights || whole_device(dev, sm_count);
         p.tiles_per_cta = tiles / grid;
         p.tiles_rem = tiles % grid;
         p.row_bytes = k / 2;
@@ -1089,7 +1093,7 @@ cudaError_t launch_int4_gemv_kblocks(const void* x_bf16, const void* w_packed, c
         cudaLaunchAttribute attr = {};
         dependent(attr);
         cfg.attrs = &attr;
-        cfg.numAttrs = constant_weights || whole_device(dev, sm_count) ? 1 : 0;
+        cfg.numAttrs = p.early ? 1 : 0;
         e = cudaLaunchKernelEx(&cfg, kernels[m <= 2 ? 0 : 1][blk == 4096 ? 0 : 1][(last ? out_f32 != 0 : true) ? 1 : 0], p);
         kb += blk;
     }

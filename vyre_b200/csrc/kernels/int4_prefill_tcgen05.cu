@@ -83,6 +83,7 @@ struct Params {
     uint32_t group_inv;      // G = 0: group / 64 > 1: (i * group_inv) >> 32 = i / (group / 64) for the 64-k blocks i of a row; else 0
     uint32_t groups;         // of a row
     uint32_t tile0;          // first weight tile of this launch
+    uint32_t early;          // the next launch may start beside this one
     // unpack_word's, from here so that they stay in registers: an instruction takes one immediate, and the compiler makes a second one
     // anew before every use (three instructions a word)
     uint32_t mask, mul, add;
@@ -175,7 +176,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
-    lets_next_start();
+    if (p.early) lets_next_start();
     // Every role waits for the launches before this one before it waits for anything with a limit: their time is not this launch's. (One wait
     // here for all roles but the prefetching ones costs the exact forms 72 bytes of spilled registers: 8 x 6400 -> 14336 20.7 / 28 us.)
     auto done_wait = [&](uint32_t i) { return mbar_wait(smem_u32(&bars->done[i % DONE]), (i / DONE) & 1, abort_flag); };
@@ -477,7 +478,8 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     dependent(attr[1]);
     cfg.attrs = attr;
-    cfg.numAttrs = all_sms ? 2 : 1;
+    p.early = all_sms;
+    cfg.numAttrs = p.early ? 2 : 1;
     // A caller that wants an SM left free (sm_count below the device's) gets launches that fit the other SMs at once: a second wave of one
     // launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
     const uint32_t step = all_sms ? tiles : slots;

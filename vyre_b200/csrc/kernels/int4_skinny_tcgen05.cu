@@ -85,6 +85,7 @@ struct Params {
     uint32_t m, n, k, split;
     uint32_t tile0;          // first weight tile of this launch
     uint32_t constant;       // weights and scales may be read before the launches before this one are complete
+    uint32_t early;          // the next launch may start beside this one
 };
 
 template <int BN, bool OUT_F32>
@@ -132,7 +133,7 @@ int4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     // only now, with this CTA's tensor memory in hand, may the next launch's CTA take the rest of it
-    lets_next_start();
+    if (p.early) lets_next_start();
     // Before any wait with a limit: the time that the launches before this one still take is not this one's. Only constant weights (warp 0) and
     // scales (from warp 12 on) are read before.
     if (warp != 0 && !(p.constant && warp >= 12)) waits_for_previous();
@@ -371,8 +372,9 @@ cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t o
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     dependent(attr[1]);
     cfg.attrs = attr;
-    cfg.numAttrs = constant_weights || all_sms ? 2 : 1;
     p.constant = constant_weights;
+    p.early = constant_weights || all_sms;
+    cfg.numAttrs = p.early ? 2 : 1;
     // A caller that wants an SM left free (sm_count below the device's, VYB_LAUNCH_LEAVE_ONE_SM) gets launches that fit the other SMs at once:
     // a second wave of one launch would fill every SM as the first one drains. Anybody else: one launch for all tiles.
     const uint32_t step = all_sms ? tiles : slots;
