@@ -100,3 +100,10 @@ def test_a_launch_that_leaves_an_sm_free_lets_nobody_start(f):
     launches, early = re.findall(r"cfg\.numAttrs = ([^;]*);", s), re.findall(r"p\.early = ([^;]*);", s)
     assert launches and set(launches) <= {"p.early ? 1 : 0", "p.early ? 2 : 1"} and len(early) == len(launches)
     assert set(early) <= {"all_sms", "constant_weights || all_sms", "constant_weights || whole_device(dev, sm_count)"}
+
+
+def test_kernels_that_read_twice_keep_l1():
+    """A preferred split of shared memory is a property of a kernel, whatever its size: what reads a row again from L1 must not have it."""
+    between = re.findall(r"launch_between<([^;()]*)>\(", SOURCES["ref_ops.cu"])
+    assert set(between) == {"residual_add_kernel", "swiglu_kernel", "rms_norm_tree_regs_kernel<16>", "rms_norm_tree_regs_kernel<32>", "rms_norm_kernel<true>"}
+    assert "if (rows <= 64) return launch_between<rms_norm_kernel<true>>(" in SOURCES["ref_ops.cu"]

@@ -397,6 +397,8 @@ __global__ void residual_add_kernel(const void* residual, const void* branch, vo
 // invocation, one f32 chain over the row in index order; here one block owns a row: its threads stage the row through
 // shared memory (coalesced), thread 0 runs that same chain once, and all threads then normalise (x * (1 / sqrt(mean +
 // eps)), rounded to dtype, times f32(weight), times gate / (1 + exp(-gate)) with a gate, one cast). Same values.
+// SPLIT: the form that is launched with its neighbours' split of shared memory (launch_between)
+template <bool SPLIT>
 __global__ void rms_norm_kernel(const void* input, const void* weight, const void* gate, void* out, uint32_t hidden, float eps,
                                 uint32_t dt, uint32_t wdt) {
     waits_for_previous();
@@ -691,8 +693,13 @@ cudaError_t launch_rms_norm(const void* input, const void* weight, const void* g
         return launch_between<rms_norm_tree_regs_kernel<16>>(dim3(rows), dim3(256), 0, s, input, weight, out, hidden, eps, dtype, weight_dtype);
     if (tree && !gate && few && hidden <= 8192)
         return launch_between<rms_norm_tree_regs_kernel<32>>(dim3(rows), dim3(256), 0, s, input, weight, out, hidden, eps, dtype, weight_dtype);
-    if (tree) return launch_between<rms_norm_tree_kernel>(dim3(rows), dim3(256), 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
-    return launch_between<rms_norm_kernel>(dim3(rows), dim3(256), 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
+    // These read a row twice, the second time from L1, which their neighbours' split of shared memory leaves 28 KB of an SM (us, with that split /
+    // with L1: 8 x 14336 21.5 / 14.1, 600 x 4096 8.7 / 6.8, 300 x 8192 14.9 / 10.7, 4096 x 4096 33.7 / 22.5, 8192 x 6144 85.8 / 57.5, 4096 x 1024
+    // 30.7 / 29.0): only short rows of a decode batch, 8 x 1024 6.3 / 6.2, take it, for the early start between projections.
+    const dim3 grid(rows), block(256);
+    if (tree) return launch_dependent(rms_norm_tree_kernel, grid, block, 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
+    if (rows <= 64) return launch_between<rms_norm_kernel<true>>(grid, block, 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
+    return launch_dependent(rms_norm_kernel<false>, grid, block, 0, s, input, weight, gate, out, hidden, eps, dtype, weight_dtype);
 }
 cudaError_t launch_k_quant_unpack(const uint32_t* packed, const float* scales, const float* mins, float* out, uint32_t n,
                                   uint32_t bits, cudaStream_t s) {
