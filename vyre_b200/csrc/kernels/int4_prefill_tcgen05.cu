@@ -532,22 +532,13 @@ cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const
 
 cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
                                 uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
-    // The CTA-pair GEMM from 129 rows on, except where tiles are so few that this kernel splits the k range over idle SMs (pair / this, us:
-    // 256 x 4096 -> 4096 18.1 / 16.0, 256 x 3072 -> 2658 14.7 / 11.9; 256 x 3072 -> 8192 16.1 / 18.6, 512 x 3072 -> 2658 15.5 / 18.2)
-    const uint64_t items = uint64_t((n + 127) / 128) * ((m + 127) / 128);
-    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > uint64_t(sm_count) / 2)
+    // The CTA-pair GEMM from 129 rows on, except where this kernel splits the k range over SMs that few tiles leave idle, and in short rows whose tiles
+    // all run at once: one tile's way through the pair's pipeline is longer (pair / this, us: 256 x 4096 -> 4096 18.1 / 16.0, 256 x 3072 -> 2658 14.7 /
+    // 11.9, 200 x 512 -> 8192 11.7 / 10.6, 512 x 1024 -> 4096 12.7 / 12.5, 384 x 1536 -> 6272 18.8 / 14.7; 512 x 3072 -> 4096 18.8 / 19.0, f32
+    // 1024 x 2048 -> 2048 14.7 / 15.4, 256 x 3072 -> 8192 16.1 / 18.6).
+    const uint64_t items = uint64_t((n + 127) / 128) * ((m + 127) / 128), sms = uint64_t(sm_count);
+    if (int4_gemm_pair_supported(m, n, k, group) && sm_count >= 2 && items > (k <= 1536 ? sms : sms / 2))
         return launch_int4_gemm_pair(x_bf16, w_packed, scale_bf16, y, m, n, k, group, out_f32, 0, 1, nullptr, nullptr, n, sm_count, stream, status);
-    // Rows are the grid's y dimension, which ends at 65535 tiles: more rows are further launches
-    constexpr uint32_t MAX_ROWS = 65535u * 128u;
-    if (m > MAX_ROWS) {
-        for (uint64_t r0 = 0; r0 < m; r0 += MAX_ROWS) {
-            const cudaError_t e = launch_int4_prefill(static_cast<const uint16_t*>(x_bf16) + r0 * k, w_packed, scale_bf16,
-                                                      static_cast<uint8_t*>(y) + r0 * n * (out_f32 ? 4 : 2), uint32_t(m - r0 < MAX_ROWS ? m - r0 : MAX_ROWS), n,
-                                                      k, group, out_f32, sm_count, stream, status);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    }
     Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
     const uint32_t per = group / 64;
     if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
