@@ -1,5 +1,5 @@
-"""A submission's device time: both ends are taken on one stream, it is read while the submission is waited for if it is there by then, and an event whose
-record may still be to come is not recorded again. The moments between cannot be arranged from outside, so this reads the source."""
+"""A submission's device time: both ends are taken on one stream, it is read while the submission is waited for if it is there by then, and no event
+is recorded on two streams. The moments between cannot be arranged from outside, so this reads the source."""
 import os
 import re
 
@@ -23,18 +23,20 @@ def test_start_and_end_are_taken_on_one_stream():
     assert "if (!queued) cudaEventRecord(sub->end->event, inst->stream);" in s and "cudaEventRecord(sub->end->event, inst->clock);" in s
 
 
-def test_times_are_read_when_the_submission_is_waited_for():
+def test_times_that_are_there_are_read_when_the_submission_is_waited_for():
     w = body("vyb_submission_wait")
-    # the newest submission of a chain alone may leave it to its completion: its end is still on the way between the streams
-    assert "if (e == cudaSuccess && !(s->beside && inst->tail == s)) timed = inst->read_times(s->start, s->end, &ns);" in w
-    assert w.index("read_times") < w.index("inst->tail = nullptr;")
+    # an end beside the stream is still on its way then, and is read when it is asked for
+    assert "if (e == cudaSuccess && !s->beside) timed = inst->read_times(s->start, s->end, &ns);" in w
     g = body("vyb_completion_device_ns")
     assert "if (!c->has_device_ns && c->start) {" in g and g.index("cudaEventSynchronize(c->end->event)") < g.index("read_times") and "std::lock_guard" in g
 
 
-def test_an_event_is_not_recorded_again_before_its_record_is_there():
-    assert "(there ? time_points : late_points).push_back(t)" in body("release_time")
+def test_an_event_is_recorded_on_one_stream_alone():
+    """A record that is still to come is not overtaken by the event's next one."""
+    assert "time_points[t->beside].push_back(t)" in body("release_time")
     a = body("acquire_time")
-    assert "query_event(late_points[i]->event) == cudaSuccess" in a
-    # who gives back times without having read them does not know
-    assert not re.search(r"release_time\((?!sub->end|start|end)[^,;]+, true\)", RUNTIME) and "c->inst->release_time(c->end, false);" in RUNTIME
+    assert "t->beside = beside;" in a and "time_points[beside].back()" in a
+    s = body("vyb_submit")
+    assert "sub->end = inst->acquire_time(queued);" in s and "sub->start = inst->acquire_time(queued);" in s
+    records = re.findall(r"cudaEventRecord\((sub->(?:start|end)->event), ([^)]*)\)", RUNTIME)
+    assert records == [("sub->start->event", "queued ? inst->clock : inst->stream"), ("sub->end->event", "inst->stream"), ("sub->end->event", "inst->clock")]

@@ -77,6 +77,7 @@ namespace {
 
 struct PinnedBuf {
     void* ptr = nullptr;
+    void* dev = nullptr;  // the device's address of it, asked for once
     size_t cap = 0;
     bool in_use = false;
 };
@@ -89,6 +90,7 @@ struct DeviceBuf {
 struct TimePoint {
     cudaEvent_t event = nullptr;
     int users = 0;
+    bool beside = false;  // recorded on the clock stream, always: a record that is still to come there is never overtaken by the next one
 };
 // Asking for an event while a stream is captured anywhere in the process (cudaStreamCaptureModeGlobal) is refused and ends that capture, unless
 // the thread says that the question has nothing to do with it.
@@ -124,8 +126,7 @@ struct vyb_instance {
     uint32_t injected_status = 0;     // word that a kernel of the next submission raises (vyb_instance_inject_status)
 
     // events are recycled: creating and destroying three per submission costs more than the launch itself
-    std::vector<TimePoint*> time_points;
-    std::vector<TimePoint*> late_points;  // whose record may still be to come on the clock stream: not to be recorded again before
+    std::vector<TimePoint*> time_points[2];  // of this stream, of the clock stream
     std::vector<cudaEvent_t> plain_events;
     cudaEvent_t acquire_event() {
         cudaEvent_t e = nullptr;
@@ -140,25 +141,21 @@ struct vyb_instance {
     void release_event(cudaEvent_t e) {
         if (e) plain_events.push_back(e);
     }
-    TimePoint* acquire_time() {
+    TimePoint* acquire_time(bool beside) {
         TimePoint* t;
-        for (size_t i = late_points.size(); time_points.empty() && i-- > 0;)
-            if (query_event(late_points[i]->event) == cudaSuccess) {
-                time_points.push_back(late_points[i]);
-                late_points.erase(late_points.begin() + i);
-            }
-        if (time_points.empty()) {
+        if (time_points[beside].empty()) {
             t = new TimePoint;
+            t->beside = beside;
             cudaEventCreate(&t->event);
         } else {
-            t = time_points.back();
-            time_points.pop_back();
+            t = time_points[beside].back();
+            time_points[beside].pop_back();
         }
         t->users = 1;
         return t;
     }
-    void release_time(TimePoint* t, bool there) {
-        if (t && --t->users == 0) (there ? time_points : late_points).push_back(t);
+    void release_time(TimePoint* t) {
+        if (t && --t->users == 0) time_points[t->beside].push_back(t);
     }
     // Reads a submission's times and gives them back; false while its end is still to come
     bool read_times(TimePoint*& start, TimePoint*& end, uint64_t* ns) {
@@ -167,8 +164,8 @@ struct vyb_instance {
             cudaGetLastError();
             return false;
         }
-        release_time(start, true);
-        release_time(end, true);
+        release_time(start);
+        release_time(end);
         start = end = nullptr;
         *ns = uint64_t(double(ms) * 1.0e6);
         return true;
@@ -206,10 +203,19 @@ struct vyb_instance {
             }
         PinnedBuf b;
         if (cudaHostAlloc(&b.ptr, std::max<size_t>(len, 256), cudaHostAllocDefault) != cudaSuccess) return nullptr;
+        if (cudaHostGetDevicePointer(&b.dev, b.ptr, 0) != cudaSuccess) {
+            cudaGetLastError();
+            b.dev = nullptr;
+        }
         b.cap = std::max<size_t>(len, 256);
         b.in_use = true;
         pinned.push_back(b);
         return b.ptr;
+    }
+    void* device_address(const void* p) const {
+        for (const auto& b : pinned)
+            if (b.ptr == p) return b.dev;
+        return nullptr;
     }
     void release_pinned(void* p) {
         for (auto& b : pinned)
@@ -254,8 +260,8 @@ void instance_unref(vyb_instance* i) {
         std::lock_guard<std::mutex> lk(i->dev->mu);
         i->dev->clock_streams.push_back(i->clock);
     }
-    for (auto* pool : {&i->time_points, &i->late_points})
-        for (TimePoint* t : *pool) {
+    for (auto& pool : i->time_points)
+        for (TimePoint* t : pool) {
             cudaEventDestroy(t->event);
             delete t;
         }
@@ -1008,9 +1014,8 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
     // slot, so a word raised by one submission is never reported for another and nothing has to be copied or cleared on the
     // stream between two submissions: the copy and the memset that did it took 12 us of every submission in a chain.
     sub->status_host = static_cast<uint32_t*>(inst->acquire_pinned(16));
-    void* own_status = nullptr;
-    if (!sub->status_host || cudaHostGetDevicePointer(&own_status, sub->status_host, 0) != cudaSuccess) {
-        cudaGetLastError();
+    void* own_status = inst->device_address(sub->status_host);
+    if (!own_status) {
         cleanup();
         return fail_oom(16, 0);
     }
@@ -1024,13 +1029,13 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         for (const OutputSlot& o : inst->tail->outputs) queued = queued && !o.host;
     queued = queued && inst->clock_stream() != nullptr;
     sub->beside = queued;
-    sub->end = inst->acquire_time();
+    sub->end = inst->acquire_time(queued);
     sub->done = inst->acquire_event();
     if (queued && inst->tail->beside) {
         sub->start = inst->tail->end;
         ++sub->start->users;
     } else {  // both times on one stream: the way from one to the other takes some microseconds
-        sub->start = inst->acquire_time();
+        sub->start = inst->acquire_time(queued);
         if (queued) cudaStreamWaitEvent(inst->clock, inst->tail->done, 0);
         cudaEventRecord(sub->start->event, queued ? inst->clock : inst->stream);
     }
@@ -1046,8 +1051,8 @@ int32_t vyb_submit(vyb_instance* inst, const uint8_t artifact_digest[32], const 
         cudaGetLastError();
         cudaStreamSynchronize(inst->stream);
         cleanup();
-        inst->release_time(sub->start, !queued);
-        inst->release_time(sub->end, true);
+        inst->release_time(sub->start);
+        inst->release_time(sub->end);
         inst->release_event(sub->done);
         if (e == cudaErrorNotSupported) return fail_unsupported("operator `" + p.op_id + "`");
         return fail_dispatch(int(e), "kernel launch failed: " + cuda_msg(e));
@@ -1099,9 +1104,10 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
         for (void* t : s->staged) inst->release_pinned(t);
         if (!prep && s->status_host) inst->release_pinned(s->status_host);
         if (!prep) {
-            // An end that is taken beside the stream is there 6 us after the submission's own event. In a chain that is waited for in order only the
-            // last one's is still to come: the completion reads it when it is asked (waiting for it here: 149 / 156 us a chain of eight).
-            if (e == cudaSuccess && !(s->beside && inst->tail == s)) timed = inst->read_times(s->start, s->end, &ns);
+            // An end that is taken beside the stream is there 6 us after the submission's own event: the completion reads it when it is asked (us,
+            // waiting for it here: eight linears at 48 rows 149 / 156; reading what is there and asking events before their next use: four
+            // small Q4_K linears 54 / 68).
+            if (e == cudaSuccess && !s->beside) timed = inst->read_times(s->start, s->end, &ns);
             inst->release_event(s->done);
             if (inst->tail == s) inst->tail = nullptr;
         }
@@ -1120,8 +1126,8 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
             prep->busy = false;
             return;
         }
-        inst->release_time(s->start, false);
-        inst->release_time(s->end, false);
+        inst->release_time(s->start);
+        inst->release_time(s->end);
         for (auto& o : s->outputs)
             if (o.host) inst->release_pinned(o.host);
     };
@@ -1196,8 +1202,8 @@ void vyb_completion_free(vyb_completion* c) {
         if (c->prepared) {
             c->prepared->busy = false;  // its buffers may be written by the next replay
         } else {
-            c->inst->release_time(c->start, false);
-            c->inst->release_time(c->end, false);
+            c->inst->release_time(c->start);
+            c->inst->release_time(c->end);
             for (auto& o : c->outputs)
                 if (o.host) c->inst->release_pinned(o.host);
         }
