@@ -45,9 +45,9 @@ constexpr int TMEM_COLS = 512;
 constexpr int CTRL_BYTES = 512, ALIGN_SLACK = 1024;
 constexpr uint32_t PREFETCH_STAGES = 24;
 
-// BN: activation rows of a tile. G: exact weights, pairs of scales in a stage (group 128: 1, group 64: 2); 0: rounded weights, one accumulator
-// for the whole row. SETS: accumulators of a stage, one per group or, with twice as many, per half of a group.
-template <int BN, int G, int SETS_>
+// BN: activation rows of a tile. G: exact weights, an accumulator per 128 k (1) or per 64 k (2; an instance of its own for groups of 128 with
+// two accumulators each spills 108 bytes); 0: rounded weights, one accumulator for the whole row.
+template <int BN, int G>
 struct Cfg {
     static constexpr int X_BYTES = BN * KB * 2;
     // Weights and activations have rings of their own: a stage of weights is free as soon as it is unpacked, one of activations when its MMAs
@@ -55,7 +55,7 @@ struct Cfg {
     static constexpr int STAGES = BN == 16 ? 10 : BN == 32 ? 9 : BN == 64 ? 6 : 5, X_STAGES = BN == 16 ? 6 : BN <= 64 ? 4 : 2;
     static constexpr int RING_BYTES = STAGES * RAW_BYTES + X_STAGES * X_BYTES;
     static constexpr int SMEM_BYTES = RING_BYTES + CTRL_BYTES + ALIGN_SLACK;
-    static constexpr int SETS = SETS_;
+    static constexpr int SETS = G == 0 ? 1 : 2 * G;            // accumulators of a stage
     static constexpr int A_COL = G == 0 ? BN : 2 * SETS * BN;  // accumulators (of two stages) come first
     static constexpr int A_SLOTS = 3;                          // unpacked stages (8 x 4096 -> 14336: 13.4 us with two, 12.1 with three)
     static_assert(A_COL + A_SLOTS * 128 <= TMEM_COLS && X_STAGES <= DONE && STAGES <= 10, "tensor memory, barriers");
@@ -73,6 +73,21 @@ struct Bars {
 };
 static_assert(sizeof(Bars) <= CTRL_BYTES, "control block");
 
+// The bytes of a row's scales that `stages` stages from `stage` on need
+struct Range {
+    uint32_t first, last;
+};
+__host__ __device__ constexpr Range scale_bytes(uint32_t stage, uint32_t stages, uint32_t group, uint32_t groups) {
+    const uint32_t end = uint32_t((uint64_t(stage + stages) * KB + group - 1) / group);
+    return {uint32_t(uint64_t(stage) * KB / group) * 2, (end < groups ? end : groups) * 2};
+}
+constexpr bool same(Range a, uint32_t first, uint32_t last) { return a.first == first && a.last == last; }
+// two parts of 4096 k: each half of the row's scales, whatever the group; a group that spans both; a last stage past the row's end
+static_assert(same(scale_bytes(0, 8, 64, 64), 0, 64) && same(scale_bytes(8, 8, 64, 64), 64, 128), "groups of 64");
+static_assert(same(scale_bytes(0, 8, 128, 32), 0, 32) && same(scale_bytes(8, 8, 128, 32), 32, 64), "groups of 128");
+static_assert(same(scale_bytes(8, 8, 512, 8), 8, 16) && same(scale_bytes(8, 8, 4096, 1), 0, 2), "long groups");
+static_assert(same(scale_bytes(2, 2, 192, 5), 4, 10) && same(scale_bytes(6, 1, 64, 25), 48, 50), "a group on a part's border, ends");
+
 struct Params {
     const uint16_t* x;       // bf16 [m][k] and packed weights [n][k / 8], for by_definition
     const uint32_t* w;
@@ -81,7 +96,8 @@ struct Params {
     uint32_t* status;
     uint32_t m, n, k, split;
     uint32_t group_inv;      // G = 0: group / 64 > 1: (i * group_inv) >> 32 = i / (group / 64) for the 64-k blocks i of a row; else 0
-    uint32_t groups;         // of a row
+    uint32_t group, groups;  // k of a group, groups of a row
+    uint32_t halves;         // G = 2: 1 if a group is two accumulators' k
     uint32_t tile0;          // first weight tile of this launch
     uint32_t early;          // the next launch may start beside this one
     // unpack_word's, from here so that they stay in registers: an instruction takes one immediate, and the compiler makes a second one
@@ -103,12 +119,12 @@ __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.40282347e
 
 // One output of exact weights by the definition, as int4_linear_generic_kernel computes it (a lane's words in ascending order, then the lanes
 // as the shuffles add them): a group's sum, or a scale times 64, can leave f32's range where no term does. An output that does not come out
-// finite is computed anew, so that an infinity or NaN stands only where the definition has one. Out of line: next to nothing takes it.
-__device__ __noinline__ float by_definition(const Params& p, uint32_t m, uint32_t n) {
+// finite is computed anew, so that an infinity or NaN stands only where the definition has one.
+__device__ float by_definition(const Params& p, uint32_t m, uint32_t n) {
     const uint16_t* x = p.x + size_t(m) * p.k;
     const uint32_t* w = p.w + size_t(n) * (p.k / 8);
     const uint16_t* scales = p.scales + size_t(n) * p.groups;
-    const uint32_t k = p.k, group = k / p.groups;
+    const uint32_t k = p.k, group = p.group;
     float part[32];
 #pragma unroll 1
     for (uint32_t lane = 0; lane < 32; ++lane) {
@@ -127,10 +143,28 @@ __device__ __noinline__ float by_definition(const Params& p, uint32_t m, uint32_
     return part[0];
 }
 
-template <int BN, int G, int SETS, bool OUT_F32>
+// Those of a tile that are not finite: columns `part`, `part` + `split` and so on are this block's. Out of line, since next to nothing takes it, and its
+// parameters by value: a reference would need the kernel's in memory (16 x 4096 -> 14336 with f32 outputs 14.7 / 15.4 us).
+template <int BN, bool OUT_F32>
+__device__ __noinline__ void redo_tile(const Params p, uint32_t m0, uint32_t n0, uint32_t part) {
+    for (uint32_t idx = threadIdx.x; idx < BN * BM; idx += THREADS) {
+        const uint32_t m = m0 + idx / BM * p.split + part, n = n0 + idx % BM;
+        if (idx / BM * p.split + part >= BN || m >= p.m || n >= p.n) continue;
+        const size_t at = size_t(m) * p.n + n;
+        if constexpr (OUT_F32) {
+            float* y = static_cast<float*>(p.y) + at;
+            if (!finite(*y)) *y = by_definition(p, m, n);
+        } else {
+            __nv_bfloat16* y = static_cast<__nv_bfloat16*>(p.y) + at;
+            if (!finite(__bfloat162float(*y))) *y = __float2bfloat16_rn(by_definition(p, m, n));
+        }
+    }
+}
+
+template <int BN, int G, bool OUT_F32>
 __global__ void __launch_bounds__(THREADS, 1)
-int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ Params p) {
-    using C = Cfg<BN, G, SETS>;
+int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
+    using C = Cfg<BN, G>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* x_tiles = tiles + C::STAGES * RAW_BYTES;
@@ -145,11 +179,6 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const size_t at = size_t(m0 + c) * p.n + row;
         if constexpr (OUT_F32) static_cast<float*>(p.y)[at] = v;
         else static_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
-    };
-    auto stored = [&](uint32_t c, uint32_t row) {
-        const size_t at = size_t(m0 + c) * p.n + row;
-        if constexpr (OUT_F32) return static_cast<const float*>(p.y)[at];
-        else return __bfloat162float(static_cast<const __nv_bfloat16*>(p.y)[at]);
     };
 
     if (threadIdx.x == 0) {
@@ -216,9 +245,10 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         __syncwarp();
     } else if (warp == 3) {
         // ---- scales into L2: a row's share is a few sectors, read two bytes at a time ----
-        const uint32_t row_bytes = p.groups * 2, per = G == 0 ? 8 : 4 * G, first = kb0 * per, last = min(row_bytes, first + kbs * per);
+        const uint32_t row_bytes = p.groups * 2;
+        const Range range = scale_bytes(kb0, kbs, p.group, p.groups);
         for (uint32_t r = lane; r < BM && n0 + r < p.n; r += 32)
-            for (uint32_t at = first; at < last; at += 32)
+            for (uint32_t at = range.first; at < range.last; at += 32)
                 prefetch_l2(reinterpret_cast<const uint8_t*>(p.scales) + size_t(n0 + r) * row_bytes + at);
         waits_for_previous();
     } else if (warp == 1) {
@@ -350,8 +380,8 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         auto load_scales = [&](uint32_t i, uint32_t (&q)[G]) {
 #pragma unroll
             for (int h = 0; h < G; ++h) {  // past the row's last group the activations are zeros
-                const uint32_t g = g0 + (i * G + h) * 2;
-                q[h] = (g < groups ? uint32_t(sp[g]) : 0u) | (g + 1 < groups ? uint32_t(sp[g + 1]) << 16 : 0u);
+                const uint32_t set = g0 + (i * G + h) * 2, g = G == 2 ? set >> p.halves : set, g1 = G == 2 ? (set + 1) >> p.halves : set + 1;
+                q[h] = (g < groups ? uint32_t(sp[g]) : 0u) | (g1 < groups ? uint32_t(sp[g1]) << 16 : 0u);
             }
         };
 #pragma unroll
@@ -372,8 +402,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 tc_fence_after();
 #pragma unroll
                 for (int h = 0; h < C::SETS; ++h) {
-                    const int g = h * 2 * G / C::SETS;
-                    const float s = __uint_as_float(g & 1 ? bits[g / 2] & 0xFFFF0000u : bits[g / 2] << 16) * 64.0f;  // tensor memory holds (q - 8) / 64
+                    const float s = __uint_as_float(h & 1 ? bits[h / 2] & 0xFFFF0000u : bits[h / 2] << 16) * 64.0f;  // tensor memory holds (q - 8) / 64
                     uint32_t v[BN];
                     tmem_ld_32x16(tmem + ((quad * 32) << 16) + (d * C::SETS + h) * BN, v);
                     tmem_ld_wait();
@@ -382,8 +411,12 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         __syncwarp();
                         if (lane == 0) mbar_arrive(smem_u32(&bars->b_full[(i + 2) % READY]));  // for the stage after the next
                     }
+                    // the sums before the next loads: moved past them, they keep both sets' registers and spill
 #pragma unroll
-                    for (int c = 0; c < BN; ++c) acc[c] = fmaf(s, __uint_as_float(v[c]), acc[c]);
+                    for (int c = 0; c < BN; ++c) {
+                        acc[c] = fmaf(s, __uint_as_float(v[c]), acc[c]);
+                        asm volatile("" : "+f"(acc[c]));
+                    }
                 }
             }
         }
@@ -419,18 +452,14 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
             for (uint32_t q = 1; q < MAX_SPLIT; ++q)
                 if (q < p.split) sum += v[q];
-            if (G != 0 && !finite(sum)) sum = by_definition(p, m0 + c, n0 + o);
             store(c, n0 + o, sum);
+            if (G != 0 && !finite(sum)) bars->redo = 1;
         }
         cluster_sync();  // no CTA leaves while another still reads its shared memory
     } else {
         __syncthreads();
-        if (G != 0 && bars->redo)  // here, where the epilogue's registers are free
-            for (uint32_t idx = threadIdx.x; idx < BN * BM; idx += THREADS) {
-                const uint32_t c = idx / BM, row = n0 + idx % BM;
-                if (m0 + c < p.m && row < p.n && !finite(stored(c, row))) store(c, row, by_definition(p, m0 + c, row));
-            }
     }
+    if (G != 0 && bars->redo) redo_tile<BN, OUT_F32>(p, m0, n0, part);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);
@@ -442,16 +471,16 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
 }
 
-template <int BN, int G, int SETS, bool OUT_F32>
+template <int BN, int G, bool OUT_F32>
 cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cudaStream_t stream) {
-    using C = Cfg<BN, G, SETS>;
+    using C = Cfg<BN, G>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        const void* f = (const void*)int4_tmem_kernel<BN, G, SETS, OUT_F32>;
+        const void* f = (const void*)int4_tmem_kernel<BN, G, OUT_F32>;
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
@@ -485,7 +514,7 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     const uint32_t step = all_sms ? tiles : slots;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split, rows);
-        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, SETS, OUT_F32>, mw, mx, p);
+        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, OUT_F32>, mw, mx, p);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -501,6 +530,7 @@ Params make_params(const void* x, const void* w, const void* scale, void* y, uin
     p.m = m;
     p.n = n;
     p.k = k;
+    p.group = group;
     p.groups = k / group;
     p.mask = 0x00F0000Fu;
     p.mul = 0x7D007F00u;  // 2^123 | 2^127
@@ -521,13 +551,12 @@ bool int4_few_rows_supported(const void* x, const void* w, const void* scale, ui
 
 cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
                                  uint32_t group, uint32_t out_f32, int sm_count, cudaStream_t stream, uint32_t* status) {
-    const Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
+    Params p = make_params(x_bf16, w_packed, scale_bf16, y, m, n, k, group, status);
+    p.halves = group == 128;
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
-    if (group == 64) return launch(launch_cfg<16, 2, 4, true>, launch_cfg<16, 2, 4, false>);
-    // Up to eight rows of groups of 128: sums in the tensor core over 64 k (run_int4_linear, which sends bf16 outputs alone, has the errors). More
-    // rows: over a whole group, as the kernel has them that takes 17 rows on.
-    if (m <= 8 && !out_f32) return launch_cfg<16, 1, 4, false>(x_bf16, w_packed, p, sm_count, stream);
-    return launch(launch_cfg<16, 1, 2, true>, launch_cfg<16, 1, 2, false>);
+    // Up to eight rows: sums in the tensor core over 64 k (run_int4_linear has the errors). More: over a whole group, as the kernel has them that
+    // takes 17 rows on.
+    return group == 64 || m <= 8 ? launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
 }
 
 cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
@@ -543,9 +572,9 @@ cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const 
     const uint32_t per = group / 64;
     if (per > 1) p.group_inv = uint32_t((0x100000000ull + per - 1) / per);
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
-    if (m <= 16) return launch(launch_cfg<16, 0, 1, true>, launch_cfg<16, 0, 1, false>);
-    if (m <= 32) return launch(launch_cfg<32, 0, 1, true>, launch_cfg<32, 0, 1, false>);
-    return m <= 64 ? launch(launch_cfg<64, 0, 1, true>, launch_cfg<64, 0, 1, false>) : launch(launch_cfg<128, 0, 1, true>, launch_cfg<128, 0, 1, false>);
+    if (m <= 16) return launch(launch_cfg<16, 0, true>, launch_cfg<16, 0, false>);
+    if (m <= 32) return launch(launch_cfg<32, 0, true>, launch_cfg<32, 0, false>);
+    return m <= 64 ? launch(launch_cfg<64, 0, true>, launch_cfg<64, 0, false>) : launch(launch_cfg<128, 0, true>, launch_cfg<128, 0, false>);
 }
 
 }  // namespace vybk
