@@ -107,3 +107,9 @@ def test_kernels_that_read_twice_keep_l1():
     between = re.findall(r"launch_between<([^;()]*)>\(", SOURCES["ref_ops.cu"])
     assert set(between) == {"residual_add_kernel", "swiglu_kernel", "rms_norm_tree_regs_kernel<16>", "rms_norm_tree_regs_kernel<32>", "rms_norm_kernel<true>"}
     assert "if (rows <= 64) return launch_between<rms_norm_kernel<true>>(" in SOURCES["ref_ops.cu"]
+
+
+def test_no_instance_without_a_caller():
+    """f32 outputs of up to 16 rows: int4_few_rows and the integer kernels."""
+    s = SOURCES["int4_skinny_tcgen05.cu"]
+    assert "int4_skinny_kernel<BN, BN != 16>" in s and "if (m <= 16 && !out_f32) return launch_bn<16>" in s

@@ -411,12 +411,8 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                         __syncwarp();
                         if (lane == 0) mbar_arrive(smem_u32(&bars->b_full[(i + 2) % READY]));  // for the stage after the next
                     }
-                    // the sums before the next loads: moved past them, they keep both sets' registers and spill
 #pragma unroll
-                    for (int c = 0; c < BN; ++c) {
-                        acc[c] = fmaf(s, __uint_as_float(v[c]), acc[c]);
-                        asm volatile("" : "+f"(acc[c]));
-                    }
+                    for (int c = 0; c < BN; ++c) acc[c] = fmaf(s, __uint_as_float(v[c]), acc[c]);
                 }
             }
         }

@@ -334,7 +334,7 @@ template <int BN>
 cudaError_t launch_bn(const void* x, const void* w, const Params& p0, uint32_t out_f32, int sm_count, cudaStream_t stream, bool constant_weights) {
     using C = Cfg<BN>;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const Params);
-    static const Kernel kernels[2] = {int4_skinny_kernel<BN, false>, int4_skinny_kernel<BN, true>};
+    static const Kernel kernels[2] = {int4_skinny_kernel<BN, false>, int4_skinny_kernel<BN, BN != 16>};  // sixteen columns: bf16 outputs alone
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -403,7 +403,8 @@ cudaError_t launch_int4_skinny(const void* x_bf16, const void* w_packed, const v
     p.n = n;
     p.k = k;
     // 17..32 rows take the 48-column form: a 32-column form with two CTAs per SM measured 18.7 us at 14336 x 4096, 48 columns 15.7
-    if (m <= 16) return launch_bn<16>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
+    // f32 outputs of up to 16 rows come from other kernels (run_int4_linear, launch_int4_gemv); called for here, they take 48 columns too
+    if (m <= 16 && !out_f32) return launch_bn<16>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
     if (m <= 48) return launch_bn<48>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
     return launch_bn<64>(x_bf16, w_packed, p, out_f32, sm_count, stream, constant_weights);
 }
