@@ -180,3 +180,47 @@ def test_sums_then_prefill_gemm(m, n, k):
         ffi.check(L.vyb_k_int4_prefill_gemm(p(x), p(w), p(scale), p(y[i]), m, n, k, 64, ffi.DT_BF16, s, None))
 
     unwaited(step, lambda i: [y[i]])
+
+
+def test_captured_with_forks_and_copies():
+    """Early launches in a graph whose nodes also wait for copies, memsets and a second stream."""
+    m, k = 64, 4096
+    L, g = ffi.lib(), torch.Generator(device="cuda").manual_seed(8)
+    bf = lambda *sh: torch.randn(*sh, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    a, b, w, x, n1, n2 = bf(m, k), bf(m, k), bf(k), bf(m, k), bf(m, k), bf(m, k)
+    q, sc, kept = torch.empty(2, m, k, dtype=torch.int8, device="cuda"), torch.empty(2, m, device="cuda"), torch.empty(2, m, k, dtype=torch.int8, device="cuda")
+    s, t = torch.cuda.Stream(), torch.cuda.Stream()
+    cs, ct = C.c_void_p(s.cuda_stream), C.c_void_p(t.cuda_stream)
+
+    def work():
+        with torch.cuda.stream(s):
+            ffi.check(L.vyb_k_residual_add(p(a), p(b), p(x), m * k, ffi.DT_BF16, cs))
+            t.wait_stream(s)
+            with torch.cuda.stream(t):
+                ffi.check(L.vyb_k_rms_norm(p(x), p(w), p(n1), m, k, 1e-5, ffi.DT_BF16, ct))
+                n2.copy_(n1)                                                             # a copy behind an early kernel
+                ffi.check(L.vyb_k_swiglu(p(n2), p(n1), p(n1), m * k, ffi.DT_BF16, ct))   # and an early kernel behind a copy
+            q.zero_()
+            ffi.check(L.vyb_k_quantize_per_token_int8(p(x), p(q[0]), p(sc[0]), m, k, cs))
+            s.wait_stream(t)
+            ffi.check(L.vyb_k_quantize_per_token_int8(p(n1), p(q[1]), p(sc[1]), m, k, cs))  # behind kernels of two streams
+            kept.copy_(q)
+
+    torch.cuda.synchronize()
+    work()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        work()
+    for _ in range(4):
+        a.copy_(bf(m, k))
+        torch.cuda.synchronize()
+        work()
+        torch.cuda.synchronize()
+        want = [v.clone() for v in (kept, sc, n1)]
+        for v in (x, n1, n2, q, sc, kept):
+            v.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(u, v) for u, v in zip((kept, sc, n1), want)) and kept.any()
