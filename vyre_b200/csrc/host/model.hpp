@@ -133,7 +133,7 @@ bool profile_equal(const vyb_target_profile& a, const vyb_target_profile& b);
 
 // kernel variants recorded in the payload module
 enum KernelVariant : uint32_t {
-    KV_GENERIC = 0,
+    KV_GENERIC = 0,                      // no kernel named; the int4 linear's runs warp per row or, up to eight rows, with weights in tensor memory (run_int4_linear)
     KV_INT4_GEMV_TMA = 1,
     KV_INT4_PREFILL_TCGEN05 = 2,
     KV_INT8_GEMM_TCGEN05 = 3,

@@ -13,14 +13,16 @@
 // weight row, each set a pass in four; eight warps drain the one accumulator, half of its columns each (the unpacking of the next tile's first
 // four passes lies under it).
 // bf16 results pass through 64 KB of shared memory, so that the accumulator is free as soon as it is read (about 1200 cycles): with SwiGLU and 2-byte
-// stores between its read and its release 4096 tokens of eight experts took 3220 us a layer, now 2733 (2992 with the weights through shared memory).
+// stores between its read and its release 4096 tokens of eight experts took 3220 us a layer, now 2700 to 2810 (2990 with the weights through shared memory).
 // In glu mode lanes 0-63 of a CTA hold gate rows and lanes 64-127 the same up rows; they meet where the results pass through shared memory.
 // The activation rows of a plain tile are chosen so that the tiles fill whole waves of pairs (choose_bn).
 //
-// What bounds it: at 2048 and more rows of wide projections the power cap (cuBLAS sustains 1.40 PFLOP/s there, this 1.37); below, the MMAs (1024
-// cycles a pass; unpacking takes 830 to 1500, four passes at once) and the last wave. Measured, us in a stream, with the weights unpacked into shared
-// memory / into tensor memory: 2048 x 4096 -> 14336 187 / 175, 1024 x 4096 -> 14336 152 / 94, 512 x 4096 -> 14336 90 / 51, 2048 x 4096 -> 4096 89 / 53,
-// 2048 x 3072 -> 2658 118 / 30, 4096 x 4096 -> 14336 394 / 364.
+// What bounds it: at 2048 and more rows of wide projections the power cap (2048 x 4096 -> 14336 takes 171 us in a burst of a dozen, at 1.965 GHz, and
+// 204 in a stream of sixty or more, at 1.40 to 1.45 GHz); below, the MMAs (1024 cycles a pass; unpacking takes 830 to 1500, four passes at once) and how full the
+// waves of tiles are; in short rows the one accumulator, whose read and release take about as long as three passes. Measured, us in a burst, with the
+// weights unpacked into shared memory / into tensor memory: 2048 x 4096 -> 14336 187 / 171, 1024 x 4096 -> 14336 152 / 94, 512 x 4096 -> 14336 90 / 51, 2048 x
+// 4096 -> 4096 89 / 53, 2048 x 3072 -> 2658 118 / 30, 4096 x 4096 -> 14336 394 / 340, 4096 x 1024 -> 14336 114 / 103, 8192 x 1088 -> 14336 437 / 285 (before, a
+// single-CTA kernel); 4096 x 256 -> 14336 64 / 68 and 8192 x 320 -> 14336 170 / 188 are what the one accumulator costs.
 //
 // Every wait is clock-bounded; on expiry the CTA raises a status word, drains and frees its TMEM. No multicast.
 //
@@ -450,7 +452,10 @@ bool int4_gemm_pair_supported(uint32_t m, uint32_t n, uint32_t k, uint32_t group
 
 namespace {
 
-// Activation rows of a plain tile: what makes the waves of pairs shortest, a tile's time being its rows and about 24 rows' worth of epilogue
+// Activation rows of a plain tile: what makes the waves of pairs shortest, a tile's time being its rows and about 24 rows' worth of epilogue (us at 128,
+// 160, 192, 224 and 256 rows, * what is taken: 2048 x 4096 -> 14336 187 / 171* / 173 / 175 / 169, 1024 x 4096 -> 14336 110 / 119 / 112 / 99* / 113, 512 x 4096 -> 14336
+// 73 / 82 / 74 / 84 / 62*, 2048 x 4096 -> 4096 74 / 69* / 78 / 91 / 68, 2048 x 3072 -> 2658 53 / 49* / 53 / 60 / 63, 300 x 4096 -> 8192 39 / 30* / 35 / 37 / 37, 1400 x 7168 -> 10000
+// 151* / 143 / 155 / 148 / 162, 2048 x 1024 -> 14336 71 / 68* / 72 / 65 / 64)
 uint32_t choose_bn(uint32_t m, uint32_t n_tiles, uint32_t pairs) {
     uint32_t best = MAX_BN;
     uint64_t cost = ~0ull;

@@ -1,4 +1,5 @@
-// Group-quantized int4 linear with the weights in tensor memory (tcgen05, sm_100a): prefill batches, and few rows of any row length.
+// Group-quantized int4 linear with the weights in tensor memory on single CTAs (tcgen05, sm_100a): prefill batches of up to 128 rows or of few or
+// short tiles (launch_int4_prefill; the CTA-pair GEMM has the rest), and few rows of any row length.
 //
 //   rounded (prefill):  y[m, n] = cast( sum_k x[m, k] * bf16((q[n, k] - 8) * s[n, g(k)]) )          any group of whole 64 k, f32 sums
 //   exact (few rows):   y[m, n] = cast( sum_g s[n, g] * sum_{k in g} x[m, k] * (q[n, k] - 8) )      groups of 64 or 128, up to 16 rows

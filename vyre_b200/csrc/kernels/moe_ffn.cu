@@ -407,9 +407,9 @@ cudaError_t launch_moe_ffn_int4(const void* x_bf16, const void* w_router_bf16, c
                          experts, skinny);
     if (e != cudaSuccess) return e;
     // Few rows per expert: weight rows on the M side of single CTAs, 32 or 64 activation rows a chunk. This / the pair GEMM, us a layer, at 64, 96, 112
-    // and 128 rows per expert: 8 experts of 4096 / 14336 401 / 464, 490 / 475, 492 / 490, 628 / 497; 16 of 2048 / 4096 173 / 198, 190 / 215, 205 / 210,
-    // 240 / 211; 16 of 3328 / 2816 190 / 221, 234 / 240, 256 / 243, 274 / 248; 32 of 2048 / 2048 180 / 228, 227 / 234, 244 / 239, 275 / 245; four of
-    // 1280 / 1536, whose 48 pair tiles leave 26 of 74 pairs idle, 51 / 65 at all four.
+    // and 128 rows per expert: 8 experts of 4096 / 14336 413 / 463, 503 / 487, 522 / 519, 671 / 558; 16 of 2048 / 4096 183 / 229, 204 / 239, 205 / 224,
+    // 253 / 209; 16 of 3328 / 2816 177 / 214, 213 / 217, 225 / 220, 252 / 220; 32 of 2048 / 2048 182 / 226, 228 / 231, 246 / 234, 278 / 239; four of
+    // 1280 / 1536, whose 48 pair tiles leave 26 of 74 pairs idle, 48 / 56 at all four.
     // The line is the average, which the host knows: with all tokens on one or two experts this form can be
     // slower than the pair GEMM (wide: 512 tokens on two of 8 experts 500 against 449 us; narrow: 160 tokens on two of 16 experts, 4096 / 4096,
     // 160 against 130 us, balanced 193 against 459). A choice by the plan kernel, both forms launched and one returning at once,
