@@ -589,7 +589,7 @@ int32_t vyb_submission_is_ready(const vyb_submission* s);
 int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion);
 /* Completion (artifact_lifecycle.rs:100-109): host bytes per output value, device_ns when measured. device_ns runs from the end of the
  * instance's work before (from the launch, if there was none under way) to the end of the submission's own kernels, so that those of a
- * chain add up to the chain's time. For the newest submission of a chain the call may have to wait some microseconds for the end's time. */
+ * chain add up to the chain's time. In a chain of submissions the call may have to wait some microseconds for the time of the end. */
 int32_t vyb_completion_output(const vyb_completion* c, uint32_t value_id, const uint8_t** bytes, size_t* len);
 uint32_t vyb_completion_output_count(const vyb_completion* c);
 int32_t vyb_completion_device_ns(const vyb_completion* c, uint64_t* ns);

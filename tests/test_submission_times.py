@@ -1,4 +1,4 @@
-"""A submission's device time: both ends are taken on one stream, it is read while the submission is waited for if it is there by then, and no event
+"""A submission's device time: both ends are taken on one stream, it is read while a submission by itself is waited for, and no event
 is recorded on two streams. The moments between cannot be arranged from outside, so this reads the source."""
 import os
 import re
@@ -25,8 +25,9 @@ def test_start_and_end_are_taken_on_one_stream():
 
 def test_times_that_are_there_are_read_when_the_submission_is_waited_for():
     w = body("vyb_submission_wait")
-    # an end beside the stream is still on its way then, and is read when it is asked for
-    assert "if (e == cudaSuccess && !s->beside) timed = inst->read_times(s->start, s->end, &ns);" in w
+    # in a chain they are read when they are asked for: an end beside the stream is still on its way
+    assert "if (e == cudaSuccess && !s->beside && inst->tail == s) timed = inst->read_times(s->start, s->end, &ns);" in w
+    assert w.index("read_times") < w.index("inst->tail = nullptr;")
     g = body("vyb_completion_device_ns")
     assert "if (!c->has_device_ns && c->start) {" in g and g.index("cudaEventSynchronize(c->end->event)") < g.index("read_times") and "std::lock_guard" in g
 

@@ -1104,10 +1104,10 @@ int32_t vyb_submission_wait(vyb_submission* s, vyb_completion** completion) {
         for (void* t : s->staged) inst->release_pinned(t);
         if (!prep && s->status_host) inst->release_pinned(s->status_host);
         if (!prep) {
-            // An end that is taken beside the stream is there 6 us after the submission's own event: the completion reads it when it is asked (us,
-            // waiting for it here: eight linears at 48 rows 149 / 156; reading what is there and asking events before their next use: four
-            // small Q4_K linears 54 / 68).
-            if (e == cudaSuccess && !s->beside) timed = inst->read_times(s->start, s->end, &ns);
+            // A submission by itself: its times are there. In a chain the completion reads them when it is asked: an end that is taken beside the
+            // stream is there 6 us after the submission's own event, and the host has the next ones to wait for (us: eight linears at 48 rows 149,
+            // waiting for the ends here 156; four small Q4_K linears 54, reading what is there 58, asking for all 67).
+            if (e == cudaSuccess && !s->beside && inst->tail == s) timed = inst->read_times(s->start, s->end, &ns);
             inst->release_event(s->done);
             if (inst->tail == s) inst->tail = nullptr;
         }
