@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) int8_weight_only_kernel(const float* x,
                 }
             }
         } else {
+#pragma unroll 4
             for (uint32_t kk = lane; kk < k; kk += 32) {
                 const float wv = float(wr[kk]);
 #pragma unroll
