@@ -46,8 +46,8 @@ constexpr int TMEM_COLS = 512;
 constexpr int CTRL_BYTES = 512, ALIGN_SLACK = 1024;
 constexpr uint32_t PREFETCH_STAGES = 24;
 
-// BN: activation rows of a tile. G: exact weights, an accumulator per 128 k (1) or per 64 k (2; an instance of its own for groups of 128 with
-// two accumulators each spills 108 bytes); 0: rounded weights, one accumulator for the whole row.
+// BN: activation rows of a tile. G: exact weights, an accumulator per 128 k (1) or per 64 k (2; HALVES: a group is two of them); 0: rounded
+// weights, one accumulator for the whole row.
 template <int BN, int G>
 struct Cfg {
     static constexpr int X_BYTES = BN * KB * 2;
@@ -98,7 +98,7 @@ struct Params {
     uint32_t m, n, k, split;
     uint32_t group_inv;      // G = 0: group / 64 > 1: (i * group_inv) >> 32 = i / (group / 64) for the 64-k blocks i of a row; else 0
     uint32_t group, groups;  // k of a group, groups of a row
-    uint32_t halves;         // G = 2: 1 if a group is two accumulators' k
+    uint32_t halves;         // HALVES: 1, read from here, as a constant shift makes an instance that spills 108 bytes
     uint32_t tile0;          // first weight tile of this launch
     uint32_t early;          // the next launch may start beside this one
     // unpack_word's, from here so that they stay in registers: an instruction takes one immediate, and the compiler makes a second one
@@ -162,7 +162,7 @@ __device__ __noinline__ void redo_tile(const Params p, uint32_t m0, uint32_t n0,
     }
 }
 
-template <int BN, int G, bool OUT_F32>
+template <int BN, int G, bool HALVES, bool OUT_F32>
 __global__ void __launch_bounds__(THREADS, 1)
 int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
     using C = Cfg<BN, G>;
@@ -381,7 +381,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         auto load_scales = [&](uint32_t i, uint32_t (&q)[G]) {
 #pragma unroll
             for (int h = 0; h < G; ++h) {  // past the row's last group the activations are zeros
-                const uint32_t set = g0 + (i * G + h) * 2, g = G == 2 ? set >> p.halves : set, g1 = G == 2 ? (set + 1) >> p.halves : set + 1;
+                const uint32_t set = g0 + (i * G + h) * 2, g = HALVES ? set >> p.halves : set, g1 = HALVES ? (set + 1) >> p.halves : set + 1;
                 q[h] = (g < groups ? uint32_t(sp[g]) : 0u) | (g1 < groups ? uint32_t(sp[g1]) << 16 : 0u);
             }
         };
@@ -468,7 +468,7 @@ int4_tmem_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
 }
 
-template <int BN, int G, bool OUT_F32>
+template <int BN, int G, bool OUT_F32, bool HALVES = false>
 cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cudaStream_t stream) {
     using C = Cfg<BN, G>;
     static std::atomic<uint64_t> configured{0};
@@ -477,7 +477,7 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     if (e != cudaSuccess) return e;
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        const void* f = (const void*)int4_tmem_kernel<BN, G, OUT_F32>;
+        const void* f = (const void*)int4_tmem_kernel<BN, G, HALVES, OUT_F32>;
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
@@ -511,7 +511,7 @@ cudaError_t launch_cfg(const void* x, const void* w, Params p, int sm_count, cud
     const uint32_t step = all_sms ? tiles : slots;
     for (p.tile0 = 0; p.tile0 < tiles; p.tile0 += step) {
         cfg.gridDim = dim3((tiles - p.tile0 < step ? tiles - p.tile0 : step) * p.split, rows);
-        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, OUT_F32>, mw, mx, p);
+        e = cudaLaunchKernelEx(&cfg, int4_tmem_kernel<BN, G, HALVES, OUT_F32>, mw, mx, p);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -553,7 +553,8 @@ cudaError_t launch_int4_few_rows(const void* x_bf16, const void* w_packed, const
     const auto launch = [&](auto f32, auto bf16) { return out_f32 ? f32(x_bf16, w_packed, p, sm_count, stream) : bf16(x_bf16, w_packed, p, sm_count, stream); };
     // Up to eight rows: sums in the tensor core over 64 k (run_int4_linear has the errors). More: over a whole group, as the kernel has them that
     // takes 17 rows on.
-    return group == 64 || m <= 8 ? launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
+    if (group == 64) return launch(launch_cfg<16, 2, true>, launch_cfg<16, 2, false>);
+    return m <= 8 ? launch(launch_cfg<16, 2, true, true>, launch_cfg<16, 2, false, true>) : launch(launch_cfg<16, 1, true>, launch_cfg<16, 1, false>);
 }
 
 cudaError_t launch_int4_prefill(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m, uint32_t n, uint32_t k,
