@@ -15,7 +15,8 @@ torch = pytest.importorskip("torch")
 # more tiles than SMs, so that pairs take them: one 64-k block, one pass and a bit, one fetch and a bit, three passes of four; groups of several blocks;
 # rows of outputs that are multiples of eight, four, two and one; a last tile of one row
 @pytest.mark.parametrize("m,n,k,group", [(1000, 2562, 64, 64), (700, 3332, 192, 192), (520, 5003, 320, 64), (300, 9600, 1088, 64), (641, 4100, 704, 64), (513, 4001, 256, 128),
-                                         (257, 9606, 1344, 192), (700, 3336, 1600, 320)])
+                                         (257, 9606, 1344, 192), (700, 3336, 1600, 320),
+                                         (384, 6200, 1536, 128), (385, 4700, 1536, 128)])  # 147 and 148 tiles of single CTAs, all of which run at once
 def test_row_lengths_and_row_starts(m, n, k, group):
     x, w, s = synth.int4_linear_inputs(m, n, k, group=group, seed=m + n + k)
     want = oracle.int4_rowmajor_linear(x, w, s, m, n, k, group=group, out_dtype=oracle.DT_F32, mode=1).reshape(m, n).astype(np.float64)
