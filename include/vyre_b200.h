@@ -693,7 +693,8 @@ int32_t vyb_k_int4_gemv(const void* x_bf16, const void* w_packed, const void* sc
 #define VYB_LAUNCH_CONSTANT_WEIGHTS 1u
 /* Launch no more blocks at a time than one SM fewer than the device has would hold, so that a small kernel of another stream
  * (vyb_k_allgather_push) finds room and a memory pipeline that is not saturated by the weight stream. (A call with more output
- * rows than those SMs take at once is several launches in a row on the tensor-memory kernel; the other kernels walk their rows.) */
+ * rows than those SMs take at once is several launches in a row on the tensor-memory kernel; the other kernels walk their rows.)
+ * Nor does the next launch of the stream start beside it, unless the weights are said to be constant. */
 #define VYB_LAUNCH_LEAVE_ONE_SM 2u
 int32_t vyb_k_int4_gemv_ex(const void* x_bf16, const void* w_packed, const void* scale_bf16, void* y, uint32_t m,
                            uint32_t n, uint32_t k, uint32_t group_size, uint32_t out_dtype, uint32_t flags,
